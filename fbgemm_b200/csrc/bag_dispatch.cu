@@ -1,0 +1,238 @@
+// Which bag kernel (bag_kernel.cuh) takes a lookup, and how many tables go into
+// one launch.
+#include <algorithm>
+#include <vector>
+
+#include "bag_kernel.cuh"
+
+namespace fbgemm_b200 {
+
+namespace {
+
+struct VariantInfo {
+  int fmt, vb, cpl, g;
+};
+constexpr VariantInfo kVariantInfo[] = {
+#define INFO(FMT, VB, CPL, G) {bag::FMT, VB, CPL, G},
+    FBGEMM_B200_BAG_VARIANTS(INFO)
+#undef INFO
+};
+
+// Largest power of two, 16 at most, that divides v.
+int alignment_of(uint64_t v) {
+  return v % 16 == 0 ? 16 : v % 8 == 0 ? 8 : v % 4 == 0 ? 4 : v % 2 == 0 ? 2 : 1;
+}
+
+int format_of(const SpmdmParams& p, int bit_rate) {
+  switch (p.in_kind) {
+    case FBGEMM_B200_IN_QUANTIZED: return bit_rate;
+    case FBGEMM_B200_IN_F32: return bag::kF32;
+    case FBGEMM_B200_IN_F16: return bag::kF16;
+    case FBGEMM_B200_IN_BF16: return bag::kBf16;
+    default: return bag::kFp8;
+  }
+}
+
+void bag_table_of(const SpmdmParams& p, BagTable* t) {
+  t->data = p.table + p.data_row_off;
+  t->indices = p.indices;
+  t->offsets = p.offsets;
+  t->weights = p.weights;
+  t->cit = p.cit;
+  t->out = p.out;
+  t->status = p.status;
+  t->data_size = p.data_size;
+  t->bags = p.output_size;
+  t->index_size = p.index_size;
+  const int esize = (p.flags & (kOutHalf | kOutBf16)) ? 2 : 4;
+  t->out_pitch = p.output_stride * esize;
+  t->bags_per_peer = p.bags_per_peer;
+  t->sb_off = p.sb_row_off - p.data_row_off;
+  t->stride = p.input_stride;
+  t->cols = p.block_size;
+  t->data_bytes = p.data_bytes;
+  t->flags = p.flags;
+  const uint64_t sb = reinterpret_cast<uintptr_t>(p.table + p.sb_row_off) | (uint64_t)p.input_stride;
+  t->sb_align = (int16_t)std::min(8, alignment_of(sb));
+  uint64_t o = (uint64_t)t->out_pitch;
+  for (int i = 0; i < p.num_peers; ++i) {
+    o |= reinterpret_cast<uintptr_t>(p.peer_out[i]);
+  }
+  if (p.num_peers <= 0) {
+    o |= reinterpret_cast<uintptr_t>(p.out);
+  }
+  t->num_peers = p.num_peers;
+  t->out_align = (int16_t)alignment_of(o);
+  t->fp8_exponent_bits = (int16_t)p.fp8_exponent_bits;
+  t->fp8_exponent_bias = (int16_t)p.fp8_exponent_bias;
+}
+
+// Row offsets that do not fit 32 bits.  (A row-wise sparse call says how many
+// rows its map has, not how many its table holds: no more than those.)
+bool is_wide(const BagTable& t) {
+  return (unsigned __int128)t.data_size * (uint64_t)t.stride > 0xffffffffull;
+}
+
+// Whole warps per bag while every bag of the launch finds a resident warp: the
+// fewer lanes share a bag, the longer its rows take, and nothing else is there
+// to run.  Beyond that narrow rows take half warps (one and the same walk serves
+// two bags), the narrowest quarter warps.  Measured, us, on bags of 30 rows at
+// 12 M rows: 4-bit D = 64, 4096 bags 7.0 / 8.9 / 10.9 with 32 / 16 / 8 lanes;
+// 8192 bags 11.6 / 10.0 / 12.2; 65536 bags 61.8 / 51.9 / 48.7.  4-bit D = 128,
+// 65536 bags 80.9 / 72.8 / 78.3.  Wider rows always want whole warps.
+constexpr int64_t kResidentWarps = 148 * bag::kBlocksPerSm * bag::kWarps;
+
+int pick_variant(const BagTable& t, int fmt, int64_t bags_in_launch, int* tiles) {
+  const int align = alignment_of(reinterpret_cast<uintptr_t>(t.data) | (uint64_t)t.stride);
+  const int least_g = bags_in_launch <= kResidentWarps ? 32 : bags_in_launch <= 4 * kResidentWarps ? 16 : 8;
+  int best = -1;
+  double best_cost = 0;
+  for (int i = 0; i < bag::kVariants; ++i) {
+    const VariantInfo& v = kVariantInfo[i];
+    if (v.fmt != fmt || v.vb > align || v.g < least_g) {
+      continue;
+    }
+    // the last chunk may run into scale,bias behind the payload, but not beyond the row
+    if (t.data_bytes % v.vb != 0 && !(bag::is_quantized(fmt) && t.sb_off > 0 && v.vb <= 4)) {
+      continue;
+    }
+    const int tile = v.vb * v.cpl * v.g;
+    const int n = (t.data_bytes + tile - 1) / tile;
+    if (n > 1 && v.g < 32) {
+      continue;
+    }
+    // instructions per row: what a row costs besides its columns, its loads, and 2.5 per column of a lane
+    const double cols = (double)v.vb * v.cpl * 8 / bag::column_bits(fmt);
+    const double cost = n * (6.0 + 1.5 * v.cpl + 2.5 * cols) * v.g;
+    if (best < 0 || cost < best_cost) {
+      best = i;
+      best_cost = cost;
+      *tiles = n;
+    }
+  }
+  return best;
+}
+
+int64_t blocks_of(const BagTable& t, int variant) {
+  const int64_t per_block = (int64_t)bag::kWarps * (32 / kVariantInfo[variant].g);
+  return (t.bags + per_block - 1) / per_block;
+}
+
+bag::BagFn single_kernel(int variant, bool wide, bool deep) {
+  struct All {
+    bag::BagFn fn[bag::kVariants][4] = {};
+    All() {
+      bag_kernels_8(fn);
+      bag_kernels_4(fn);
+      bag_kernels_2(fn);
+      bag_kernels_plain(fn);
+    }
+  };
+  static const All all;
+  return all.fn[variant][wide + 2 * deep];
+}
+
+}  // namespace
+
+cudaError_t launch_bags(const SpmdmParams& p, int bit_rate, cudaStream_t stream) {
+  bag::BagCall c;
+  bag_table_of(p, &c.t);
+  for (int i = 0; i < p.num_peers; ++i) {
+    c.peers[i] = p.peer_out[i];
+  }
+  int tiles = 0;
+  const int v = pick_variant(c.t, format_of(p, bit_rate), p.output_size, &tiles);
+  const int64_t blocks = blocks_of(c.t, v);
+  if (blocks <= 0 || blocks > 0x7fffffffLL || tiles > 65535) {
+    return cudaErrorInvalidValue;
+  }
+  const bool deep = kVariantInfo[v].g == 32 && blocks * tiles <= 148 * bag::kDeepBlocksPerSm;
+  single_kernel(v, is_wide(c.t), deep)<<<dim3((unsigned)blocks, (unsigned)tiles), bag::kThreads, 0, stream>>>(c);
+  g_launch_count.fetch_add(1, std::memory_order_relaxed);
+  return cudaGetLastError();
+}
+
+// ---- several tables per launch --------------------------------------------------
+
+struct UnitsLaunch {
+  bag::BagUnits units;
+  unsigned blocks;
+  bool wide;
+};
+
+MultiPlan::MultiPlan() = default;
+MultiPlan::~MultiPlan() = default;
+
+// One launch takes up to kMaxUnits column tiles of tables of any row formats.
+cudaError_t build_multi_plan(const SpmdmParams* tables, const int* bit_rates, size_t count, MultiPlan* plan) {
+  int64_t bags = 0;
+  for (size_t t = 0; t < count; ++t) {
+    bags += tables[t].output_size;
+  }
+  struct Unit {
+    size_t table;
+    int variant, tile;
+    int64_t blocks;
+    bool wide;
+    double work;
+  };
+  std::vector<Unit> order;
+  std::vector<BagTable> bag_tables(count);
+  for (size_t t = 0; t < count; ++t) {
+    if (tables[t].output_size <= 0) {
+      continue;  // nothing to pool, nothing to store
+    }
+    int tiles = 0;
+    bag_table_of(tables[t], &bag_tables[t]);
+    const int v = pick_variant(bag_tables[t], format_of(tables[t], bit_rates[t]), bags, &tiles);
+    const int64_t blocks = blocks_of(bag_tables[t], v);
+    if (blocks > 0x7fffffffLL || tiles > 65535) {
+      return cudaErrorInvalidValue;
+    }
+    for (int i = 0; i < tiles; ++i) {
+      order.push_back({t, v, i, blocks, is_wide(bag_tables[t]),
+                       (double)tables[t].index_size / std::max<int64_t>(1, blocks) * bag_tables[t].data_bytes});
+    }
+  }
+  // Tables beyond 4 GB go together.  Among the others the longest-running blocks come first: the short ones fill
+  // the last wave.
+  std::stable_sort(order.begin(), order.end(), [](const Unit& a, const Unit& b) {
+    return a.wide != b.wide ? a.wide : a.work > b.work;
+  });
+  for (size_t i = 0; i < order.size();) {
+    plan->launches.emplace_back(new UnitsLaunch);
+    UnitsLaunch& l = *plan->launches.back();
+    bag::BagUnits& u = l.units;
+    u.count = 0;
+    l.wide = order[i].wide;
+    int64_t blocks = 0;
+    for (; i < order.size() && order[i].wide == l.wide && u.count < bag::kMaxUnits &&
+         blocks + order[i].blocks <= 0x7fffffffLL; ++i) {
+      const int k = u.count++;
+      const SpmdmParams& p = tables[order[i].table];
+      u.first_block[k] = (int32_t)blocks;
+      u.variant[k] = (uint16_t)order[i].variant;
+      u.tile[k] = (uint16_t)order[i].tile;
+      u.t[k] = bag_tables[order[i].table];
+      std::copy(p.peer_out, p.peer_out + p.num_peers, u.peers[k]);
+      blocks += order[i].blocks;
+    }
+    u.first_block[u.count] = (int32_t)blocks;
+    l.blocks = (unsigned)blocks;
+  }
+  return cudaSuccess;
+}
+
+cudaError_t launch_multi_plan(const MultiPlan& plan, cudaStream_t stream) {
+  for (const auto& l : plan.launches) {
+    (l->wide ? bag_units_wide() : bag_units_narrow())<<<l->blocks, bag::kThreads, 0, stream>>>(l->units);
+    g_launch_count.fetch_add(1, std::memory_order_relaxed);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) {
+      return e;
+    }
+  }
+  return cudaSuccess;
+}
+
+}  // namespace fbgemm_b200

@@ -1,0 +1,745 @@
+// The pooled lookup: one lane group (a warp, or a half or quarter of one) per
+// bag and column tile.
+//
+// Arithmetic as in the scalar reference (src/RefImplementations.cc:1290-1346,
+// :1427-1541, :1617-1688, :1746-1822 of FBGEMM), so fp32 results are bit-equal:
+// per output column, rows strictly in index order,
+//     acc = fma(w*scale, q, acc + w*bias)
+// two columns at a time with the packed fp32 instructions of sm_100
+// (add.rn.f32x2, fma.rn.f32x2), which round each half like the scalar forms.
+//
+// What bounds a lookup is the chain offsets -> index -> row of every bag and
+// instruction issue, not bytes.  Hence the layout:
+//  * The columns of a row are spread over the lane group, 1 to 16 bytes of
+//    payload per lane.  A row in flight costs a lane one or two registers, so
+//    8 to 12 rows of a bag are in flight with a full set of warps on the SM.
+//  * Everything that is per row and not per column is done ONCE per row, by the
+//    lane that owns the row in the walk over the bag's indices (one index per
+//    lane at a time, coalesced): index load, range check, pruning map, weight,
+//    scale and bias load, their conversion and weighting.  The results go
+//    through shared memory: where the row lies, and {scale, scale, bias, bias}
+//    ready for the packed instructions - one 16-byte broadcast load per row.
+//  * Rows that an index does not name (pruned, -1, out of range) drop out of
+//    that queue by ballot and popcount, so the row loop knows no skipped rows.
+//  * Row loads are issued ahead of the arithmetic, four rows at a time.
+#pragma once
+
+#include <cuda_fp16.h>
+
+#include <type_traits>
+
+#include "internal.h"
+
+namespace fbgemm_b200 {
+namespace bag {
+
+constexpr int kWarps = 4;
+constexpr int kThreads = kWarps * 32;
+
+using u64 = unsigned long long;
+
+__device__ __forceinline__ u64 pack2(float lo, float hi) {
+  u64 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack2(u64 v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ u64 add2(u64 a, u64 b) {
+  u64 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ u64 mul2(u64 a, u64 b) {
+  u64 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) {
+  u64 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
+__device__ __forceinline__ int64_t load_int(const void* p, int64_t i, bool is64) {
+  return is64 ? (int64_t)__ldg(reinterpret_cast<const long long*>(p) + i)
+              : (int64_t)__ldg(reinterpret_cast<const int*>(p) + i);
+}
+
+// Inlined: a call in the row walk would put the kernel's registers under the calling convention.
+__device__ __forceinline__ void report(int32_t* st, int code, int64_t bag, int64_t pos, int64_t val) {
+  if (atomicCAS(st, 0, code) == 0) {
+    st[1] = (int32_t)bag;
+    st[2] = (int32_t)pos;
+    st[3] = (int32_t)val;
+  }
+}
+
+// fp32 -> fp16 (round to nearest even, cpu_float2half_rn) or bf16 the way the
+// reference does it: (bits + 0x8000) >> 16 (cpu_float2bfloat16,
+// include/fbgemm/FloatConversion.h:312-315).
+__device__ __forceinline__ uint32_t to_16bit(float v, bool bf16) {
+  return bf16 ? (__float_as_uint(v) + 0x8000u) >> 16 : (uint32_t)__half_as_ushort(__float2half_rn(v));
+}
+
+// VB payload bytes of one row, as loaded by one lane.
+template <int VB>
+struct Bytes {
+  uint32_t w[VB < 4 ? 1 : VB / 4];
+  __device__ __forceinline__ void load(const uint8_t* p) {
+    if constexpr (VB == 1) {
+      w[0] = __ldg(p);
+    } else if constexpr (VB == 2) {
+      w[0] = __ldg(reinterpret_cast<const unsigned short*>(p));
+    } else if constexpr (VB == 4) {
+      w[0] = __ldg(reinterpret_cast<const uint32_t*>(p));
+    } else if constexpr (VB == 8) {
+      const uint2 v = __ldg(reinterpret_cast<const uint2*>(p));
+      w[0] = v.x;
+      w[1] = v.y;
+    } else {
+      const uint4 v = __ldg(reinterpret_cast<const uint4*>(p));
+      w[0] = v.x;
+      w[1] = v.y;
+      w[2] = v.z;
+      w[3] = v.w;
+    }
+  }
+};
+
+// Row formats.  Quantized rows are named by their bit width.
+enum : int { kInt8 = 8, kInt4 = 4, kInt2 = 2, kF32 = 32, kF16 = 16, kBf16 = 17, kFp8 = 9 };
+__host__ __device__ constexpr bool is_quantized(int fmt) { return fmt <= 8; }
+__host__ __device__ constexpr int column_bits(int fmt) { return fmt == kBf16 ? 16 : fmt == kFp8 ? 8 : fmt; }
+
+// Integer -> float: column K's bits are planted, where they lie, in the
+// mantissa of the power of two whose last place has their weight, which is then
+// subtracted: one logic instruction per column and half a packed addition.
+// 8-bit columns go through a byte permute (any byte of the word to bits 0-7).
+template <int BITS, int K>
+struct Plant {
+  static constexpr int kPerWord = 32 / BITS;
+  static constexpr int kWord = K / kPerWord;
+  static constexpr int kInWord = K % kPerWord;
+  static constexpr int kHalf = kPerWord / 2;                     // columns per 16 bits
+  static constexpr int kStep = BITS == 8 ? 0 : kInWord % kHalf;  // which power of two
+  static constexpr int kShift = kStep * BITS;                    // where the bits lie in the mantissa
+};
+
+// What a format keeps in registers: the powers of two (the logic instruction
+// has room for one immediate, the mask), or how FP8 widens to fp32.
+template <int FMT, int COLS>
+struct Constants {
+  static constexpr int BITS = FMT;
+  static constexpr int kHalf = 16 / BITS;
+  static constexpr int kCount = BITS == 8 ? 1 : (COLS < kHalf ? COLS : kHalf);
+  uint32_t m[kCount];
+  __device__ __forceinline__ void init(const BagTable&) {
+#pragma unroll
+    for (int i = 0; i < kCount; ++i) {
+      asm volatile("mov.b32 %0, %1;" : "=r"(m[i]) : "r"((uint32_t)(127 + 23 - i * (BITS == 8 ? 0 : BITS)) << 23));
+    }
+  }
+  template <int K>
+  __device__ __forceinline__ float plant(const uint32_t* w) const {
+    using P = Plant<BITS, K>;
+    if constexpr (BITS == 8) {
+      return __uint_as_float(__byte_perm(w[P::kWord], m[0], 0x7540u | P::kInWord));
+    } else {
+      const uint32_t x = P::kInWord >= P::kHalf ? w[P::kWord] >> 16 : w[P::kWord];
+      uint32_t r;
+      asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(x), "n"(((1 << BITS) - 1) << P::kShift), "r"(m[P::kStep]));
+      return __uint_as_float(r);
+    }
+  }
+  template <int K>
+  __device__ __forceinline__ static u64 minus() {  // the negated powers of two of columns K, K + 1
+    constexpr float a = -(float)(1u << (23 - Plant<BITS, K>::kShift));
+    constexpr float b = -(float)(1u << (23 - Plant<BITS, K + 1>::kShift));
+    return pack2(a, b);
+  }
+};
+template <int COLS>
+struct Constants<kF32, COLS> {
+  __device__ __forceinline__ void init(const BagTable&) {}
+};
+template <int COLS>
+struct Constants<kF16, COLS> : Constants<kF32, COLS> {};
+template <int COLS>
+struct Constants<kBf16, COLS> : Constants<kF32, COLS> {};
+// FP8 -> fp32 as Float8ToFloat_ref (src/RefImplementations.cc:184-215): the seven low bits shifted into fp32's
+// exponent and mantissa, times 2^(127 - bias), sign OR-ed in.
+template <int COLS>
+struct Constants<kFp8, COLS> {
+  float mult;
+  int shift;
+  __device__ __forceinline__ void init(const BagTable& p) {
+    mult = __uint_as_float((uint32_t)(254 - p.fp8_exponent_bias) << 23);
+    shift = 24 - (8 - p.fp8_exponent_bits);
+  }
+};
+
+// The columns a lane owns of a row: CPL chunks of VB payload bytes, chunk c at
+// byte (c * G + lane) * VB of the tile.  acc[] holds them as fp32 pairs: the
+// columns of a chunk in order, or (where a chunk is one column) the columns of
+// two chunks.
+template <int FMT, int VB, int CPL>
+struct Cols {
+  static constexpr int BITS = column_bits(FMT);
+  static constexpr int kPerChunk = VB * 8 / BITS;
+  static constexpr int kPairs = kPerChunk * CPL / 2;
+  static_assert(kPerChunk * CPL % 2 == 0, "whole pairs");
+  using M = Constants<FMT, kPerChunk>;
+
+  // Column k of an unquantized chunk.
+  __device__ __forceinline__ static float value(const M& m, const uint32_t* w, int k) {
+    const uint32_t x = w[k * BITS / 32] >> (k * BITS % 32);
+    if constexpr (FMT == kF32) {
+      return __uint_as_float(x);
+    } else if constexpr (FMT == kF16) {
+      return __half2float(__ushort_as_half((unsigned short)(x & 0xffffu)));
+    } else if constexpr (FMT == kBf16) {
+      return __uint_as_float(x << 16);
+    } else {
+      const float mag = __fmul_rn(__uint_as_float((x & 0x7fu) << m.shift), m.mult);
+      return __uint_as_float(__float_as_uint(mag) | ((x & 0x80u) << 24));
+    }
+  }
+  template <int K>
+  __device__ __forceinline__ static void pool_chunk(const M& m, u64* acc, const uint32_t* w, u64 s2, u64 b2) {
+    if constexpr (K < kPerChunk) {
+      const u64 q = add2(pack2(m.template plant<K>(w), m.template plant<K + 1>(w)), M::template minus<K>());
+      acc[K / 2] = fma2(s2, q, add2(acc[K / 2], b2));
+      pool_chunk<K + 2>(m, acc, w, s2, b2);
+    }
+  }
+  // One row.  Quantized: acc = fma(scale, q, acc + bias); otherwise acc = fma(w, x, acc) with w in `s2`
+  // (src/RefImplementations.cc:1347-1424, :1543-1615).
+  __device__ __forceinline__ static void pool(const M& m, u64 (&acc)[kPairs], const Bytes<VB> (&d)[CPL], u64 s2, u64 b2) {
+    if constexpr (!is_quantized(FMT)) {
+#pragma unroll
+      for (int i = 0; i < kPairs; ++i) {
+        constexpr int n = kPerChunk;
+        const float lo = value(m, d[2 * i / n].w, 2 * i % n);
+        const float hi = value(m, d[(2 * i + 1) / n].w, (2 * i + 1) % n);
+        acc[i] = fma2(s2, pack2(lo, hi), acc[i]);
+      }
+    } else if constexpr (kPerChunk == 1) {
+#pragma unroll
+      for (int c = 0; c < CPL; c += 2) {
+        const u64 q = add2(pack2(__uint_as_float(d[c].w[0] | m.m[0]), __uint_as_float(d[c + 1].w[0] | m.m[0])),
+                           M::template minus<0>());
+        acc[c / 2] = fma2(s2, q, add2(acc[c / 2], b2));
+      }
+    } else {
+#pragma unroll
+      for (int c = 0; c < CPL; ++c) {
+        pool_chunk<0>(m, acc + c * kPerChunk / 2, d[c].w, s2, b2);
+      }
+    }
+  }
+};
+
+// Four little-endian bytes at p, whose address is a multiple of `align`.
+__device__ __forceinline__ uint32_t load_u32(const uint8_t* p, int align) {
+  if (align >= 4) {
+    return __ldg(reinterpret_cast<const uint32_t*>(p));
+  }
+  if (align == 2) {
+    const unsigned short* h = reinterpret_cast<const unsigned short*>(p);
+    return (uint32_t)__ldg(h) | ((uint32_t)__ldg(h + 1) << 16);
+  }
+  return (uint32_t)__ldg(p) | ((uint32_t)__ldg(p + 1) << 8) | ((uint32_t)__ldg(p + 2) << 16) |
+      ((uint32_t)__ldg(p + 3) << 24);
+}
+
+// Store N consecutive columns of an output row, all of them inside the row, at
+// an address that is a multiple of `align` bytes or of the N columns' size.
+template <int N>
+__device__ __forceinline__ void store_f32(float* o, const float* v, int align) {
+  if (N >= 4 && align >= 16) {
+#pragma unroll
+    for (int i = 0; i + 4 <= N; i += 4) {
+      *reinterpret_cast<float4*>(o + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+    }
+  } else if (N >= 2 && align >= 8) {
+#pragma unroll
+    for (int i = 0; i + 2 <= N; i += 2) {
+      *reinterpret_cast<float2*>(o + i) = make_float2(v[i], v[i + 1]);
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      o[i] = v[i];
+    }
+  }
+}
+template <int N>
+__device__ __forceinline__ void store_u16(uint16_t* o, const uint32_t* h, int align) {
+  if (N >= 8 && align >= 16) {
+#pragma unroll
+    for (int i = 0; i + 8 <= N; i += 8) {
+      *reinterpret_cast<uint4*>(o + i) = make_uint4(h[i] | (h[i + 1] << 16), h[i + 2] | (h[i + 3] << 16),
+                                                    h[i + 4] | (h[i + 5] << 16), h[i + 6] | (h[i + 7] << 16));
+    }
+  } else if (N >= 4 && align >= 8) {
+#pragma unroll
+    for (int i = 0; i + 4 <= N; i += 4) {
+      *reinterpret_cast<uint2*>(o + i) = make_uint2(h[i] | (h[i + 1] << 16), h[i + 2] | (h[i + 3] << 16));
+    }
+  } else if (N >= 2 && align >= 4) {
+#pragma unroll
+    for (int i = 0; i + 2 <= N; i += 2) {
+      *reinterpret_cast<uint32_t*>(o + i) = h[i] | (h[i + 1] << 16);
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      o[i] = (uint16_t)h[i];
+    }
+  }
+}
+
+template <int N>
+__device__ __forceinline__ void store_columns(const BagTable& p, char* row, int col0, const float* v) {
+  const int left = p.cols - col0;
+  if (p.flags & (kOutHalf | kOutBf16)) {
+    const bool bf16 = p.flags & kOutBf16;
+    uint16_t* o = reinterpret_cast<uint16_t*>(row) + col0;
+    uint32_t h[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      h[i] = to_16bit(v[i], bf16);
+    }
+    if (left >= N) {
+      store_u16<N>(o, h, p.out_align);
+    } else {
+#pragma unroll
+      for (int i = 0; i < N; ++i) {
+        if (i < left) {
+          o[i] = (uint16_t)h[i];
+        }
+      }
+    }
+  } else {
+    float* o = reinterpret_cast<float*>(row) + col0;
+    if (left >= N) {
+      store_f32<N>(o, v, p.out_align);
+    } else {
+#pragma unroll
+      for (int i = 0; i < N; ++i) {
+        if (i < left) {
+          o[i] = v[i];
+        }
+      }
+    }
+  }
+}
+
+// Where rows lie: byte offsets from row 0, in 32 bits where the table allows
+// (WIDE = false: one 32-bit addition per row and chunk, 10 % of the instructions
+// less than 64-bit addresses), else in 64.
+template <bool WIDE>
+using Row = typename std::conditional<WIDE, unsigned long long, uint32_t>::type;
+
+// Where a lane finds its chunks of a row; lanes whose chunk lies beyond the
+// payload read chunk 0 instead and do not store.
+template <int VB, int CPL, int G, bool WIDE>
+struct LaneData {
+  uint32_t at[CPL];
+  const uint8_t* base;
+  __device__ __forceinline__ void init(const uint8_t* data, int tile_at, int gl, int data_bytes) {
+    base = data;
+#pragma unroll
+    for (int c = 0; c < CPL; ++c) {
+      const int a = tile_at + (c * G + gl) * VB;
+      at[c] = a < data_bytes ? a : 0;
+    }
+  }
+  __device__ __forceinline__ void load(Bytes<VB> (&d)[CPL], Row<WIDE> row) const {
+#pragma unroll
+    for (int c = 0; c < CPL; ++c) {
+      d[c].load(base + (Row<WIDE>)(row + at[c]));
+    }
+  }
+};
+
+// Queue of a warp: the rows that its lanes found, in index order.
+template <bool WIDE>
+struct __align__(16) Queue {
+  Row<WIDE> row[32];
+  ulonglong2 sb[32];  // {scale, scale}, {bias, bias}; {weight, weight} of unquantized rows
+};
+
+// Groups of four rows whose loads are issued ahead of the arithmetic.  Measured on 65536 bags of 30 rows: with half or
+// quarter warps per bag none is best for 4- and 2-bit rows (72.8 against 76.2 us at D = 128, 4 bits), one for 8-bit
+// rows (82 against 102 us at D = 128); whole warps want one.
+__host__ __device__ constexpr int rows_ahead(int fmt, int g) { return g == 32 || (g == 16 && fmt == kInt8) ? 1 : 0; }
+constexpr int kDeepAhead = 2;
+
+// One block's work on table `p`: bags block * kWarps * (32 / G) onwards, columns of tile `tile` of the row.
+template <int FMT, int VB, int CPL, int G, bool WIDE, int kAhead = rows_ahead(FMT, G)>
+__device__ __forceinline__ void pool_bags(const BagTable& p, void* const* peers, int64_t block, int tile,
+                                          Queue<WIDE> (&queues)[kWarps]) {
+  using C = Cols<FMT, VB, CPL>;
+
+  constexpr int kTileBytes = G * VB * CPL;
+  constexpr unsigned kGroupMask = G == 32 ? 0xffffffffu : (1u << (G % 32)) - 1u;
+  constexpr bool kQuantized = is_quantized(FMT);
+  const int lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5;
+  const int gl = lane % G;
+  const int grp = lane / G;
+  Row<WIDE>* q_row = queues[warp].row + grp * G;
+  ulonglong2* q_sb = queues[warp].sb + grp * G;
+  const bool idx64 = p.flags & kIdx64;
+  const bool off64 = p.flags & kOff64;
+  const bool weighted = p.flags & kWeighted;
+  const bool positional = p.flags & kPositional;
+  const bool pruned = p.flags & kPruned;
+  const bool no_bag = p.flags & kNoBag;
+  const bool minus_one_skips = FMT != kFp8 && (p.flags & (kSbFirst | kNoBag)) == kSbFirst;
+  const bool half_sb = FMT != kInt8 || (p.flags & kSbFirst);
+
+  // rebasing to offsets[0] (the functor's convention) unless the offsets are absolute
+  const bool rebase = !(p.flags & (kNoBag | kAbsOffsets));
+  const int64_t off_base = rebase ? load_int(p.offsets, 0, off64) : 0;
+  if (block == 0 && threadIdx.x == 0 && rebase) {
+    // `return current == index_size` of the reference
+    const int64_t total = load_int(p.offsets, p.bags, off64) - off_base;
+    if (total != p.index_size) {
+      report(p.status, FBGEMM_B200_STATUS_SIZE_MISMATCH, p.bags, total, p.index_size);
+    }
+  }
+  int64_t pos = 0;  // of this lane's next candidate: one in every G indices of the bag
+  int len = 0;
+  {
+    const int64_t bag = (block * kWarps + warp) * (32 / G) + grp;
+    if (bag < p.bags) {
+      // no_bag: output row m is the single row indices[m]
+      const int64_t o0 = no_bag ? bag : load_int(p.offsets, bag, off64);
+      const int64_t o1 = no_bag ? bag + 1 : load_int(p.offsets, bag + 1, off64);
+      pos = o0 - off_base;
+      const int bag_len = (int)(o1 - o0);  // the reference narrows to 32 bits too
+      len = bag_len < 0 ? 0 : bag_len;
+      // Offsets that step backwards: the reference, which walks the index array
+      // with a running position, ends up past index_size and returns false.
+      if (bag_len < 0 || pos < 0 || pos + len > p.index_size) {
+        if (gl == 0) {
+          report(p.status, FBGEMM_B200_STATUS_BAG_OVERRUN, bag, pos, len);
+        }
+        len = 0;  // never read past the caller's arrays
+      }
+      pos += gl;
+    }
+  }
+  int longest = len;
+#pragma unroll
+  for (int d = G; d < 32; d <<= 1) {
+    longest = max(longest, __shfl_xor_sync(0xffffffffu, longest, d));
+  }
+
+  LaneData<VB, CPL, G, WIDE> lane_data;
+  lane_data.init(p.data, tile * kTileBytes, gl, p.data_bytes);
+  const uint8_t* sb_data = p.data + p.sb_off;
+  typename C::M constants;
+  constants.init(p);
+  u64 acc[C::kPairs];
+#pragma unroll
+  for (int k = 0; k < C::kPairs; ++k) {
+    acc[k] = 0ull;  // (+0.f, +0.f)
+  }
+
+  const uint32_t limit = (uint32_t)min((unsigned long long)p.data_size, idx64 ? 0xfffffffeull : 0x80000000ull);
+  auto fetch = [&](int c) -> uint2 {
+    uint2 r = make_uint2(0u, 0u);
+    if (c < len) {
+      if (idx64) {
+        r = __ldg(static_cast<const uint2*>(p.indices) + pos);
+      } else {
+        r.x = __ldg(static_cast<const uint32_t*>(p.indices) + pos);
+      }
+    }
+    return r;
+  };
+  uint2 raw = fetch(gl);
+  for (int c0 = 0; c0 < longest; c0 += G) {
+    const int c = c0 + gl;
+    const bool in_bag = c < len;
+    float w = 1.f;
+    if (weighted && in_bag) {
+      w = __ldg(p.weights + (positional ? (int64_t)c : pos));
+    }
+    bool keep;
+    if constexpr (WIDE) {
+      const long long v = idx64 ? (long long)(((u64)raw.y << 32) | raw.x) : (long long)(int)raw.x;
+      keep = in_bag && (u64)v < (u64)p.data_size;
+    } else {
+      keep = in_bag && raw.y == 0 && raw.x < limit;
+    }
+    Row<WIDE> id = 0;
+    if (keep) {
+      id = raw.x;
+      if constexpr (WIDE) {
+        id |= (u64)raw.y << 32;
+      }
+    }
+    if (in_bag && !keep && !(minus_one_skips && raw.x == 0xffffffffu && (!idx64 || raw.y == 0xffffffffu))) {
+      report(p.status, FBGEMM_B200_STATUS_BAD_INDEX, (block * kWarps + warp) * (32 / G) + grp, pos, (int32_t)raw.x);
+    }
+    if (pruned && keep) {
+      const int32_t m = __ldg(p.cit + id);
+      keep = m >= 0;
+      id = keep ? (uint32_t)m : 0u;
+    }
+    pos += G;
+    raw = fetch(c + G);  // the next stretch's, on its way during this one's arithmetic
+
+    // Kept rows to the front of the queue in order, the other lanes' slots behind them.  Those hold row 0 with scale
+    // and bias 0, which leave every sum as it is (x + 0 = x, and no sum is ever -0), so that groups of four rows
+    // need no special case for the last one.
+    const unsigned ballot = __ballot_sync(0xffffffffu, keep);
+    const unsigned kept = G == 32 ? ballot : (ballot >> (grp * G)) & kGroupMask;
+    const int count = __popc(kept);
+    int most = count;
+    const unsigned below = (1u << gl) - 1u;
+    const int at = keep ? __popc(kept & below) : most + __popc(~kept & below);
+    if constexpr (G < 32) {
+#pragma unroll
+      for (int g = 0; g < 32 / G; ++g) {
+        most = max(most, __popc((ballot >> (g * G)) & kGroupMask));
+      }
+    }
+    uint32_t sb_lo = 0, sb_hi = 0;
+    const Row<WIDE> row_at = id * (Row<WIDE>)p.stride;
+    q_row[at] = row_at;
+    if (kQuantized && keep) {
+      const uint8_t* s = sb_data + row_at;
+      if (half_sb) {
+        sb_lo = load_u32(s, p.sb_align);
+      } else if (p.sb_align >= 8) {
+        const uint2 v = __ldg(reinterpret_cast<const uint2*>(s));
+        sb_lo = v.x;
+        sb_hi = v.y;
+      } else {
+        sb_lo = load_u32(s, p.sb_align);
+        sb_hi = load_u32(s + 4, p.sb_align);
+      }
+    }
+    __syncwarp();
+
+    // The row loop, four rows at a time, the loads kAhead groups ahead of the arithmetic.
+    Bytes<VB> d[kAhead + 1][4][CPL];
+    auto load = [&](Bytes<VB> (&to)[4][CPL], int r) {
+      if constexpr (WIDE) {
+        const ulonglong2 ab = *reinterpret_cast<const ulonglong2*>(q_row + r);
+        const ulonglong2 cd = *reinterpret_cast<const ulonglong2*>(q_row + r + 2);
+        lane_data.load(to[0], ab.x);
+        lane_data.load(to[1], ab.y);
+        lane_data.load(to[2], cd.x);
+        lane_data.load(to[3], cd.y);
+      } else {
+        const uint4 rows = *reinterpret_cast<const uint4*>(q_row + r);
+        lane_data.load(to[0], rows.x);
+        lane_data.load(to[1], rows.y);
+        lane_data.load(to[2], rows.z);
+        lane_data.load(to[3], rows.w);
+      }
+    };
+#pragma unroll
+    for (int g = 0; g < kAhead; ++g) {
+      if (4 * g < most) {
+        load(d[g], 4 * g);
+      }
+    }
+    if constexpr (kQuantized) {
+      float scale, bias;
+      if (half_sb) {
+        scale = __half2float(__ushort_as_half((unsigned short)(sb_lo & 0xffffu)));
+        bias = __half2float(__ushort_as_half((unsigned short)(sb_lo >> 16)));
+      } else {
+        scale = __uint_as_float(sb_lo);
+        bias = __uint_as_float(sb_hi);
+      }
+      if (weighted && keep) {
+        scale = __fmul_rn(w, scale);
+        bias = __fmul_rn(w, bias);
+      }
+      q_sb[at] = make_ulonglong2(pack2(scale, scale), pack2(bias, bias));
+    } else {
+      q_sb[at].x = pack2(w, w);
+    }
+    __syncwarp();
+#pragma unroll 1
+    for (int r0 = 0; r0 < most; r0 += 4 * (kAhead + 1)) {
+#pragma unroll
+      for (int g = 0; g <= kAhead; ++g) {
+        const int r = r0 + 4 * g;
+        if (g > 0 && r >= most) {
+          break;
+        }
+        if (r + 4 * kAhead < most) {
+          load(d[(g + kAhead) % (kAhead + 1)], r + 4 * kAhead);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          if constexpr (kQuantized) {
+            const ulonglong2 s = q_sb[r + u];
+            C::pool(constants, acc, d[g][u], s.x, s.y);
+          } else if (r + u < count) {  // (row 0 times 0 is no harmless addition when its values may be infinite)
+            C::pool(constants, acc, d[g][u], q_sb[r + u].x, 0ull);
+          }
+        }
+      }
+    }
+    __syncwarp();  // the queue is rewritten by the next stretch
+  }
+
+  const int64_t bag = (block * kWarps + warp) * (32 / G) + grp;
+  if (bag >= p.bags) {
+    return;
+  }
+  int bag_len = 0;
+  if (p.flags & kNormalize) {
+    bag_len = (int)(load_int(p.offsets, bag + 1, off64) - load_int(p.offsets, bag, off64));
+  }
+  if (bag_len != 0) {
+    const float inv = __fdiv_rn(1.f, (float)bag_len);
+    const u64 inv2 = pack2(inv, inv);
+#pragma unroll
+    for (int k = 0; k < C::kPairs; ++k) {
+      acc[k] = mul2(acc[k], inv2);
+    }
+  }
+  char* row;
+  if (p.num_peers > 0) {
+    const int64_t d = bag / p.bags_per_peer;
+    row = static_cast<char*>(peers[d]) + (bag - d * p.bags_per_peer) * p.out_pitch;
+  } else {
+    row = static_cast<char*>(p.out) + bag * p.out_pitch;
+  }
+  float v[2 * C::kPairs];
+#pragma unroll
+  for (int k = 0; k < C::kPairs; ++k) {
+    unpack2(acc[k], v[2 * k], v[2 * k + 1]);
+  }
+#pragma unroll
+  for (int c = 0; c < CPL; ++c) {
+    const int col = tile * (kTileBytes * 8 / C::BITS) + (c * G + gl) * C::kPerChunk;
+    if (col < p.cols) {
+      store_columns<C::kPerChunk>(p, row, col, v + c * C::kPerChunk);
+    }
+  }
+}
+
+// 12 blocks of 4 warps per SM, i.e. 40 registers: a lookup waits for memory, and resident warps are what hides it.
+// 65536 bags of 30 rows took 82 / 112 / 77 us (8-bit D = 128, 4-bit D = 256, 4-bit D = 128) against 95 / 144 / 121 us
+// with the 60 to 100 registers the compiler takes when left alone; 16 blocks (32 registers) were no better.
+constexpr int kBlocksPerSm = 12;
+
+// One table per launch: its parameters travel in constant memory, blockIdx.y is the column tile.
+struct BagCall {
+  BagTable t;
+  void* peers[FBGEMM_B200_MAX_PEERS];
+};
+
+template <int FMT, int VB, int CPL, int G, bool WIDE>
+__global__ void __launch_bounds__(kThreads, kBlocksPerSm) bag_kernel(const __grid_constant__ BagCall c) {
+  __shared__ Queue<WIDE> queues[kWarps];
+  pool_bags<FMT, VB, CPL, G, WIDE>(c.t, c.peers, blockIdx.x, blockIdx.y, queues);
+}
+
+// The same for launches whose warps are all resident with 64 registers each:
+// residency costs nothing there, so they go into more rows in flight per bag.
+// 10 bags of 100 rows (8-bit D = 64) 7.4 against 8.7 us, 4096 ragged bags (4-bit
+// D = 64) 8.0 against 8.6 us.
+constexpr int kDeepBlocksPerSm = 8;
+template <int FMT, int VB, int CPL, int G, bool WIDE>
+__global__ void __launch_bounds__(kThreads, kDeepBlocksPerSm) bag_kernel_deep(const __grid_constant__ BagCall c) {
+  __shared__ Queue<WIDE> queues[kWarps];
+  pool_bags<FMT, VB, CPL, G, WIDE, kDeepAhead>(c.t, c.peers, blockIdx.x, blockIdx.y, queues);
+}
+
+// The compiled combinations of row format, payload bytes per lane and chunk,
+// chunks per lane and lanes per bag.  Whole warps (32 lanes) for every format
+// and alignment, wide rows in several tiles; half and quarter warps for the
+// narrow rows of large batches (see pick_variant in bag_dispatch.cu).
+#define FBGEMM_B200_BAG_VARIANTS_8(X)                                                                       \
+  X(kInt8, 2, 1, 16) X(kInt8, 1, 2, 16) X(kInt8, 4, 1, 16) X(kInt8, 8, 1, 16) X(kInt8, 4, 2, 16)              \
+  X(kInt8, 2, 1, 32) X(kInt8, 1, 2, 32) X(kInt8, 4, 1, 32) X(kInt8, 2, 2, 32) X(kInt8, 1, 4, 32)              \
+  X(kInt8, 8, 1, 32) X(kInt8, 4, 2, 32)
+#define FBGEMM_B200_BAG_VARIANTS_4(X)                                                                       \
+  X(kInt4, 2, 1, 8) X(kInt4, 4, 1, 8) X(kInt4, 1, 1, 16) X(kInt4, 2, 1, 16) X(kInt4, 4, 1, 16)                \
+  X(kInt4, 1, 1, 32) X(kInt4, 2, 1, 32) X(kInt4, 1, 2, 32) X(kInt4, 4, 1, 32) X(kInt4, 2, 2, 32) X(kInt4, 1, 4, 32)
+#define FBGEMM_B200_BAG_VARIANTS_2(X)                                                                       \
+  X(kInt2, 2, 1, 8) X(kInt2, 1, 1, 16) X(kInt2, 2, 1, 16)                                                     \
+  X(kInt2, 1, 1, 32) X(kInt2, 2, 1, 32) X(kInt2, 1, 2, 32)
+#define FBGEMM_B200_BAG_VARIANTS_PLAIN(X)                                                                   \
+  X(kF32, 16, 1, 32) X(kF32, 8, 1, 32) X(kF32, 4, 2, 32)                                                      \
+  X(kF16, 8, 1, 32) X(kF16, 4, 1, 32) X(kF16, 2, 2, 32)                                                       \
+  X(kBf16, 8, 1, 32) X(kBf16, 4, 1, 32) X(kBf16, 2, 2, 32)                                                    \
+  X(kFp8, 4, 1, 32) X(kFp8, 2, 1, 32) X(kFp8, 1, 2, 32)
+#define FBGEMM_B200_BAG_VARIANTS(X) \
+  FBGEMM_B200_BAG_VARIANTS_8(X) FBGEMM_B200_BAG_VARIANTS_4(X) FBGEMM_B200_BAG_VARIANTS_2(X) FBGEMM_B200_BAG_VARIANTS_PLAIN(X)
+
+#define FBGEMM_B200_BAG_ID(FMT, VB, CPL, G) id_##FMT##_##VB##_##CPL##_##G,
+enum VariantId : int { FBGEMM_B200_BAG_VARIANTS(FBGEMM_B200_BAG_ID) kVariants };
+#undef FBGEMM_B200_BAG_ID
+
+// Several tables per launch (what the reference's multi-table caller does with
+// a loop of functor calls, fbgemm_gpu/codegen/inference/embedding_forward_quantized_cpu_template.cpp:343-473):
+// unit u - one column tile of one table - owns the blocks [first_block[u],
+// first_block[u + 1]), whatever the tables' row formats.  The units arrive by
+// value, in constant memory; a block finds its own by bisection.
+constexpr int kMaxUnits = 64;
+struct BagUnits {
+  int32_t count;
+  int32_t first_block[kMaxUnits + 1];
+  uint16_t variant[kMaxUnits];
+  uint16_t tile[kMaxUnits];
+  BagTable t[kMaxUnits];
+  void* peers[kMaxUnits][FBGEMM_B200_MAX_PEERS];
+};
+static_assert(sizeof(BagUnits) < 32764, "one kernel argument");
+
+template <bool WIDE>
+__global__ void __launch_bounds__(kThreads, kBlocksPerSm) bag_units_kernel(const __grid_constant__ BagUnits a) {
+  __shared__ Queue<WIDE> queues[kWarps];
+  int lo = 0, hi = a.count;
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if ((int)blockIdx.x >= a.first_block[mid]) {
+      lo = mid;
+    } else {
+      hi = mid;
+    }
+  }
+  const BagTable& t = a.t[lo];
+  const int64_t block = (int)blockIdx.x - a.first_block[lo];
+  switch (a.variant[lo]) {
+#define FBGEMM_B200_BAG_CASE(FMT, VB, CPL, G)                                   \
+  case id_##FMT##_##VB##_##CPL##_##G:                                           \
+    pool_bags<FMT, VB, CPL, G, WIDE>(t, a.peers[lo], block, a.tile[lo], queues); \
+    break;
+    FBGEMM_B200_BAG_VARIANTS(FBGEMM_B200_BAG_CASE)
+#undef FBGEMM_B200_BAG_CASE
+  }
+}
+
+using BagFn = void (*)(const BagCall);
+using BagUnitsFn = void (*)(const BagUnits);
+
+}  // namespace bag
+
+// The single-table kernels by variant id, indexed by whether rows lie beyond 4
+// GB, plus 2 for the deep form (whole warps per bag only); one translation unit
+// per group of formats (bag_kernel_*.cu).
+void bag_kernels_8(bag::BagFn (*fn)[4]);
+void bag_kernels_4(bag::BagFn (*fn)[4]);
+void bag_kernels_2(bag::BagFn (*fn)[4]);
+void bag_kernels_plain(bag::BagFn (*fn)[4]);
+bag::BagUnitsFn bag_units_narrow();
+bag::BagUnitsFn bag_units_wide();
+
+}  // namespace fbgemm_b200

@@ -684,7 +684,7 @@ int fbgemm_b200_multi_plan_create(
     return FBGEMM_B200_ENOMEM;
   }
   plan->device = ctx->device;
-  const cudaError_t e = build_multi_plan(params, bit_rates, &plan->plan);
+  const cudaError_t e = build_multi_plan(params.data(), bit_rates.data(), params.size(), &plan->plan);
   if (e != cudaSuccess) {
     delete plan;
     return fail_cuda(e, "multi-table plan");
@@ -707,7 +707,7 @@ int fbgemm_b200_multi_plan_launch(fbgemm_b200_multi_plan* plan, void* stream) {
 }
 
 int fbgemm_b200_multi_plan_num_launches(const fbgemm_b200_multi_plan* plan) {
-  return plan ? (int)(plan->plan.groups.size() + plan->plan.singles.size()) : 0;
+  return plan ? (int)plan->plan.launches.size() : 0;
 }
 
 void fbgemm_b200_multi_plan_destroy(fbgemm_b200_multi_plan* plan) {

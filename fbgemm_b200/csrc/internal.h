@@ -5,6 +5,7 @@
 
 #include <atomic>
 #include <cstdint>
+#include <memory>
 #include <string>
 #include <utility>
 #include <vector>
@@ -77,49 +78,52 @@ __device__ __forceinline__ char* output_row(const SpmdmParams& p, int64_t bag, i
   return static_cast<char*>(p.out) + bag * p.output_stride * esize;
 }
 
+// One table of a lookup as the bag kernels (bag_kernel.cuh) take it.
+struct BagTable {
+  const uint8_t* data;        // first payload byte of row 0
+  const void* indices;
+  const void* offsets;
+  const float* weights;
+  const int32_t* cit;
+  void* out;
+  int32_t* status;
+  int64_t data_size;
+  int64_t bags;
+  int64_t index_size;
+  int64_t out_pitch;          // bytes between output rows
+  int64_t bags_per_peer;
+  int64_t stride;             // bytes between table rows
+  int32_t sb_off;             // scale,bias relative to `data`
+  int32_t cols;               // D
+  int32_t data_bytes;         // packed payload bytes per row
+  uint32_t flags;
+  int16_t sb_align;           // address alignment of scale,bias: 8, 4, 2 or 1
+  int16_t out_align;          // address alignment of output rows: 16 ... 1
+  int32_t num_peers;
+  int16_t fp8_exponent_bits;
+  int16_t fp8_exponent_bias;
+};
+
 // One lookup kernel launch (spmdm_kernels.cu).  Returns cudaSuccess or the
 // launch error; never synchronises.
 cudaError_t launch_spmdm(const SpmdmParams& p, int bit_rate, cudaStream_t stream);
 
-// The argument of one multi-table launch: up to kMultiTables tables of the
-// same kernel variant, passed by value so that, like the single-table
-// kernel's, their parameters live in constant memory.  Table t owns the blocks
-// [first_block[t], first_block[t + 1]).
-constexpr int kMultiTables = 16;
-struct MultiArgs {
-  int32_t count;
-  int32_t first_block[kMultiTables + 1];
-  SpmdmParams t[kMultiTables];
-};
-static_assert(sizeof(MultiArgs) <= 4096, "one kernel argument, within the classic 4 KB of parameter space");
+// The bag kernel for this lookup (bag_dispatch.cu).
+cudaError_t launch_bags(const SpmdmParams& p, int bit_rate, cudaStream_t stream);
 
-// Several tables per call (spmdm_kernels.cu): the tables grouped by kernel
-// variant, each group cut into launches of up to kMultiTables tables.  Built
-// once for a fixed set of pointers, launched as often as wanted.
+// Several tables per call (bag_dispatch.cu): up to 64 column tiles of tables of
+// any row formats per launch.  Built for a fixed set of pointers, launched as
+// often as wanted.
+struct UnitsLaunch;
 struct MultiPlan {
-  struct Launch {
-    void (*fn)(const MultiArgs);
-    unsigned blocks;    // grid size
-    MultiArgs args;
-  };
-  std::vector<Launch> groups;
-  std::vector<std::pair<SpmdmParams, int>> singles;  // (parameters, bit rate): one launch each
-  // The launches of one call overlap: all but the first go to side streams
-  // that fork from, and join, the caller's stream through these events.
-  static constexpr int kSideStreams = 3;
-  cudaStream_t side[kSideStreams] = {};
-  cudaEvent_t fork = nullptr;
-  cudaEvent_t join[kSideStreams] = {};
-  MultiPlan() = default;
+  std::vector<std::unique_ptr<UnitsLaunch>> launches;
+  MultiPlan();
   MultiPlan(const MultiPlan&) = delete;
   MultiPlan& operator=(const MultiPlan&) = delete;
   ~MultiPlan();
 };
-cudaError_t build_multi_plan(const std::vector<SpmdmParams>& tables, const std::vector<int>& bit_rates, MultiPlan* plan);
+cudaError_t build_multi_plan(const SpmdmParams* tables, const int* bit_rates, size_t count, MultiPlan* plan);
 cudaError_t launch_multi_plan(const MultiPlan& plan, cudaStream_t stream);
-
-// The lookup on a table that is not row-wise quantized (plain_kernels.cu).
-cudaError_t launch_plain_rows(const SpmdmParams& p, cudaStream_t stream);
 
 // no_bag with 8-bit output: byte copies of the indexed rows (plain_kernels.cu).
 cudaError_t launch_rows_copy(

@@ -7,11 +7,9 @@
 //
 //     acc[j] = fma(w*scale, q[j], acc[j] + w*bias)    rows in index order
 //
-// This file holds (1) the staged kernel, which takes every shape and option,
-// (2) the dispatcher that sends a lookup to one of the register-resident
-// direct kernels (spmdm_direct.cuh; dense or compacting) when a variant fits
-// the row width, else to the staged kernel, and (3) the multi-table plans that
-// put up to 16 tables of the same variant into one launch.
+// This file holds the staged kernel, which fbgemm_b200_set_kernel_choice(GENERIC)
+// selects for quantized rows of every shape and option.  All other lookups go
+// to the bag kernels (bag_kernel.cuh, bag_dispatch.cu).
 //
 // Scheduling of the staged kernel.  A bag is owned by a group of LPB lanes (8,
 // 16 or a full warp,
@@ -29,14 +27,7 @@
 // have no role here.
 #include <cuda_fp16.h>
 
-#include <cstdlib>
-#include <cstring>
-
-#include <algorithm>
-#include <vector>
-
 #include "internal.h"
-#include "spmdm_direct.cuh"
 
 namespace fbgemm_b200 {
 
@@ -435,20 +426,6 @@ const Variant* variants(int* count) {
   }
 }
 
-// Overrides of the variant choice exist only in tuning builds
-// (-DFBGEMM_B200_TUNING, which also instantiates variants the dispatcher never
-// picks); the product's launch path reads no environment variable.
-#ifdef FBGEMM_B200_TUNING
-int env_int(const char* name, int dflt) {
-  const char* s = std::getenv(name);
-  return (s && *s) ? std::atoi(s) : dflt;
-}
-#else
-constexpr int env_int(const char*, int dflt) {
-  return dflt;
-}
-#endif
-
 }  // namespace
 
 std::atomic<uint64_t> g_launch_count{0};
@@ -458,240 +435,9 @@ int max_chunks_per_bag(int bit_rate) {
   return 32 * (bit_rate == 8 ? 8 : bit_rate == 4 ? 4 : 2);
 }
 
-// The variant of the direct kernel (spmdm_direct.cuh) for this call, or null
-// when the rows do not allow 4- or 8-byte vector loads.
-static const direct::Variant* pick_direct(const SpmdmParams& p, int bit_rate) {
-  if (p.in_kind != 0) {
-    return nullptr;  // not a quantized row format
-  }
-  const uintptr_t base = reinterpret_cast<uintptr_t>(p.table);
-  auto divides = [&](int v) {
-    return base % 4 == 0 && (base + p.data_row_off) % v == 0 && p.input_stride % v == 0 && p.data_bytes % v == 0;
-  };
-  // Row ids travel between lanes as 32-bit values and skipped rows read row 0.
-  if (!divides(4) || p.data_bytes == 0 || p.data_size == 0 || p.data_size > 0xfffffffeLL ||
-      p.input_stride > 0xffffffffLL) {
-    return nullptr;
-  }
-  int vec = divides(8) ? 8 : 4;
-  const int env_vec = env_int("FBGEMM_B200_VEC", 0);
-  if (env_vec == 4) {
-    vec = 4;
-  }
-  int count = 0;
-  const direct::Variant* v = bit_rate == 8 ? direct_variants_8(&count)
-      : bit_rate == 4                      ? direct_variants_4(&count)
-                                           : direct_variants_2(&count);
-  const int cpc = vec * 8 / bit_rate;      // columns per chunk
-  const int nchunks = p.data_bytes / vec;
-  int cpl_max = 0;
-  for (int i = 0; i < count; ++i) {
-    if (v[i].vec == vec && v[i].cpl > cpl_max) {
-      cpl_max = v[i].cpl;
-    }
-  }
-  // Columns per lane: narrow lane groups amortise the per-row work that does
-  // not scale with D, wide ones keep registers (and so resident warps) in
-  // check.  Measured best on B200: 32 columns for 8-bit rows, 16 for 4- and
-  // 2-bit rows (whose unpacking needs more registers per column).
-  // Rows of 256 and more 8-bit columns do better with 16 again (two bags per
-  // warp instead of four: 67 against 73 ps per row at D = 256, the ragged bags
-  // of a warp wait less for each other).
-  const int cols_target = bit_rate == 8 ? (p.data_bytes >= 256 ? 16 : 32) : 16;
-  int cpl_target = cols_target / cpc < 1 ? 1 : cols_target / cpc;
-  cpl_target = cpl_target > cpl_max ? cpl_max : cpl_target;
-  // At least 4 lanes per bag: with 2 (sixteen bags per warp) an 8-bit D=64
-  // table measured 32 us per 16384-bag call against 25.5 us with 4.
-  int lpb = 4;
-  while (lpb < 32 && lpb * cpl_target < nchunks) {
-    lpb *= 2;
-  }
-  int cpl = 1;
-  while (lpb * cpl < nchunks) {
-    cpl *= 2;
-  }
-  const int env_lpb = env_int("FBGEMM_B200_LPB", 0);
-  const int env_cpl = env_int("FBGEMM_B200_CPL", 0);
-  if (env_lpb > 0 && env_cpl > 0 && env_lpb * env_cpl >= nchunks) {
-    lpb = env_lpb;
-    cpl = env_cpl;
-  }
-  const direct::Variant* pick = nullptr;
-  for (int i = 0; i < count; ++i) {
-    if (v[i].vec == vec && v[i].lpb == lpb && v[i].cpl == cpl) {
-      pick = &v[i];
-    }
-  }
-  return pick;
-}
-
-// 1 when the row's payload is exactly the variant's LPB * CPL chunks.
-static int direct_exact(const direct::Variant* v, const SpmdmParams& p) {
-  return p.data_bytes == v->vec * v->lpb * v->cpl ? 1 : 0;
-}
-
-static int64_t direct_blocks(const direct::Variant* v, int64_t bags) {
-  const int64_t bags_per_block = (int64_t)direct::kWarpsPerBlock * (32 / v->lpb);
-  return (bags + bags_per_block - 1) / bags_per_block;
-}
-
-// One table, one launch; returns cudaErrorNotSupported when the direct kernel
-// cannot take the rows.
-static cudaError_t launch_direct(const SpmdmParams& p, int bit_rate, cudaStream_t stream) {
-  const direct::Variant* pick = pick_direct(p, bit_rate);
-  if (!pick) {
-    return cudaErrorNotSupported;
-  }
-  const int64_t blocks = direct_blocks(pick, p.output_size);
-  if (blocks <= 0 || blocks > 0x7fffffffLL) {
-    return cudaErrorInvalidValue;
-  }
-  // Tables in which an index may name no row (a pruning map, or the layout in
-  // which -1 is a pruned index) take the compacting kernel; the plain one has
-  // no notion of a skipped row.
-  const bool compact = (p.flags & (kPruned | kSbFirst)) || env_int("FBGEMM_B200_COMPACT", 0) == 1;
-  const int exact = direct_exact(pick, p);
-  (compact ? pick->compact[exact] : pick->fn[exact])<<<(unsigned)blocks, direct::kThreads, 0, stream>>>(p);
-  g_launch_count.fetch_add(1, std::memory_order_relaxed);
-  return cudaGetLastError();
-}
-
-// ---- several tables per launch --------------------------------------------------
-
-MultiPlan::~MultiPlan() {
-  for (int i = 0; i < kSideStreams; ++i) {
-    if (side[i]) {
-      cudaStreamDestroy(side[i]);
-    }
-    if (join[i]) {
-      cudaEventDestroy(join[i]);
-    }
-  }
-  if (fork) {
-    cudaEventDestroy(fork);
-  }
-}
-
-// Tables that share a kernel variant go into one launch (up to kMultiTables of
-// them): their parameters travel as the kernel's argument and the grid is the
-// sum of their blocks.  Tables the direct kernel cannot take keep a launch of
-// their own.
-cudaError_t build_multi_plan(const std::vector<SpmdmParams>& tables, const std::vector<int>& bit_rates, MultiPlan* plan) {
-  std::vector<const direct::Variant*> variant(tables.size());
-  std::vector<size_t> order;
-  for (size_t t = 0; t < tables.size(); ++t) {
-    variant[t] = tables[t].output_size > 0 ? pick_direct(tables[t], bit_rates[t]) : nullptr;
-    if (tables[t].output_size <= 0) {
-      continue;  // nothing to pool, nothing to store
-    }
-    if (variant[t]) {
-      order.push_back(t);
-    } else {
-      plan->singles.push_back({tables[t], bit_rates[t]});
-    }
-  }
-  // what decides a table's kernel besides the variant: 2 = rows may be skipped, 1 = exact-fit addressing
-  auto form = [&](size_t t) {
-    return ((tables[t].flags & (kPruned | kSbFirst)) != 0 ? 2 : 0) + direct_exact(variant[t], tables[t]);
-  };
-  std::stable_sort(order.begin(), order.end(), [&](size_t a, size_t b) {
-    return variant[a] != variant[b] ? variant[a] < variant[b] : form(a) < form(b);
-  });
-  for (size_t i = 0; i < order.size();) {
-    const direct::Variant* v = variant[order[i]];
-    const int f = form(order[i]);
-    plan->groups.emplace_back();
-    MultiPlan::Launch& g = plan->groups.back();
-    g.fn = (f & 2) ? v->compact_multi[f & 1] : v->multi[f & 1];
-    g.args = MultiArgs{};
-    int64_t blocks = 0;
-    for (; i < order.size() && variant[order[i]] == v && form(order[i]) == f && g.args.count < kMultiTables; ++i) {
-      const int64_t b = direct_blocks(v, tables[order[i]].output_size);
-      if (blocks + b > 0x7fffffffLL) {
-        break;  // the rest of this variant's tables start a new launch
-      }
-      g.args.first_block[g.args.count] = (int32_t)blocks;
-      g.args.t[g.args.count] = tables[order[i]];
-      blocks += b;
-      ++g.args.count;
-    }
-    if (g.args.count == 0) {
-      return cudaErrorInvalidValue;  // a single table with more than 2^31 blocks
-    }
-    g.args.first_block[g.args.count] = (int32_t)blocks;
-    g.blocks = (unsigned)blocks;
-  }
-  // largest grid first: the short launches fill the tail of the long ones
-  std::stable_sort(plan->groups.begin(), plan->groups.end(),
-                   [](const MultiPlan::Launch& a, const MultiPlan::Launch& b) { return a.blocks > b.blocks; });
-  if (plan->groups.size() + plan->singles.size() > 1) {
-    cudaError_t e = cudaEventCreateWithFlags(&plan->fork, cudaEventDisableTiming);
-    for (int i = 0; i < MultiPlan::kSideStreams && e == cudaSuccess; ++i) {
-      e = cudaStreamCreateWithFlags(&plan->side[i], cudaStreamNonBlocking);
-      if (e == cudaSuccess) {
-        e = cudaEventCreateWithFlags(&plan->join[i], cudaEventDisableTiming);
-      }
-    }
-    if (e != cudaSuccess) {
-      return e;
-    }
-  }
-  return cudaSuccess;
-}
-
-cudaError_t launch_multi_plan(const MultiPlan& plan, cudaStream_t stream) {
-  const size_t launches = plan.groups.size() + plan.singles.size();
-  const bool spread = launches > 1 && plan.fork;
-  cudaError_t e = cudaSuccess;
-  if (spread) {
-    e = cudaEventRecord(plan.fork, stream);
-    for (int i = 0; i < MultiPlan::kSideStreams && e == cudaSuccess; ++i) {
-      e = cudaStreamWaitEvent(plan.side[i], plan.fork, 0);
-    }
-    if (e != cudaSuccess) {
-      return e;
-    }
-  }
-  size_t n = 0;  // launch n goes to the caller's stream (n % 4 == 0) or to side stream n % 4 - 1
-  auto stream_of = [&](size_t i) {
-    const size_t k = i % (MultiPlan::kSideStreams + 1);
-    return (!spread || k == 0) ? stream : plan.side[k - 1];
-  };
-  for (const MultiPlan::Launch& g : plan.groups) {
-    g.fn<<<g.blocks, direct::kThreads, 0, stream_of(n++)>>>(g.args);
-    g_launch_count.fetch_add(1, std::memory_order_relaxed);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) {
-      return e;
-    }
-  }
-  for (const auto& single : plan.singles) {
-    e = launch_spmdm(single.first, single.second, stream_of(n++));
-    if (e != cudaSuccess) {
-      return e;
-    }
-  }
-  if (spread) {
-    for (int i = 0; i < MultiPlan::kSideStreams && e == cudaSuccess; ++i) {
-      e = cudaEventRecord(plan.join[i], plan.side[i]);
-      if (e == cudaSuccess) {
-        e = cudaStreamWaitEvent(stream, plan.join[i], 0);
-      }
-    }
-  }
-  return e;
-}
-
 cudaError_t launch_spmdm(const SpmdmParams& p_in, int bit_rate, cudaStream_t stream) {
-  if (p_in.in_kind != 0) {
-    return launch_plain_rows(p_in, stream);
-  }
-  const bool staged_only = g_kernel_choice.load(std::memory_order_relaxed) == FBGEMM_B200_KERNEL_GENERIC;
-  if (!staged_only) {
-    const cudaError_t e = launch_direct(p_in, bit_rate, stream);
-    if (e != cudaErrorNotSupported) {
-      return e;
-    }
+  if (p_in.in_kind != 0 || g_kernel_choice.load(std::memory_order_relaxed) != FBGEMM_B200_KERNEL_GENERIC) {
+    return launch_bags(p_in, bit_rate, stream);
   }
   SpmdmParams p = p_in;
   int count = 0;
@@ -704,12 +450,6 @@ cudaError_t launch_spmdm(const SpmdmParams& p_in, int bit_rate, cudaStream_t str
   int want_cpl = 1;
   while (want_lpb * want_cpl < nchunks) {
     want_cpl *= 2;
-  }
-  const int env_lpb = env_int("FBGEMM_B200_LPB", 0);
-  const int env_cpl = env_int("FBGEMM_B200_CPL", 0);
-  if (env_lpb > 0 && env_cpl > 0 && env_lpb * env_cpl >= nchunks) {
-    want_lpb = env_lpb;
-    want_cpl = env_cpl;
   }
   const Variant* pick = nullptr;
   for (int i = 0; i < count; ++i) {
@@ -724,8 +464,8 @@ cudaError_t launch_spmdm(const SpmdmParams& p_in, int bit_rate, cudaStream_t str
   // Shared-memory stage: per bag slot `rows_per_wave` rows, their byte offsets
   // (8 B) and weights (4 B).
   const int gpw = 32 / pick->lpb;
-  const int warp_budget = env_int("FBGEMM_B200_SMEM_PER_WARP", 6144);
-  const int max_rows = env_int("FBGEMM_B200_WAVE_ROWS", 64);
+  const int warp_budget = 6144;
+  const int max_rows = 64;
   int rows = (warp_budget / gpw) / (p.pitch + 12);
   rows = rows < 1 ? 1 : rows > max_rows ? max_rows : rows;
   p.rows_per_wave = rows;

@@ -1,0 +1,115 @@
+"""The pooled lookup at the edges of its kernels: row widths around the column
+tiles, every alignment of a row, bags around the 32 (16, 8) indices a lane group
+walks at a time, batches for whole, half and quarter warps per bag, rows beyond
+4 GB, and more tables than one launch takes.  Bit for bit against the CPU
+oracle."""
+import numpy as np
+import pytest
+import torch
+
+import fbgemm_b200 as F
+from conftest import bits
+from helpers import random_fused_table, row_bytes
+
+pytestmark = pytest.mark.gpu
+EDGE_LENGTHS = np.array([0, 1, 3, 4, 5, 7, 8, 9, 12, 15, 16, 17, 31, 32, 33, 47, 64, 65])
+
+
+def dev(a):
+    return None if a is None else torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+
+def generate(bit_rate, dim, weighted, sb_last, stride):
+    kw = dict(index_dtype=np.int64, offset_dtype=np.int32, out_dtype=np.float32)
+    if bit_rate == 8:
+        return F.GenerateEmbeddingSpMDMWithStrides(dim, weighted, False, 16, False, True, -1, stride, sb_last, **kw)
+    return F.GenerateEmbeddingSpMDMNBitWithStrides(bit_rate, dim, weighted, False, 16, False, True, -1, stride, sb_last, **kw)
+
+
+def check(oracle, rng, bit_rate, dim, batch, sb_last, pad, weighted=True, rows=150):
+    natural = (dim * bit_rate + 7) // 8 + (8 if bit_rate == 8 and sb_last else 4)
+    stride = natural + pad
+    table = random_fused_table(rng, rows, dim, bit_rate, stride, not sb_last)
+    lengths = rng.choice(EDGE_LENGTHS, batch) if batch < 1000 else rng.integers(0, 4, batch)
+    if batch >= 1000:
+        lengths[rng.integers(0, batch, 60)] = rng.choice(EDGE_LENGTHS, 60)
+    n = int(lengths.sum())
+    indices = rng.integers(0, rows, n)
+    if not sb_last:
+        indices[rng.random(n) < 0.3] = -1
+    offsets = np.concatenate([[0], np.cumsum(lengths)]).astype(np.int32)
+    w = rng.standard_normal(n).astype(np.float32) if weighted else None
+    ok_ref, ref = oracle.spmdm_ex(bit_rate, dim, rows, table, indices, offsets, w, False, "f32", False, True, -1, stride,
+                                  sb_last, False, output_size=batch, index_size=n)
+    out = torch.ones(batch * dim + 8, device="cuda")
+    ok = generate(bit_rate, dim, weighted, sb_last, stride)(batch, n, rows, dev(table), dev(indices), dev(offsets), dev(w), out)
+    assert ok and ok_ref
+    got = out.cpu().numpy()
+    assert (got[batch * dim:] == 1).all(), "wrote past the output"
+    np.testing.assert_array_equal(bits(got[:batch * dim]), bits(ref[:batch * dim]))
+
+
+@pytest.mark.parametrize("bit_rate", [8, 4, 2])
+@pytest.mark.parametrize("sb_last", [True, False])
+def test_row_widths_and_alignments(gpu_ctx, oracle, bit_rate, sb_last):
+    rng = np.random.default_rng(100 * bit_rate + sb_last)
+    for dim in (1, 2, 15, 16, 17, 31, 32, 33, 63, 64, 65, 127, 128, 129, 255, 256, 257, 300, 520, 1024):
+        for pad in (0, 1, 2, 4):
+            check(oracle, rng, bit_rate, dim, 40, sb_last, pad, weighted=(dim + pad) % 2 == 0)
+
+
+@pytest.mark.parametrize("bit_rate", [8, 4, 2])
+@pytest.mark.parametrize("batch", [7104, 7105, 28416, 28417])
+def test_lanes_per_bag(gpu_ctx, oracle, bit_rate, batch):
+    rng = np.random.default_rng(7 * bit_rate + batch)
+    for dim in (20, 32, 64, 128):
+        check(oracle, rng, bit_rate, dim, batch, dim != 64, 0)
+
+
+@pytest.mark.parametrize("bit_rate", [8, 4])
+def test_rows_beyond_4gb(gpu_ctx, oracle, bit_rate):
+    """Few rows, far apart: the table's pitch puts them beyond 32-bit offsets."""
+    rng = np.random.default_rng(bit_rate)
+    dim, rows, stride, batch = 64, 70_000, 65_536, 50
+    used = np.sort(rng.choice(rows, 64, replace=False))
+    used[-1] = rows - 1
+    compact = random_fused_table(rng, len(used), dim, bit_rate)
+    table = torch.zeros(rows * stride, dtype=torch.uint8, device="cuda").view(rows, stride)
+    table[torch.from_numpy(used).cuda(), :row_bytes(bit_rate, dim)] = dev(compact)
+    lengths = rng.choice(EDGE_LENGTHS, batch)
+    n = int(lengths.sum())
+    pick = rng.integers(0, len(used), n)
+    offsets = np.concatenate([[0], np.cumsum(lengths)]).astype(np.int32)
+    w = rng.standard_normal(n).astype(np.float32)
+    ok_ref, ref = oracle.spmdm(bit_rate, dim, len(used), compact, pick, offsets, w, False, np.float32, False, True,
+                               output_size=batch, index_size=n)
+    out = torch.zeros(batch * dim, device="cuda")
+    kern = generate(bit_rate, dim, True, True, stride)
+    assert kern(batch, n, rows, table, dev(used[pick]), dev(offsets), dev(w), out) and ok_ref
+    np.testing.assert_array_equal(bits(out.cpu().numpy()), bits(ref))
+    bad = used[pick].copy()
+    bad[0] = rows
+    assert not kern(batch, n, rows, table, dev(bad), dev(offsets), dev(w), out)
+
+
+def test_more_tables_than_one_launch_takes(gpu_ctx, oracle):
+    rng = np.random.default_rng(9)
+    calls, want = [], []
+    for t in range(70):
+        bit_rate, dim, batch, rows = (8, 4, 2)[t % 3], (64, 20, 300, 128)[t % 4], 33 + t, 50
+        table = random_fused_table(rng, rows, dim, bit_rate)
+        lengths = rng.choice(EDGE_LENGTHS, batch)
+        n = int(lengths.sum())
+        indices = rng.integers(0, rows, n)
+        offsets = np.concatenate([[0], np.cumsum(lengths)]).astype(np.int32)
+        w = rng.standard_normal(n).astype(np.float32)
+        want.append(oracle.spmdm(bit_rate, dim, rows, table, indices, offsets, w, False, np.float32, False, True,
+                                 output_size=batch, index_size=n)[1])
+        calls.append((generate(bit_rate, dim, True, True, -1), batch, n, rows, dev(table), dev(indices), dev(offsets),
+                      dev(w), torch.zeros(batch * dim, device="cuda"), None))
+    plan = F.MultiTablePlan(calls)
+    plan.launch()
+    assert F.status_read(0)[0]
+    for c, ref in zip(calls, want):
+        np.testing.assert_array_equal(bits(c[8].cpu().numpy()), bits(ref))
+    plan.close()
