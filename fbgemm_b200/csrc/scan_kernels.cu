@@ -4,8 +4,10 @@
 // sequentially (`current += len`, src/RefImplementations.cc:1290-1298); on the
 // GPU every bag has to know its start up front.
 //
-// Three small launches: per-tile scan, scan of the tile totals by one block,
-// add-back.  Each length is narrowed to 32 bits first, as `int len` does in
+// Bound by launches, not by the few kilobytes: up to kOneBlockTiles tiles one
+// block walks them with a running total (one launch; 3001 bags took three
+// launches and 9.1 us), beyond that every tile is scanned by its own block and a
+// second launch adds the total of the tiles before it.  Each length is narrowed to 32 bits first, as `int len` does in
 // the reference, and a negative length advances nothing.
 #include "internal.h"
 
@@ -16,6 +18,7 @@ namespace {
 constexpr int kScanThreads = 1024;
 constexpr int kItemsPerThread = 4;
 constexpr int kTile = kScanThreads * kItemsPerThread;
+constexpr int kOneBlockTiles = 4;
 
 __device__ __forceinline__ int64_t load_len(const void* p, int64_t i, bool is64, int64_t n) {
   if (i >= n) {
@@ -89,36 +92,54 @@ scan_tiles(const void* lengths, int is64, int64_t n, int64_t* offsets, int64_t* 
   }
 }
 
-// One block turns tile_sums[0..m) into its exclusive scan, in place, and
-// writes the grand total to offsets[n].
 __global__ void __launch_bounds__(kScanThreads)
-scan_tile_sums(int64_t* tile_sums, int64_t m, int64_t* offsets, int64_t n) {
+scan_one_block(const void* lengths, int is64, int64_t n, int64_t* offsets) {
   __shared__ int64_t total;
   int64_t carry = 0;
-  for (int64_t base = 0; base < m; base += kScanThreads) {
-    const int64_t i = base + threadIdx.x;
-    const int64_t v = i < m ? tile_sums[i] : 0;
-    const int64_t prefix = block_exclusive_scan(v, &total);
-    if (i < m) {
-      tile_sums[i] = carry + prefix;
+  for (int64_t tile = 0; tile < n; tile += kTile) {
+    const int64_t base = tile + (int64_t)threadIdx.x * kItemsPerThread;
+    int64_t v[kItemsPerThread];
+    int64_t sum = 0;
+#pragma unroll
+    for (int i = 0; i < kItemsPerThread; ++i) {
+      v[i] = load_len(lengths, base + i, is64 != 0, n);
+      sum += v[i];
+    }
+    int64_t prefix = carry + block_exclusive_scan(sum, &total);
+#pragma unroll
+    for (int i = 0; i < kItemsPerThread; ++i) {
+      if (base + i < n) {
+        offsets[base + i] = prefix;
+      }
+      prefix += v[i];
     }
     carry += total;
-    __syncthreads();
+    __syncthreads();  // `total` is rewritten by the next tile's scan
   }
   if (threadIdx.x == 0) {
     offsets[n] = carry;
   }
 }
 
+// Tile b's offsets moved up by the lengths of the tiles before it; the last block also writes the grand total.
 __global__ void __launch_bounds__(kScanThreads)
 add_tile_prefix(int64_t* offsets, const int64_t* tile_sums, int64_t n) {
-  const int64_t add = tile_sums[blockIdx.x];
+  __shared__ int64_t total;
+  int64_t before = 0;
+  for (int64_t i = threadIdx.x; i < blockIdx.x; i += kScanThreads) {
+    before += tile_sums[i];
+  }
+  block_exclusive_scan(before, &total);
+  const int64_t add = total;
   const int64_t base = (int64_t)blockIdx.x * kTile + (int64_t)threadIdx.x * kItemsPerThread;
 #pragma unroll
   for (int i = 0; i < kItemsPerThread; ++i) {
     if (base + i < n) {
       offsets[base + i] += add;
     }
+  }
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
+    offsets[n] = add + tile_sums[blockIdx.x];
   }
 }
 
@@ -139,10 +160,14 @@ cudaError_t launch_length_scan(
   if (tiles <= 0 || tiles > 0x7fffffffLL) {
     return cudaErrorInvalidValue;
   }
+  if (tiles <= kOneBlockTiles) {
+    scan_one_block<<<1, kScanThreads, 0, stream>>>(lengths, length_bytes == 8, n, offsets);
+    g_launch_count.fetch_add(1, std::memory_order_relaxed);
+    return cudaGetLastError();
+  }
   scan_tiles<<<(unsigned)tiles, kScanThreads, 0, stream>>>(lengths, length_bytes == 8, n, offsets, tile_sums);
-  scan_tile_sums<<<1, kScanThreads, 0, stream>>>(tile_sums, tiles, offsets, n);
   add_tile_prefix<<<(unsigned)tiles, kScanThreads, 0, stream>>>(offsets, tile_sums, n);
-  g_launch_count.fetch_add(3, std::memory_order_relaxed);
+  g_launch_count.fetch_add(2, std::memory_order_relaxed);
   return cudaGetLastError();
 }
 
