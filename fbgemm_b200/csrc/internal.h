@@ -222,6 +222,7 @@ cudaError_t launch_sequence_lookup(
     bool scale_bias_last,
     int fp8_exponent_bits,
     int fp8_exponent_bias,
+    bool fill,
     int32_t* status,
     cudaStream_t stream);
 

@@ -25,6 +25,13 @@
 // are most of the traffic, 4 or 2 bytes per column against 1/4 to 4 read - are
 // coalesced and wide; widths that are no multiple of 4 and unaligned rows go
 // column by column.
+//
+// Bound by memory: rows read once, output rows written once.  Where the 32
+// positions of a warp name rows of one type (all but the warps at a table's
+// border), it walks them several at a time (walk_rows): rows narrower than 128
+// columns side by side, kInFlight loads issued before the first store.  One row
+// at a time 4.2 M rows of 128 int8 columns to fp16 took 519 us, most of it
+// waiting.
 #include <cuda_fp16.h>
 
 #include "internal.h"
@@ -58,6 +65,7 @@ struct SeqArgs {
   int32_t sb_last;
   int32_t fp8_exponent_bits;
   int32_t fp8_exponent_bias;
+  int32_t fill;      // rows that get nothing else are set to zero
   int32_t by_fours;  // D % 4 == 0 and output rows aligned for 8- / 16-byte stores
 };
 
@@ -109,56 +117,112 @@ __device__ __forceinline__ void store_column(uint8_t* orow, int j, float v) {
   }
 }
 
+// Four consecutive columns of one row: the 1-16 bytes that hold them, and their values.
+template <int TYPE>
+struct Four {
+  static constexpr int kWords = TYPE == kFP32 ? 4 : (TYPE == kFP16 ? 2 : 1);
+  uint32_t w[kWords];
+  __device__ __forceinline__ void load(const uint8_t* data, int u) {
+    if constexpr (TYPE == kFP32) {
+      const uint4 v = __ldg(reinterpret_cast<const uint4*>(data) + u);
+      w[0] = v.x;
+      w[1] = v.y;
+      w[2] = v.z;
+      w[3] = v.w;
+    } else if constexpr (TYPE == kFP16) {
+      const uint2 v = __ldg(reinterpret_cast<const uint2*>(data) + u);
+      w[0] = v.x;
+      w[1] = v.y;
+    } else if constexpr (TYPE == kINT4) {
+      w[0] = __ldg(reinterpret_cast<const unsigned short*>(data) + u);
+    } else if constexpr (TYPE == kINT2) {
+      w[0] = __ldg(data + u);
+    } else {
+      w[0] = __ldg(reinterpret_cast<const uint32_t*>(data) + u);
+    }
+  }
+  __device__ __forceinline__ float value(int c, float scale, float start, float fp8_mult, int fp8_shift) const {
+    if constexpr (TYPE == kFP32) {
+      return from_x(__uint_as_float(w[c]));
+    } else if constexpr (TYPE == kFP16) {
+      return from_x(__half2float(__ushort_as_half((unsigned short)(w[c >> 1] >> (16 * (c & 1))))));
+    } else if constexpr (TYPE == kFP8) {
+      return from_fp8((w[0] >> (8 * c)) & 0xffu, fp8_mult, fp8_shift);
+    } else {
+      constexpr int bits = TYPE == kINT8 ? 8 : (TYPE == kINT4 ? 4 : 2);
+      return from_q((w[0] >> (bits * c)) & ((1u << bits) - 1u), scale, start);
+    }
+  }
+};
+
+template <int OUT>
+__device__ __forceinline__ void store_four(uint8_t* orow, int u, const float (&v)[4]) {
+  if constexpr (OUT == kToF32) {
+    __stcs(reinterpret_cast<float4*>(orow) + u, make_float4(v[0], v[1], v[2], v[3]));
+  } else {
+    constexpr bool bf = OUT == kToBf16;
+    __stcs(reinterpret_cast<uint2*>(orow) + u,
+           make_uint2((uint32_t)to_16bit(v[0], bf) | ((uint32_t)to_16bit(v[1], bf) << 16),
+                      (uint32_t)to_16bit(v[2], bf) | ((uint32_t)to_16bit(v[3], bf) << 16)));
+  }
+}
+
 // Four consecutive columns per lane and step: one load of the 1-16 bytes that hold them, one store of
 // 8 or 16 bytes.  The caller has checked that D is a multiple of 4 and that loads and stores are aligned.
 template <int TYPE, int OUT>
 __device__ __forceinline__ void emit_row_by_fours(const uint8_t* data, uint8_t* orow, int D, float scale, float start,
                                                   float fp8_mult, int fp8_shift, int lane) {
   for (int u = lane; u < (D >> 2); u += 32) {
+    Four<TYPE> d;
+    d.load(data, u);
     float v[4];
-    if constexpr (TYPE == kINT8) {
-      const uint32_t w = __ldg(reinterpret_cast<const uint32_t*>(data) + u);
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        v[c] = from_q((w >> (8 * c)) & 0xffu, scale, start);
-      }
-    } else if constexpr (TYPE == kINT4) {
-      const uint32_t w = __ldg(reinterpret_cast<const unsigned short*>(data) + u);
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        v[c] = from_q((w >> (4 * c)) & 0xfu, scale, start);
-      }
-    } else if constexpr (TYPE == kINT2) {
-      const uint32_t w = __ldg(data + u);
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        v[c] = from_q((w >> (2 * c)) & 0x3u, scale, start);
-      }
-    } else if constexpr (TYPE == kFP32) {
-      const uint4 w = __ldg(reinterpret_cast<const uint4*>(data) + u);
-      v[0] = from_x(__uint_as_float(w.x));
-      v[1] = from_x(__uint_as_float(w.y));
-      v[2] = from_x(__uint_as_float(w.z));
-      v[3] = from_x(__uint_as_float(w.w));
-    } else if constexpr (TYPE == kFP16) {
-      const uint2 w = __ldg(reinterpret_cast<const uint2*>(data) + u);
-      v[0] = from_x(__half2float(__ushort_as_half((unsigned short)(w.x & 0xffffu))));
-      v[1] = from_x(__half2float(__ushort_as_half((unsigned short)(w.x >> 16))));
-      v[2] = from_x(__half2float(__ushort_as_half((unsigned short)(w.y & 0xffffu))));
-      v[3] = from_x(__half2float(__ushort_as_half((unsigned short)(w.y >> 16))));
-    } else {
-      const uint32_t w = __ldg(reinterpret_cast<const uint32_t*>(data) + u);
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        v[c] = from_fp8((w >> (8 * c)) & 0xffu, fp8_mult, fp8_shift);
-      }
+    for (int c = 0; c < 4; ++c) {
+      v[c] = d.value(c, scale, start, fp8_mult, fp8_shift);
     }
-    if constexpr (OUT == kToF32) {
-      reinterpret_cast<float4*>(orow)[u] = make_float4(v[0], v[1], v[2], v[3]);
-    } else {
-      constexpr bool bf = OUT == kToBf16;
-      reinterpret_cast<uint2*>(orow)[u] = make_uint2((uint32_t)to_16bit(v[0], bf) | ((uint32_t)to_16bit(v[1], bf) << 16),
-                                                     (uint32_t)to_16bit(v[2], bf) | ((uint32_t)to_16bit(v[3], bf) << 16));
+    store_four<OUT>(orow, u, v);
+  }
+}
+
+// All rows of the warp's 32 positions, which are of type TYPE (or pruned: `pruned` has their bits) and take the
+// four-column path: 1 << log_side rows side by side, kInFlight of those at a time.
+template <int TYPE, int OUT>
+__device__ __forceinline__ void walk_rows(const SeqArgs& a, const uint8_t* my_data, float my_scale, float my_start,
+                                          unsigned pruned, uint8_t* out_rows, int lane, float fp8_mult, int fp8_shift) {
+  constexpr int kInFlight = TYPE == kFP32 ? 4 : 8;
+  const int units = a.D >> 2;
+  const int log_side = units <= 8 ? 2 : (units <= 16 ? 1 : 0);
+  const int lanes = 32 >> log_side;              // per row
+  const int side = lane / lanes, ul = lane - side * lanes;
+  for (int u0 = 0; u0 < units; u0 += lanes) {    // one round for up to 128 columns
+    const int u = u0 + ul;
+    const bool in_row = u < units;
+#pragma unroll 1
+    for (int i0 = 0; i0 < 32 >> log_side; i0 += kInFlight) {
+      Four<TYPE> d[kInFlight];
+#pragma unroll
+      for (int j = 0; j < kInFlight; ++j) {
+        const int i = ((i0 + j) << log_side) + side;
+        const uint8_t* data = reinterpret_cast<const uint8_t*>(
+            __shfl_sync(0xffffffffu, (unsigned long long)reinterpret_cast<uintptr_t>(my_data), i));
+        if (in_row) {
+          d[j].load(data, u);
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < kInFlight; ++j) {
+        const int i = ((i0 + j) << log_side) + side;
+        const float scale = __shfl_sync(0xffffffffu, my_scale, i);
+        const float start = __shfl_sync(0xffffffffu, my_start, i);
+        if (in_row) {
+          float v[4];
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            v[c] = (pruned >> i) & 1u ? 0.f : d[j].value(c, scale, start, fp8_mult, fp8_shift);
+          }
+          store_four<OUT>(out_rows + i * a.out_row_bytes, u, v);
+        }
+      }
     }
   }
 }
@@ -265,6 +329,32 @@ __global__ void __launch_bounds__(kThreads) sequence_rows_kernel(const SeqArgs a
     }
   }
 
+  if constexpr (!copy) {
+    // One row type in all 32 positions: walked several rows at a time.
+    const unsigned rows = __ballot_sync(0xffffffffu, my_state == kRow);
+    const unsigned zeros = __ballot_sync(0xffffffffu, my_state == kZeros);
+    if (rows != 0 && (rows | zeros) == 0xffffffffu) {
+      const int leader = __ffs(rows) - 1;
+      const int type = __shfl_sync(0xffffffffu, my_type, leader);
+      const uint8_t* any = reinterpret_cast<const uint8_t*>(
+          __shfl_sync(0xffffffffu, (unsigned long long)reinterpret_cast<uintptr_t>(my_row), leader));
+      if (__all_sync(0xffffffffu, my_state == kZeros || (my_type == type && my_fours))) {
+        const bool quantized = type == kINT8 || type == kINT4 || type == kINT2;
+        const uint8_t* my_data = (my_state == kZeros ? any : my_row) + (quantized && !a.sb_last ? 4 : 0);
+        uint8_t* out_rows = a.out + first * a.out_row_bytes;
+        switch (type) {
+          case kINT8: walk_rows<kINT8, OUT>(a, my_data, my_scale, my_start, zeros, out_rows, lane, fp8_mult, fp8_shift); break;
+          case kINT4: walk_rows<kINT4, OUT>(a, my_data, my_scale, my_start, zeros, out_rows, lane, fp8_mult, fp8_shift); break;
+          case kINT2: walk_rows<kINT2, OUT>(a, my_data, my_scale, my_start, zeros, out_rows, lane, fp8_mult, fp8_shift); break;
+          case kFP32: walk_rows<kFP32, OUT>(a, my_data, my_scale, my_start, zeros, out_rows, lane, fp8_mult, fp8_shift); break;
+          case kFP16: walk_rows<kFP16, OUT>(a, my_data, my_scale, my_start, zeros, out_rows, lane, fp8_mult, fp8_shift); break;
+          default: walk_rows<kFP8, OUT>(a, my_data, my_scale, my_start, zeros, out_rows, lane, fp8_mult, fp8_shift); break;
+        }
+        return;
+      }
+    }
+  }
+
   // what the warp needs to know first about a position, in one word: state | type << 2 | four-column path << 5
   const int my_code = my_state | (my_type << 2) | ((int)my_fours << 5);
   const int count = (int)(a.index_size - first < 32 ? a.index_size - first : 32);
@@ -272,13 +362,10 @@ __global__ void __launch_bounds__(kThreads) sequence_rows_kernel(const SeqArgs a
   for (int i = 0; i < count; ++i, orow += a.out_row_bytes) {
     const int code = __shfl_sync(0xffffffffu, my_code, i);
     const int state = code & 3;
-    if (state == kSkip) {
-      continue;
-    }
-    if (state == kZeros) {
-      if constexpr (!copy) {
-        for (int j = lane; j < a.D; j += 32) {
-          store_column<OUT>(orow, j, 0.f);
+    if (state == kSkip || state == kZeros) {
+      if (state == kZeros || a.fill) {
+        for (int64_t b = lane; b < a.out_row_bytes; b += 32) {
+          orow[b] = 0;
         }
       }
       continue;
@@ -302,6 +389,9 @@ __global__ void __launch_bounds__(kThreads) sequence_rows_kernel(const SeqArgs a
         for (int64_t b = lane; b < width; b += 32) {
           orow[b] = __ldg(row + b);
         }
+      }
+      for (int64_t b = width + lane; a.fill && b < a.out_row_bytes; b += 32) {
+        orow[b] = 0;
       }
     } else {
       const bool quantized = type == kINT8 || type == kINT4 || type == kINT2;
@@ -343,6 +433,7 @@ cudaError_t launch_sequence_lookup(
     int out_kind,
     int64_t out_row_bytes,
     bool scale_bias_last,
+    bool fill,
     int fp8_exponent_bits,
     int fp8_exponent_bias,
     int32_t* status,
@@ -365,6 +456,7 @@ cudaError_t launch_sequence_lookup(
   a.out_kind = out_kind;
   a.index64 = index_bytes == 8;
   a.sb_last = scale_bias_last;
+  a.fill = fill;
   a.fp8_exponent_bits = fp8_exponent_bits;
   a.fp8_exponent_bias = fp8_exponent_bias;
   const int64_t per_block = (int64_t)kWarps * kPerWarp;

@@ -350,12 +350,15 @@ class IntNBitSequenceEmbedding:
         B = (offsets.numel() - 1) // self.T
         n = indices.numel()
         if output is None:
-            output = torch.zeros((n, self.out_cols), dtype=self.out_dtype, device=self.device)
+            output = torch.empty((n, self.out_cols), dtype=self.out_dtype, device=self.device)
+            lookup = E._capi.lib().fbgemm_b200_sequence_lookup_filled
+            if B == 0:
+                output.zero_()
         assert output.is_contiguous() and output.dtype == self.out_dtype and output.numel() == n * self.out_cols
         if B == 0 or n == 0:
             return output
         ctx = E.get_context(self.device.index)
-        rc = E._capi.lib().fbgemm_b200_sequence_lookup(
+        rc = lookup(
             ctx.handle, self.dev_weights.data_ptr(), self._desc.data_ptr(), self.T, B, self.D, indices.data_ptr(),
             offsets.data_ptr(), indices.element_size(), n, output.data_ptr(), self.out_code, self.out_row_bytes,
             int(self.scale_bias_last), self.fp8[0], self.fp8[1], slot,
@@ -371,6 +374,7 @@ def int_nbit_split_embedding_nobag_codegen_forward_unweighted(
     """One call with the reference operator's arguments (placement and UVM
     arguments left out; ``pooling_mode`` is accepted and, bags being one row
     long, changes nothing)."""
+        lookup = E._capi.lib().fbgemm_b200_sequence_lookup
     op = IntNBitSequenceEmbedding(dev_weights, weights_offsets, weights_tys, D, row_alignment, output_dtype,
                                   scale_bias_last, fp8_exponent_bits, fp8_exponent_bias)
     return op.forward(indices, offsets)

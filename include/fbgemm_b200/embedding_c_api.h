@@ -564,6 +564,28 @@ FBGEMM_B200_API const void* fbgemm_b200_table_device_ptr(fbgemm_b200_ctx* ctx, c
  * (FBGEMM_B200_EBUSY if the lane has un-waited work). */
 FBGEMM_B200_API int fbgemm_b200_spmdm_host_submit(
     fbgemm_b200_ctx* ctx,
+/* The same for an output buffer that holds nothing yet: rows of positions that
+ * no table covers, or whose index is out of range, and bytes behind a copied
+ * row are set to zero, so that the buffer need not be cleared first. */
+FBGEMM_B200_API int fbgemm_b200_sequence_lookup_filled(
+    fbgemm_b200_ctx* ctx,
+    const void* dev_weights,
+    const fbgemm_b200_sequence_table* tables,
+    int32_t T,
+    int32_t B,
+    int32_t D,
+    const void* indices,
+    const void* offsets,
+    int32_t index_bytes,
+    int64_t index_size,
+    void* out,
+    int32_t out_dtype,
+    int64_t out_row_bytes,
+    int32_t scale_bias_last,
+    int32_t fp8_exponent_bits,
+    int32_t fp8_exponent_bias,
+    int32_t slot,
+    void* stream);
     int lane,
     const fbgemm_b200_spmdm_config* cfg,
     int64_t output_size,
