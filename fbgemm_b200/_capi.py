@@ -104,6 +104,9 @@ SIGNATURES = {
     "fbgemm_b200_multi_plan_launch": (C.c_int, [_p, _p]),
     "fbgemm_b200_multi_plan_num_launches": (C.c_int, [_p]),
     "fbgemm_b200_multi_plan_destroy": (None, [_p]),
+    "fbgemm_b200_table_set_create": (C.c_int, [_p, C.POINTER(TableCall), C.POINTER(_i64), C.c_int32, C.POINTER(_p)]),
+    "fbgemm_b200_table_set_forward": (C.c_int, [_p, _i64, _p, _i64, _p, _p, _p, C.c_int, _p]),
+    "fbgemm_b200_table_set_destroy": (None, [_p]),
     "fbgemm_b200_status_read": (C.c_int, [_p, C.c_int, _p, C.POINTER(C.c_int32)]),
     "fbgemm_b200_spmdm": (C.c_int, [_p, _cfgp, _i64, _i64, _i64, _p, _p, _p, _p, _p, _p, _p]),
     "fbgemm_b200_spmdm_lengths_noalloc": (C.c_int, [_cfgp, _i64, _i64, _i64, _p, _p, _p, _p, _p, _p, _p]),
@@ -115,11 +118,11 @@ SIGNATURES = {
                                                   _p, _p, C.c_int32, _p]),
     "fbgemm_b200_sequence_lookup": (C.c_int, [_p, _p, _p, C.c_int32, C.c_int32, C.c_int32, _p, _p, C.c_int32, _i64, _p,
                                               C.c_int32, _i64, C.c_int32, C.c_int32, C.c_int32, C.c_int32, _p]),
+    "fbgemm_b200_sequence_lookup_filled": (C.c_int, [_p, _p, _p, C.c_int32, C.c_int32, C.c_int32, _p, _p, C.c_int32, _i64, _p,
+                                              C.c_int32, _i64, C.c_int32, C.c_int32, C.c_int32, C.c_int32, _p]),
     "fbgemm_b200_pruned_hashmap_insert": (C.c_int, [_p, C.c_int32, C.c_int32, _p, _p, _p, C.c_int32, _i64, _p, C.c_int32,
                                                     _p, C.c_int32, _p]),
     "fbgemm_b200_pruned_hashmap_insert_host": (C.c_int, [C.c_int32, C.c_int32, _p, _p, _p, C.c_int32, _p, C.c_int32,
-    "fbgemm_b200_sequence_lookup_filled": (C.c_int, [_p, _p, _p, C.c_int32, C.c_int32, C.c_int32, _p, _p, C.c_int32, _i64, _p,
-                                              C.c_int32, _i64, C.c_int32, C.c_int32, C.c_int32, C.c_int32, _p]),
                                                          _p]),
     "fbgemm_b200_table_register": (C.c_int, [_p, _p, C.c_size_t]),
     "fbgemm_b200_table_unregister": (C.c_int, [_p, _p]),
@@ -147,6 +150,19 @@ SIGNATURES = {
 }
 
 _lib = None
+_native = None
+
+
+def native():
+    """The CPython extension with the calls a serving loop makes (native_calls.c): the same entry points of the library,
+    without ctypes' argument conversion."""
+    global _native
+    if _native is None:
+        lib()
+        from . import _native_calls
+
+        _native = _native_calls
+    return _native
 
 
 def lib() -> C.CDLL:

@@ -14,6 +14,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(PKG_DIR)
@@ -26,7 +27,9 @@ CUDA_SOURCES = ["bag_units_narrow.cu", "bag_units_wide.cu", "bag_kernel_8.cu", "
                 "bag_kernel_plain.cu", "bag_dispatch.cu", "spmdm_kernels.cu", "rows_copy_kernels.cu", "scan_kernels.cu",
                 "quantize_kernels.cu", "remap_kernels.cu", "pruned_lookup_kernels.cu", "sequence_kernels.cu", "stage_kernels.cu",
                 "c_api.cu", "noalloc_entry.cu", "peer_sync_kernels.cu", "multi_host.cu"]
-CXX_SOURCES = ["generators.cc"]
+CXX_SOURCES = ["generators.cc", "host_copy.cc"]
+NATIVE_SOURCE = "native_calls.c"  # the CPython extension, linked against the library beside it
+NATIVE_PATH = os.path.join(PKG_DIR, "_native_calls.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -52,7 +55,7 @@ def _sources():
 
 def _fingerprint() -> str:
     h = hashlib.sha256()
-    paths = _sources()
+    paths = _sources() + [os.path.join(CSRC, NATIVE_SOURCE)]
     for d in (CSRC, os.path.join(INCLUDE, "fbgemm_b200")):
         for name in sorted(os.listdir(d)):
             if name.endswith((".h", ".cuh")):
@@ -66,7 +69,7 @@ def _fingerprint() -> str:
 
 
 def needs_build() -> bool:
-    if not os.path.exists(LIB_PATH) or not os.path.exists(STAMP_PATH):
+    if not all(os.path.exists(p) for p in (LIB_PATH, NATIVE_PATH, STAMP_PATH)):
         return True
     with open(STAMP_PATH) as f:
         return f.read().strip() != _fingerprint()
@@ -106,6 +109,9 @@ def build(force: bool = False, verbose: bool = False) -> str:
     link = [nvcc, "-shared", "-o", LIB_PATH, *objs, "-gencode", "arch=compute_100a,code=sm_100a",
             "-Xcompiler", "-fPIC"]
     subprocess.run(link, check=True)
+    subprocess.run([shutil.which("gcc") or "cc", "-O2", "-Wall", "-shared", "-fPIC", "-I", INCLUDE,
+                    "-I", sysconfig.get_paths()["include"], os.path.join(CSRC, NATIVE_SOURCE), "-o", NATIVE_PATH,
+                    "-L", PKG_DIR, "-l:" + os.path.basename(LIB_PATH), "-Wl,-rpath,$ORIGIN"], check=True)
     with open(STAMP_PATH, "w") as f:
         f.write(_fingerprint())
     return LIB_PATH

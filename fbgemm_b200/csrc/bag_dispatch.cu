@@ -235,4 +235,19 @@ cudaError_t launch_multi_plan(const MultiPlan& plan, cudaStream_t stream) {
   return cudaSuccess;
 }
 
+cudaError_t launch_tables(const SpmdmParams* tables, const int* bit_rates, size_t count, cudaStream_t stream) {
+  if (g_kernel_choice.load(std::memory_order_relaxed) == FBGEMM_B200_KERNEL_GENERIC) {
+    for (size_t t = 0; t < count; ++t) {
+      const cudaError_t e = tables[t].output_size > 0 ? launch_spmdm(tables[t], bit_rates[t], stream) : cudaSuccess;
+      if (e != cudaSuccess) {
+        return e;
+      }
+    }
+    return cudaSuccess;
+  }
+  MultiPlan plan;
+  const cudaError_t e = build_multi_plan(tables, bit_rates, count, &plan);
+  return e == cudaSuccess ? launch_multi_plan(plan, stream) : e;
+}
+
 }  // namespace fbgemm_b200

@@ -728,6 +728,14 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm) bag_units_kernel(const
 }
 
 using BagFn = void (*)(const BagCall);
+template <int FMT, int VB, int CPL, int G, bool WIDE>
+BagFn deep_kernel() {
+  if constexpr (G == 32) {
+    return bag_kernel_deep<FMT, VB, CPL, G, WIDE>;
+  } else {
+    return nullptr;
+  }
+}
 using BagUnitsFn = void (*)(const BagUnits);
 
 }  // namespace bag

@@ -8,10 +8,8 @@ void bag_kernels_2(bag::BagFn (*fn)[4]) {
 #define ENTRY(FMT, VB, CPL, G)                                                         \
   fn[id_##FMT##_##VB##_##CPL##_##G][0] = bag_kernel<FMT, VB, CPL, G, false>;          \
   fn[id_##FMT##_##VB##_##CPL##_##G][1] = bag_kernel<FMT, VB, CPL, G, true>;           \
-  if constexpr (G == 32) {                                                            \
-    fn[id_##FMT##_##VB##_##CPL##_##G][2] = bag_kernel_deep<FMT, VB, CPL, G, false>;   \
-    fn[id_##FMT##_##VB##_##CPL##_##G][3] = bag_kernel_deep<FMT, VB, CPL, G, true>;    \
-  }
+  fn[id_##FMT##_##VB##_##CPL##_##G][2] = deep_kernel<FMT, VB, CPL, G, false>();       \
+  fn[id_##FMT##_##VB##_##CPL##_##G][3] = deep_kernel<FMT, VB, CPL, G, true>();
   FBGEMM_B200_BAG_VARIANTS_2(ENTRY)
 #undef ENTRY
 }

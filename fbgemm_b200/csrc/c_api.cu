@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "context.h"
+#include "host_copy.h"
 
 namespace fbgemm_b200 {
 
@@ -359,6 +360,43 @@ int fbgemm_b200::enqueue_lookup(
 
 namespace {
 
+// The code of an error record in page-locked host memory, which is cleared.
+// The kernels that may write to it have completed.
+int32_t take_record(int32_t* record) {
+  const int32_t code = *static_cast<volatile int32_t*>(record);
+  if (code != 0) {
+    std::memset(record, 0, 4 * sizeof(int32_t));
+  }
+  return code;
+}
+
+// One functor call on device pointers, at least one bag.
+int enqueue_on_stream(
+    fbgemm_b200_ctx* ctx,
+    const fbgemm_b200_spmdm_config* cfg,
+    int64_t output_size,
+    int64_t index_size,
+    int64_t data_size,
+    const void* input,
+    const void* indices,
+    const void* offsets_or_lengths,
+    const float* weights,
+    void* out,
+    const int32_t* cit,
+    int32_t* status,
+    cudaStream_t stream) {
+  if (cfg && !cfg->use_offsets && !cfg->no_bag) {
+    // Lengths mode: the scanned offsets live in scratch that belongs to the
+    // stream, so that launches on different streams never share it.
+    std::lock_guard<std::mutex> lock(ctx->mu);
+    return enqueue_lookup(cfg, output_size, index_size, data_size, input, indices, offsets_or_lengths, weights, out, cit,
+                          status, scan_scratch_of(ctx, stream), stream);
+  }
+  DeviceBuffer unused;  // only lengths mode touches the scratch
+  return enqueue_lookup(cfg, output_size, index_size, data_size, input, indices, offsets_or_lengths, weights, out, cit,
+                        status, unused, stream);
+}
+
 int pruned_lookup(
     bool hashmap,
     fbgemm_b200_ctx* ctx,
@@ -396,44 +434,6 @@ int pruned_lookup(
   return 0;
 }
 
-template <typename Index, typename Hash>
-bool hashmap_insert(
-    int32_t T,
-    int32_t B,
-    const Index* indices,
-    const Index* dense,
-    const Index* offsets,
-    Hash* table,
-    const int64_t* table_offsets) {
-  using Unsigned = typename std::make_unsigned<Index>::type;
-  bool ok = true;
-  for (int32_t t = 0; t < T; ++t) {
-    const int64_t first = table_offsets[t];
-    const uint64_t capacity = (uint64_t)(table_offsets[t + 1] - first);
-    if (capacity == 0) {
-      continue;
-    }
-    Hash* slots = table + 2 * first;
-    for (int64_t k = offsets[(int64_t)t * B]; k < (int64_t)offsets[(int64_t)(t + 1) * B]; ++k) {
-      if (dense[k] == -1) {
-        continue;
-      }
-      const Unsigned key = (Unsigned)indices[k];
-      uint64_t h;
-      if (sizeof(Index) == 8) {
-        uint64_t x = (uint64_t)key;
-        x ^= x >> 33;
-        x *= 0xff51afd7ed558ccdULL;
-        x ^= x >> 33;
-        x *= 0xc4ceb9fe1a85ec53ULL;
-        x ^= x >> 33;
-        h = x;
-      } else {
-        uint32_t x = (uint32_t)key;
-        x ^= x >> 16;
-        x *= 0x85ebca6bu;
-        x ^= x >> 13;
-        x *= 0xc2b2ae35u;
 int sequence_lookup(
     bool fill,
     fbgemm_b200_ctx* ctx,
@@ -486,6 +486,44 @@ int sequence_lookup(
   return 0;
 }
 
+template <typename Index, typename Hash>
+bool hashmap_insert(
+    int32_t T,
+    int32_t B,
+    const Index* indices,
+    const Index* dense,
+    const Index* offsets,
+    Hash* table,
+    const int64_t* table_offsets) {
+  using Unsigned = typename std::make_unsigned<Index>::type;
+  bool ok = true;
+  for (int32_t t = 0; t < T; ++t) {
+    const int64_t first = table_offsets[t];
+    const uint64_t capacity = (uint64_t)(table_offsets[t + 1] - first);
+    if (capacity == 0) {
+      continue;
+    }
+    Hash* slots = table + 2 * first;
+    for (int64_t k = offsets[(int64_t)t * B]; k < (int64_t)offsets[(int64_t)(t + 1) * B]; ++k) {
+      if (dense[k] == -1) {
+        continue;
+      }
+      const Unsigned key = (Unsigned)indices[k];
+      uint64_t h;
+      if (sizeof(Index) == 8) {
+        uint64_t x = (uint64_t)key;
+        x ^= x >> 33;
+        x *= 0xff51afd7ed558ccdULL;
+        x ^= x >> 33;
+        x *= 0xc4ceb9fe1a85ec53ULL;
+        x ^= x >> 33;
+        h = x;
+      } else {
+        uint32_t x = (uint32_t)key;
+        x ^= x >> 16;
+        x *= 0x85ebca6bu;
+        x ^= x >> 13;
+        x *= 0xc2b2ae35u;
         x ^= x >> 16;
         h = x;
       }
@@ -549,6 +587,12 @@ int fbgemm_b200_ctx_create(int device, fbgemm_b200_ctx** out) {
   if (e == cudaSuccess) {
     e = cudaMallocHost(&ctx->status_host, sbytes);
   }
+  if (e == cudaSuccess) {
+    e = cudaMallocHost(&ctx->sync_status, 4 * sizeof(int32_t));
+  }
+  if (e == cudaSuccess) {
+    std::memset(ctx->sync_status, 0, 4 * sizeof(int32_t));
+  }
   if (e != cudaSuccess) {
     fbgemm_b200_ctx_destroy(ctx);
     return fail_cuda(e, "status slots");
@@ -573,6 +617,11 @@ void fbgemm_b200_ctx_destroy(fbgemm_b200_ctx* ctx) {
     cudaFreeHost(l.h_in.ptr);
     cudaFreeHost(l.h_out.ptr);
     cudaFreeHost(l.h_status.ptr);
+    for (cudaEvent_t ev : l.piece_done) {
+      if (ev) {
+        cudaEventDestroy(ev);
+      }
+    }
   }
   for (auto& kv : ctx->tables) {
     cudaFree(kv.second.buf.ptr);
@@ -583,6 +632,7 @@ void fbgemm_b200_ctx_destroy(fbgemm_b200_ctx* ctx) {
   cudaFree(ctx->remap_scratch.ptr);
   cudaFree(ctx->status);
   cudaFreeHost(ctx->status_host);
+  cudaFreeHost(ctx->sync_status);
   delete ctx;
 }
 
@@ -641,17 +691,8 @@ int fbgemm_b200_spmdm_launch(
     }
     return 0;
   }
-  if (cfg && !cfg->use_offsets && !cfg->no_bag) {
-    // Lengths mode: the scanned offsets live in scratch that belongs to the
-    // stream, so that launches on different streams never share it.
-    std::lock_guard<std::mutex> lock(ctx->mu);
-    return enqueue_lookup(cfg, output_size, index_size, data_size, input, indices, offsets_or_lengths, weights, out,
-                          compressed_indices_table, ctx->status + 4 * slot,
-                          scan_scratch_of(ctx, static_cast<cudaStream_t>(stream)), static_cast<cudaStream_t>(stream));
-  }
-  DeviceBuffer unused;  // only lengths mode touches the scratch
-  return enqueue_lookup(cfg, output_size, index_size, data_size, input, indices, offsets_or_lengths, weights, out,
-                        compressed_indices_table, ctx->status + 4 * slot, unused, static_cast<cudaStream_t>(stream));
+  return enqueue_on_stream(ctx, cfg, output_size, index_size, data_size, input, indices, offsets_or_lengths, weights, out,
+                           compressed_indices_table, ctx->status + 4 * slot, static_cast<cudaStream_t>(stream));
 }
 
 int fbgemm_b200_spmdm_launch_sharded(
@@ -769,6 +810,90 @@ void fbgemm_b200_multi_plan_destroy(fbgemm_b200_multi_plan* plan) {
   }
 }
 
+int fbgemm_b200_table_set_create(
+    fbgemm_b200_ctx* ctx,
+    const fbgemm_b200_table_call* tables,
+    const int64_t* out_columns,
+    int32_t num_tables,
+    fbgemm_b200_table_set** out) {
+  if (out) {
+    *out = nullptr;
+  }
+  if (!ctx || !tables || !out_columns || num_tables <= 0 || !out) {
+    set_error("table_set_create: bad argument");
+    return FBGEMM_B200_EINVAL;
+  }
+  auto* set = new (std::nothrow) fbgemm_b200_table_set;
+  if (!set) {
+    set_error("out of host memory");
+    return FBGEMM_B200_ENOMEM;
+  }
+  set->ctx = ctx;
+  for (int t = 0; t < num_tables; ++t) {
+    const fbgemm_b200_table_call& c = tables[t];
+    int rc = fbgemm_b200_spmdm_check_config(&c.cfg);
+    const auto& first = tables[0].cfg;
+    if (rc == 0 && (!c.cfg.absolute_offsets || !c.input || c.data_size < 0 || out_columns[t] < 0 ||
+                    c.cfg.index_bytes != first.index_bytes || c.cfg.offset_bytes != first.offset_bytes ||
+                    c.cfg.has_weight != first.has_weight || c.cfg.out_dtype != first.out_dtype)) {
+      set_error("table_set_create: tables take absolute offsets and share index, offset and output types");
+      rc = FBGEMM_B200_EINVAL;
+    }
+    if (rc) {
+      delete set;
+      return rc;
+    }
+    set->tables.push_back(c);
+    set->out_columns.push_back(out_columns[t]);
+  }
+  *out = set;
+  return 0;
+}
+
+int fbgemm_b200_table_set_forward(
+    fbgemm_b200_table_set* set,
+    int64_t bags,
+    const void* indices,
+    int64_t index_size,
+    const void* offsets,
+    const float* weights,
+    void* out,
+    int slot,
+    void* stream) {
+  if (!set || slot < 0 || slot >= FBGEMM_B200_USER_SLOTS || bags < 0 || !offsets || !out) {
+    set_error("table_set_forward: bad argument");
+    return FBGEMM_B200_EINVAL;
+  }
+  if (bags == 0) {
+    return 0;
+  }
+  const size_t T = set->tables.size();
+  std::vector<SpmdmParams> params(T);
+  std::vector<int> bit_rates(T);
+  const auto& first = set->tables[0].cfg;
+  const int64_t esize = first.out_dtype == FBGEMM_B200_OUT_F32 ? 4 : 2;
+  for (size_t t = 0; t < T; ++t) {
+    const fbgemm_b200_table_call& c = set->tables[t];
+    const int rc = build_lookup_params(&c.cfg, bags, index_size, c.data_size, c.input, indices,
+                                       c.cfg.has_weight ? weights : nullptr,
+                                       static_cast<char*>(out) + set->out_columns[t] * esize, nullptr,
+                                       set->ctx->status + 4 * slot, nullptr, 0, 0, &params[t]);
+    if (rc) {
+      return rc;
+    }
+    params[t].offsets = static_cast<const char*>(offsets) + (int64_t)t * bags * first.offset_bytes;
+    params[t].flags |= first.offset_bytes == 8 ? kOff64 : 0;
+    bit_rates[t] = c.cfg.bit_rate;
+  }
+  DeviceGuard guard(set->ctx->device);
+  const cudaError_t e = launch_tables(params.data(), bit_rates.data(), T, static_cast<cudaStream_t>(stream));
+  return e == cudaSuccess ? 0 : fail_cuda(e, "table set launch");
+}
+
+void fbgemm_b200_table_set_destroy(fbgemm_b200_table_set* set) {
+  delete set;
+}
+
 int fbgemm_b200_status_read(fbgemm_b200_ctx* ctx, int slot, void* stream, int32_t* info) {
   if (!ctx || slot < 0 || slot >= FBGEMM_B200_STATUS_SLOTS) {
     set_error("bad context or status slot");
@@ -814,15 +939,26 @@ int fbgemm_b200_spmdm(
     set_error("null context");
     return FBGEMM_B200_EINVAL;
   }
-  // Slot 0 is shared by all synchronous calls of this context.
+  DeviceGuard guard(ctx->device);
+  if (output_size == 0) {
+    const int rc = check_config(cfg, nullptr);
+    return rc ? rc : index_size == 0 ? 1 : 0;  // no bag to pool: the reference returns `0 == index_size`
+  }
+  // One record is shared by all synchronous calls of this context.  It lies in page-locked host memory and the kernels
+  // write to it in place, on errors only: copying a device record back took 3.2 us on the device and a second wait.
   static std::mutex sync_mu;
   std::lock_guard<std::mutex> lock(sync_mu);
-  int rc = fbgemm_b200_spmdm_launch(ctx, cfg, output_size, index_size, data_size, input, indices,
-                                    offsets_or_lengths, weights, out, compressed_indices_table, 0, stream);
+  const int rc = enqueue_on_stream(ctx, cfg, output_size, index_size, data_size, input, indices, offsets_or_lengths,
+                                   weights, out, compressed_indices_table, ctx->sync_status,
+                                   static_cast<cudaStream_t>(stream));
   if (rc) {
     return rc;
   }
-  return fbgemm_b200_status_read(ctx, 0, stream, nullptr);
+  const cudaError_t e = cudaStreamSynchronize(static_cast<cudaStream_t>(stream));
+  if (e != cudaSuccess) {
+    return fail_cuda(e, "lookup");
+  }
+  return take_record(ctx->sync_status) == 0 ? 1 : 0;
 }
 
 int fbgemm_b200_compressed_indices_remap(
@@ -1183,6 +1319,7 @@ int fbgemm_b200_spmdm_host_submit(
       return fail_cuda(e, "lane status");
     }
   }
+  std::memset(L.h_status.ptr, 0, 16);
   L.trivially_true = L.trivially_false = false;
   L.user_out = out;
   L.out_rows = 0;
@@ -1299,24 +1436,26 @@ int fbgemm_b200_spmdm_host_submit(
       return fail_cuda(e, "lane staging buffers");
     }
     uint8_t* h = static_cast<uint8_t*>(L.h_in.ptr);
-    if (idx_bytes) {
-      std::memcpy(h, indices, idx_bytes);
-    }
-    std::memcpy(h + off_at, offsets_or_lengths, off_bytes);
-    if (n_w) {
-      std::memcpy(h + w_at, weights, n_w * sizeof(float));
-    }
+    std::vector<CopySlice> slices;
+    auto add = [&](uint8_t* dst, const void* src, size_t bytes) {
+      constexpr size_t kSlice = 128 * 1024;
+      for (size_t at = 0; at < bytes; at += kSlice) {
+        slices.push_back({dst + at, static_cast<const uint8_t*>(src) + at, std::min(kSlice, bytes - at)});
+      }
+    };
+    add(h, indices, idx_bytes);
+    add(h + off_at, offsets_or_lengths, off_bytes);
+    add(h + w_at, weights, n_w * sizeof(float));
+    copy_slices(slices.data(), (int)slices.size(), [](int) { return true; });
     e = cudaMemcpyAsync(di, h, in_bytes, cudaMemcpyHostToDevice, L.stream);
   }
   if (e != cudaSuccess) {
     return fail_cuda(e, "input upload");
   }
 
-  // Status of this lane: the last FBGEMM_B200_HOST_LANES slots of the context.
-  const int slot = FBGEMM_B200_STATUS_SLOTS - FBGEMM_B200_HOST_LANES + lane_id;
   rc = enqueue_lookup(cfg, output_size, index_size, data_size, d_table, di, di + off_at,
                       cfg->has_weight ? reinterpret_cast<const float*>(di + w_at) : nullptr, L.d_out.ptr, d_cit,
-                      ctx->status + 4 * slot, L.d_scan, L.stream);
+                      static_cast<int32_t*>(L.h_status.ptr), L.d_scan, L.stream);
   if (rc) {
     return rc;
   }
@@ -1336,23 +1475,33 @@ int fbgemm_b200_spmdm_host_submit(
     L.out_pitch_bytes = out_pitch;
   }
   const size_t row_bytes = (size_t)cfg->block_size * esize;
-  if (row_bytes == out_pitch) {
+  L.pieces = 0;
+  if (row_bytes == out_pitch && !user_pinned) {
+    // In pieces: each is copied on to the caller's buffer while the next ones come down (host_wait).
+    constexpr size_t kPiece = 512 * 1024;
+    const size_t n = std::min<size_t>(Lane::kMaxPieces, (out_bytes + kPiece - 1) / kPiece);
+    L.piece_bytes = ((out_bytes + n - 1) / n + 255) / 256 * 256;
+    e = cudaSuccess;
+    for (size_t at = 0; at < out_bytes && e == cudaSuccess; at += L.piece_bytes) {
+      cudaEvent_t& done = L.piece_done[L.pieces++];
+      if (!done) {
+        e = cudaEventCreateWithFlags(&done, cudaEventDisableTiming);
+      }
+      if (e == cudaSuccess) {
+        e = cudaMemcpyAsync(static_cast<uint8_t*>(dst) + at, static_cast<uint8_t*>(L.d_out.ptr) + at,
+                            std::min(L.piece_bytes, out_bytes - at), cudaMemcpyDeviceToHost, L.stream);
+      }
+      if (e == cudaSuccess) {
+        e = cudaEventRecord(done, L.stream);
+      }
+    }
+  } else if (row_bytes == out_pitch) {
     e = cudaMemcpyAsync(dst, L.d_out.ptr, out_bytes, cudaMemcpyDeviceToHost, L.stream);
   } else {
     // Only block_size columns of each row are this call's: the caller's rows
     // may hold other tables' columns in between (output_stride).
     e = cudaMemcpy2DAsync(dst, out_pitch, L.d_out.ptr, out_pitch, row_bytes, (size_t)output_size,
                           cudaMemcpyDeviceToHost, L.stream);
-  }
-  if (e == cudaSuccess) {
-    // The status record follows the rows.  As a DMA copy it takes its turn in the copy engine behind the other
-    // lanes' rows; where the uploads are the larger transfer that wait is what holds the lane back, and a one-warp
-    // kernel writes the record to the page-locked word instead (measured on the 4-bit configuration with 8 lanes:
-    // 31.8 -> 27.5 us per call).  Where the rows are the larger transfer the copy stays: with the kernel the 8-bit
-    // configuration ran 9 % faster and the pruned 2-bit one 15 % slower.
-    e = upload_dominant
-            ? launch_status_to_host(ctx->status + 4 * slot, static_cast<int32_t*>(L.h_status.ptr), L.stream)
-            : cudaMemcpyAsync(L.h_status.ptr, ctx->status + 4 * slot, 16, cudaMemcpyDeviceToHost, L.stream);
   }
   if (e != cudaSuccess) {
     return fail_cuda(e, "result download");
@@ -1379,29 +1528,34 @@ int fbgemm_b200_spmdm_host_wait(fbgemm_b200_ctx* ctx, int lane_id) {
     return 0;
   }
   DeviceGuard guard(ctx->device);
-  cudaError_t e = cudaStreamSynchronize(L.stream);
+  cudaError_t e = cudaSuccess;
+  const uint8_t* src = static_cast<const uint8_t*>(L.h_out.ptr);
+  uint8_t* dst = static_cast<uint8_t*>(L.user_out);
+  if (L.out_rows && L.pieces) {
+    CopySlice slices[Lane::kMaxPieces];
+    const size_t bytes = (size_t)L.out_rows * L.out_pitch_bytes;
+    for (int i = 0; i < L.pieces; ++i) {
+      const size_t at = (size_t)i * L.piece_bytes;
+      slices[i] = {dst + at, src + at, std::min(L.piece_bytes, bytes - at)};
+    }
+    copy_slices(slices, L.pieces, [&](int i) {
+      e = cudaEventSynchronize(L.piece_done[i]);
+      return e == cudaSuccess;
+    });
+  } else {
+    e = cudaStreamSynchronize(L.stream);
+  }
   if (e != cudaSuccess) {
     return fail_cuda(e, "lane synchronize");
   }
-  if (L.out_rows) {
+  if (L.out_rows && !L.pieces) {
     // Only the block_size columns of each row belong to this call: the user's
     // buffer may hold other tables' columns between them (output_stride).
-    const uint8_t* src = static_cast<const uint8_t*>(L.h_out.ptr);
-    uint8_t* dst = static_cast<uint8_t*>(L.user_out);
-    if (L.out_row_bytes == L.out_pitch_bytes) {
-      std::memcpy(dst, src, (size_t)L.out_rows * L.out_pitch_bytes);
-    } else {
-      for (int64_t r = 0; r < L.out_rows; ++r) {
-        std::memcpy(dst + r * L.out_pitch_bytes, src + r * L.out_pitch_bytes, L.out_row_bytes);
-      }
+    for (int64_t r = 0; r < L.out_rows; ++r) {
+      std::memcpy(dst + r * L.out_pitch_bytes, src + r * L.out_pitch_bytes, L.out_row_bytes);
     }
   }
-  const int32_t code = static_cast<const int32_t*>(L.h_status.ptr)[0];
-  if (code != 0) {
-    const int slot = FBGEMM_B200_STATUS_SLOTS - FBGEMM_B200_HOST_LANES + lane_id;
-    cudaMemsetAsync(ctx->status + 4 * slot, 0, 16, L.stream);
-  }
-  return code == 0 ? 1 : 0;
+  return take_record(static_cast<int32_t*>(L.h_status.ptr)) == 0 ? 1 : 0;
 }
 
 int fbgemm_b200_spmdm_host(

@@ -57,9 +57,15 @@ struct Lane {
   DeviceBuffer d_scan;  // lengths-mode scratch of this lane
   PinnedBuffer h_in;
   PinnedBuffer h_out;
+  // The call's error record.  The kernels write to it where it lies, in page-locked host memory, and only when there
+  // is an error, so that nothing has to be copied back.
   PinnedBuffer h_status;
   bool busy = false;
   // what to do at wait()
+  static constexpr int kMaxPieces = 16;
+  cudaEvent_t piece_done[kMaxPieces] = {};  // rows in pageable memory come down in pieces
+  int pieces = 0;
+  size_t piece_bytes = 0;
   void* user_out = nullptr;
   size_t out_row_bytes = 0;   // bytes of one pooled row (block_size elements)
   size_t out_pitch_bytes = 0; // bytes between rows in the user's buffer
@@ -114,6 +120,7 @@ struct fbgemm_b200_ctx {
   std::mutex mu;
   int32_t* status = nullptr;         // device, FBGEMM_B200_STATUS_SLOTS x 4
   int32_t* status_host = nullptr;    // pinned, same shape (read-back)
+  int32_t* sync_status = nullptr;    // pinned, one record: the awaited device-pointer call's
   // Lengths-mode scratch of the device-pointer path, one buffer per stream:
   // calls on one stream are ordered, calls on different streams must not
   // share the scanned offsets.
@@ -121,6 +128,13 @@ struct fbgemm_b200_ctx {
   fbgemm_b200::DeviceBuffer remap_scratch;        // fbgemm_b200_compressed_indices_remap (one call at a time, it synchronises)
   std::unordered_map<const void*, fbgemm_b200::ResidentTable> tables;
   fbgemm_b200::Lane lanes[FBGEMM_B200_HOST_LANES];
+};
+
+// The tables of one table-batched operator (fbgemm_b200_table_set_*).
+struct fbgemm_b200_table_set {
+  fbgemm_b200_ctx* ctx = nullptr;
+  std::vector<fbgemm_b200_table_call> tables;
+  std::vector<int64_t> out_columns;
 };
 
 struct fbgemm_b200_multi_plan {

@@ -124,6 +124,8 @@ struct MultiPlan {
 };
 cudaError_t build_multi_plan(const SpmdmParams* tables, const int* bit_rates, size_t count, MultiPlan* plan);
 cudaError_t launch_multi_plan(const MultiPlan& plan, cudaStream_t stream);
+// The same without keeping the plan.
+cudaError_t launch_tables(const SpmdmParams* tables, const int* bit_rates, size_t count, cudaStream_t stream);
 
 // no_bag with 8-bit output: byte copies of the indexed rows (plain_kernels.cu).
 cudaError_t launch_rows_copy(
@@ -220,9 +222,9 @@ cudaError_t launch_sequence_lookup(
     int out_kind,
     int64_t out_row_bytes,
     bool scale_bias_last,
+    bool fill,
     int fp8_exponent_bits,
     int fp8_exponent_bias,
-    bool fill,
     int32_t* status,
     cudaStream_t stream);
 

@@ -4,7 +4,7 @@
 // with the tables resident in HBM.  One step of a handle:
 //
 //   indices / offsets / weights of every table  --H2D-->  the handle's staging block
-//   one lookup per table (spread over side streams), pooled rows stored into
+//   the tables' lookups, up to 64 of them in a launch, pooled rows stored into
 //   `out_dev` - or, table-wise sharded, into the peers' buffers
 //   [sharded]  publish "my rows for step s are stored" to every peer, wait
 //              until every peer has published the same for my slice
@@ -25,7 +25,6 @@
 using namespace fbgemm_b200;
 
 namespace {
-constexpr int kSideStreams = 3;
 size_t up16(size_t v) {
   return (v + 15) & ~size_t(15);
 }
@@ -60,9 +59,6 @@ struct fbgemm_b200_multi_host {
   uint64_t timeout_us = 0;
   uint64_t step = 0;
   cudaStream_t stream = nullptr;
-  cudaStream_t side[kSideStreams] = {};
-  cudaEvent_t fork = nullptr;
-  cudaEvent_t join[kSideStreams] = {};
   PinnedBuffer h_status;
   bool busy = false;
   cudaEvent_t mark[4] = {};  // step start, uploads done, rows complete, download done
@@ -71,38 +67,28 @@ struct fbgemm_b200_multi_host {
 
 namespace {
 
-// One lookup per table on device arrays, round-robin over `stream` and the handle's side streams, which are forked
-// from `stream` and joined back into it.
-int fan_out_lookups(fbgemm_b200_multi_host* h, cudaStream_t stream, const void* const* idx, const void* const* off,
-                    const float* const* w, const int64_t* index_sizes, int32_t* status) {
-  cudaError_t e = cudaEventRecord(h->fork, stream);
-  for (int i = 0; i < kSideStreams && e == cudaSuccess; ++i) {
-    e = cudaStreamWaitEvent(h->side[i], h->fork, 0);
-  }
-  if (e != cudaSuccess) {
-    return fail_cuda(e, "multi-table step: fork");
-  }
-  DeviceBuffer unused;  // offsets mode: no scan scratch
+// The lookups of all tables on device arrays.
+int enqueue_tables(fbgemm_b200_multi_host* h, cudaStream_t stream, const void* const* idx, const void* const* off,
+                   const float* const* w, const int64_t* index_sizes, int32_t* status) {
   const size_t T = h->calls.size();
+  std::vector<SpmdmParams> params(T);
+  std::vector<int> bit_rates(T);
   for (size_t t = 0; t < T; ++t) {
     const fbgemm_b200_table_call& c = h->calls[t];
-    const size_t k = t % (kSideStreams + 1);
-    cudaStream_t s = k == 0 ? stream : h->side[k - 1];
-    const int rc = enqueue_lookup(&c.cfg, c.output_size, index_sizes[t], c.data_size, c.input, idx[t], off[t],
-                                  c.cfg.has_weight ? w[t] : nullptr, h->num_peers > 0 ? nullptr : c.out,
-                                  c.compressed_indices_table, status, unused, s,
-                                  h->num_peers > 0 ? h->peer_out[t].data() : nullptr, h->num_peers, h->bags_per_peer);
+    const bool peers = h->num_peers > 0;
+    const int rc = build_lookup_params(&c.cfg, c.output_size, index_sizes[t], c.data_size, c.input, idx[t],
+                                       c.cfg.has_weight ? w[t] : nullptr, peers ? nullptr : c.out,
+                                       c.compressed_indices_table, status, peers ? h->peer_out[t].data() : nullptr,
+                                       h->num_peers, h->bags_per_peer, &params[t]);
     if (rc) {
       return rc;
     }
+    params[t].offsets = off[t];
+    params[t].flags |= c.cfg.offset_bytes == 8 ? kOff64 : 0;
+    bit_rates[t] = c.cfg.bit_rate;
   }
-  for (int i = 0; i < kSideStreams && e == cudaSuccess; ++i) {
-    e = cudaEventRecord(h->join[i], h->side[i]);
-    if (e == cudaSuccess) {
-      e = cudaStreamWaitEvent(stream, h->join[i], 0);
-    }
-  }
-  return e == cudaSuccess ? 0 : fail_cuda(e, "multi-table step: join");
+  const cudaError_t e = launch_tables(params.data(), bit_rates.data(), T, stream);
+  return e == cudaSuccess ? 0 : fail_cuda(e, "multi-table step");
 }
 
 }  // namespace
@@ -116,17 +102,6 @@ void fbgemm_b200_multi_host_destroy(fbgemm_b200_multi_host* h) {
   DeviceGuard guard(h->device);
   if (h->stream) {
     cudaStreamSynchronize(h->stream);
-  }
-  for (int i = 0; i < kSideStreams; ++i) {
-    if (h->side[i]) {
-      cudaStreamDestroy(h->side[i]);
-    }
-    if (h->join[i]) {
-      cudaEventDestroy(h->join[i]);
-    }
-  }
-  if (h->fork) {
-    cudaEventDestroy(h->fork);
   }
   for (cudaEvent_t m : h->mark) {
     if (m) {
@@ -221,15 +196,6 @@ int fbgemm_b200_multi_host_create(
   cudaError_t e = reserve(h->staging, at);
   if (e == cudaSuccess) {
     e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
-  }
-  if (e == cudaSuccess) {
-    e = cudaEventCreateWithFlags(&h->fork, cudaEventDisableTiming);
-  }
-  for (int i = 0; i < kSideStreams && e == cudaSuccess; ++i) {
-    e = cudaStreamCreateWithFlags(&h->side[i], cudaStreamNonBlocking);
-    if (e == cudaSuccess) {
-      e = cudaEventCreateWithFlags(&h->join[i], cudaEventDisableTiming);
-    }
   }
   for (int i = 0; i < 4 && e == cudaSuccess; ++i) {
     e = cudaEventCreate(&h->mark[i]);
@@ -342,7 +308,7 @@ int fbgemm_b200_multi_host_submit(
     h->d_off[t] = st + h->off_at[t];
     h->d_w[t] = reinterpret_cast<const float*>(st + h->w_at[t]);
   }
-  if (const int rc = fan_out_lookups(h, h->stream, h->d_idx.data(), h->d_off.data(), h->d_w.data(), index_sizes, status)) {
+  if (const int rc = enqueue_tables(h, h->stream, h->d_idx.data(), h->d_off.data(), h->d_w.data(), index_sizes, status)) {
     return rc;
   }
   if (e == cudaSuccess && h->has_sync) {
@@ -413,7 +379,7 @@ int64_t fbgemm_b200_multi_host_step_device(
   for (size_t t = 0; t < T; ++t) {
     h->d_w[t] = weights ? weights[t] : nullptr;
   }
-  if (const int rc = fan_out_lookups(h, stream, indices, offsets, h->d_w.data(), index_sizes, status)) {
+  if (const int rc = enqueue_tables(h, stream, indices, offsets, h->d_w.data(), index_sizes, status)) {
     return rc;
   }
   if (h->has_sync) {

@@ -42,6 +42,8 @@ class Context:
 
     def close(self):
         if self._h:
+            if _handles.get(self.device) == self._h.value:
+                del _handles[self.device]
             _capi.lib().fbgemm_b200_ctx_destroy(self._h)
             self._h = C.c_void_p()
 
@@ -71,6 +73,25 @@ def get_context(device: int | None = None) -> Context:
         if ctx is None:
             ctx = _ctxs[device] = Context(device)
         return ctx
+
+
+_handles: dict[int, int] = {}  # device -> address of its context
+
+
+def _handle_of(device: int) -> int:
+    h = _handles.get(device)
+    if h is None:
+        h = _handles[device] = get_context(device).handle.value
+    return h
+
+
+def _current_stream(device: int) -> int:
+    """Raw handle of torch's current stream."""
+    global _current_stream
+    import torch
+
+    _current_stream = torch._C._cuda_getCurrentRawStream   # the next call goes straight there
+    return _current_stream(device)
 
 
 def launch_count() -> int:
@@ -119,6 +140,7 @@ class SpmdmKernel:
     def __init__(self, cfg: SpmdmConfig, rowwise_sparse: bool):
         self.cfg = cfg
         self.rowwise_sparse = rowwise_sparse
+        self._cfg_addr = C.addressof(cfg)
         _capi.check(_capi.lib().fbgemm_b200_spmdm_check_config(C.byref(cfg)), "generator arguments")
 
     # -- the reference's functor signature ----------------------------------
@@ -129,20 +151,14 @@ class SpmdmKernel:
         if not self.rowwise_sparse and compressed_indices_table is not None:
             raise ValueError("this kernel was not generated for row-wise sparse tables")
         self._check_dtypes(indices, offsets_or_lengths)
-        lib = _capi.lib()
         if _is_tensor(input):
-            import torch
-
-            dev = input.device.index
-            ctx = get_context(dev)
-            stream = torch.cuda.current_stream(dev).cuda_stream
-            rc = lib.fbgemm_b200_spmdm(
-                ctx.handle, C.byref(self.cfg), output_size, index_size, data_size, _ptr(input), _ptr(indices),
-                _ptr(offsets_or_lengths), _ptr(weights) if self.cfg.has_weight else None, _ptr(out),
-                _ptr(compressed_indices_table), stream)
+            dev = input.get_device()
+            rc = _capi.native().spmdm(
+                _handle_of(dev), self._cfg_addr, output_size, index_size, data_size, input, indices, offsets_or_lengths,
+                weights if self.cfg.has_weight else None, out, compressed_indices_table, _current_stream(dev))
         else:
             ctx = get_context()
-            rc = lib.fbgemm_b200_spmdm_host(
+            rc = _capi.lib().fbgemm_b200_spmdm_host(
                 ctx.handle, C.byref(self.cfg), output_size, index_size, data_size, _ptr(input), _ptr(indices),
                 _ptr(offsets_or_lengths), _ptr(weights) if self.cfg.has_weight else None, _ptr(out),
                 _ptr(compressed_indices_table))
@@ -153,16 +169,11 @@ class SpmdmKernel:
                compressed_indices_table=None, slot: int = 0, stream=None) -> None:
         """Enqueue on ``stream`` (int handle; default torch's current stream)
         without synchronising; errors land in status slot ``slot``."""
-        import torch
-
-        dev = input.device.index
-        ctx = get_context(dev)
-        if stream is None:
-            stream = torch.cuda.current_stream(dev).cuda_stream
-        rc = _capi.lib().fbgemm_b200_spmdm_launch(
-            ctx.handle, C.byref(self.cfg), output_size, index_size, data_size, _ptr(input), _ptr(indices),
-            _ptr(offsets_or_lengths), _ptr(weights) if self.cfg.has_weight else None, _ptr(out),
-            _ptr(compressed_indices_table), slot, stream)
+        dev = input.get_device()
+        rc = _capi.native().spmdm_launch(
+            _handle_of(dev), self._cfg_addr, output_size, index_size, data_size, input, indices, offsets_or_lengths,
+            weights if self.cfg.has_weight else None, out, compressed_indices_table, slot,
+            _current_stream(dev) if stream is None else stream)
         _capi.check(rc, "fbgemm_b200_spmdm_launch")
 
     def host_submit(self, lane, output_size, index_size, data_size, input, indices, offsets_or_lengths,

@@ -6,12 +6,12 @@ of FBGEMM).  Same arguments, same result; the tensors live in HBM.
 
 The reference walks the tables on host threads and calls one generated kernel
 per table with ``output + D_start``, ``output_stride = total_D`` and the slice
-``offsets[t*B : (t+1)*B + 1]`` of the ``T*B + 1`` offsets.  Here every table is
-one launch of the same lookup kernel with *absolute* offsets (the kernel is
-given the whole index array and the slice of offsets, so nothing has to be
-read back to the host to find where a table's indices start), all launches
-enqueued without a synchronisation; or, for callers whose input buffers keep
-their addresses, one multi-table plan that is built once and replayed.
+``offsets[t*B : (t+1)*B + 1]`` of the ``T*B + 1`` offsets.  Here up to 64 tables
+are one launch with *absolute* offsets (the kernel is given the whole index
+array and the slice of offsets, so nothing has to be read back to the host to
+find where a table's indices start), enqueued without a synchronisation by one
+call into the library; or, for callers whose input buffers keep their addresses,
+one multi-table plan that is built once and replayed.
 
 Rows are INT8 / INT4 / INT2 with fp16 scale and bias *first* (the layout of
 table-batched embeddings, ``scale_bias_last = False``), or scale and bias last
@@ -23,6 +23,7 @@ reference's nobag operator and is refused.
 """
 from __future__ import annotations
 
+import ctypes as C
 import enum
 
 import numpy as np
@@ -133,8 +134,32 @@ class IntNBitTableBatchedEmbeddingBags:
                                                             self.total_D, D_bytes, scale_bias_last, bf16, **kw)
             k.cfg.absolute_offsets = 1
             self.kernels.append(k)
-        self._streams = [torch.cuda.Stream(device=self.device) for _ in range(4)]
         self._plans: dict = {}
+        # every output column belongs to a table: the kernels write all of the output, which then need not be cleared
+        self._covers_output = self.T > 0 and self.D_offsets[0] == 0 and self.D_offsets[-1] == self.total_D
+        self._set = self._make_set()
+
+    def _make_set(self):
+        """The library's handle for these tables (``fbgemm_b200_table_set_*``)."""
+        calls = (E._capi.TableCall * self.T)()
+        columns = (C.c_int64 * self.T)()
+        for t in range(self.T):
+            calls[t].cfg = self.kernels[t].cfg
+            calls[t].data_size = self.rows[t]
+            calls[t].input = self.tables[t].data_ptr()
+            columns[t] = int(self.D_offsets[t])
+        handle = C.c_void_p()
+        E._capi.check(E._capi.lib().fbgemm_b200_table_set_create(
+            E.get_context(self.device.index).handle, calls, columns, self.T, C.byref(handle)), "fbgemm_b200_table_set_create")
+        return handle.value
+
+    def __del__(self):
+        try:
+            if self._set:
+                E._capi.lib().fbgemm_b200_table_set_destroy(self._set)
+                self._set = None
+        except Exception:
+            pass
 
     def _calls(self, B, indices, offsets, indice_weights, output):
         flat = output.view(-1)
@@ -156,11 +181,12 @@ class IntNBitTableBatchedEmbeddingBags:
         if self.weighted:
             assert indice_weights is not None and indice_weights.dtype == torch.float32
         if output is None:
-            output = torch.zeros((B, self.total_D), dtype=self.out_dtype, device=self.device)
+            make = torch.empty if self._covers_output else torch.zeros
+            output = make((B, self.total_D), dtype=self.out_dtype, device=self.device)
         if B == 0:
             return output
-        calls = self._calls(B, indices, offsets, indice_weights, output)
         if use_plan:
+            calls = self._calls(B, indices, offsets, indice_weights, output)
             key = (indices.data_ptr(), offsets.data_ptr(), indice_weights.data_ptr() if self.weighted else 0,
                    output.data_ptr(), B, indices.numel(), slot)
             plan = self._plans.pop(key, None)
@@ -171,14 +197,10 @@ class IntNBitTableBatchedEmbeddingBags:
             self._plans[key] = plan
             plan.launch()
             return output
-        cur = torch.cuda.current_stream(self.device)
-        for s in self._streams:
-            s.wait_stream(cur)
-        for t, (k, b, n, rows, table, idx, off, w, out, _) in enumerate(calls):
-            k.launch(b, n, rows, table, idx, off, w, out, slot=slot,
-                     stream=self._streams[t % len(self._streams)].cuda_stream)
-        for s in self._streams:
-            cur.wait_stream(s)
+        rc = E._capi.native().table_set_forward(self._set, B, indices, indices.numel(), offsets,
+                                                indice_weights if self.weighted else None, output, slot,
+                                                E._current_stream(self.device.index))
+        E._capi.check(rc, "fbgemm_b200_table_set_forward")
         return output
 
 
@@ -349,6 +371,7 @@ class IntNBitSequenceEmbedding:
         assert (offsets.numel() - 1) % self.T == 0
         B = (offsets.numel() - 1) // self.T
         n = indices.numel()
+        lookup = E._capi.lib().fbgemm_b200_sequence_lookup
         if output is None:
             output = torch.empty((n, self.out_cols), dtype=self.out_dtype, device=self.device)
             lookup = E._capi.lib().fbgemm_b200_sequence_lookup_filled
@@ -374,7 +397,6 @@ def int_nbit_split_embedding_nobag_codegen_forward_unweighted(
     """One call with the reference operator's arguments (placement and UVM
     arguments left out; ``pooling_mode`` is accepted and, bags being one row
     long, changes nothing)."""
-        lookup = E._capi.lib().fbgemm_b200_sequence_lookup
     op = IntNBitSequenceEmbedding(dev_weights, weights_offsets, weights_tys, D, row_alignment, output_dtype,
                                   scale_bias_last, fp8_exponent_bits, fp8_exponent_bias)
     return op.forward(indices, offsets)

@@ -235,9 +235,9 @@ FBGEMM_B200_API int fbgemm_b200_spmdm_launch_sharded(
  * output_stride = total_D
  * (fbgemm_gpu/codegen/inference/embedding_forward_quantized_cpu_template.cpp:343-473;
  * the reference library itself has no multi-table entry point).  A plan is
- * built once for a fixed set of device pointers: the tables are grouped by
- * kernel variant and every group becomes ONE launch whose grid covers all bags
- * of all its tables.  Launching the plan again pools whatever the index,
+ * built once for a fixed set of device pointers: up to 64 tables (column tiles
+ * of them, where rows are wide) of whatever row formats are ONE launch whose
+ * grid covers all their bags.  Launching the plan again pools whatever the index,
  * offset and weight arrays hold by then.
  *
  * One fbgemm_b200_table_call per table: the arguments of
@@ -275,6 +275,40 @@ FBGEMM_B200_API int fbgemm_b200_multi_plan_launch(fbgemm_b200_multi_plan* plan, 
 /* Kernel launches one fbgemm_b200_multi_plan_launch enqueues. */
 FBGEMM_B200_API int fbgemm_b200_multi_plan_num_launches(const fbgemm_b200_multi_plan* plan);
 FBGEMM_B200_API void fbgemm_b200_multi_plan_destroy(fbgemm_b200_multi_plan* plan);
+
+/* The tables of one table-batched operator (the reference's
+ * int_nbit_split_embedding_codegen_forward_*_cpu,
+ * fbgemm_gpu/codegen/inference/embedding_forward_quantized_cpu_template.cpp:205-520):
+ * one indices array, one offsets array of num_tables * bags + 1 entries (table
+ * after table) and one weights array for all of them, pooled rows side by side
+ * in one output.  Of each fbgemm_b200_table_call only cfg (absolute_offsets set,
+ * output_stride = columns of the whole output; index, offset and output types
+ * and has_weight the same for all tables), data_size and input are read;
+ * out_columns[t] is the output column table t starts at.  Nothing else is
+ * fixed: a forward call takes any batch and any arrays, allocates nothing on
+ * the device and may run on several streams and threads at once.  The context
+ * outlives the set. */
+typedef struct fbgemm_b200_table_set fbgemm_b200_table_set;
+
+FBGEMM_B200_API int fbgemm_b200_table_set_create(
+    fbgemm_b200_ctx* ctx,
+    const fbgemm_b200_table_call* tables,
+    const int64_t* out_columns,
+    int32_t num_tables,
+    fbgemm_b200_table_set** set);
+/* Pools `bags` bags of every table; asynchronous, errors in status slot `slot`.
+ * Returns 0 or a negative code. */
+FBGEMM_B200_API int fbgemm_b200_table_set_forward(
+    fbgemm_b200_table_set* set,
+    int64_t bags,
+    const void* indices,
+    int64_t index_size,
+    const void* offsets,
+    const float* weights, /* NULL unless has_weight */
+    void* out,
+    int slot,
+    void* stream);
+FBGEMM_B200_API void fbgemm_b200_table_set_destroy(fbgemm_b200_table_set* set);
 
 /* Waits for `stream`, reads status slot `slot` into info[4] = {code, bag,
  * position in indices, offending value (low 32 bits)} and clears the slot.
@@ -530,6 +564,28 @@ FBGEMM_B200_API int fbgemm_b200_sequence_lookup(
     int32_t fp8_exponent_bias,
     int32_t slot,
     void* stream);
+/* The same for an output buffer that holds nothing yet: rows of positions that
+ * no table covers, or whose index is out of range, and bytes behind a copied
+ * row are set to zero, so that the buffer need not be cleared first. */
+FBGEMM_B200_API int fbgemm_b200_sequence_lookup_filled(
+    fbgemm_b200_ctx* ctx,
+    const void* dev_weights,
+    const fbgemm_b200_sequence_table* tables,
+    int32_t T,
+    int32_t B,
+    int32_t D,
+    const void* indices,
+    const void* offsets,
+    int32_t index_bytes,
+    int64_t index_size,
+    void* out,
+    int32_t out_dtype,
+    int64_t out_row_bytes,
+    int32_t scale_bias_last,
+    int32_t fp8_exponent_bits,
+    int32_t fp8_exponent_bias,
+    int32_t slot,
+    void* stream);
 
 /* ---- pooled lookup, host pointers -------------------------------------- */
 
@@ -564,28 +620,6 @@ FBGEMM_B200_API const void* fbgemm_b200_table_device_ptr(fbgemm_b200_ctx* ctx, c
  * (FBGEMM_B200_EBUSY if the lane has un-waited work). */
 FBGEMM_B200_API int fbgemm_b200_spmdm_host_submit(
     fbgemm_b200_ctx* ctx,
-/* The same for an output buffer that holds nothing yet: rows of positions that
- * no table covers, or whose index is out of range, and bytes behind a copied
- * row are set to zero, so that the buffer need not be cleared first. */
-FBGEMM_B200_API int fbgemm_b200_sequence_lookup_filled(
-    fbgemm_b200_ctx* ctx,
-    const void* dev_weights,
-    const fbgemm_b200_sequence_table* tables,
-    int32_t T,
-    int32_t B,
-    int32_t D,
-    const void* indices,
-    const void* offsets,
-    int32_t index_bytes,
-    int64_t index_size,
-    void* out,
-    int32_t out_dtype,
-    int64_t out_row_bytes,
-    int32_t scale_bias_last,
-    int32_t fp8_exponent_bits,
-    int32_t fp8_exponent_bias,
-    int32_t slot,
-    void* stream);
     int lane,
     const fbgemm_b200_spmdm_config* cfg,
     int64_t output_size,
