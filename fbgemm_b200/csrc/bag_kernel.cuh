@@ -308,9 +308,19 @@ __device__ __forceinline__ void store_columns(const BagTable& p, char* row, int 
     const bool bf16 = p.flags & kOutBf16;
     uint16_t* o = reinterpret_cast<uint16_t*>(row) + col0;
     uint32_t h[N];
+    if (!bf16 && N % 2 == 0) {
 #pragma unroll
-    for (int i = 0; i < N; ++i) {
-      h[i] = to_16bit(v[i], bf16);
+      for (int i = 0; i + 1 < N; i += 2) {
+        const __half2 two = __floats2half2_rn(v[i], v[i + 1]);  // one instruction for both
+        const uint32_t bits = *reinterpret_cast<const uint32_t*>(&two);
+        h[i] = bits & 0xffffu;
+        h[i + 1] = bits >> 16;
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < N; ++i) {
+        h[i] = to_16bit(v[i], bf16);
+      }
     }
     if (left >= N) {
       store_u16<N>(o, h, p.out_align);
@@ -372,18 +382,34 @@ struct __align__(16) Queue {
   ulonglong2 sb[32];  // {scale, scale}, {bias, bias}; {weight, weight} of unquantized rows
 };
 
-// Groups of four rows whose loads are issued ahead of the arithmetic.  Measured on 65536 bags of 30 rows: with half or
-// quarter warps per bag none is best for 4- and 2-bit rows (72.8 against 76.2 us at D = 128, 4 bits), one for 8-bit
-// rows (82 against 102 us at D = 128); whole warps want one.
-__host__ __device__ constexpr int rows_ahead(int fmt, int g) { return g == 32 || (g == 16 && fmt == kInt8) ? 1 : 0; }
-constexpr int kDeepAhead = 2;
+// What a kernel is compiled for.
+//  kLean  bags by offsets, weights per index, every index a row of the table
+//  kFull  besides: pruning maps, -1 as a pruned index, no_bag, positional weights
+//  kWide  the same where positions, bags (31 bits) or row offsets (32) need more
+// The lean form saves the queue's compaction and half of the tests, a tenth of
+// the time of 65536 bags of 30 rows (8-bit D = 128 76.4 against 83.6 us).
+enum : int { kLean = 0, kFull = 1, kWide = 2 };
+
+// Groups of four rows whose loads are issued ahead of the arithmetic.  Measured on 65536 bags of 30 rows: with half
+// warps per bag none is best for 4-bit rows (67.9 against 69.4 us at D = 128), one for 8- and 2-bit rows (82 against
+// 102 us, 66 against 68); quarter warps want none, whole warps one.  Launches whose warps are all resident with more
+// registers each (kDeep) take one more with whole warps.
+__host__ __device__ constexpr int rows_ahead(int fmt, int g, bool deep) {
+  return g == 32 ? (deep ? 2 : 1) : deep ? 1 : g == 16 && (fmt == kInt8 || fmt == kInt2) ? 1 : 0;
+}
+
+// The stream's next launch may be set up while this one drains; it waits here until all results of this one are there.
+__device__ __forceinline__ void wait_for_previous_launch() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_launch_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // One block's work on table `p`: bags block * kWarps * (32 / G) onwards, columns of tile `tile` of the row.
-template <int FMT, int VB, int CPL, int G, bool WIDE, int kAhead = rows_ahead(FMT, G)>
-__device__ __forceinline__ void pool_bags(const BagTable& p, void* const* peers, int64_t block, int tile,
-                                          Queue<WIDE> (&queues)[kWarps]) {
+template <int FMT, int VB, int CPL, int G, int MODE, bool kDeep>
+__device__ __forceinline__ void pool_bags(const BagTable& p, void* const* peers, uint32_t block, int tile,
+                                          Queue<MODE == kWide> (&queues)[kWarps]) {
+  constexpr bool WIDE = MODE == kWide, FULL = MODE != kLean;
+  constexpr int kAhead = rows_ahead(FMT, G, kDeep);
   using C = Cols<FMT, VB, CPL>;
-
+  using Pos = typename std::conditional<WIDE, int64_t, int32_t>::type;  // bags and positions
   constexpr int kTileBytes = G * VB * CPL;
   constexpr unsigned kGroupMask = G == 32 ? 0xffffffffu : (1u << (G % 32)) - 1u;
   constexpr bool kQuantized = is_quantized(FMT);
@@ -396,62 +422,63 @@ __device__ __forceinline__ void pool_bags(const BagTable& p, void* const* peers,
   const bool idx64 = p.flags & kIdx64;
   const bool off64 = p.flags & kOff64;
   const bool weighted = p.flags & kWeighted;
-  const bool positional = p.flags & kPositional;
-  const bool pruned = p.flags & kPruned;
-  const bool no_bag = p.flags & kNoBag;
-  const bool minus_one_skips = FMT != kFp8 && (p.flags & (kSbFirst | kNoBag)) == kSbFirst;
+  const bool positional = FULL && (p.flags & kPositional);
+  const bool pruned = FULL && (p.flags & kPruned);
+  const bool no_bag = FULL && (p.flags & kNoBag);
+  const bool minus_one_skips = FULL && FMT != kFp8 && (p.flags & (kSbFirst | kNoBag)) == kSbFirst;
   const bool half_sb = FMT != kInt8 || (p.flags & kSbFirst);
 
-  // rebasing to offsets[0] (the functor's convention) unless the offsets are absolute
-  const bool rebase = !(p.flags & (kNoBag | kAbsOffsets));
-  const int64_t off_base = rebase ? load_int(p.offsets, 0, off64) : 0;
-  if (block == 0 && threadIdx.x == 0 && rebase) {
-    // `return current == index_size` of the reference
-    const int64_t total = load_int(p.offsets, p.bags, off64) - off_base;
-    if (total != p.index_size) {
-      report(p.status, FBGEMM_B200_STATUS_SIZE_MISMATCH, p.bags, total, p.index_size);
-    }
-  }
-  int64_t pos = 0;  // of this lane's next candidate: one in every G indices of the bag
-  int len = 0;
-  {
-    const int64_t bag = (block * kWarps + warp) * (32 / G) + grp;
-    if (bag < p.bags) {
-      // no_bag: output row m is the single row indices[m]
-      const int64_t o0 = no_bag ? bag : load_int(p.offsets, bag, off64);
-      const int64_t o1 = no_bag ? bag + 1 : load_int(p.offsets, bag + 1, off64);
-      pos = o0 - off_base;
-      const int bag_len = (int)(o1 - o0);  // the reference narrows to 32 bits too
-      len = bag_len < 0 ? 0 : bag_len;
-      // Offsets that step backwards: the reference, which walks the index array
-      // with a running position, ends up past index_size and returns false.
-      if (bag_len < 0 || pos < 0 || pos + len > p.index_size) {
-        if (gl == 0) {
-          report(p.status, FBGEMM_B200_STATUS_BAG_OVERRUN, bag, pos, len);
-        }
-        len = 0;  // never read past the caller's arrays
-      }
-      pos += gl;
-    }
-  }
-  int longest = len;
-#pragma unroll
-  for (int d = G; d < 32; d <<= 1) {
-    longest = max(longest, __shfl_xor_sync(0xffffffffu, longest, d));
-  }
-
+  const Pos bag = (Pos)block * (kWarps * (32 / G)) + warp * (32 / G) + grp;
   LaneData<VB, CPL, G, WIDE> lane_data;
   lane_data.init(p.data, tile * kTileBytes, gl, p.data_bytes);
   const uint8_t* sb_data = p.data + p.sb_off;
   typename C::M constants;
   constants.init(p);
+  wait_for_previous_launch();
+
+  Pos pos = 0;  // of this lane's next candidate: one in every G indices of the bag
+  int len = 0;
+  {
+    // rebasing to offsets[0] (the functor's convention) unless the offsets are absolute
+    const bool rebase = !(p.flags & (kNoBag | kAbsOffsets));
+    const int64_t off_base = rebase ? load_int(p.offsets, 0, off64) : 0;
+    if (block == 0 && threadIdx.x == 0 && rebase) {
+      // `return current == index_size` of the reference
+      const int64_t total = load_int(p.offsets, p.bags, off64) - off_base;
+      if (total != p.index_size) {
+        report(p.status, FBGEMM_B200_STATUS_SIZE_MISMATCH, p.bags, total, p.index_size);
+      }
+    }
+    int64_t start = 0;
+    int bag_len = 0;
+    if (bag < (Pos)p.bags) {
+      // no_bag: output row m is the single row indices[m]
+      const int64_t o0 = no_bag ? bag : load_int(p.offsets, bag, off64);
+      const int64_t o1 = no_bag ? (int64_t)bag + 1 : load_int(p.offsets, (int64_t)bag + 1, off64);
+      start = o0 - off_base;
+      bag_len = (int)(o1 - o0);  // the reference narrows to 32 bits too
+    }
+    // Offsets that step backwards: the reference, which walks the index array
+    // with a running position, ends up past index_size and returns false.
+    if (bag_len < 0 || start < 0 || start + bag_len > p.index_size) {
+      if (gl == 0) {
+        report(p.status, FBGEMM_B200_STATUS_BAG_OVERRUN, bag, start, bag_len < 0 ? 0 : bag_len);
+      }
+      start = bag_len = 0;  // never read past the caller's arrays
+    }
+    pos = (Pos)start + gl;
+    len = bag_len;
+  }
+  // Uniform to the compiler too (a redux result, unlike a shuffle's): the row loop then branches without
+  // reconvergence barriers and keeps its constants in uniform registers (2-bit D = 256 107 against 127 us).
+  const int longest = (int)__reduce_max_sync(0xffffffffu, (unsigned)len);
+
   u64 acc[C::kPairs];
 #pragma unroll
   for (int k = 0; k < C::kPairs; ++k) {
     acc[k] = 0ull;  // (+0.f, +0.f)
   }
 
-  const uint32_t limit = (uint32_t)min((unsigned long long)p.data_size, idx64 ? 0xfffffffeull : 0x80000000ull);
   auto fetch = [&](int c) -> uint2 {
     uint2 r = make_uint2(0u, 0u);
     if (c < len) {
@@ -464,19 +491,20 @@ __device__ __forceinline__ void pool_bags(const BagTable& p, void* const* peers,
     return r;
   };
   uint2 raw = fetch(gl);
+#pragma unroll 1
   for (int c0 = 0; c0 < longest; c0 += G) {
     const int c = c0 + gl;
     const bool in_bag = c < len;
     float w = 1.f;
     if (weighted && in_bag) {
-      w = __ldg(p.weights + (positional ? (int64_t)c : pos));
+      w = __ldg(p.weights + (positional ? (Pos)c : pos));
     }
     bool keep;
     if constexpr (WIDE) {
       const long long v = idx64 ? (long long)(((u64)raw.y << 32) | raw.x) : (long long)(int)raw.x;
       keep = in_bag && (u64)v < (u64)p.data_size;
     } else {
-      keep = in_bag && raw.y == 0 && raw.x < limit;
+      keep = in_bag && raw.y == 0 && raw.x < p.limit;
     }
     Row<WIDE> id = 0;
     if (keep) {
@@ -486,7 +514,7 @@ __device__ __forceinline__ void pool_bags(const BagTable& p, void* const* peers,
       }
     }
     if (in_bag && !keep && !(minus_one_skips && raw.x == 0xffffffffu && (!idx64 || raw.y == 0xffffffffu))) {
-      report(p.status, FBGEMM_B200_STATUS_BAD_INDEX, (block * kWarps + warp) * (32 / G) + grp, pos, (int32_t)raw.x);
+      report(p.status, FBGEMM_B200_STATUS_BAD_INDEX, bag, pos, (int32_t)raw.x);
     }
     if (pruned && keep) {
       const int32_t m = __ldg(p.cit + id);
@@ -496,20 +524,28 @@ __device__ __forceinline__ void pool_bags(const BagTable& p, void* const* peers,
     pos += G;
     raw = fetch(c + G);  // the next stretch's, on its way during this one's arithmetic
 
-    // Kept rows to the front of the queue in order, the other lanes' slots behind them.  Those hold row 0 with scale
-    // and bias 0, which leave every sum as it is (x + 0 = x, and no sum is ever -0), so that groups of four rows
-    // need no special case for the last one.
-    const unsigned ballot = __ballot_sync(0xffffffffu, keep);
-    const unsigned kept = G == 32 ? ballot : (ballot >> (grp * G)) & kGroupMask;
-    const int count = __popc(kept);
-    int most = count;
-    const unsigned below = (1u << gl) - 1u;
-    const int at = keep ? __popc(kept & below) : most + __popc(~kept & below);
-    if constexpr (G < 32) {
+    // Where this lane's row goes in the queue, how many rows the group has, and the most that a group of the warp has.
+    // Slots behind a group's rows hold row 0 with scale and bias 0, which leave every sum as it is (x + 0 = x, and no
+    // sum is ever -0), so that groups of four rows need no special case for the last one.
+    int at, count, most;
+    if constexpr (FULL) {
+      // kept rows to the front of the queue in order, the other lanes' slots behind them
+      const unsigned ballot = __ballot_sync(0xffffffffu, keep);
+      const unsigned kept = G == 32 ? ballot : (ballot >> (grp * G)) & kGroupMask;
+      const unsigned below = (1u << gl) - 1u;
+      count = __popc(kept);
+      at = keep ? __popc(kept & below) : count + __popc(~kept & below);
+      most = count;
+      if constexpr (G < 32) {
 #pragma unroll
-      for (int g = 0; g < 32 / G; ++g) {
-        most = max(most, __popc((ballot >> (g * G)) & kGroupMask));
+        for (int g = 0; g < 32 / G; ++g) {
+          most = max(most, __popc((ballot >> (g * G)) & kGroupMask));
+        }
       }
+    } else {
+      at = gl;
+      count = len - c0;
+      most = min(longest - c0, G);
     }
     uint32_t sb_lo = 0, sb_hi = 0;
     const Row<WIDE> row_at = id * (Row<WIDE>)p.stride;
@@ -596,13 +632,15 @@ __device__ __forceinline__ void pool_bags(const BagTable& p, void* const* peers,
     __syncwarp();  // the queue is rewritten by the next stretch
   }
 
-  const int64_t bag = (block * kWarps + warp) * (32 / G) + grp;
-  if (bag >= p.bags) {
+  if constexpr (!kDeep) {
+    let_next_launch_start();  // (small launches gain nothing from it: 8.1 against 7.6 us for 4096 ragged bags)
+  }
+  if (bag >= (Pos)p.bags) {
     return;
   }
   int bag_len = 0;
   if (p.flags & kNormalize) {
-    bag_len = (int)(load_int(p.offsets, bag + 1, off64) - load_int(p.offsets, bag, off64));
+    bag_len = (int)(load_int(p.offsets, (int64_t)bag + 1, off64) - load_int(p.offsets, bag, off64));
   }
   if (bag_len != 0) {
     const float inv = __fdiv_rn(1.f, (float)bag_len);
@@ -644,21 +682,21 @@ struct BagCall {
   void* peers[FBGEMM_B200_MAX_PEERS];
 };
 
-template <int FMT, int VB, int CPL, int G, bool WIDE>
+template <int FMT, int VB, int CPL, int G, int MODE>
 __global__ void __launch_bounds__(kThreads, kBlocksPerSm) bag_kernel(const __grid_constant__ BagCall c) {
-  __shared__ Queue<WIDE> queues[kWarps];
-  pool_bags<FMT, VB, CPL, G, WIDE>(c.t, c.peers, blockIdx.x, blockIdx.y, queues);
+  __shared__ Queue<MODE == kWide> queues[kWarps];
+  pool_bags<FMT, VB, CPL, G, MODE, false>(c.t, c.peers, blockIdx.x, blockIdx.y, queues);
 }
 
-// The same for launches whose warps are all resident with 64 registers each:
+// The same for launches whose warps are all resident with 56 registers each:
 // residency costs nothing there, so they go into more rows in flight per bag.
-// 10 bags of 100 rows (8-bit D = 64) 7.4 against 8.7 us, 4096 ragged bags (4-bit
-// D = 64) 8.0 against 8.6 us.
-constexpr int kDeepBlocksPerSm = 8;
-template <int FMT, int VB, int CPL, int G, bool WIDE>
+// 10 bags of 100 rows (8-bit D = 64) 7.7 against 8.7 us, 10 000 bags of 20 rows
+// (8-bit D = 128, half warps) 11.6 against 13.9 us.
+constexpr int kDeepBlocksPerSm = 9;
+template <int FMT, int VB, int CPL, int G, int MODE>
 __global__ void __launch_bounds__(kThreads, kDeepBlocksPerSm) bag_kernel_deep(const __grid_constant__ BagCall c) {
-  __shared__ Queue<WIDE> queues[kWarps];
-  pool_bags<FMT, VB, CPL, G, WIDE, kDeepAhead>(c.t, c.peers, blockIdx.x, blockIdx.y, queues);
+  __shared__ Queue<MODE == kWide> queues[kWarps];
+  pool_bags<FMT, VB, CPL, G, MODE, true>(c.t, c.peers, blockIdx.x, blockIdx.y, queues);
 }
 
 // The compiled combinations of row format, payload bytes per lane and chunk,
@@ -703,9 +741,9 @@ struct BagUnits {
 };
 static_assert(sizeof(BagUnits) < 32764, "one kernel argument");
 
-template <bool WIDE>
+template <int MODE>
 __global__ void __launch_bounds__(kThreads, kBlocksPerSm) bag_units_kernel(const __grid_constant__ BagUnits a) {
-  __shared__ Queue<WIDE> queues[kWarps];
+  __shared__ Queue<MODE == kWide> queues[kWarps];
   int lo = 0, hi = a.count;
   while (hi - lo > 1) {
     const int mid = (lo + hi) >> 1;
@@ -716,11 +754,11 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm) bag_units_kernel(const
     }
   }
   const BagTable& t = a.t[lo];
-  const int64_t block = (int)blockIdx.x - a.first_block[lo];
+  const uint32_t block = blockIdx.x - a.first_block[lo];
   switch (a.variant[lo]) {
 #define FBGEMM_B200_BAG_CASE(FMT, VB, CPL, G)                                   \
-  case id_##FMT##_##VB##_##CPL##_##G:                                           \
-    pool_bags<FMT, VB, CPL, G, WIDE>(t, a.peers[lo], block, a.tile[lo], queues); \
+  case id_##FMT##_##VB##_##CPL##_##G:                                                  \
+    pool_bags<FMT, VB, CPL, G, MODE, false>(t, a.peers[lo], block, a.tile[lo], queues); \
     break;
     FBGEMM_B200_BAG_VARIANTS(FBGEMM_B200_BAG_CASE)
 #undef FBGEMM_B200_BAG_CASE
@@ -728,26 +766,19 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm) bag_units_kernel(const
 }
 
 using BagFn = void (*)(const BagCall);
-template <int FMT, int VB, int CPL, int G, bool WIDE>
-BagFn deep_kernel() {
-  if constexpr (G == 32) {
-    return bag_kernel_deep<FMT, VB, CPL, G, WIDE>;
-  } else {
-    return nullptr;
-  }
-}
+constexpr int kForms = 5;  // kLean, kFull, kWide, and the deep forms of kLean and kFull
 using BagUnitsFn = void (*)(const BagUnits);
 
 }  // namespace bag
 
-// The single-table kernels by variant id, indexed by whether rows lie beyond 4
-// GB, plus 2 for the deep form (whole warps per bag only); one translation unit
-// per group of formats (bag_kernel_*.cu).
-void bag_kernels_8(bag::BagFn (*fn)[4]);
-void bag_kernels_4(bag::BagFn (*fn)[4]);
-void bag_kernels_2(bag::BagFn (*fn)[4]);
-void bag_kernels_plain(bag::BagFn (*fn)[4]);
-bag::BagUnitsFn bag_units_narrow();
+// The single-table kernels by variant id and form; one translation unit per
+// group of formats (bag_kernel_*.cu).
+void bag_kernels_8(bag::BagFn (*fn)[bag::kForms]);
+void bag_kernels_4(bag::BagFn (*fn)[bag::kForms]);
+void bag_kernels_2(bag::BagFn (*fn)[bag::kForms]);
+void bag_kernels_plain(bag::BagFn (*fn)[bag::kForms]);
+bag::BagUnitsFn bag_units_lean();
+bag::BagUnitsFn bag_units_full();
 bag::BagUnitsFn bag_units_wide();
 
 }  // namespace fbgemm_b200

@@ -3,13 +3,14 @@
 
 namespace fbgemm_b200 {
 
-void bag_kernels_2(bag::BagFn (*fn)[4]) {
+void bag_kernels_2(bag::BagFn (*fn)[bag::kForms]) {
   using namespace bag;
-#define ENTRY(FMT, VB, CPL, G)                                                         \
-  fn[id_##FMT##_##VB##_##CPL##_##G][0] = bag_kernel<FMT, VB, CPL, G, false>;          \
-  fn[id_##FMT##_##VB##_##CPL##_##G][1] = bag_kernel<FMT, VB, CPL, G, true>;           \
-  fn[id_##FMT##_##VB##_##CPL##_##G][2] = deep_kernel<FMT, VB, CPL, G, false>();       \
-  fn[id_##FMT##_##VB##_##CPL##_##G][3] = deep_kernel<FMT, VB, CPL, G, true>();
+#define ENTRY(FMT, VB, CPL, G)                                                        \
+  fn[id_##FMT##_##VB##_##CPL##_##G][0] = bag_kernel<FMT, VB, CPL, G, kLean>;         \
+  fn[id_##FMT##_##VB##_##CPL##_##G][1] = bag_kernel<FMT, VB, CPL, G, kFull>;         \
+  fn[id_##FMT##_##VB##_##CPL##_##G][2] = bag_kernel<FMT, VB, CPL, G, kWide>;         \
+  fn[id_##FMT##_##VB##_##CPL##_##G][3] = bag_kernel_deep<FMT, VB, CPL, G, kLean>;    \
+  fn[id_##FMT##_##VB##_##CPL##_##G][4] = bag_kernel_deep<FMT, VB, CPL, G, kFull>;
   FBGEMM_B200_BAG_VARIANTS_2(ENTRY)
 #undef ENTRY
 }

@@ -97,6 +97,7 @@ struct BagTable {
   int32_t cols;               // D
   int32_t data_bytes;         // packed payload bytes per row
   uint32_t flags;
+  uint32_t limit;             // indices name rows below this (forms other than kWide)
   int16_t sb_align;           // address alignment of scale,bias: 8, 4, 2 or 1
   int16_t out_align;          // address alignment of output rows: 16 ... 1
   int32_t num_peers;
