@@ -5,12 +5,14 @@
 //   N-bit + fp16 scale,bias  src/QuantUtils.cc:534-611
 // (fp32 subtract, fp32 multiply by the inverse scale, round half to even).
 //
-// Bound by memory: 4 bytes read per column, 1/4 to 1 written.  The vector form
-// (rows of whole, aligned float4s, up to 1024 columns) therefore reads a row
-// once, into registers - 8, 16 or 32 lanes per row, several rows per lane group
-// in flight - and stores the codes of four columns at a time; the row-by-row form
-// with a second pass over the row and byte stores took 248 us for 1 M x 128
-// columns (8-bit), where the memory needs 99 us.  Other widths keep that form.
+// Bound by memory: 4 bytes read per column, 1/4 to 1 written.  Rows follow one
+// another without gaps, so a block takes 16 KB of them as one stretch of bytes,
+// whatever their width: 16-byte asynchronous copies bring them to shared memory,
+// lane groups of 8 (wide rows: 32) quantize row by row from there into the bytes
+// of the fused rows, and those leave as 16-byte stores of whole sectors.  8 blocks
+// per SM keep 128 KB on their way.  A warp per row that read its row twice and
+// stored single bytes took 248 us for 1 M x 128 columns (8-bit), rows held in
+// registers and stored by words 129 us, this 102 us; memory needs 99 us.
 #include <cuda_fp16.h>
 
 #include "internal.h"
@@ -89,75 +91,107 @@ struct Coder {
   }
 };
 
-// Rows of whole, aligned float4s.  LPR lanes per row, NV float4s per lane, R
-// rows per lane group, all their loads issued before the first use.
-template <int BITS, bool FP32_SB, int LPR, int NV, int R>
+__device__ __forceinline__ void copy_async(void* smem, const void* global, int bytes) {
+  const uint32_t dst = (uint32_t)__cvta_generic_to_shared(smem);
+  if (bytes == 16) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(global) : "memory");
+  } else {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(global) : "memory");
+  }
+}
+
+// Block b quantizes rows b * per_block onwards, which start 16-byte aligned on both sides if the tables do.  LPR lanes per row.
+template <int BITS, bool FP32_SB, int LPR>
 __global__ void __launch_bounds__(kQuantThreads)
-quantize_vector_kernel(const float* __restrict__ in, int64_t rows, int cols, uint8_t* __restrict__ out) {
-  const int gl = threadIdx.x % LPR;
-  const int64_t group = (int64_t)blockIdx.x * (kQuantThreads / LPR) + threadIdx.x / LPR;
-  const int64_t groups = (int64_t)gridDim.x * (kQuantThreads / LPR);
-  const int n4 = cols >> 2;
-  const int data_bytes = cols * BITS / 8;
-  const int64_t pitch = data_bytes + (FP32_SB ? 8 : 4);
-  float4 v[R][NV];
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const int64_t row = min(group + r * groups, rows - 1);
-    const float4* x = reinterpret_cast<const float4*>(in + row * cols);
-#pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      const int k = gl + i * LPR;
-      v[r][i] = __ldcs(x + (k < n4 ? k : 0));  // lanes beyond the row repeat its first columns
+quantize_block_kernel(const float* __restrict__ in, int64_t rows, int cols, uint8_t* __restrict__ out, int per_block) {
+  extern __shared__ __align__(16) float smem[];
+  constexpr int EPB = 8 / BITS;
+  const int data_bytes = cols / EPB;
+  const int pitch = data_bytes + (FP32_SB ? 8 : 4);
+  const int64_t row0 = (int64_t)blockIdx.x * per_block;
+  const int n = (int)min((int64_t)per_block, rows - row0);
+  const float* x = in + row0 * cols;
+  uint8_t* o = out + row0 * pitch;
+  uint8_t* coded = reinterpret_cast<uint8_t*>(smem + (int64_t)per_block * cols);
+
+  const int values = n * cols;
+  int done = 0;
+  if (reinterpret_cast<uintptr_t>(x) % 16 == 0) {
+    done = values & ~3;
+    for (int i = 4 * threadIdx.x; i < done; i += 4 * kQuantThreads) {
+      copy_async(smem + i, x + i, 16);
     }
   }
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    float lo = v[r][0].x, hi = lo;
-#pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      lo = fminf(fminf(lo, fminf(v[r][i].x, v[r][i].y)), fminf(v[r][i].z, v[r][i].w));
-      hi = fmaxf(fmaxf(hi, fmaxf(v[r][i].x, v[r][i].y)), fmaxf(v[r][i].z, v[r][i].w));
+  for (int i = done + threadIdx.x; i < values; i += kQuantThreads) {
+    copy_async(smem + i, x + i, 4);
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();
+
+  const int gl = threadIdx.x % LPR;
+  const unsigned mask = LPR == 32 ? 0xffffffffu : ((1u << (LPR % 32)) - 1u) << (threadIdx.x % 32 / LPR * LPR);
+  for (int r = threadIdx.x / LPR; r < n; r += kQuantThreads / LPR) {
+    const float* row = smem + r * cols;
+    uint8_t* c = coded + r * pitch;
+    float lo = row[0], hi = lo;
+    if (cols % 4 == 0) {
+      for (int k = gl; k < cols / 4; k += LPR) {
+        const float4 v = reinterpret_cast<const float4*>(row)[k];
+        lo = fminf(fminf(lo, fminf(v.x, v.y)), fminf(v.z, v.w));
+        hi = fmaxf(fmaxf(hi, fmaxf(v.x, v.y)), fmaxf(v.z, v.w));
+      }
+    } else {
+      for (int k = gl; k < cols; k += LPR) {
+        lo = fminf(lo, row[k]);
+        hi = fmaxf(hi, row[k]);
+      }
     }
 #pragma unroll
     for (int d = LPR / 2; d > 0; d >>= 1) {
-      lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, d));
-      hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, d));
-    }
-    const int64_t row = group + r * groups;
-    if (row >= rows) {
-      continue;
+      lo = fminf(lo, __shfl_xor_sync(mask, lo, d));
+      hi = fmaxf(hi, __shfl_xor_sync(mask, hi, d));
     }
     Coder<BITS, FP32_SB> coder;
     coder.init(lo, hi);
-    uint8_t* o = out + row * pitch;
-#pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      const int k = gl + i * LPR;
-      if (k < n4) {
-        const uint32_t c = coder.code(v[r][i].x) | (coder.code(v[r][i].y) << BITS) | (coder.code(v[r][i].z) << (2 * BITS)) |
-            (coder.code(v[r][i].w) << (3 * BITS));
+    if (cols % 4 == 0) {
+      for (int k = gl; k < cols / 4; k += LPR) {
+        const float4 v = reinterpret_cast<const float4*>(row)[k];
+        const uint32_t four =
+            coder.code(v.x) | (coder.code(v.y) << BITS) | (coder.code(v.z) << (2 * BITS)) | (coder.code(v.w) << (3 * BITS));
         if constexpr (BITS == 8) {
-          reinterpret_cast<uint32_t*>(o)[k] = c;
+          reinterpret_cast<uint32_t*>(c)[k] = four;
         } else if constexpr (BITS == 4) {
-          reinterpret_cast<uint16_t*>(o)[k] = (uint16_t)c;
+          reinterpret_cast<uint16_t*>(c)[k] = (uint16_t)four;
         } else {
-          o[k] = (uint8_t)c;
+          c[k] = (uint8_t)four;
         }
+      }
+    } else {
+      for (int b = gl; b < data_bytes; b += LPR) {
+        uint32_t packed = 0;
+#pragma unroll
+        for (int e = 0; e < EPB; ++e) {
+          packed |= coder.code(row[b * EPB + e]) << (e * BITS);
+        }
+        c[b] = (uint8_t)packed;
       }
     }
     if (gl < (FP32_SB ? 2 : 1)) {
-      uint8_t* s = o + data_bytes + 4 * gl;
-      const uint32_t w = coder.sb[FP32_SB ? gl : 0];
-      if constexpr (BITS == 8) {
-        *reinterpret_cast<uint32_t*>(s) = w;
-      } else if constexpr (BITS == 4) {
-        reinterpret_cast<uint16_t*>(s)[0] = (uint16_t)w;
-        reinterpret_cast<uint16_t*>(s)[1] = (uint16_t)(w >> 16);
-      } else {
-        store_u32_bytes(s, w);
-      }
+      store_u32_bytes(c + data_bytes + 4 * gl, coder.sb[FP32_SB ? gl : 0]);
     }
+  }
+  __syncthreads();
+
+  const int bytes = n * pitch;
+  int copied = 0;
+  if (reinterpret_cast<uintptr_t>(o) % 16 == 0) {
+    copied = bytes & ~15;
+    for (int i = 16 * threadIdx.x; i < copied; i += 16 * kQuantThreads) {
+      *reinterpret_cast<uint4*>(o + i) = *reinterpret_cast<const uint4*>(coded + i);
+    }
+  }
+  for (int i = copied + threadIdx.x; i < bytes; i += kQuantThreads) {
+    o[i] = coded[i];
   }
 }
 
@@ -191,29 +225,37 @@ quantize_row_kernel(const float* __restrict__ in, int64_t rows, int cols, uint8_
   }
 }
 
-// The vector form where rows are whole float4s and codes can be stored four columns at a time.
+// By blocks of about 16 KB of whole rows that start on 16-byte boundaries on both sides; rows too wide for that row by
+// row.  Lanes per row: as many as give every lane of the block a row to work on, so that narrow rows share a warp and
+// its divisions and exchanges (4 M rows of 32 columns: 169 us with 8 lanes per row, 136 with 4).
 template <int BITS, bool FP32_SB>
 cudaError_t launch_quantize(const float* in, int64_t rows, int cols, uint8_t* out, cudaStream_t s) {
-  const bool vector = cols % 4 == 0 && cols <= 1024 && reinterpret_cast<uintptr_t>(in) % 16 == 0 &&
-      reinterpret_cast<uintptr_t>(out) % (BITS == 8 ? 4 : BITS == 4 ? 2 : 1) == 0;
-  const int rows_per_block = !vector ? kQuantThreads / 32
-      : cols <= 32                   ? kQuantThreads / 8 * 4
-      : cols <= 64                   ? kQuantThreads / 16 * 4
-      : cols <= 128                  ? kQuantThreads / 32 * 4
-      : cols <= 256                  ? kQuantThreads / 32 * 2
-                                     : kQuantThreads / 32;
-  const int64_t blocks = (rows + rows_per_block - 1) / rows_per_block;
+  constexpr int kBlockBytes = 16384;
+  const int pitch = (int)((int64_t)cols * BITS / 8) + (FP32_SB ? 8 : 4);
+  int step = 1;  // rows after which both sides are back on a 16-byte boundary
+  while ((int64_t)step * pitch % 16 != 0 || (int64_t)step * cols % 4 != 0) {
+    step *= 2;
+  }
+  const bool by_blocks = (int64_t)step * cols * 4 <= 2 * kBlockBytes;
+  int per_block = kQuantThreads / 32;
+  if (by_blocks) {
+    per_block = kBlockBytes / (4 * cols) / step * step;
+    per_block = per_block < step ? step : per_block > 512 ? 512 : per_block;
+  }
+  const int64_t blocks = (rows + per_block - 1) / per_block;
   if (blocks <= 0 || blocks > 0x7fffffffLL) {
     return cudaErrorInvalidValue;
   }
-  void (*fn)(const float*, int64_t, int, uint8_t*) = !vector ? quantize_row_kernel<BITS, FP32_SB>
-      : cols <= 32                                           ? quantize_vector_kernel<BITS, FP32_SB, 8, 1, 4>
-      : cols <= 64                                           ? quantize_vector_kernel<BITS, FP32_SB, 16, 1, 4>
-      : cols <= 128                                          ? quantize_vector_kernel<BITS, FP32_SB, 32, 1, 4>
-      : cols <= 256                                          ? quantize_vector_kernel<BITS, FP32_SB, 32, 2, 2>
-      : cols <= 512                                          ? quantize_vector_kernel<BITS, FP32_SB, 32, 4, 1>
-                                                             : quantize_vector_kernel<BITS, FP32_SB, 32, 8, 1>;
-  fn<<<(unsigned)blocks, kQuantThreads, 0, s>>>(in, rows, cols, out);
+  if (by_blocks) {
+    const int smem = per_block * (4 * cols + pitch);  // 44 KB at most: 32 KB and its codes, or 16 KB and theirs
+    (per_block >= 64         ? quantize_block_kernel<BITS, FP32_SB, 4>
+         : per_block > 16 ? quantize_block_kernel<BITS, FP32_SB, 8>
+         : per_block > 8  ? quantize_block_kernel<BITS, FP32_SB, 16>
+                          : quantize_block_kernel<BITS, FP32_SB, 32>)
+        <<<(unsigned)blocks, kQuantThreads, smem, s>>>(in, rows, cols, out, per_block);
+  } else {
+    quantize_row_kernel<BITS, FP32_SB><<<(unsigned)blocks, kQuantThreads, 0, s>>>(in, rows, cols, out);
+  }
   g_launch_count.fetch_add(1, std::memory_order_relaxed);
   return cudaGetLastError();
 }

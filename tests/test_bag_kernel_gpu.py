@@ -113,3 +113,23 @@ def test_more_tables_than_one_launch_takes(gpu_ctx, oracle):
     for c, ref in zip(calls, want):
         np.testing.assert_array_equal(bits(c[8].cpu().numpy()), bits(ref))
     plan.close()
+
+
+@pytest.mark.parametrize("cols", [4, 7, 8, 33, 64, 100, 129, 256, 300, 512, 520, 1024, 1032, 2052])
+def test_quantizer_blocks(gpu_ctx, oracle, cols):
+    """Widths around the choices of rows per block and lanes per row, row counts around a block, and tables that start
+    off a 16-byte boundary."""
+    rng = np.random.default_rng(cols)
+    for rows in (1, 17, 300):
+        x = rng.standard_normal((rows, cols)).astype(np.float32)
+        x[0] = 1.5  # no range
+        for off in (0, 1):
+            src = torch.empty(rows * cols + 4, device="cuda")[off:off + rows * cols].view(rows, cols)
+            src.copy_(torch.from_numpy(x))
+            out = torch.empty(rows * (cols + 8) + 8, dtype=torch.uint8, device="cuda")[off:off + rows * (cols + 8)]
+            got = F.FloatToFused8BitRowwiseQuantizedSBFloat(src, out.view(rows, cols + 8)).cpu().numpy()
+            np.testing.assert_array_equal(got, oracle.quantize_8bit(x))
+        for b in (4, 2):
+            if cols % (8 // b) == 0:
+                got = F.FloatToFusedNBitRowwiseQuantizedSBHalf(b, dev(x)).cpu().numpy()
+                np.testing.assert_array_equal(got, oracle.quantize_nbit(b, x))
