@@ -5,6 +5,7 @@
 #include <mutex>
 #include <unordered_map>
 
+#include "host_copy.h"
 #include "internal.h"
 
 namespace fbgemm_b200 {
@@ -62,10 +63,12 @@ struct Lane {
   PinnedBuffer h_status;
   bool busy = false;
   // what to do at wait()
-  static constexpr int kMaxPieces = 16;
-  cudaEvent_t piece_done[kMaxPieces] = {};  // rows in pageable memory come down in pieces
+  static constexpr int kMaxPieces = kCopyParts;
+  cudaStream_t up = nullptr;                // uploads of a call that goes in parts
+  cudaEvent_t piece_up[kMaxPieces] = {};
+  cudaEvent_t piece_done[kMaxPieces] = {};  // rows for pageable memory come down in pieces
   int pieces = 0;
-  size_t piece_bytes = 0;
+  size_t piece_end[kMaxPieces] = {};        // bytes
   void* user_out = nullptr;
   size_t out_row_bytes = 0;   // bytes of one pooled row (block_size elements)
   size_t out_pitch_bytes = 0; // bytes between rows in the user's buffer

@@ -4,6 +4,10 @@
 // call's copy copies alone.
 #include "host_copy.h"
 
+#if defined(__x86_64__)
+#include <emmintrin.h>
+#endif
+
 #include <atomic>
 #include <chrono>
 #include <condition_variable>
@@ -17,6 +21,7 @@ namespace fbgemm_b200 {
 namespace {
 
 constexpr int kHelpers = 3;
+constexpr size_t kWorthHelp = 512 * 1024;  // waking the helpers costs the copy of a few hundred KB
 constexpr auto kIdle = std::chrono::seconds(1);
 
 class Helpers {
@@ -32,22 +37,45 @@ class Helpers {
     }
   }
 
-  bool copy(const CopySlice* slices, int count, const std::function<bool(int)>& ready) {
+  bool copy(const CopySlice* slices, int count, int parts, bool ahead, const std::function<bool(int)>& ready,
+            const std::function<bool(int)>& done) {
     // One copy at a time has the helpers.
     std::unique_lock<std::mutex> mine(in_use_, std::try_to_lock);
-    const bool helped = mine.owns_lock() && count > 1 && open(slices, count);
-    bool ok = true;
-    int next = 0;  // without helpers
+    size_t bytes = 0;
     for (int i = 0; i < count; ++i) {
-      ok = ready(i);
-      if (!ok) {
-        break;
+      bytes += slices[i].bytes;
+    }
+    const bool helped = mine.owns_lock() && bytes >= kWorthHelp && open(slices, count, ahead ? count : 0);
+    bool ok = true;
+    int end = 0;  // slices of the parts so far
+    for (int p = 0; p < parts && ok; ++p) {
+      if (!ahead && ready) {
+        ok = ready(p);
+        if (!ok) {
+          break;
+        }
+      }
+      const int begin = end;
+      while (end < count && slices[end].part <= p) {
+        ++end;
       }
       if (helped) {
-        ready_.store(i + 1, std::memory_order_release);
+        if (!ahead) {
+          ready_.store(end, std::memory_order_release);
+        }
+        if (done) {
+          while (left_[p].load(std::memory_order_acquire) > 0) {
+            if (!claim_one()) {
+              pause();
+            }
+          }
+        }
       } else {
-        take(slices[next++]);
+        for (int i = begin; i < end; ++i) {
+          take(slices[i]);
+        }
       }
+      ok = !done || done(p);
     }
     if (helped) {
       while (claim_one()) {
@@ -58,7 +86,35 @@ class Helpers {
   }
 
  private:
-  static void take(const CopySlice& s) { std::memcpy(s.dst, s.src, s.bytes); }
+  // Past the caches: neither side of the copy is read again from them, and the lines of the destination need not be
+  // fetched first (253 -> 218 us for the call of 10 000 bags below).
+  static void take(const CopySlice& s) {
+    size_t done = 0;
+#if defined(__x86_64__)
+    if (reinterpret_cast<uintptr_t>(s.dst) % 16 == 0) {
+      const __m128i* from = static_cast<const __m128i*>(s.src);
+      __m128i* to = static_cast<__m128i*>(s.dst);
+      for (; done + 64 <= s.bytes; done += 64, from += 4, to += 4) {
+        const __m128i a = _mm_loadu_si128(from), b = _mm_loadu_si128(from + 1);
+        const __m128i c = _mm_loadu_si128(from + 2), d = _mm_loadu_si128(from + 3);
+        _mm_stream_si128(to, a);
+        _mm_stream_si128(to + 1, b);
+        _mm_stream_si128(to + 2, c);
+        _mm_stream_si128(to + 3, d);
+      }
+      _mm_sfence();
+    }
+#endif
+    std::memcpy(static_cast<char*>(s.dst) + done, static_cast<const char*>(s.src) + done, s.bytes - done);
+  }
+
+  static void pause() {
+#if defined(__x86_64__)
+    __builtin_ia32_pause();
+#else
+    std::this_thread::yield();
+#endif
+  }
 
   // Takes the next slice that is ready; false if there is none.
   bool claim_one() {
@@ -66,13 +122,14 @@ class Helpers {
     while (i < ready_.load(std::memory_order_acquire)) {
       if (claimed_.compare_exchange_weak(i, i + 1, std::memory_order_acq_rel)) {
         take(slices_[i]);
+        left_[slices_[i].part].fetch_sub(1, std::memory_order_acq_rel);
         return true;
       }
     }
     return false;
   }
 
-  bool open(const CopySlice* slices, int count) {
+  bool open(const CopySlice* slices, int count, int ready) {
     std::lock_guard<std::mutex> l(mu_);
     if (stop_) {
       return false;
@@ -93,9 +150,14 @@ class Helpers {
       return false;
     }
     slices_ = slices;
-    (void)count;
+    for (auto& l : left_) {
+      l.store(0, std::memory_order_relaxed);
+    }
+    for (int i = 0; i < count; ++i) {
+      left_[slices[i].part].fetch_add(1, std::memory_order_relaxed);
+    }
     claimed_.store(0, std::memory_order_relaxed);
-    ready_.store(0, std::memory_order_relaxed);
+    ready_.store(ready, std::memory_order_release);
     open_.store(true, std::memory_order_release);
     wake_.notify_all();
     return true;
@@ -135,11 +197,7 @@ class Helpers {
       l.unlock();
       while (open_.load(std::memory_order_acquire)) {
         if (!claim_one()) {
-#if defined(__x86_64__)
-          __builtin_ia32_pause();
-#else
-          std::this_thread::yield();
-#endif
+          pause();
         }
       }
       l.lock();
@@ -158,14 +216,16 @@ class Helpers {
   int busy_ = 0;
   std::atomic<bool> open_{false};
   std::atomic<int> claimed_{0}, ready_{0};
+  std::atomic<int> left_[kCopyParts] = {};  // slices of each part that are not copied yet
   const CopySlice* slices_ = nullptr;
 };
 
 }  // namespace
 
-bool copy_slices(const CopySlice* slices, int count, const std::function<bool(int)>& ready) {
+bool copy_slices(const CopySlice* slices, int count, int parts, bool ahead, const std::function<bool(int)>& ready,
+                 const std::function<bool(int)>& done) {
   static Helpers helpers;
-  return helpers.copy(slices, count, ready);
+  return helpers.copy(slices, count, parts, ahead, ready, done);
 }
 
 }  // namespace fbgemm_b200

@@ -4,7 +4,7 @@
 // One thread copies at about 17 GB/s, a third of what the link moves: the 5.1 MB
 // of rows of a 10 000-bag call took 300 us to leave the staging block after a
 // transfer of 93 us.  A few helpers bring the copy down to the transfer's time,
-// and slices are copied while later ones are still on their way.
+// and the transfers of a call's parts overlap the copies of the others.
 #pragma once
 
 #include <cstddef>
@@ -16,11 +16,15 @@ struct CopySlice {
   void* dst;
   const void* src;
   size_t bytes;
+  int part;  // 0, 1, ... < kCopyParts, not decreasing from slice to slice
 };
+constexpr int kCopyParts = 16;
 
-// Copies all slices, in order of arrival: slice i is copied once ready(i) has
-// returned, which is called on the calling thread for i = 0, 1, ... (and may
-// wait; false ends the whole copy early).  Returns false if ready() did.
-bool copy_slices(const CopySlice* slices, int count, const std::function<bool(int)>& ready);
+// Copies all slices.  Before the slices of part p are copied ready(p) is called, and once they are copied done(p), both
+// on the calling thread, part after part (a part may have no slices); they return false to end the whole copy early.
+// With `ahead` the slices of all parts may be copied at once (ready() is not called), otherwise only those of parts
+// that are ready.  Returns false if a callback did.
+bool copy_slices(const CopySlice* slices, int count, int parts, bool ahead, const std::function<bool(int)>& ready,
+                 const std::function<bool(int)>& done);
 
 }  // namespace fbgemm_b200

@@ -133,3 +133,43 @@ def test_quantizer_blocks(gpu_ctx, oracle, cols):
             if cols % (8 // b) == 0:
                 got = F.FloatToFusedNBitRowwiseQuantizedSBHalf(b, dev(x)).cpu().numpy()
                 np.testing.assert_array_equal(got, oracle.quantize_nbit(b, x))
+
+
+@pytest.mark.parametrize("dim,out_dt,weighting", [(128, np.float32, "unweighted"), (64, np.float16, "weighted"),
+                                                  (86, np.float16, "weighted"), (128, np.float32, "positional")])
+def test_pageable_calls_in_parts(gpu_ctx, oracle, dim, out_dt, weighting):
+    """Host arrays large enough to go up, through the lookup and down in parts of consecutive bags, some of them without
+    any index; calls whose offsets do not cover the indices, or step back, return false."""
+    rng = np.random.default_rng(dim)
+    rows, batch = 3000, 30_001
+    table = random_fused_table(rng, rows, dim, 8)
+    lengths = rng.integers(0, 30, batch)
+    lengths[5000:20000] = 0
+    n = int(lengths.sum())
+    indices = rng.integers(0, rows, n)
+    offsets = np.concatenate([[0], np.cumsum(lengths)]).astype(np.int64)
+    w = rng.standard_normal(n).astype(np.float32)
+    positional = weighting == "positional"
+    kern = F.GenerateEmbeddingSpMDMWithStrides(dim, weighting != "unweighted", True, 16, positional, True,
+                                               index_dtype=np.int64, offset_dtype=np.int64, out_dtype=out_dt)
+    ok_ref, ref = oracle.spmdm(8, dim, rows, table, indices, offsets, w if weighting != "unweighted" else None, True, out_dt,
+                               positional, True, output_size=batch, index_size=n)
+    out = np.zeros(batch * dim, dtype=out_dt)
+    gpu_ctx.register_table(table)
+    for _ in range(2):
+        out[:] = 0
+        assert kern(batch, n, rows, table, indices, offsets, w, out) and ok_ref
+        np.testing.assert_array_equal(bits(out), bits(ref[:batch * dim]))
+    for bad in (n - 1, n + 1):
+        o = offsets.copy()
+        o[-1] = bad
+        assert not kern(batch, n, rows, table, indices, o, w, out)
+    o = offsets.copy()
+    o[batch // 2] = n
+    assert not kern(batch, n, rows, table, indices, o, w, out)
+    i = indices.copy()
+    i[n // 2] = rows
+    assert not kern(batch, n, rows, table, i, offsets, w, out)
+    assert kern(batch, n, rows, table, indices, offsets, w, out)
+    np.testing.assert_array_equal(bits(out), bits(ref[:batch * dim]))
+    gpu_ctx.unregister_table(table)
