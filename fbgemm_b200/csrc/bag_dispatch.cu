@@ -74,7 +74,7 @@ void bag_table_of(const SpmdmParams& p, BagTable* t) {
 int form_of(const BagTable& t) {
   const bool wide = (unsigned __int128)t.data_size * (uint64_t)t.stride > 0xffffffffull || t.bags > 0x7fffff00LL ||
       t.index_size > 0x7fffff00LL;
-  const bool options = t.flags & (kPruned | kSbFirst | kNoBag | kPositional);
+  const bool options = t.flags & (kPruned | kSbFirst | kNoBag | kPositional | kLengths);
   return wide ? bag::kWide : options || t.data_size == 0 ? bag::kFull : bag::kLean;
 }
 

@@ -384,7 +384,8 @@ struct __align__(16) Queue {
 
 // What a kernel is compiled for.
 //  kLean  bags by offsets, weights per index, every index a row of the table
-//  kFull  besides: pruning maps, -1 as a pruned index, no_bag, positional weights
+//  kFull  besides: pruning maps, -1 as a pruned index, no_bag, positional
+//         weights, lengths in place of offsets
 //  kWide  the same where positions, bags (31 bits) or row offsets (32) need more
 // The lean form saves the queue's compaction and half of the tests, a tenth of
 // the time of 65536 bags of 30 rows (8-bit D = 128 76.4 against 83.6 us).
@@ -401,6 +402,50 @@ __host__ __device__ constexpr int rows_ahead(int fmt, int g, bool deep) {
 // The stream's next launch may be set up while this one drains; it waits here until all results of this one are there.
 __device__ __forceinline__ void wait_for_previous_launch() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void let_next_launch_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// Where a bag starts, from the lengths alone (kLengths): the block adds up those of all bags before its own, coalesced
+// and from L2, then every lane those between.
+template <int G>
+__device__ __forceinline__ void bag_from_lengths(const BagTable& p, int64_t first, int64_t bag, int64_t& start, int& length) {
+  __shared__ long long sums[kWarps];
+  const bool is64 = p.flags & kOff64;
+  auto at = [&](int64_t i) {
+    const int v = (int)load_int(p.offsets, i, is64);  // the reference narrows to 32 bits too
+    return v < 0 ? 0 : v;
+  };
+  long long sum = 0;
+#pragma unroll 4
+  for (int64_t i = threadIdx.x; i < first; i += kThreads) {
+    sum += at(i);
+  }
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) {
+    sum += __shfl_xor_sync(0xffffffffu, sum, d);
+  }
+  if (threadIdx.x % 32 == 0) {
+    sums[threadIdx.x / 32] = sum;
+  }
+  __syncthreads();
+  sum = 0;
+#pragma unroll
+  for (int i = 0; i < kWarps; ++i) {
+    sum += sums[i];
+  }
+  if (first + kWarps * (32 / G) >= p.bags && threadIdx.x == 0) {  // the last block: `return current == index_size`
+    long long total = sum;
+    for (int64_t i = first; i < p.bags; ++i) {
+      total += at(i);
+    }
+    if (total != p.index_size) {
+      report(p.status, FBGEMM_B200_STATUS_SIZE_MISMATCH, p.bags, total, p.index_size);
+    }
+  }
+  for (int64_t i = first; i < bag && i < p.bags; ++i) {
+    sum += at(i);
+  }
+  start = sum;
+  length = bag < p.bags ? at(bag) : 0;
+}
 
 // One block's work on table `p`: bags block * kWarps * (32 / G) onwards, columns of tile `tile` of the row.
 template <int FMT, int VB, int CPL, int G, int MODE, bool kDeep>
@@ -425,6 +470,7 @@ __device__ __forceinline__ void pool_bags(const BagTable& p, void* const* peers,
   const bool positional = FULL && (p.flags & kPositional);
   const bool pruned = FULL && (p.flags & kPruned);
   const bool no_bag = FULL && (p.flags & kNoBag);
+  const bool by_lengths = FULL && (p.flags & kLengths);
   const bool minus_one_skips = FULL && FMT != kFp8 && (p.flags & (kSbFirst | kNoBag)) == kSbFirst;
   const bool half_sb = FMT != kInt8 || (p.flags & kSbFirst);
 
@@ -439,24 +485,28 @@ __device__ __forceinline__ void pool_bags(const BagTable& p, void* const* peers,
   Pos pos = 0;  // of this lane's next candidate: one in every G indices of the bag
   int len = 0;
   {
-    // rebasing to offsets[0] (the functor's convention) unless the offsets are absolute
-    const bool rebase = !(p.flags & (kNoBag | kAbsOffsets));
-    const int64_t off_base = rebase ? load_int(p.offsets, 0, off64) : 0;
-    if (block == 0 && threadIdx.x == 0 && rebase) {
-      // `return current == index_size` of the reference
-      const int64_t total = load_int(p.offsets, p.bags, off64) - off_base;
-      if (total != p.index_size) {
-        report(p.status, FBGEMM_B200_STATUS_SIZE_MISMATCH, p.bags, total, p.index_size);
-      }
-    }
     int64_t start = 0;
     int bag_len = 0;
-    if (bag < (Pos)p.bags) {
-      // no_bag: output row m is the single row indices[m]
-      const int64_t o0 = no_bag ? bag : load_int(p.offsets, bag, off64);
-      const int64_t o1 = no_bag ? (int64_t)bag + 1 : load_int(p.offsets, (int64_t)bag + 1, off64);
-      start = o0 - off_base;
-      bag_len = (int)(o1 - o0);  // the reference narrows to 32 bits too
+    if (by_lengths) {
+      bag_from_lengths<G>(p, (int64_t)block * (kWarps * (32 / G)), bag, start, bag_len);
+    } else {
+      // rebasing to offsets[0] (the functor's convention) unless the offsets are absolute
+      const bool rebase = !(p.flags & (kNoBag | kAbsOffsets));
+      const int64_t off_base = rebase ? load_int(p.offsets, 0, off64) : 0;
+      if (block == 0 && threadIdx.x == 0 && rebase) {
+        // `return current == index_size` of the reference
+        const int64_t total = load_int(p.offsets, p.bags, off64) - off_base;
+        if (total != p.index_size) {
+          report(p.status, FBGEMM_B200_STATUS_SIZE_MISMATCH, p.bags, total, p.index_size);
+        }
+      }
+      if (bag < (Pos)p.bags) {
+        // no_bag: output row m is the single row indices[m]
+        const int64_t o0 = no_bag ? bag : load_int(p.offsets, bag, off64);
+        const int64_t o1 = no_bag ? (int64_t)bag + 1 : load_int(p.offsets, (int64_t)bag + 1, off64);
+        start = o0 - off_base;
+        bag_len = (int)(o1 - o0);  // the reference narrows to 32 bits too
+      }
     }
     // Offsets that step backwards: the reference, which walks the index array
     // with a running position, ends up past index_size and returns false.
@@ -640,7 +690,8 @@ __device__ __forceinline__ void pool_bags(const BagTable& p, void* const* peers,
   }
   int bag_len = 0;
   if (p.flags & kNormalize) {
-    bag_len = (int)(load_int(p.offsets, (int64_t)bag + 1, off64) - load_int(p.offsets, bag, off64));
+    bag_len = by_lengths ? (int)load_int(p.offsets, bag, off64)
+                         : (int)(load_int(p.offsets, (int64_t)bag + 1, off64) - load_int(p.offsets, bag, off64));
   }
   if (bag_len != 0) {
     const float inv = __fdiv_rn(1.f, (float)bag_len);

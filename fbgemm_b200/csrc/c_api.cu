@@ -334,6 +334,10 @@ int fbgemm_b200::enqueue_lookup(
   } else if (cfg->use_offsets) {
     p.offsets = offsets_or_lengths;
     flags |= cfg->offset_bytes == 8 ? kOff64 : 0;
+  } else if (output_size <= kMaxBagsByLengths &&
+             g_kernel_choice.load(std::memory_order_relaxed) == FBGEMM_B200_KERNEL_AUTO) {
+    p.offsets = offsets_or_lengths;
+    flags |= kLengths | (cfg->offset_bytes == 8 ? kOff64 : 0);
   } else {
     // lengths -> int64 offsets in scratch
     const size_t need = ((size_t)output_size + 1 + scan_scratch_elems(output_size)) * sizeof(int64_t);

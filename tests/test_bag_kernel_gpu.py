@@ -173,3 +173,24 @@ def test_pageable_calls_in_parts(gpu_ctx, oracle, dim, out_dt, weighting):
     assert kern(batch, n, rows, table, indices, offsets, w, out)
     np.testing.assert_array_equal(bits(out), bits(ref[:batch * dim]))
     gpu_ctx.unregister_table(table)
+
+
+@pytest.mark.parametrize("batch", [1, 3, 33, 5000, 12_288, 12_289])
+def test_lengths_without_a_scan(gpu_ctx, oracle, batch):
+    rng = np.random.default_rng(batch)
+    rows, dim = 400, 64
+    table = random_fused_table(rng, rows, dim, 4)
+    lengths = rng.integers(0, 6, batch)
+    lengths[rng.integers(0, batch, 3)] = 40
+    n = int(lengths.sum())
+    indices = rng.integers(0, rows, n).astype(np.int32)
+    w = rng.standard_normal(n).astype(np.float32)
+    for odt in (np.int32, np.int64):
+        kern = F.GenerateEmbeddingSpMDMNBit(4, dim, True, True, use_offsets=False, index_dtype=np.int32, offset_dtype=odt)
+        ok_ref, ref = oracle.spmdm(4, dim, rows, table, indices, lengths.astype(odt), w, True, np.float32, False, False,
+                                   output_size=batch, index_size=n)
+        out = torch.zeros(batch * dim, device="cuda")
+        args = (dev(table), dev(indices), dev(lengths.astype(odt)), dev(w), out)
+        assert kern(batch, n, rows, *args) and ok_ref
+        np.testing.assert_array_equal(bits(out.cpu().numpy()), bits(ref))
+        assert not kern(batch, n - 1, rows, *args)       # the lengths do not add up to index_size
