@@ -187,7 +187,8 @@ struct UnitsLaunch {
 MultiPlan::MultiPlan() = default;
 MultiPlan::~MultiPlan() = default;
 
-// One launch takes up to kMaxUnits column tiles of tables of any row formats.
+// One launch takes up to kMaxTables tables of any row formats with kMaxUnits
+// column tiles in all.
 cudaError_t build_multi_plan(const SpmdmParams* tables, const int* bit_rates, size_t count, MultiPlan* plan) {
   int64_t bags = 0;
   for (size_t t = 0; t < count; ++t) {
@@ -222,6 +223,7 @@ cudaError_t build_multi_plan(const SpmdmParams* tables, const int* bit_rates, si
   std::stable_sort(order.begin(), order.end(), [](const Unit& a, const Unit& b) {
     return a.form != b.form ? a.form > b.form : a.work > b.work;
   });
+  std::vector<int> place(count);  // of a table in the launch being filled
   for (size_t i = 0; i < order.size();) {
     plan->launches.emplace_back(new UnitsLaunch);
     UnitsLaunch& l = *plan->launches.back();
@@ -229,15 +231,23 @@ cudaError_t build_multi_plan(const SpmdmParams* tables, const int* bit_rates, si
     u.count = 0;
     l.form = order[i].form;
     int64_t blocks = 0;
+    int tables_in = 0;
+    std::fill(place.begin(), place.end(), -1);
     for (; i < order.size() && order[i].form == l.form && u.count < bag::kMaxUnits &&
          blocks + order[i].blocks <= 0x7fffffffLL; ++i) {
+      int& at = place[order[i].table];
+      if (at < 0) {
+        if (tables_in == bag::kMaxTables) {
+          break;
+        }
+        at = tables_in++;
+        const SpmdmParams& p = tables[order[i].table];
+        u.t[at] = bag_tables[order[i].table];
+        std::copy(p.peer_out, p.peer_out + p.num_peers, u.peers[at]);
+      }
       const int k = u.count++;
-      const SpmdmParams& p = tables[order[i].table];
       u.first_block[k] = (int32_t)blocks;
-      u.variant[k] = (uint16_t)order[i].variant;
-      u.tile[k] = (uint16_t)order[i].tile;
-      u.t[k] = bag_tables[order[i].table];
-      std::copy(p.peer_out, p.peer_out + p.num_peers, u.peers[k]);
+      u.unit[k] = {(uint8_t)order[i].variant, (uint8_t)at, (uint16_t)order[i].tile};
       blocks += order[i].blocks;
     }
     u.first_block[u.count] = (int32_t)blocks;

@@ -781,15 +781,18 @@ enum VariantId : int { FBGEMM_B200_BAG_VARIANTS(FBGEMM_B200_BAG_ID) kVariants };
 // unit u - one column tile of one table - owns the blocks [first_block[u],
 // first_block[u + 1]), whatever the tables' row formats.  The units arrive by
 // value, in constant memory; a block finds its own by bisection.
-constexpr int kMaxUnits = 64;
+constexpr int kMaxUnits = 128, kMaxTables = 64;
 struct BagUnits {
   int32_t count;
   int32_t first_block[kMaxUnits + 1];
-  uint16_t variant[kMaxUnits];
-  uint16_t tile[kMaxUnits];
-  BagTable t[kMaxUnits];
-  void* peers[kMaxUnits][FBGEMM_B200_MAX_PEERS];
+  struct Unit {
+    uint8_t variant, table;
+    uint16_t tile;
+  } unit[kMaxUnits];
+  BagTable t[kMaxTables];
+  void* peers[kMaxTables][FBGEMM_B200_MAX_PEERS];
 };
+static_assert(kVariants <= 256, "a variant is a byte");
 static_assert(sizeof(BagUnits) < 32764, "one kernel argument");
 
 template <int MODE>
@@ -804,12 +807,13 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm) bag_units_kernel(const
       hi = mid;
     }
   }
-  const BagTable& t = a.t[lo];
+  const BagUnits::Unit u = a.unit[lo];
+  const BagTable& t = a.t[u.table];
   const uint32_t block = blockIdx.x - a.first_block[lo];
-  switch (a.variant[lo]) {
+  switch (u.variant) {
 #define FBGEMM_B200_BAG_CASE(FMT, VB, CPL, G)                                   \
   case id_##FMT##_##VB##_##CPL##_##G:                                                  \
-    pool_bags<FMT, VB, CPL, G, MODE, false>(t, a.peers[lo], block, a.tile[lo], queues); \
+    pool_bags<FMT, VB, CPL, G, MODE, false>(t, a.peers[u.table], block, u.tile, queues); \
     break;
     FBGEMM_B200_BAG_VARIANTS(FBGEMM_B200_BAG_CASE)
 #undef FBGEMM_B200_BAG_CASE

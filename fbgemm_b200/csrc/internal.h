@@ -113,7 +113,7 @@ cudaError_t launch_spmdm(const SpmdmParams& p, int bit_rate, cudaStream_t stream
 // The bag kernel for this lookup (bag_dispatch.cu).
 cudaError_t launch_bags(const SpmdmParams& p, int bit_rate, cudaStream_t stream);
 
-// Several tables per call (bag_dispatch.cu): up to 64 column tiles of tables of
+// Several tables per call (bag_dispatch.cu): up to 64 tables (128 column tiles) of
 // any row formats per launch.  Built for a fixed set of pointers, launched as
 // often as wanted.
 struct UnitsLaunch;
