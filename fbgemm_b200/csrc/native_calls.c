@@ -111,10 +111,60 @@ static PyObject* table_set_forward(PyObject* self, PyObject* const* args, Py_ssi
   return PyLong_FromLong(fbgemm_b200_table_set_forward(set, bags, indices, index_size, t[0], t[1], t[2], (int)slot, stream));
 }
 
+/* quantize(bit_rate, x, rows, cols, out, stream); bit_rate 0: 8-bit rows with fp32 scale and bias */
+static PyObject* quantize(PyObject* self, PyObject* const* args, Py_ssize_t n) {
+  (void)self;
+  int64_t bits, size[2];
+  void *x, *t[2];
+  if (arity(n, 6) || integers(args, 0, 1, &bits) || addresses(args, 1, 1, &x) || integers(args, 2, 2, size) ||
+      addresses(args, 4, 2, t)) {
+    return NULL;
+  }
+  return PyLong_FromLong(bits == 0 ? fbgemm_b200_float_to_fused_8bit_rowwise(x, size[0], (int32_t)size[1], t[0], t[1])
+                                   : fbgemm_b200_float_to_fused_nbit_rowwise((int32_t)bits, x, size[0], (int32_t)size[1], t[0],
+                                                                             t[1]));
+}
+
+/* pruned_lookup(hashmap, ctx, T, B, indices, offsets, index_bytes, index_size, map, map_bytes, map_offsets, dense, slot,
+ * stream) */
+static PyObject* pruned_lookup(PyObject* self, PyObject* const* args, Py_ssize_t n) {
+  (void)self;
+  int64_t hashmap, size[2], index[2], map_bytes, slot;
+  void *ctx, *in[2], *map, *t[2], *stream;
+  if (arity(n, 14) || integers(args, 0, 1, &hashmap) || addresses(args, 1, 1, &ctx) || integers(args, 2, 2, size) ||
+      addresses(args, 4, 2, in) || integers(args, 6, 2, index) || addresses(args, 8, 1, &map) ||
+      integers(args, 9, 1, &map_bytes) || addresses(args, 10, 2, t) || integers(args, 12, 1, &slot) ||
+      addresses(args, 13, 1, &stream)) {
+    return NULL;
+  }
+  return PyLong_FromLong((hashmap ? fbgemm_b200_pruned_hashmap_lookup : fbgemm_b200_pruned_array_lookup)(
+      ctx, (int32_t)size[0], (int32_t)size[1], in[0], in[1], (int32_t)index[0], index[1], map, (int32_t)map_bytes, t[0], t[1],
+      (int32_t)slot, stream));
+}
+
+/* sequence_lookup(filled, ctx, weights, tables, T, B, D, indices, offsets, index_bytes, index_size, out, out_dtype,
+ * out_row_bytes, scale_bias_last, fp8_exponent_bits, fp8_exponent_bias, slot, stream) */
+static PyObject* sequence_lookup(PyObject* self, PyObject* const* args, Py_ssize_t n) {
+  (void)self;
+  int64_t filled, size[3], index[2], out[6];
+  void *t[3], *in[2], *rows, *stream;
+  if (arity(n, 19) || integers(args, 0, 1, &filled) || addresses(args, 1, 3, t) || integers(args, 4, 3, size) ||
+      addresses(args, 7, 2, in) || integers(args, 9, 2, index) || addresses(args, 11, 1, &rows) ||
+      integers(args, 12, 6, out) || addresses(args, 18, 1, &stream)) {
+    return NULL;
+  }
+  return PyLong_FromLong((filled ? fbgemm_b200_sequence_lookup_filled : fbgemm_b200_sequence_lookup)(
+      t[0], t[1], t[2], (int32_t)size[0], (int32_t)size[1], (int32_t)size[2], in[0], in[1], (int32_t)index[0], index[1], rows,
+      (int32_t)out[0], out[1], (int32_t)out[2], (int32_t)out[3], (int32_t)out[4], (int32_t)out[5], stream));
+}
+
 static PyMethodDef methods[] = {
     {"spmdm_launch", (PyCFunction)(void (*)(void))spmdm_launch, METH_FASTCALL, "fbgemm_b200_spmdm_launch"},
     {"spmdm", (PyCFunction)(void (*)(void))spmdm, METH_FASTCALL, "fbgemm_b200_spmdm"},
     {"table_set_forward", (PyCFunction)(void (*)(void))table_set_forward, METH_FASTCALL, "fbgemm_b200_table_set_forward"},
+    {"quantize", (PyCFunction)(void (*)(void))quantize, METH_FASTCALL, "fbgemm_b200_float_to_fused_*_rowwise"},
+    {"pruned_lookup", (PyCFunction)(void (*)(void))pruned_lookup, METH_FASTCALL, "fbgemm_b200_pruned_*_lookup"},
+    {"sequence_lookup", (PyCFunction)(void (*)(void))sequence_lookup, METH_FASTCALL, "fbgemm_b200_sequence_lookup*"},
     {NULL, NULL, 0, NULL}};
 
 static struct PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native_calls", NULL, -1, methods, NULL, NULL, NULL, NULL};

@@ -549,6 +549,17 @@ def GenerateEmbeddingSpMDMNBitRowWiseSparse(bit_rate, block_size, has_weight, no
 
 # ---- quantizers (device tensors) ---------------------------------------------
 
+def _quantize(bit_rate, x, out, what) -> None:
+    import torch
+
+    dev = x.get_device()
+    if dev != torch.cuda.current_device():
+        with torch.cuda.device(dev):
+            return _quantize(bit_rate, x, out, what)
+    rows, cols = x.shape
+    _capi.check(_capi.native().quantize(bit_rate, x, rows, cols, out, _current_stream(dev)), what)
+
+
 def FloatToFused8BitRowwiseQuantizedSBFloat(x, out=None):
     """fbgemm::FloatOrHalfToFused8BitRowwiseQuantizedSBFloat<float>
     (include/fbgemm/QuantUtils.h:312) on a CUDA fp32 tensor [rows, cols] ->
@@ -559,10 +570,7 @@ def FloatToFused8BitRowwiseQuantizedSBFloat(x, out=None):
     rows, cols = x.shape
     if out is None:
         out = torch.empty((rows, cols + 8), dtype=torch.uint8, device=x.device)
-    with torch.cuda.device(x.device):
-        stream = torch.cuda.current_stream().cuda_stream
-        _capi.check(_capi.lib().fbgemm_b200_float_to_fused_8bit_rowwise(
-            x.data_ptr(), rows, cols, out.data_ptr(), stream), "8-bit quantizer")
+    _quantize(0, x, out, "8-bit quantizer")
     return out
 
 
@@ -579,10 +587,7 @@ def FloatToFusedNBitRowwiseQuantizedSBHalf(bit_rate, x, out=None):
         raise ValueError("Unsupported number of columns")  # src/QuantUtils.cc:624-627
     if out is None:
         out = torch.empty((rows, cols // epb + 4), dtype=torch.uint8, device=x.device)
-    with torch.cuda.device(x.device):
-        stream = torch.cuda.current_stream().cuda_stream
-        _capi.check(_capi.lib().fbgemm_b200_float_to_fused_nbit_rowwise(
-            bit_rate, x.data_ptr(), rows, cols, out.data_ptr(), stream), "N-bit quantizer")
+    _quantize(bit_rate, x, out, "N-bit quantizer")
     return out
 
 

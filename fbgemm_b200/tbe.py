@@ -231,12 +231,12 @@ def _pruned_lookup(fn_name, indices, offsets, mapping, mapping_offsets, slot):
     B = (offsets.numel() - 1) // T
     if B <= 0:
         raise ValueError("B must be positive")
-    ctx = E.get_context(indices.device.index)
     dense = torch.empty_like(indices)
-    fn = getattr(E._capi.lib(), fn_name)
-    rc = fn(ctx.handle, T, B, E._ptr(indices), E._ptr(offsets), indices.element_size(), indices.numel(),
-            E._ptr(mapping), mapping.element_size(), E._ptr(mapping_offsets), E._ptr(dense), slot,
-            torch.cuda.current_stream(indices.device).cuda_stream)
+    dev = indices.get_device()
+    rc = E._capi.native().pruned_lookup(
+        int(fn_name == "fbgemm_b200_pruned_hashmap_lookup"), E._handle_of(dev), T, B, indices, offsets,
+        indices.element_size(), indices.numel(), mapping, mapping.element_size(), mapping_offsets, dense, slot,
+        E._current_stream(dev))
     E._capi.check(rc, fn_name)
     return dense
 
@@ -371,21 +371,18 @@ class IntNBitSequenceEmbedding:
         assert (offsets.numel() - 1) % self.T == 0
         B = (offsets.numel() - 1) // self.T
         n = indices.numel()
-        lookup = E._capi.lib().fbgemm_b200_sequence_lookup
-        if output is None:
+        filled = output is None   # nothing in it yet: the kernel also writes the rows that no index fills
+        if filled:
             output = torch.empty((n, self.out_cols), dtype=self.out_dtype, device=self.device)
-            lookup = E._capi.lib().fbgemm_b200_sequence_lookup_filled
             if B == 0:
                 output.zero_()
         assert output.is_contiguous() and output.dtype == self.out_dtype and output.numel() == n * self.out_cols
         if B == 0 or n == 0:
             return output
-        ctx = E.get_context(self.device.index)
-        rc = lookup(
-            ctx.handle, self.dev_weights.data_ptr(), self._desc.data_ptr(), self.T, B, self.D, indices.data_ptr(),
-            offsets.data_ptr(), indices.element_size(), n, output.data_ptr(), self.out_code, self.out_row_bytes,
-            int(self.scale_bias_last), self.fp8[0], self.fp8[1], slot,
-            torch.cuda.current_stream(self.device).cuda_stream)
+        rc = E._capi.native().sequence_lookup(
+            int(filled), E._handle_of(self.device.index), self.dev_weights, self._desc, self.T, B, self.D, indices, offsets,
+            indices.element_size(), n, output, self.out_code, self.out_row_bytes, int(self.scale_bias_last), self.fp8[0],
+            self.fp8[1], slot, E._current_stream(self.device.index))
         E._capi.check(rc, "fbgemm_b200_sequence_lookup")
         return output
 
