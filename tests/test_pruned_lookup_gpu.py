@@ -53,6 +53,28 @@ def test_a_full_table_without_the_key_ends_with_minus_one(gpu_ctx):
     assert got.cpu().tolist() == [-1, 2]
 
 
+@pytest.mark.parametrize("idt", [np.int32, np.int64])
+@pytest.mark.parametrize("hdt", [np.int32, np.int64])
+@pytest.mark.parametrize("capacity,free,skip", [(1, 0, 0), (4, 0, 1), (5, 1, 3), (8, 0, 0), (9, 0, 1), (37, 0, 2), (40, 1, 5),
+                                                (333, 0, 1), (1000, 3, 0), (5000, 20, 7)])
+def test_long_probe_sequences(gpu_ctx, oracle, idt, hdt, capacity, free, skip):
+    """Maps (almost) without empty slots, which no sector boundary need begin."""
+    rng = np.random.default_rng(1550 + capacity)
+    T, keys = 3, capacity - free
+    picked = [rng.choice(4 * capacity, keys, replace=False) for _ in range(T)]
+    indices = np.concatenate(picked).astype(idt)
+    dense = np.concatenate([rng.permutation(keys) for _ in range(T)]).astype(idt)
+    offsets = (np.arange(T + 1) * keys).astype(idt)
+    hto = np.arange(T + 1, dtype=np.int64) * capacity + skip
+    table = np.full((hto[-1] + 2, 2), -1, dtype=hdt)
+    assert oracle.pruned_hashmap_insert(T, 1, indices, dense, offsets, table, hto)
+    looked = np.stack([np.concatenate([p, rng.integers(0, 8 * capacity, 100)]) for p in picked]).astype(idt)
+    off2 = (np.arange(T + 1) * looked.shape[1]).astype(idt)
+    want = oracle.pruned_hashmap_lookup(T, 1, looked.reshape(-1), off2, table, hto)
+    got = tbe.pruned_hashmap_lookup(dev(looked.reshape(-1)), dev(off2), dev(table), dev(hto))
+    np.testing.assert_array_equal(got.cpu().numpy(), want)
+
+
 def test_positions_outside_the_offsets_are_left_alone(gpu_ctx, oracle):
     rng = np.random.default_rng(1600)
     indices, dense, offsets, table, hto = pruning_case(rng, 3, 10, 6, np.int64, np.int64)
