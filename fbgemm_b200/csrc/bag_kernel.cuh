@@ -577,8 +577,12 @@ __device__ __forceinline__ void pool_bags(const BagTable& p, void* const* peers,
     // Where this lane's row goes in the queue, how many rows the group has, and the most that a group of the warp has.
     // Slots behind a group's rows hold row 0 with scale and bias 0, which leave every sum as it is (x + 0 = x, and no
     // sum is ever -0), so that groups of four rows need no special case for the last one.
-    int at, count, most;
-    if constexpr (FULL) {
+    int at = gl, count = len - c0, most = min(longest - c0, G);
+    bool gaps = FULL;
+    if constexpr (!FULL && !kQuantized) {
+      gaps = __any_sync(0xffffffffu, in_bag && !keep);  // an index out of range pools nothing
+    }
+    if (gaps) {
       // kept rows to the front of the queue in order, the other lanes' slots behind them
       const unsigned ballot = __ballot_sync(0xffffffffu, keep);
       const unsigned kept = G == 32 ? ballot : (ballot >> (grp * G)) & kGroupMask;
@@ -592,10 +596,6 @@ __device__ __forceinline__ void pool_bags(const BagTable& p, void* const* peers,
           most = max(most, __popc((ballot >> (g * G)) & kGroupMask));
         }
       }
-    } else {
-      at = gl;
-      count = len - c0;
-      most = min(longest - c0, G);
     }
     uint32_t sb_lo = 0, sb_hi = 0;
     const Row<WIDE> row_at = id * (Row<WIDE>)p.stride;

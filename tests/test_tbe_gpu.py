@@ -145,3 +145,24 @@ def test_operator_matches_the_reference_operator_fixtures(gpu_ctx):
             want = g[k + "out"]
             np.testing.assert_array_equal(got.view(np.uint32 if out.dtype == torch.float32 else np.uint16),
                                           want.view(np.uint32) if want.dtype == np.float32 else want, err_msg=k)
+
+
+@pytest.mark.parametrize("idt", [np.int32, np.int64])
+def test_an_index_out_of_range_pools_nothing_from_unquantized_tables(gpu_ctx, idt):
+    """The call reports it; the other rows of the bag are pooled as if it were not there."""
+    rng = np.random.default_rng(8350)
+    tys = [tbe.SparseType.FP16, tbe.SparseType.FP8, tbe.SparseType.FP32]
+    dims, rows, B = [64, 200, 24], [300, 150, 100], 300
+    tables, blob, w_off, D_off, offsets, indices, weights = build_op_inputs(rng, tys, dims, rows, B, 40, 16, True, idt)
+    op = tbe.IntNBitTableBatchedEmbeddingBags(torch.from_numpy(blob).cuda(), w_off, np.array([int(t) for t in tys], np.uint8),
+                                              D_off, int(D_off[-1]), tbe.PoolingMode.SUM, 16, tbe.SparseType.FP32, True, True,
+                                              torch.from_numpy(indices).dtype, 5, 15)
+    bad = rng.random(len(indices)) < 0.2
+    broken = np.where(bad, np.where(rng.random(len(indices)) < 0.5, -1, 10_000), indices).astype(idt)
+    got = op.forward(*(torch.from_numpy(a).cuda() for a in (broken, offsets, weights)), slot=23).clone()
+    assert not F.status_read(23)[0]
+    gone = np.concatenate([[0], np.cumsum(bad)])
+    kept = (indices[~bad], (offsets - gone[offsets]).astype(idt), weights[~bad])
+    want = op.forward(*(torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in kept), slot=23)
+    assert F.status_read(23)[0]
+    assert torch.equal(got, want)
