@@ -747,7 +747,7 @@ def main_multi(args):
         with torch.cuda.stream(lanes[b]):
             streams = [lanes[b]] + side[b]
             if p2p and step_calls:
-                # ack wait, the lookups over four streams, ready signal and wait, release: one call
+                # ack wait, the lookups, ready signal and wait, release: one call
                 step_calls[b].step_device(step_args[s], True, lanes[b].cuda_stream)
             elif p2p:
                 n = sl.step(sets[s], buffer=b, slot_base=(j % 4) * 100, streams=None if plans else streams,
@@ -1023,7 +1023,7 @@ def main_multi(args):
                                           "stores), ready/ack counters between the ranks on the device" if p2p else
                                           "NCCL all_to_all_single after the lookups"),
                        "launch": (f"multi-table plan, {launches_per_batch} kernel launches per global batch" if plans else
-                                  f"one launch per table over 4 streams ({launches_per_batch} kernel launches per "
+                                  f"one call per global batch ({launches_per_batch} kernel launches per "
                                   "global batch and rank, counters included)") + f"; {nbuf} global batches in flight, "
                                  "one per output buffer",
                        "l2": "tables are far larger than L2; the input sets rotate"},
@@ -1042,7 +1042,7 @@ def main_multi(args):
                          "traffic": traffic["bytes_per_global_batch"] / world if traffic_ok else None,
                          "traffic_source": traffic["source"] if traffic_ok else None, "peak_source": peak_src,
                          "note": "per GPU: gathered-row bytes of one global batch / device time per global batch (the "
-                                 "tables' launches overlap on 4 streams); traffic = DRAM bytes of all lookup kernels of "
+                                 "global batches in flight overlap); traffic = DRAM bytes of all lookup kernels of "
                                  "one global batch per GPU"},
             "e2e": e2e, "cpu_baseline": cpu, "single_table": single,
             "peer_store_ab": dict(peer_ab, peer_stores_ms_per_global_batch=ms / nbatches,

@@ -57,7 +57,7 @@ struct SpmdmParams {
   int32_t group_smem;         // shared-memory bytes per bag slot
   int32_t copy_width;         // 16/8/4: cp.async granule; 0: byte-wise path
   uint32_t flags;
-  // Tables that are not row-wise quantized (plain_kernels.cu): 0 = quantized,
+  // Tables that are not row-wise quantized (the plain formats of bag_kernel.cuh): 0 = quantized,
   // else FBGEMM_B200_IN_F32 / _F16 / _BF16 / _FP8 and the FP8 format.
   int32_t in_kind;
   int32_t fp8_exponent_bits;
@@ -129,7 +129,7 @@ cudaError_t launch_multi_plan(const MultiPlan& plan, cudaStream_t stream);
 // The same without keeping the plan.
 cudaError_t launch_tables(const SpmdmParams* tables, const int* bit_rates, size_t count, cudaStream_t stream);
 
-// no_bag with 8-bit output: byte copies of the indexed rows (plain_kernels.cu).
+// no_bag with 8-bit output: byte copies of the indexed rows (rows_copy_kernels.cu).
 cudaError_t launch_rows_copy(
     const uint8_t* table,
     const void* indices,
