@@ -84,12 +84,15 @@ int form_of(const BagTable& t) {
 // two bags), the narrowest quarter warps.  Measured, us, on bags of 30 rows at
 // 12 M rows: 4-bit D = 64, 4096 bags 7.0 / 8.9 / 10.9 with 32 / 16 / 8 lanes;
 // 8192 bags 11.6 / 10.0 / 12.2; 65536 bags 61.8 / 51.9 / 48.7.  4-bit D = 128,
-// 65536 bags 80.9 / 72.8 / 78.3.  Wider rows always want whole warps.
+// 65536 bags 80.9 / 72.8 / 78.3.  Wider rows always want whole warps.  Quarter
+// warps from 8 bags per resident warp on: 33000 bags of 2-bit D = 64 take 39.5 us
+// with them and 33.6 without, 4-bit 40.4 and 38.7, 64 mixed tables of 512 bags
+// 53.3 and 50.6; 100000 bags of 4-bit D = 64 86.5 and 91.9.
 constexpr int64_t kResidentWarps = 148 * bag::kBlocksPerSm * bag::kWarps;
 
 int pick_variant(const BagTable& t, int fmt, int64_t bags_in_launch, int* tiles) {
   const int align = alignment_of(reinterpret_cast<uintptr_t>(t.data) | (uint64_t)t.stride);
-  const int least_g = bags_in_launch <= kResidentWarps ? 32 : bags_in_launch <= 4 * kResidentWarps ? 16 : 8;
+  const int least_g = bags_in_launch <= kResidentWarps ? 32 : bags_in_launch <= 8 * kResidentWarps ? 16 : 8;
   int best = -1;
   double best_cost = 0;
   for (int i = 0; i < bag::kVariants; ++i) {

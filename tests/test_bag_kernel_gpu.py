@@ -59,7 +59,7 @@ def test_row_widths_and_alignments(gpu_ctx, oracle, bit_rate, sb_last):
 
 
 @pytest.mark.parametrize("bit_rate", [8, 4, 2])
-@pytest.mark.parametrize("batch", [7104, 7105, 28416, 28417])
+@pytest.mark.parametrize("batch", [7104, 7105, 28416, 56832, 56833])
 def test_lanes_per_bag(gpu_ctx, oracle, bit_rate, batch):
     rng = np.random.default_rng(7 * bit_rate + batch)
     for dim in (20, 32, 64, 128):
