@@ -173,7 +173,11 @@ cudaError_t launch_bags(const SpmdmParams& p, int bit_rate, cudaStream_t stream)
     return cudaErrorInvalidValue;
   }
   int form = form_of(c.t);
-  if (form != bag::kWide && blocks * tiles <= 148 * bag::kDeepBlocksPerSm) {
+  // The deep form while the launch fits the chip at once; with a pruning map, one more trip to memory in every stretch,
+  // up to two such launches' worth: 2-bit D = 128, 11000 bags 16.9 against 14.5 us, 14000 20.0 / 18.5, 20000 27.6 / 25.5.
+  // (Dense tables lose there: 8-bit D = 128, 14000 bags 29.7 against 33.6.)
+  const int64_t fit = 148 * bag::kDeepBlocksPerSm * (c.t.flags & kPruned ? 2 : 1);
+  if (form != bag::kWide && blocks * tiles <= fit) {
     form += 3;
   }
   return launch<bag::BagCall>(single_kernel(v, form), dim3((unsigned)blocks, (unsigned)tiles), c, stream);

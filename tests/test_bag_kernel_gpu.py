@@ -194,3 +194,21 @@ def test_lengths_without_a_scan(gpu_ctx, oracle, batch):
         assert kern(batch, n, rows, *args) and ok_ref
         np.testing.assert_array_equal(bits(out.cpu().numpy()), bits(ref))
         assert not kern(batch, n - 1, rows, *args)       # the lengths do not add up to index_size
+
+
+@pytest.mark.parametrize("batch", [10_656, 10_657, 21_312, 21_313])
+def test_pruned_launches_around_what_fits_the_chip(gpu_ctx, oracle, batch):
+    rng = np.random.default_rng(batch)
+    kept, full, dim = 400, 900, 128
+    table = random_fused_table(rng, kept, dim, 2)
+    mapping = np.full(full, -1, dtype=np.int32)
+    mapping[rng.choice(full, kept, replace=False)] = np.arange(kept, dtype=np.int32)
+    lengths = rng.integers(0, 4, batch)
+    lengths[rng.integers(0, batch, 60)] = rng.choice(EDGE_LENGTHS, 60)
+    offsets = np.concatenate([[0], np.cumsum(lengths)]).astype(np.int32)
+    indices = rng.integers(0, full, offsets[-1]).astype(np.int64)
+    kern = F.GenerateEmbeddingSpMDMNBitRowWiseSparse(2, dim, False, True, index_dtype=np.int64, offset_dtype=np.int32)
+    ok_ref, ref = oracle.spmdm_rowwise_sparse(2, dim, full, table, indices, mapping, offsets, None, True)
+    out = torch.zeros(batch * dim, device="cuda")
+    assert kern(batch, len(indices), full, dev(table), dev(indices), dev(offsets), None, out, dev(mapping)) and ok_ref
+    np.testing.assert_array_equal(bits(out.cpu().numpy()), bits(ref))
