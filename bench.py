@@ -1307,6 +1307,8 @@ def main():
 
     if not torch.cuda.is_available():
         emit(({"error": "no CUDA device: fbgemm_b200 has no CPU path"}))
+        if int(os.environ.get("WORLD_SIZE", "1")) > 1:
+            time.sleep(5)   # the launcher ends every rank when the first one does: let the others say it too
         return 1
     if args.workload == 5:
         return main_callers(args)
