@@ -140,7 +140,6 @@ class SpmdmKernel:
     def __init__(self, cfg: SpmdmConfig, rowwise_sparse: bool):
         self.cfg = cfg
         self.rowwise_sparse = rowwise_sparse
-        self._cfg_addr = C.addressof(cfg)
         _capi.check(_capi.lib().fbgemm_b200_spmdm_check_config(C.byref(cfg)), "generator arguments")
 
     # -- the reference's functor signature ----------------------------------
@@ -154,7 +153,7 @@ class SpmdmKernel:
         if _is_tensor(input):
             dev = input.get_device()
             rc = _capi.native().spmdm(
-                _handle_of(dev), self._cfg_addr, output_size, index_size, data_size, input, indices, offsets_or_lengths,
+                _handle_of(dev), C.addressof(self.cfg), output_size, index_size, data_size, input, indices, offsets_or_lengths,
                 weights if self.cfg.has_weight else None, out, compressed_indices_table, _current_stream(dev))
         else:
             ctx = get_context()
@@ -171,7 +170,7 @@ class SpmdmKernel:
         without synchronising; errors land in status slot ``slot``."""
         dev = input.get_device()
         rc = _capi.native().spmdm_launch(
-            _handle_of(dev), self._cfg_addr, output_size, index_size, data_size, input, indices, offsets_or_lengths,
+            _handle_of(dev), C.addressof(self.cfg), output_size, index_size, data_size, input, indices, offsets_or_lengths,
             weights if self.cfg.has_weight else None, out, compressed_indices_table, slot,
             _current_stream(dev) if stream is None else stream)
         _capi.check(rc, "fbgemm_b200_spmdm_launch")
