@@ -69,6 +69,15 @@ static int arity(Py_ssize_t got, Py_ssize_t want) {
   return 0;
 }
 
+/* Runs CALL, which gives an int, without the interpreter's lock: a launch waits when the stream's queue is full, and lengths
+ * mode takes the context's lock and may allocate. */
+#define WITHOUT_LOCK(CALL)    \
+  int rc;                     \
+  Py_BEGIN_ALLOW_THREADS      \
+  rc = (CALL);                \
+  Py_END_ALLOW_THREADS        \
+  return PyLong_FromLong(rc)
+
 /* spmdm_launch(ctx, cfg, output_size, index_size, data_size, input, indices, offsets, weights, out, map, slot, stream) */
 static PyObject* spmdm_launch(PyObject* self, PyObject* const* args, Py_ssize_t n) {
   (void)self;
@@ -78,8 +87,8 @@ static PyObject* spmdm_launch(PyObject* self, PyObject* const* args, Py_ssize_t 
       integers(args, 11, 1, &slot) || addresses(args, 12, 1, &stream)) {
     return NULL;
   }
-  return PyLong_FromLong(fbgemm_b200_spmdm_launch(h[0], h[1], size[0], size[1], size[2], t[0], t[1], t[2], t[3], t[4], t[5],
-                                                  (int)slot, stream));
+  WITHOUT_LOCK(fbgemm_b200_spmdm_launch(h[0], h[1], size[0], size[1], size[2], t[0], t[1], t[2], t[3], t[4], t[5], (int)slot,
+                                        stream));
 }
 
 /* spmdm(ctx, cfg, output_size, index_size, data_size, input, indices, offsets, weights, out, map, stream): waits */
@@ -91,11 +100,7 @@ static PyObject* spmdm(PyObject* self, PyObject* const* args, Py_ssize_t n) {
       addresses(args, 11, 1, &stream)) {
     return NULL;
   }
-  int rc;
-  Py_BEGIN_ALLOW_THREADS
-  rc = fbgemm_b200_spmdm(h[0], h[1], size[0], size[1], size[2], t[0], t[1], t[2], t[3], t[4], t[5], stream);
-  Py_END_ALLOW_THREADS
-  return PyLong_FromLong(rc);
+  WITHOUT_LOCK(fbgemm_b200_spmdm(h[0], h[1], size[0], size[1], size[2], t[0], t[1], t[2], t[3], t[4], t[5], stream));
 }
 
 /* table_set_forward(set, bags, indices, index_size, offsets, weights, out, slot, stream) */
@@ -108,7 +113,7 @@ static PyObject* table_set_forward(PyObject* self, PyObject* const* args, Py_ssi
       addresses(args, 8, 1, &stream)) {
     return NULL;
   }
-  return PyLong_FromLong(fbgemm_b200_table_set_forward(set, bags, indices, index_size, t[0], t[1], t[2], (int)slot, stream));
+  WITHOUT_LOCK(fbgemm_b200_table_set_forward(set, bags, indices, index_size, t[0], t[1], t[2], (int)slot, stream));
 }
 
 /* quantize(bit_rate, x, rows, cols, out, stream); bit_rate 0: 8-bit rows with fp32 scale and bias */
@@ -120,9 +125,9 @@ static PyObject* quantize(PyObject* self, PyObject* const* args, Py_ssize_t n) {
       addresses(args, 4, 2, t)) {
     return NULL;
   }
-  return PyLong_FromLong(bits == 0 ? fbgemm_b200_float_to_fused_8bit_rowwise(x, size[0], (int32_t)size[1], t[0], t[1])
-                                   : fbgemm_b200_float_to_fused_nbit_rowwise((int32_t)bits, x, size[0], (int32_t)size[1], t[0],
-                                                                             t[1]));
+  WITHOUT_LOCK(bits == 0
+                   ? fbgemm_b200_float_to_fused_8bit_rowwise(x, size[0], (int32_t)size[1], t[0], t[1])
+                   : fbgemm_b200_float_to_fused_nbit_rowwise((int32_t)bits, x, size[0], (int32_t)size[1], t[0], t[1]));
 }
 
 /* pruned_lookup(hashmap, ctx, T, B, indices, offsets, index_bytes, index_size, map, map_bytes, map_offsets, dense, slot,
@@ -137,7 +142,7 @@ static PyObject* pruned_lookup(PyObject* self, PyObject* const* args, Py_ssize_t
       addresses(args, 13, 1, &stream)) {
     return NULL;
   }
-  return PyLong_FromLong((hashmap ? fbgemm_b200_pruned_hashmap_lookup : fbgemm_b200_pruned_array_lookup)(
+  WITHOUT_LOCK((hashmap ? fbgemm_b200_pruned_hashmap_lookup : fbgemm_b200_pruned_array_lookup)(
       ctx, (int32_t)size[0], (int32_t)size[1], in[0], in[1], (int32_t)index[0], index[1], map, (int32_t)map_bytes, t[0], t[1],
       (int32_t)slot, stream));
 }
@@ -153,7 +158,7 @@ static PyObject* sequence_lookup(PyObject* self, PyObject* const* args, Py_ssize
       integers(args, 12, 6, out) || addresses(args, 18, 1, &stream)) {
     return NULL;
   }
-  return PyLong_FromLong((filled ? fbgemm_b200_sequence_lookup_filled : fbgemm_b200_sequence_lookup)(
+  WITHOUT_LOCK((filled ? fbgemm_b200_sequence_lookup_filled : fbgemm_b200_sequence_lookup)(
       t[0], t[1], t[2], (int32_t)size[0], (int32_t)size[1], (int32_t)size[2], in[0], in[1], (int32_t)index[0], index[1], rows,
       (int32_t)out[0], out[1], (int32_t)out[2], (int32_t)out[3], (int32_t)out[4], (int32_t)out[5], stream));
 }

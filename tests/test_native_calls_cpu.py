@@ -2,14 +2,22 @@
 reaches the library, seen through stand-ins for it."""
 import copy
 import ctypes as C
+import importlib.machinery
+import importlib.util
+import os
 import pickle
+import subprocess
+import sysconfig
 
 import numpy as np
 import pytest
 
 import fbgemm_b200 as F
 from fbgemm_b200 import _capi
+from fbgemm_b200 import build
 from fbgemm_b200 import embedding as E
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 class FakeTensor:
@@ -67,3 +75,52 @@ def test_a_copied_kernel_calls_with_its_own_configuration(recorder, how):
     for name, args in recorder.calls:
         assert args[1] == C.addressof(c.cfg), name
         assert _capi.SpmdmConfig.from_address(args[1]).normalize_by_lengths == 1
+
+
+# ---- the extension itself, over stand-ins for the library's functions ------------
+
+@pytest.fixture(scope="module")
+def stubbed(tmp_path_factory):
+    path = str(tmp_path_factory.mktemp("native") / "_native_calls.so")
+    subprocess.run(["gcc", "-O1", "-Wall", "-shared", "-fPIC", "-I", build.INCLUDE, "-I", sysconfig.get_paths()["include"],
+                    os.path.join(build.CSRC, build.NATIVE_SOURCE), os.path.join(ROOT, "tests", "cpp", "native_calls_stub.c"),
+                    "-o", path], check=True)
+    loader = importlib.machinery.ExtensionFileLoader("_native_calls", path)
+    module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_native_calls", loader))
+    loader.exec_module(module)
+    return module
+
+
+class Array(FakeTensor):
+    def is_contiguous(self):
+        return True
+
+
+#: name -> arguments: "h" a handle, "t" a tensor, numbers as they are
+CALLS = {
+    "spmdm_launch": ["h", "h", 1, 1, 1, "t", "t", "t", "t", "t", "t", 0, "h"],
+    "spmdm": ["h", "h", 1, 1, 1, "t", "t", "t", "t", "t", "t", "h"],
+    "table_set_forward": ["h", 1, "t", 1, "t", "t", "t", 0, "h"],
+    "quantize": [0, "t", 1, 4, "t", "h"],
+    "pruned_lookup": [1, "h", 1, 1, "t", "t", 8, 1, "t", 8, "t", "t", 0, "h"],
+    "sequence_lookup": [1, "h", "t", "t", 1, 1, 4, "t", "t", 8, 1, "t", 0, 16, 1, 4, 7, 0, "h"],
+}
+
+
+def arguments(name):
+    return [1 << 16 if a == "h" else Array() if a == "t" else a for a in CALLS[name]]
+
+
+def test_every_call_of_the_extension_is_listed(stubbed):
+    assert set(CALLS) == {n for n in dir(stubbed) if not n.startswith("_")}
+
+
+@pytest.mark.parametrize("name", CALLS)
+@pytest.mark.parametrize("first", [0, 1, 4])   # the calls that choose between two entry points choose by it
+def test_calls_give_up_the_interpreters_lock(stubbed, name, first):
+    """A launch waits while the stream's queue is full, and lengths mode may lock or allocate: other Python threads, on
+    which that may depend, run on meanwhile."""
+    args = arguments(name)
+    if isinstance(CALLS[name][0], int):
+        args[0] = first
+    assert getattr(stubbed, name)(*args) == 0, "the lock was held"
