@@ -134,6 +134,36 @@ def _ptr(x):
     return x.ctypes.data
 
 
+def page_locked_address(x) -> int:
+    """Address of a numpy array among device tensors: the GPU reads it where it
+    lies, so it has to be page-locked memory (a pinned tensor's ``numpy()``)."""
+    if not isinstance(x, np.ndarray):
+        raise TypeError(f"a tensor is expected, got {type(x).__name__}")
+    assert x.flags["C_CONTIGUOUS"], "arrays must be contiguous"
+    if x.size and not _page_locked(x):
+        raise TypeError("beside device tensors a numpy array has to lie in page-locked memory")
+    return x.ctypes.data
+
+
+def _page_locked(x) -> bool:
+    import torch
+
+    return torch.cuda.is_available() and (x if _is_tensor(x) else torch.from_numpy(x)).is_pinned()
+
+
+def _device_of(input) -> int:
+    """The device that reads a table: its own, or for one in page-locked host
+    memory the current one."""
+    dev = input.get_device()
+    if dev < 0:
+        import torch
+
+        if not _page_locked(input):
+            raise TypeError("the table has to be a CUDA tensor, or a tensor in page-locked memory")
+        dev = torch.cuda.current_device()
+    return dev
+
+
 class SpmdmKernel:
     """The functor a generator returns.  Holds only the configuration."""
 
@@ -151,7 +181,7 @@ class SpmdmKernel:
             raise ValueError("this kernel was not generated for row-wise sparse tables")
         self._check_dtypes(indices, offsets_or_lengths)
         if _is_tensor(input):
-            dev = input.get_device()
+            dev = _device_of(input)
             rc = _capi.native().spmdm(
                 _handle_of(dev), C.addressof(self.cfg), output_size, index_size, data_size, input, indices, offsets_or_lengths,
                 weights if self.cfg.has_weight else None, out, compressed_indices_table, _current_stream(dev))
@@ -168,7 +198,7 @@ class SpmdmKernel:
                compressed_indices_table=None, slot: int = 0, stream=None) -> None:
         """Enqueue on ``stream`` (int handle; default torch's current stream)
         without synchronising; errors land in status slot ``slot``."""
-        dev = input.get_device()
+        dev = _device_of(input)
         rc = _capi.native().spmdm_launch(
             _handle_of(dev), C.addressof(self.cfg), output_size, index_size, data_size, input, indices, offsets_or_lengths,
             weights if self.cfg.has_weight else None, out, compressed_indices_table, slot,

@@ -1,0 +1,69 @@
+"""Forms of the calls that the common case does not use: tables and index arrays
+in page-locked host memory, pruning maps into larger tables, output rows farther
+apart than their columns, operators whose tables change or that are copied, and
+calls that overlap on several streams.  Bit for bit against the CPU oracle."""
+import copy
+import ctypes as C
+
+import numpy as np
+import pytest
+import torch
+
+import fbgemm_b200 as F
+from fbgemm_b200 import _capi, tbe
+from fbgemm_b200 import embedding as E
+from conftest import bits
+from helpers import build_op_inputs, oracle_op_forward, random_fused_table, random_plain_table, row_bytes
+
+pytestmark = pytest.mark.gpu
+ST = tbe.SparseType
+
+
+def dev(a):
+    return None if a is None else torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+
+def bags(rng, batch, rows, hi=40):
+    lengths = rng.integers(0, hi, batch)
+    offsets = np.concatenate([[0], np.cumsum(lengths)])
+    n = int(offsets[-1])
+    return n, rng.integers(0, rows, n).astype(np.int64), offsets.astype(np.int64)
+
+
+# ---- page-locked host memory ---------------------------------------------------
+
+@pytest.mark.parametrize("call", ["awaited", "launch"])
+def test_arrays_in_page_locked_memory(gpu_ctx, oracle, call):
+    """The GPU reads page-locked arrays where they lie: a table tensor, and index arrays as the numpy views of pinned
+    tensors."""
+    rng = np.random.default_rng(1)
+    rows, dim, batch = 200, 64, 33
+    table = random_fused_table(rng, rows, dim, 8)
+    n, indices, offsets = bags(rng, batch, rows)
+    ok_ref, ref = oracle.spmdm(8, dim, rows, table, indices, offsets, None, False, np.float32)
+    assert ok_ref
+    k = F.GenerateEmbeddingSpMDM(dim, False, False, index_dtype=np.int64, offset_dtype=np.int64)
+    pinned = [torch.from_numpy(a).pin_memory() for a in (table, indices, offsets)]
+    forms = [pinned, [dev(table), pinned[1].numpy(), pinned[2].numpy()], [pinned[0], dev(indices), pinned[2].numpy()]]
+    for t, i, o in forms:
+        out = torch.ones(batch * dim, device="cuda")
+        if call == "awaited":
+            assert k(batch, n, rows, t, i, o, None, out)
+        else:
+            k.launch(batch, n, rows, t, i, o, None, out, slot=40)
+            assert F.status_read(40)[0]
+        np.testing.assert_array_equal(bits(out.cpu().numpy()), bits(ref[:batch * dim]))
+
+
+def test_pageable_arrays_are_refused_beside_device_arrays(gpu_ctx):
+    rng = np.random.default_rng(2)
+    rows, dim, batch = 50, 32, 4
+    table = random_fused_table(rng, rows, dim, 8)
+    n, indices, offsets = bags(rng, batch, rows)
+    k = F.GenerateEmbeddingSpMDM(dim, False, False, index_dtype=np.int64, offset_dtype=np.int64)
+    out = torch.empty(batch * dim, device="cuda")
+    for call in (k, k.launch):
+        with pytest.raises(Exception):
+            call(batch, n, rows, dev(table), indices, dev(offsets), None, out)
+        with pytest.raises(Exception):
+            call(batch, n, rows, torch.from_numpy(table), dev(indices), dev(offsets), None, out)

@@ -124,3 +124,33 @@ def test_calls_give_up_the_interpreters_lock(stubbed, name, first):
     if isinstance(CALLS[name][0], int):
         args[0] = first
     assert getattr(stubbed, name)(*args) == 0, "the lock was held"
+
+
+@pytest.mark.parametrize("name", CALLS)
+def test_numbers_are_no_tensors(stubbed, name):
+    """Handles and streams are numbers; where an array is due a number is refused, not taken for its address."""
+    for i, kind in enumerate(CALLS[name]):
+        args = arguments(name)
+        if kind == "t":
+            for wrong in (0, 1 << 20, True, 1.5):
+                args[i] = wrong
+                with pytest.raises((TypeError, AttributeError)):
+                    getattr(stubbed, name)(*args)
+            args[i] = None
+            getattr(stubbed, name)(*args)
+        elif kind == "h":
+            args[i] = Array()
+            with pytest.raises(TypeError):
+                getattr(stubbed, name)(*args)
+
+
+def test_strided_tensors_and_pageable_arrays_are_refused(stubbed):
+    class Strided(FakeTensor):
+        def is_contiguous(self):
+            return False
+
+    for wrong, error in ((Strided(), AssertionError), (np.zeros(4), TypeError), (np.zeros((4, 4))[:, 1], AssertionError)):
+        args = arguments("spmdm_launch")
+        args[6] = wrong
+        with pytest.raises(error):
+            stubbed.spmdm_launch(*args)
