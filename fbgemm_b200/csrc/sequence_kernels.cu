@@ -363,10 +363,10 @@ __global__ void __launch_bounds__(kThreads) sequence_rows_kernel(const SeqArgs a
     const int code = __shfl_sync(0xffffffffu, my_code, i);
     const int state = code & 3;
     if (state == kSkip || state == kZeros) {
-      if (state == kZeros || a.fill) {
-        for (int64_t b = lane; b < a.out_row_bytes; b += 32) {
-          orow[b] = 0;
-        }
+      // a pruned row is D columns of zeros, as walk_rows stores it: what lies behind them is the caller's
+      const int64_t columns = (int64_t)a.D * (OUT == kToF32 ? 4 : 2);
+      for (int64_t b = lane, end = state == kZeros ? columns : a.fill ? a.out_row_bytes : 0; b < end; b += 32) {
+        orow[b] = 0;
       }
       continue;
     }

@@ -542,7 +542,8 @@ typedef struct fbgemm_b200_sequence_table {
  *                 out_row_bytes are written).
  * All tables share D.  Everything is a device pointer; rows of positions that
  * no table covers, or whose index is out of range (reported in status slot
- * `slot`), are left as they were.  Asynchronous on `stream`; returns 0 or a
+ * `slot`), are left as they were, and so is what an output row has behind its
+ * D columns.  Asynchronous on `stream`; returns 0 or a
  * negative code.
  */
 FBGEMM_B200_API int fbgemm_b200_sequence_lookup(

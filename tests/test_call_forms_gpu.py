@@ -67,3 +67,41 @@ def test_pageable_arrays_are_refused_beside_device_arrays(gpu_ctx):
             call(batch, n, rows, dev(table), indices, dev(offsets), None, out)
         with pytest.raises(Exception):
             call(batch, n, rows, torch.from_numpy(table), dev(indices), dev(offsets), None, out)
+
+
+# ---- sequence rows with room between them ----------------------------------------
+
+@pytest.mark.parametrize("D,n", [(16, 32), (16, 45), (10, 40), (128, 33)])
+@pytest.mark.parametrize("filled", [False, True])
+def test_sequence_rows_keep_what_lies_between_them(gpu_ctx, D, n, filled):
+    """A pruned row (-1) is D columns of zeros; the bytes up to the next row are the caller's, whatever the rows around
+    it.  Only the filled form clears rows that nothing names, in full."""
+    rng = np.random.default_rng(D + n)
+    rows, pitch_cols = 50, D + 8
+    stride = tbe.padded_row_size_in_bytes(D, ST.INT8, 4, 4)
+    table = random_fused_table(rng, rows, D, 8, stride, True)
+    idx = rng.integers(0, rows, n).astype(np.int32)
+    idx[rng.permutation(n)[:n // 3]] = -1
+    idx[n - 2] = rows + 5                              # out of range: reported, and left alone (filled: cleared)
+    op = tbe.IntNBitSequenceEmbedding(dev(table.reshape(-1)), np.zeros(1, np.int64), np.array([int(ST.INT8)], np.uint8), D, 4,
+                                      ST.FP32, False)
+    out = torch.full((n, pitch_cols), 7.0, device="cuda")
+    d_idx, d_off = dev(idx), dev(np.array([0, n], np.int32))
+    fn = _capi.lib().fbgemm_b200_sequence_lookup_filled if filled else _capi.lib().fbgemm_b200_sequence_lookup
+    rc = fn(gpu_ctx.handle, op.dev_weights.data_ptr(), op._desc.data_ptr(), 1, 1, D, d_idx.data_ptr(), d_off.data_ptr(), 4, n,
+            out.data_ptr(), op.out_code, 4 * pitch_cols, 0, 4, 7, 41, torch.cuda.current_stream().cuda_stream)
+    _capi.check(rc, "sequence lookup")
+    assert not F.status_read(41)[0]
+    got = out.cpu().numpy()
+    sb = table[:, :4].copy().view(np.float16).astype(np.float32)
+    for k in range(n):
+        if idx[k] == -1:
+            want = np.zeros(D, np.float32)
+        elif idx[k] >= rows:
+            want = np.full(D, 0.0 if filled else 7.0, np.float32)
+        else:
+            q = table[idx[k], 4:4 + D].astype(np.float64)
+            want = (np.float64(sb[idx[k], 0]) * q + np.float64(sb[idx[k], 1])).astype(np.float32)
+        np.testing.assert_array_equal(got[k, :D], want, err_msg=f"row {k}")
+        if not (filled and idx[k] >= rows):
+            assert (got[k, D:] == 7.0).all(), f"row {k}: bytes between the rows were written"
