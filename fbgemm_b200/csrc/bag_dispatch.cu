@@ -54,6 +54,7 @@ void bag_table_of(const SpmdmParams& p, BagTable* t) {
   t->flags = p.flags;
   // a 32-bit index is negative from 2^31 on
   t->limit = (uint32_t)std::min<int64_t>(p.data_size, (p.flags & kIdx64) ? 0xffffffffLL : 0x80000000LL);
+  t->map_limit = (uint32_t)(0xffffffffull / (uint64_t)p.input_stride);
   const uint64_t sb = reinterpret_cast<uintptr_t>(p.table + p.sb_row_off) | (uint64_t)p.input_stride;
   t->sb_align = (int16_t)std::min(8, alignment_of(sb));
   uint64_t o = (uint64_t)t->out_pitch;
@@ -70,12 +71,12 @@ void bag_table_of(const SpmdmParams& p, BagTable* t) {
 }
 
 // The form of a table's kernel.  (A row-wise sparse call says how many rows its
-// map has, not how many its table holds: no more than those.)
+// map has, not how many its table holds, which may be more: see pool_far_rows.)
 int form_of(const BagTable& t) {
   const bool wide = (unsigned __int128)t.data_size * (uint64_t)t.stride > 0xffffffffull || t.bags > 0x7fffff00LL ||
       t.index_size > 0x7fffff00LL;
-  const bool options = t.flags & (kPruned | kSbFirst | kNoBag | kPositional | kLengths);
-  return wide ? bag::kWide : options || t.data_size == 0 ? bag::kFull : bag::kLean;
+  const bool options = t.flags & (kSbFirst | kNoBag | kPositional | kLengths);
+  return wide ? bag::kWide : t.flags & kPruned ? bag::kMapped : options || t.data_size == 0 ? bag::kFull : bag::kLean;
 }
 
 // Whole warps per bag while every bag of the launch finds a resident warp: the
@@ -173,6 +174,7 @@ cudaError_t launch_bags(const SpmdmParams& p, int bit_rate, cudaStream_t stream)
     return cudaErrorInvalidValue;
   }
   int form = form_of(c.t);
+  form = form == bag::kMapped ? (int)bag::kFull : form;  // one kernel for both
   // The deep form while the launch fits the chip at once; with a pruning map, one more trip to memory in every stretch,
   // up to two such launches' worth: 2-bit D = 128, 11000 bags 16.9 against 14.5 us, 14000 20.0 / 18.5, 20000 27.6 / 25.5.
   // (Dense tables lose there: 8-bit D = 128, 14000 bags 29.7 against 33.6.)
@@ -265,7 +267,10 @@ cudaError_t build_multi_plan(const SpmdmParams* tables, const int* bit_rates, si
 
 cudaError_t launch_multi_plan(const MultiPlan& plan, cudaStream_t stream) {
   for (const auto& l : plan.launches) {
-    const bag::BagUnitsFn fn = l->form == bag::kWide ? bag_units_wide() : l->form == bag::kFull ? bag_units_full() : bag_units_lean();
+    const bag::BagUnitsFn fn = l->form == bag::kWide ? bag_units_wide()
+        : l->form == bag::kMapped                    ? bag_units_mapped()
+        : l->form == bag::kFull                      ? bag_units_full()
+                                                     : bag_units_lean();
     const cudaError_t e = launch<bag::BagUnits>(fn, dim3(l->blocks), l->units, stream);
     if (e != cudaSuccess) {
       return e;

@@ -190,6 +190,8 @@ struct Cols {
   static constexpr int kPerChunk = VB * 8 / BITS;
   static constexpr int kPairs = kPerChunk * CPL / 2;
   static_assert(kPerChunk * CPL % 2 == 0, "whole pairs");
+  static constexpr bool kQuantized = is_quantized(FMT);
+  static constexpr bool kHalfSb = FMT != kInt8;  // with a pruning map: those rows have scale and bias last
   using M = Constants<FMT, kPerChunk>;
 
   // Column k of an unquantized chunk.
@@ -384,12 +386,14 @@ struct __align__(16) Queue {
 
 // What a kernel is compiled for.
 //  kLean  bags by offsets, weights per index, every index a row of the table
-//  kFull  besides: pruning maps, -1 as a pruned index, no_bag, positional
+//  kFull  besides: -1 as a pruned index, no_bag, positional
 //         weights, lengths in place of offsets
+//  kMapped  besides: pruning maps (the single-table kernels know no kFull without them; for 64 table-batched tables the
+//         maps' part, unused, cost 4 %)
 //  kWide  the same where positions, bags (31 bits) or row offsets (32) need more
 // The lean form saves the queue's compaction and half of the tests, a tenth of
 // the time of 65536 bags of 30 rows (8-bit D = 128 76.4 against 83.6 us).
-enum : int { kLean = 0, kFull = 1, kWide = 2 };
+enum : int { kLean = 0, kFull = 1, kWide = 2, kMapped = 3 };
 
 // Groups of four rows whose loads are issued ahead of the arithmetic.  Measured on 65536 bags of 30 rows: with half
 // warps per bag none is best for 4-bit rows (67.9 against 69.4 us at D = 128), one for 8- and 2-bit rows (82 against
@@ -447,11 +451,59 @@ __device__ __forceinline__ void bag_from_lengths(const BagTable& p, int64_t firs
   length = bag < p.bags ? at(bag) : 0;
 }
 
+// A bag of a row-wise sparse call whose map names rows beyond 32-bit offsets (several short maps may share one large
+// table), pooled once more from its first position with 64-bit row addresses, one row at a time.  Rare, so it costs the
+// other bags one comparison per mapped row and no registers (11.3 us before and after for 8192 bags of 30 rows, 2-bit
+// D = 128), where 64-bit addresses for every pruned table would cost each of their rows the wide form's extra instructions.
+template <class C, int VB, int CPL, int G>
+__device__ __forceinline__ void pool_far_rows(const BagTable& p, const typename C::M& constants,
+                                              const LaneData<VB, CPL, G, false>& lane_data, int start, int len,
+                                              u64 (&acc)[C::kPairs]) {
+#pragma unroll
+  for (int k = 0; k < C::kPairs; ++k) {
+    acc[k] = 0ull;
+  }
+#pragma unroll 1
+  for (int c = 0; c < len; ++c) {
+    const int64_t idx = load_int(p.indices, (int64_t)start + c, p.flags & kIdx64);
+    const int32_t m = idx >= 0 && idx < p.data_size ? __ldg(p.cit + idx) : -1;
+    if (m < 0) {
+      continue;
+    }
+    const uint8_t* row = p.data + (uint64_t)(uint32_t)m * (uint64_t)p.stride;
+    const float w = p.flags & kWeighted ? __ldg(p.weights + (p.flags & kPositional ? (int64_t)c : (int64_t)start + c)) : 1.f;
+    Bytes<VB> d[CPL];
+#pragma unroll
+    for (int i = 0; i < CPL; ++i) {
+      d[i].load(row + lane_data.at[i]);
+    }
+    if constexpr (C::kQuantized) {
+      const uint8_t* sb = row + p.sb_off;
+      const uint32_t lo = load_u32(sb, p.sb_align);
+      float scale, bias;
+      if (C::kHalfSb) {
+        scale = __half2float(__ushort_as_half((unsigned short)(lo & 0xffffu)));
+        bias = __half2float(__ushort_as_half((unsigned short)(lo >> 16)));
+      } else {
+        scale = __uint_as_float(lo);
+        bias = __uint_as_float(load_u32(sb + 4, p.sb_align));
+      }
+      if (p.flags & kWeighted) {
+        scale = __fmul_rn(w, scale);
+        bias = __fmul_rn(w, bias);
+      }
+      C::pool(constants, acc, d, pack2(scale, scale), pack2(bias, bias));
+    } else {
+      C::pool(constants, acc, d, pack2(w, w), 0ull);
+    }
+  }
+}
+
 // One block's work on table `p`: bags block * kWarps * (32 / G) onwards, columns of tile `tile` of the row.
 template <int FMT, int VB, int CPL, int G, int MODE, bool kDeep>
 __device__ __forceinline__ void pool_bags(const BagTable& p, void* const* peers, uint32_t block, int tile,
                                           Queue<MODE == kWide> (&queues)[kWarps]) {
-  constexpr bool WIDE = MODE == kWide, FULL = MODE != kLean;
+  constexpr bool WIDE = MODE == kWide, FULL = MODE != kLean, MAPS = WIDE || MODE == kMapped;
   constexpr int kAhead = rows_ahead(FMT, G, kDeep);
   using C = Cols<FMT, VB, CPL>;
   using Pos = typename std::conditional<WIDE, int64_t, int32_t>::type;  // bags and positions
@@ -468,7 +520,7 @@ __device__ __forceinline__ void pool_bags(const BagTable& p, void* const* peers,
   const bool off64 = p.flags & kOff64;
   const bool weighted = p.flags & kWeighted;
   const bool positional = FULL && (p.flags & kPositional);
-  const bool pruned = FULL && (p.flags & kPruned);
+  const bool pruned = MAPS && (p.flags & kPruned);
   const bool no_bag = FULL && (p.flags & kNoBag);
   const bool by_lengths = FULL && (p.flags & kLengths);
   const bool minus_one_skips = FULL && FMT != kFp8 && (p.flags & (kSbFirst | kNoBag)) == kSbFirst;
@@ -541,6 +593,7 @@ __device__ __forceinline__ void pool_bags(const BagTable& p, void* const* peers,
     return r;
   };
   uint2 raw = fetch(gl);
+  bool far = false;  // a row of this lane's lies beyond 32-bit offsets
 #pragma unroll 1
   for (int c0 = 0; c0 < longest; c0 += G) {
     const int c = c0 + gl;
@@ -570,6 +623,12 @@ __device__ __forceinline__ void pool_bags(const BagTable& p, void* const* peers,
       const int32_t m = __ldg(p.cit + id);
       keep = m >= 0;
       id = keep ? (uint32_t)m : 0u;
+      if constexpr (!WIDE) {
+        // a table larger than its map: below, with 64-bit row addresses
+        far = far || (keep && id >= p.map_limit);
+        keep = keep && id < p.map_limit;
+        id = keep ? id : 0u;
+      }
     }
     pos += G;
     raw = fetch(c + G);  // the next stretch's, on its way during this one's arithmetic
@@ -680,6 +739,12 @@ __device__ __forceinline__ void pool_bags(const BagTable& p, void* const* peers,
       }
     }
     __syncwarp();  // the queue is rewritten by the next stretch
+  }
+
+  if constexpr (MAPS && !WIDE) {
+    if (pruned && __any_sync(0xffffffffu, far)) {
+      pool_far_rows<C, VB, CPL, G>(p, constants, lane_data, pos - gl - (longest + G - 1) / G * G, len, acc);
+    }
   }
 
   if constexpr (!kDeep) {
@@ -821,7 +886,7 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm) bag_units_kernel(const
 }
 
 using BagFn = void (*)(const BagCall);
-constexpr int kForms = 5;  // kLean, kFull, kWide, and the deep forms of kLean and kFull
+constexpr int kForms = 5;  // kLean, kMapped, kWide, and the deep forms of kLean and kMapped
 using BagUnitsFn = void (*)(const BagUnits);
 
 }  // namespace bag
@@ -834,6 +899,7 @@ void bag_kernels_2(bag::BagFn (*fn)[bag::kForms]);
 void bag_kernels_plain(bag::BagFn (*fn)[bag::kForms]);
 bag::BagUnitsFn bag_units_lean();
 bag::BagUnitsFn bag_units_full();
+bag::BagUnitsFn bag_units_mapped();
 bag::BagUnitsFn bag_units_wide();
 
 }  // namespace fbgemm_b200

@@ -1,4 +1,4 @@
-// The multi-table lookup kernel with all options (see bag_kernel.cuh).
+// The multi-table lookup kernel with all options but pruning maps (see bag_kernel.cuh).
 #include "bag_kernel.cuh"
 
 namespace fbgemm_b200 {

@@ -99,6 +99,7 @@ struct BagTable {
   int32_t data_bytes;         // packed payload bytes per row
   uint32_t flags;
   uint32_t limit;             // indices name rows below this (forms other than kWide)
+  uint32_t map_limit;         // a pruning map's rows below this lie within 32-bit byte offsets
   int16_t sb_align;           // address alignment of scale,bias: 8, 4, 2 or 1
   int16_t out_align;          // address alignment of output rows: 16 ... 1
   int32_t num_peers;

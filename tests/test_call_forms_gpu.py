@@ -105,3 +105,101 @@ def test_sequence_rows_keep_what_lies_between_them(gpu_ctx, D, n, filled):
         np.testing.assert_array_equal(got[k, :D], want, err_msg=f"row {k}")
         if not (filled and idx[k] >= rows):
             assert (got[k, D:] == 7.0).all(), f"row {k}: bytes between the rows were written"
+
+
+# ---- pruning maps into larger tables -------------------------------------------------
+
+BIG = (1 << 32) + (300 << 20)   # bytes of the table
+
+
+@pytest.fixture(scope="module")
+def big_table():
+    yield torch.zeros(BIG, dtype=torch.uint8, device="cuda")
+    torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("fmt", [8, 4, 2, "f32", "f16"])
+@pytest.mark.parametrize("batch", [40, 20_000, 60_000])
+@pytest.mark.parametrize("weights", [None, "per_index", "positional"])
+def test_pruning_map_into_a_table_beyond_4gb(gpu_ctx, oracle, big_table, fmt, batch, weights):
+    """The map is short, the table that it names rows of is not: rows on both sides of 4 GB, and the two next to it."""
+    rng = np.random.default_rng(batch + len(str(weights)))
+    dim = 128 if batch > 40 else 100
+    used_n, map_rows = 64, 300
+    quantized = fmt in (8, 4, 2)
+    compact = random_fused_table(rng, used_n, dim, fmt) if quantized else random_plain_table(rng, used_n, dim, fmt)
+    raw = compact.view(np.uint8).reshape(used_n, -1)
+    stride = raw.shape[1]
+    total = BIG // stride
+    edge = (1 << 32) // stride
+    used = np.unique(np.concatenate([[0, edge - 2, edge - 1, edge, edge + 1, total - 1],
+                                     rng.choice(total, 2 * used_n, replace=False)]))
+    used = np.sort(np.concatenate([rng.permutation(np.setdiff1d(used, [0, edge - 2, edge - 1, edge, edge + 1, total - 1]))[:used_n - 6],
+                                   [0, edge - 2, edge - 1, edge, edge + 1, total - 1]]))
+    big = big_table[:total * stride].view(total, stride)
+    big[torch.from_numpy(used).cuda()] = dev(raw)
+    to_compact = rng.integers(-1, used_n, map_rows).astype(np.int32)
+    to_big = np.where(to_compact >= 0, used[to_compact], -1).astype(np.int32)
+    lengths = rng.integers(0, 70, batch) if batch == 40 else rng.integers(0, 4, batch)
+    offsets = np.concatenate([[0], np.cumsum(lengths)]).astype(np.int32)
+    n = int(offsets[-1])
+    indices = rng.integers(0, map_rows, n).astype(np.int64)
+    positional = weights == "positional"
+    w = None if weights is None else rng.standard_normal(80 if positional else n).astype(np.float32)
+    kw = dict(index_dtype=np.int64, offset_dtype=np.int32)
+    if quantized:
+        ok_ref, ref = oracle.spmdm_rowwise_sparse(fmt, dim, map_rows, compact, indices, to_compact, offsets, w, False, positional)
+        gen = ((lambda *a: F.GenerateEmbeddingSpMDMRowWiseSparse(*a, **kw)) if fmt == 8
+               else (lambda *a: F.GenerateEmbeddingSpMDMNBitRowWiseSparse(fmt, *a, **kw)))
+    else:
+        ok_ref, ref = oracle.spmdm_plain_rowwise_sparse(fmt, dim, map_rows, compact, indices, to_compact, offsets, w, False,
+                                                        positional)
+        gen = lambda *a: F.GenerateEmbeddingSpMDMRowWiseSparse(  # noqa: E731
+            *a, in_dtype=np.float32 if fmt == "f32" else np.float16, **kw)
+    assert ok_ref
+    k = gen(dim, w is not None, False, 16, positional)
+    out = torch.ones(batch * dim, device="cuda")
+    assert k(batch, n, map_rows, big, dev(indices), dev(offsets), dev(w), out, dev(to_big))
+    big[torch.from_numpy(used).cuda()] = 0
+    np.testing.assert_array_equal(bits(out.cpu().numpy()), bits(ref[:batch * dim]))
+
+
+def test_pruning_maps_beside_other_tables_in_one_plan(gpu_ctx, oracle, big_table):
+    """Tables with and without a map, with rows on both sides of 4 GB, in one call."""
+    rng = np.random.default_rng(11)
+    dim, batch, rows, used_n = 128, 50, 200, 40
+    kw = dict(index_dtype=np.int64, offset_dtype=np.int32)
+    calls, checks = [], []
+    for t, fmt in enumerate((8, 4, 2, 4)):
+        compact = random_fused_table(rng, used_n, dim, fmt)
+        stride = compact.shape[1]
+        total, edge = BIG // stride, (1 << 32) // stride
+        used = np.unique(np.concatenate([[edge - 2, edge - 1, edge, edge + 1, total - 1 - t], t + 4 * rng.choice(total // 8, used_n - 5, replace=False)]))
+        compact = compact[:len(used)]
+        table = torch.zeros(1, dtype=torch.uint8)
+        if fmt != 4:
+            big_table.zero_() if t == 0 else None
+            table = big_table[:total * stride].view(total, stride) if t == 0 else torch.zeros((total, stride), dtype=torch.uint8, device="cuda")
+            table[torch.from_numpy(used).cuda()] = dev(compact)
+        n, indices, offsets = bags(rng, batch, rows)
+        offsets = offsets.astype(np.int32)
+        out = torch.ones(batch * dim, device="cuda")
+        if fmt == 4:      # no map
+            table, rows_of = dev(compact), len(used)
+            indices = indices % rows_of
+            ok_ref, ref = oracle.spmdm(4, dim, rows_of, compact, indices, offsets, None, False, np.float32)
+            k, cit = F.GenerateEmbeddingSpMDMNBit(4, dim, False, False, **kw), None
+        else:
+            rows_of, to_compact = rows, rng.integers(-1, len(used), rows).astype(np.int32)
+            ok_ref, ref = oracle.spmdm_rowwise_sparse(fmt, dim, rows, compact, indices, to_compact, offsets)
+            k = (F.GenerateEmbeddingSpMDMRowWiseSparse(dim, False, False, **kw) if fmt == 8
+                 else F.GenerateEmbeddingSpMDMNBitRowWiseSparse(fmt, dim, False, False, **kw))
+            cit = dev(np.where(to_compact >= 0, used[to_compact], -1).astype(np.int32))
+        assert ok_ref
+        calls.append((k, batch, n, rows_of, table, dev(indices), dev(offsets), None, out, cit))
+        checks.append((out, ref))
+    plan = F.MultiTablePlan(calls, 0, slot=45)
+    plan.launch()
+    assert F.status_read(45)[0]
+    for out, ref in checks:
+        np.testing.assert_array_equal(bits(out.cpu().numpy()), bits(ref[:batch * dim]))
