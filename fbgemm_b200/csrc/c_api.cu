@@ -635,6 +635,9 @@ void fbgemm_b200_ctx_destroy(fbgemm_b200_ctx* ctx) {
       cudaStreamDestroy(l.up);
     }
   }
+  for (fbgemm_b200_table_set* set : ctx->sets) {
+    set->ctx = nullptr;
+  }
   for (auto& kv : ctx->tables) {
     cudaFree(kv.second.buf.ptr);
   }
@@ -840,7 +843,6 @@ int fbgemm_b200_table_set_create(
     set_error("out of host memory");
     return FBGEMM_B200_ENOMEM;
   }
-  set->ctx = ctx;
   for (int t = 0; t < num_tables; ++t) {
     const fbgemm_b200_table_call& c = tables[t];
     int rc = fbgemm_b200_spmdm_check_config(&c.cfg);
@@ -858,6 +860,11 @@ int fbgemm_b200_table_set_create(
     set->tables.push_back(c);
     set->out_columns.push_back(out_columns[t]);
   }
+  {
+    std::lock_guard<std::mutex> lock(ctx->mu);
+    ctx->sets.insert(set);
+  }
+  set->ctx = ctx;
   *out = set;
   return 0;
 }
@@ -874,6 +881,10 @@ int fbgemm_b200_table_set_forward(
     void* stream) {
   if (!set || slot < 0 || slot >= FBGEMM_B200_USER_SLOTS || bags < 0 || !offsets || !out) {
     set_error("table_set_forward: bad argument");
+    return FBGEMM_B200_EINVAL;
+  }
+  if (!set->ctx) {
+    set_error("table_set_forward: the set's context was destroyed");
     return FBGEMM_B200_EINVAL;
   }
   if (bags == 0) {
@@ -903,6 +914,10 @@ int fbgemm_b200_table_set_forward(
 }
 
 void fbgemm_b200_table_set_destroy(fbgemm_b200_table_set* set) {
+  if (set && set->ctx) {
+    std::lock_guard<std::mutex> lock(set->ctx->mu);
+    set->ctx->sets.erase(set);
+  }
   delete set;
 }
 

@@ -4,6 +4,7 @@
 
 #include <mutex>
 #include <unordered_map>
+#include <unordered_set>
 
 #include "host_copy.h"
 #include "internal.h"
@@ -130,12 +131,13 @@ struct fbgemm_b200_ctx {
   std::unordered_map<cudaStream_t, fbgemm_b200::DeviceBuffer> scan;
   fbgemm_b200::DeviceBuffer remap_scratch;        // fbgemm_b200_compressed_indices_remap (one call at a time, it synchronises)
   std::unordered_map<const void*, fbgemm_b200::ResidentTable> tables;
+  std::unordered_set<fbgemm_b200_table_set*> sets;  // made with this context; they lose it when it is destroyed
   fbgemm_b200::Lane lanes[FBGEMM_B200_HOST_LANES];
 };
 
 // The tables of one table-batched operator (fbgemm_b200_table_set_*).
 struct fbgemm_b200_table_set {
-  fbgemm_b200_ctx* ctx = nullptr;
+  fbgemm_b200_ctx* ctx = nullptr;  // null once the context is destroyed
   std::vector<fbgemm_b200_table_call> tables;
   std::vector<int64_t> out_columns;
 };

@@ -286,8 +286,8 @@ FBGEMM_B200_API void fbgemm_b200_multi_plan_destroy(fbgemm_b200_multi_plan* plan
  * and has_weight the same for all tables), data_size and input are read;
  * out_columns[t] is the output column table t starts at.  Nothing else is
  * fixed: a forward call takes any batch and any arrays, allocates nothing on
- * the device and may run on several streams and threads at once.  The context
- * outlives the set. */
+ * the device and may run on several streams and threads at once.  A set whose
+ * context was destroyed is refused (and may still be destroyed). */
 typedef struct fbgemm_b200_table_set fbgemm_b200_table_set;
 
 FBGEMM_B200_API int fbgemm_b200_table_set_create(

@@ -203,3 +203,44 @@ def test_pruning_maps_beside_other_tables_in_one_plan(gpu_ctx, oracle, big_table
     assert F.status_read(45)[0]
     for out, ref in checks:
         np.testing.assert_array_equal(bits(out.cpu().numpy()), bits(ref[:batch * dim]))
+
+
+# ---- the tables of an operator -------------------------------------------------------
+
+def small_op(rng, tys=(ST.INT8, ST.INT4, ST.FP16), rows=(60, 50, 40), dims=(16, 32, 8), B=9, idt=np.int32):
+    tables, blob, w_off, D_off, offsets, indices, _ = build_op_inputs(rng, tys, dims, rows, B, 6, 4, False, idt)
+    op = tbe.IntNBitTableBatchedEmbeddingBags(dev(blob), w_off, np.array([int(t) for t in tys], np.uint8), D_off,
+                                              int(D_off[-1]), tbe.PoolingMode.SUM, 4, ST.FP32, False)
+    def want(oracle, blob=blob):
+        return oracle_op_forward(oracle, tys, dims, rows, blob, w_off, D_off, indices, offsets, None, B, False, 0, False, 4)
+    return op, blob, w_off, tables, dev(indices), dev(offsets), want
+
+
+def result(op, indices, offsets):
+    out = op.forward(indices, offsets, slot=42)
+    assert F.status_read(42)[0]
+    return out.cpu().numpy().view(np.uint32)
+
+
+def test_a_table_set_of_a_closed_context_is_refused(gpu_ctx):
+    rng = np.random.default_rng(5)
+    op, _, _, _, indices, offsets, _ = small_op(rng)
+    ctx = E.Context(0)
+    calls = (_capi.TableCall * op.T)()
+    columns = (C.c_int64 * op.T)(*[int(c) for c in op.D_offsets[:-1]])
+    for t in range(op.T):
+        calls[t].cfg, calls[t].data_size, calls[t].input = op.kernels[t].cfg, op.rows[t], op.tables[t].data_ptr()
+    sets = []
+    for _ in range(3):
+        h = C.c_void_p()
+        _capi.check(_capi.lib().fbgemm_b200_table_set_create(ctx.handle, calls, columns, op.T, C.byref(h)), "create")
+        sets.append(h)
+    out = torch.empty((9, op.total_D), device="cuda")
+    args = (9, indices.data_ptr(), indices.numel(), offsets.data_ptr(), None, out.data_ptr(), 0, None)
+    assert _capi.lib().fbgemm_b200_table_set_forward(sets[0], *args) == 0
+    torch.cuda.synchronize()
+    _capi.lib().fbgemm_b200_table_set_destroy(sets[1])   # before its context ...
+    ctx.close()
+    assert _capi.lib().fbgemm_b200_table_set_forward(sets[0], *args) == _capi.EINVAL
+    for h in (sets[0], sets[2]):                         # ... and after it
+        _capi.lib().fbgemm_b200_table_set_destroy(h)
