@@ -71,6 +71,36 @@ def _host(x, dtype):
     return np.asarray(x, dtype=dtype)
 
 
+class _TableSet:
+    """Owns one ``fbgemm_b200_table_set`` over an operator's tables."""
+
+    def __init__(self, op):
+        self.handle = None
+        self.tables = list(op.tables)   # kept alive
+        calls = (E._capi.TableCall * op.T)()
+        columns = (C.c_int64 * op.T)()
+        for t in range(op.T):
+            calls[t].cfg = op.kernels[t].cfg
+            calls[t].data_size = op.rows[t]
+            calls[t].input = E._ptr(op.tables[t])
+            columns[t] = int(op.D_offsets[t])
+        handle = C.c_void_p()
+        E._capi.check(E._capi.lib().fbgemm_b200_table_set_create(
+            E.get_context(op.device.index).handle, calls, columns, op.T, C.byref(handle)), "fbgemm_b200_table_set_create")
+        self.handle = handle.value
+
+    def __reduce__(self):
+        raise TypeError("a table set belongs to one process and one operator")
+
+    def __del__(self):
+        try:
+            if self.handle:
+                E._capi.lib().fbgemm_b200_table_set_destroy(self.handle)
+                self.handle = None
+        except Exception:
+            pass
+
+
 class IntNBitTableBatchedEmbeddingBags:
     """The tables of one table-batched operator and what does not change from
     call to call (row sizes, row counts, kernels)."""
@@ -137,29 +167,18 @@ class IntNBitTableBatchedEmbeddingBags:
         self._plans: dict = {}
         # every output column belongs to a table: the kernels write all of the output, which then need not be cleared
         self._covers_output = self.T > 0 and self.D_offsets[0] == 0 and self.D_offsets[-1] == self.total_D
-        self._set = self._make_set()
+        self._set = None   # made by the first call
 
-    def _make_set(self):
-        """The library's handle for these tables (``fbgemm_b200_table_set_*``)."""
-        calls = (E._capi.TableCall * self.T)()
-        columns = (C.c_int64 * self.T)()
-        for t in range(self.T):
-            calls[t].cfg = self.kernels[t].cfg
-            calls[t].data_size = self.rows[t]
-            calls[t].input = self.tables[t].data_ptr()
-            columns[t] = int(self.D_offsets[t])
-        handle = C.c_void_p()
-        E._capi.check(E._capi.lib().fbgemm_b200_table_set_create(
-            E.get_context(self.device.index).handle, calls, columns, self.T, C.byref(handle)), "fbgemm_b200_table_set_create")
-        return handle.value
+    def _table_set(self) -> "_TableSet":
+        """The library's handle for these tables."""
+        s = self._set
+        if s is None:
+            s = self._set = _TableSet(self)
+        return s
 
-    def __del__(self):
-        try:
-            if self._set:
-                E._capi.lib().fbgemm_b200_table_set_destroy(self._set)
-                self._set = None
-        except Exception:
-            pass
+    def __getstate__(self):
+        # a copy makes its own handles
+        return {**self.__dict__, "_set": None, "_plans": {}}
 
     def _calls(self, B, indices, offsets, indice_weights, output):
         flat = output.view(-1)
@@ -197,7 +216,8 @@ class IntNBitTableBatchedEmbeddingBags:
             self._plans[key] = plan
             plan.launch()
             return output
-        rc = E._capi.native().table_set_forward(self._set, B, indices, indices.numel(), offsets,
+        tables = self._table_set()   # (held until the call is enqueued)
+        rc = E._capi.native().table_set_forward(tables.handle, B, indices, indices.numel(), offsets,
                                                 indice_weights if self.weighted else None, output, slot,
                                                 E._current_stream(self.device.index))
         E._capi.check(rc, "fbgemm_b200_table_set_forward")

@@ -244,3 +244,22 @@ def test_a_table_set_of_a_closed_context_is_refused(gpu_ctx):
     assert _capi.lib().fbgemm_b200_table_set_forward(sets[0], *args) == _capi.EINVAL
     for h in (sets[0], sets[2]):                         # ... and after it
         _capi.lib().fbgemm_b200_table_set_destroy(h)
+
+
+# ---- copies of an operator -------------------------------------------------------------
+
+def test_copies_of_an_operator_have_tables_of_their_own(gpu_ctx, oracle):
+    rng = np.random.default_rng(4)
+    op, blob, w_off, tables, indices, offsets, want = small_op(rng)
+    ref = want(oracle)
+    np.testing.assert_array_equal(result(op, indices, offsets), ref)
+    shallow, deep = copy.copy(op), copy.deepcopy(op)
+    op.dev_weights.zero_()          # the deep copy's tables are its own
+    np.testing.assert_array_equal(result(deep, indices, offsets), ref)
+    op.dev_weights.copy_(dev(blob))
+    del op
+    np.testing.assert_array_equal(result(shallow, indices, offsets), ref)
+    del shallow
+    np.testing.assert_array_equal(result(deep, indices, offsets), ref)
+    k = copy.deepcopy(deep.kernels[0])
+    assert C.addressof(k.cfg) != C.addressof(deep.kernels[0].cfg)

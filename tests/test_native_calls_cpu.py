@@ -2,6 +2,7 @@
 reaches the library, seen through stand-ins for it."""
 import copy
 import ctypes as C
+import gc
 import importlib.machinery
 import importlib.util
 import os
@@ -11,10 +12,11 @@ import sysconfig
 
 import numpy as np
 import pytest
+import torch
 
 import fbgemm_b200 as F
 from fbgemm_b200 import _capi
-from fbgemm_b200 import build
+from fbgemm_b200 import build, tbe
 from fbgemm_b200 import embedding as E
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
@@ -75,6 +77,44 @@ def test_a_copied_kernel_calls_with_its_own_configuration(recorder, how):
     for name, args in recorder.calls:
         assert args[1] == C.addressof(c.cfg), name
         assert _capi.SpmdmConfig.from_address(args[1]).normalize_by_lengths == 1
+
+
+class FakeLibrary:
+    """Hands out table sets and counts how often each is given back."""
+
+    def __init__(self):
+        self.destroyed = {}
+
+    def fbgemm_b200_table_set_create(self, ctx, calls, columns, n, out):
+        out._obj.value = 1000 + len(self.destroyed)
+        self.destroyed[out._obj.value] = 0
+        return 0
+
+    def fbgemm_b200_table_set_destroy(self, handle):
+        self.destroyed[handle] += 1
+
+
+@pytest.mark.parametrize("how", [copy.copy, copy.deepcopy, lambda op: pickle.loads(pickle.dumps(op))])
+def test_copies_of_an_operator_give_back_one_table_set_each(monkeypatch, how):
+    library = FakeLibrary()
+    monkeypatch.setattr(_capi, "lib", lambda: library)
+    monkeypatch.setattr(E, "get_context", lambda device: type("Ctx", (), {"handle": None}))
+    k = object.__new__(F.SpmdmKernel)
+    k.cfg = _capi.SpmdmConfig()
+    op = object.__new__(tbe.IntNBitTableBatchedEmbeddingBags)
+    op.T, op.kernels, op.rows, op.D_offsets, op.device = 1, [k], [3], np.array([0, 4]), torch.device("cpu")
+    op.tables = [torch.zeros(48, dtype=torch.uint8)]
+    op._plans, op._set = {}, None
+    op._table_set()
+    other = how(op)
+    other._table_set()
+    assert other._table_set().handle is not None and len(library.destroyed) == 2
+    del op
+    gc.collect()
+    assert sorted(library.destroyed.values()) == [0, 1]
+    del other
+    gc.collect()
+    assert list(library.destroyed.values()) == [1, 1]
 
 
 # ---- the extension itself, over stand-ins for the library's functions ------------
