@@ -847,7 +847,7 @@ int fbgemm_b200_table_set_create(
     const fbgemm_b200_table_call& c = tables[t];
     int rc = fbgemm_b200_spmdm_check_config(&c.cfg);
     const auto& first = tables[0].cfg;
-    if (rc == 0 && (!c.cfg.absolute_offsets || !c.input || c.data_size < 0 || out_columns[t] < 0 ||
+    if (rc == 0 && (!c.cfg.absolute_offsets || c.data_size < 0 || out_columns[t] < 0 ||
                     c.cfg.index_bytes != first.index_bytes || c.cfg.offset_bytes != first.offset_bytes ||
                     c.cfg.has_weight != first.has_weight || c.cfg.out_dtype != first.out_dtype)) {
       set_error("table_set_create: tables take absolute offsets and share index, offset and output types");

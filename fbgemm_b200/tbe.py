@@ -25,6 +25,7 @@ from __future__ import annotations
 
 import ctypes as C
 import enum
+import operator
 
 import numpy as np
 import torch
@@ -167,12 +168,12 @@ class IntNBitTableBatchedEmbeddingBags:
         self._plans: dict = {}
         # every output column belongs to a table: the kernels write all of the output, which then need not be cleared
         self._covers_output = self.T > 0 and self.D_offsets[0] == 0 and self.D_offsets[-1] == self.total_D
-        self._set = None   # made by the first call
+        self._set = _TableSet(self) if self.T > 0 else None
 
     def _table_set(self) -> "_TableSet":
-        """The library's handle for these tables."""
+        """The library's handle for these tables, made again when one was put in place of another."""
         s = self._set
-        if s is None:
+        if s is None or len(s.tables) != len(self.tables) or not all(map(operator.is_, s.tables, self.tables)):
             s = self._set = _TableSet(self)
         return s
 

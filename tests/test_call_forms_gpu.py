@@ -246,6 +246,31 @@ def test_a_table_set_of_a_closed_context_is_refused(gpu_ctx):
         _capi.lib().fbgemm_b200_table_set_destroy(h)
 
 
+# ---- operators whose tables change, or that have none ---------------------------------
+
+def test_a_table_put_in_place_of_another_is_read(gpu_ctx, oracle):
+    rng = np.random.default_rng(3)
+    op, blob, w_off, tables, indices, offsets, want = small_op(rng)
+    np.testing.assert_array_equal(result(op, indices, offsets), want(oracle))
+    other = random_fused_table(rng, tables[1].shape[0], 32, 4, tables[1].shape[1], True)
+    op.tables[1] = dev(other.reshape(-1))
+    changed = blob.copy()
+    changed[int(w_off[1]):int(w_off[2])] = other.reshape(-1)
+    np.testing.assert_array_equal(result(op, indices, offsets), want(oracle, changed))
+    op.tables = [dev(blob[int(a):int(b)]) for a, b in zip(w_off, list(w_off[1:]) + [len(blob)])]
+    np.testing.assert_array_equal(result(op, indices, offsets), want(oracle))
+
+
+def test_operators_without_tables_and_with_empty_ones(gpu_ctx):
+    op = tbe.IntNBitTableBatchedEmbeddingBags(torch.zeros(0, dtype=torch.uint8, device="cuda"), [], [], [0], 0)
+    assert op.T == 0
+    # one table without rows: bags without indices pool to zeros
+    op = tbe.IntNBitTableBatchedEmbeddingBags(torch.zeros(0, dtype=torch.uint8, device="cuda"), [0], [int(ST.INT8)], [0, 16],
+                                              16, output_dtype=ST.FP32)
+    out = op.forward(torch.zeros(0, dtype=torch.int32, device="cuda"), torch.zeros(6, dtype=torch.int32, device="cuda"), slot=43)
+    assert F.status_read(43)[0] and out.shape == (5, 16) and (out.cpu() == 0).all()
+
+
 # ---- copies of an operator -------------------------------------------------------------
 
 def test_copies_of_an_operator_have_tables_of_their_own(gpu_ctx, oracle):
