@@ -18,6 +18,7 @@ from __future__ import annotations
 
 import ctypes as C
 import threading
+from ctypes import addressof
 
 import numpy as np
 
@@ -151,17 +152,13 @@ def _page_locked(x) -> bool:
     return torch.cuda.is_available() and (x if _is_tensor(x) else torch.from_numpy(x)).is_pinned()
 
 
-def _device_of(input) -> int:
-    """The device that reads a table: its own, or for one in page-locked host
-    memory the current one."""
-    dev = input.get_device()
-    if dev < 0:
-        import torch
+def _reading_device(input) -> int:
+    """The device that reads a table in page-locked host memory: the current one."""
+    import torch
 
-        if not _page_locked(input):
-            raise TypeError("the table has to be a CUDA tensor, or a tensor in page-locked memory")
-        dev = torch.cuda.current_device()
-    return dev
+    if not _page_locked(input):
+        raise TypeError("the table has to be a CUDA tensor, or a tensor in page-locked memory")
+    return torch.cuda.current_device()
 
 
 class SpmdmKernel:
@@ -181,9 +178,11 @@ class SpmdmKernel:
             raise ValueError("this kernel was not generated for row-wise sparse tables")
         self._check_dtypes(indices, offsets_or_lengths)
         if _is_tensor(input):
-            dev = _device_of(input)
+            dev = input.get_device()
+            if dev < 0:
+                dev = _reading_device(input)
             rc = _capi.native().spmdm(
-                _handle_of(dev), C.addressof(self.cfg), output_size, index_size, data_size, input, indices, offsets_or_lengths,
+                _handle_of(dev), addressof(self.cfg), output_size, index_size, data_size, input, indices, offsets_or_lengths,
                 weights if self.cfg.has_weight else None, out, compressed_indices_table, _current_stream(dev))
         else:
             ctx = get_context()
@@ -198,9 +197,11 @@ class SpmdmKernel:
                compressed_indices_table=None, slot: int = 0, stream=None) -> None:
         """Enqueue on ``stream`` (int handle; default torch's current stream)
         without synchronising; errors land in status slot ``slot``."""
-        dev = _device_of(input)
+        dev = input.get_device()
+        if dev < 0:
+            dev = _reading_device(input)
         rc = _capi.native().spmdm_launch(
-            _handle_of(dev), C.addressof(self.cfg), output_size, index_size, data_size, input, indices, offsets_or_lengths,
+            _handle_of(dev), addressof(self.cfg), output_size, index_size, data_size, input, indices, offsets_or_lengths,
             weights if self.cfg.has_weight else None, out, compressed_indices_table, slot,
             _current_stream(dev) if stream is None else stream)
         _capi.check(rc, "fbgemm_b200_spmdm_launch")
