@@ -16,6 +16,8 @@
 #include <thread>
 #include <vector>
 
+#include <unistd.h>
+
 namespace fbgemm_b200 {
 
 namespace {
@@ -26,6 +28,8 @@ constexpr auto kIdle = std::chrono::seconds(1);
 
 class Helpers {
  public:
+  const pid_t pid = getpid();
+
   ~Helpers() {
     {
       std::lock_guard<std::mutex> l(mu_);
@@ -40,7 +44,10 @@ class Helpers {
   bool copy(const CopySlice* slices, int count, int parts, bool ahead, const std::function<bool(int)>& ready,
             const std::function<bool(int)>& done) {
     // One copy at a time has the helpers.
-    std::unique_lock<std::mutex> mine(in_use_, std::try_to_lock);
+    std::unique_lock<std::mutex> mine(in_use_, std::defer_lock);
+    if (pid == getpid()) {
+      (void)mine.try_lock();
+    }
     size_t bytes = 0;
     for (int i = 0; i < count; ++i) {
       bytes += slices[i].bytes;
@@ -224,8 +231,18 @@ class Helpers {
 
 bool copy_slices(const CopySlice* slices, int count, int parts, bool ahead, const std::function<bool(int)>& ready,
                  const std::function<bool(int)>& done) {
-  static Helpers helpers;
-  return helpers.copy(slices, count, parts, ahead, ready, done);
+  // A forked child has neither the threads nor a use for the locks: it copies alone, and does not wait for threads that
+  // are not there when it exits.
+  struct Owner {
+    Helpers* helpers = new Helpers;
+    ~Owner() {
+      if (helpers->pid == getpid()) {
+        delete helpers;
+      }
+    }
+  };
+  static Owner owner;
+  return owner.helpers->copy(slices, count, parts, ahead, ready, done);
 }
 
 }  // namespace fbgemm_b200
