@@ -151,6 +151,7 @@ SIGNATURES = {
 
 _lib = None
 _native = None
+_build_error = None   # why the library was loaded as it was found
 
 
 def native():
@@ -159,15 +160,18 @@ def native():
     global _native
     if _native is None:
         lib()
-        from . import _native_calls
-
+        try:
+            from . import _native_calls
+        except ImportError as e:
+            built = f"; building it failed: {_build_error}" if _build_error else ""
+            raise Fbgemmb200Error(f"{_build.NATIVE_PATH} cannot be loaded: {e}{built}") from e
         _native = _native_calls
     return _native
 
 
 def lib() -> C.CDLL:
     """The loaded library (built first if the sources changed)."""
-    global _lib
+    global _lib, _build_error
     if _lib is None:
         path = _build.LIB_PATH
         if _build.needs_build():
@@ -177,6 +181,7 @@ def lib() -> C.CDLL:
                 if not os.path.exists(path):
                     raise Fbgemmb200Error(
                         f"libfbgemm_b200.so is missing and cannot be built: {e}") from e
+                _build_error = e
         handle = C.CDLL(path)
         for name, (restype, argtypes) in SIGNATURES.items():
             fn = getattr(handle, name)

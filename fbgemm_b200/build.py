@@ -29,7 +29,8 @@ CUDA_SOURCES = ["bag_units_lean.cu", "bag_units_full.cu", "bag_units_mapped.cu",
                 "c_api.cu", "noalloc_entry.cu", "peer_sync_kernels.cu", "multi_host.cu"]
 CXX_SOURCES = ["generators.cc", "host_copy.cc"]
 NATIVE_SOURCE = "native_calls.c"  # the CPython extension, linked against the library beside it
-NATIVE_PATH = os.path.join(PKG_DIR, "_native_calls.so")
+# (named and stamped for the interpreter it is built for: another one builds its own, and does not load this one)
+NATIVE_PATH = os.path.join(PKG_DIR, "_native_calls" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -65,6 +66,7 @@ def _fingerprint() -> str:
         with open(p, "rb") as f:
             h.update(f.read())
     h.update(" ".join(f for f in NVCC_FLAGS if not f.startswith(ROOT)).encode())
+    h.update(os.path.basename(NATIVE_PATH).encode())
     return h.hexdigest()
 
 
@@ -109,6 +111,9 @@ def build(force: bool = False, verbose: bool = False) -> str:
     link = [nvcc, "-shared", "-o", LIB_PATH, *objs, "-gencode", "arch=compute_100a,code=sm_100a",
             "-Xcompiler", "-fPIC"]
     subprocess.run(link, check=True)
+    unnamed = os.path.join(PKG_DIR, "_native_calls.so")   # any interpreter would load a file of this name
+    if os.path.exists(unnamed) and unnamed != NATIVE_PATH:
+        os.remove(unnamed)
     subprocess.run([shutil.which("gcc") or "cc", "-O2", "-Wall", "-shared", "-fPIC", "-I", INCLUDE,
                     "-I", sysconfig.get_paths()["include"], os.path.join(CSRC, NATIVE_SOURCE), "-o", NATIVE_PATH,
                     "-L", PKG_DIR, "-l:" + os.path.basename(LIB_PATH), "-Wl,-rpath,$ORIGIN"], check=True)

@@ -8,6 +8,7 @@ import importlib.util
 import os
 import pickle
 import subprocess
+import sys
 import sysconfig
 
 import numpy as np
@@ -115,6 +116,32 @@ def test_copies_of_an_operator_give_back_one_table_set_each(monkeypatch, how):
     del other
     gc.collect()
     assert list(library.destroyed.values()) == [1, 1]
+
+
+# ---- the extension's file ----------------------------------------------------------
+
+def test_another_interpreter_builds_its_own_extension(monkeypatch):
+    assert os.path.basename(build.NATIVE_PATH) == "_native_calls" + sysconfig.get_config_var("EXT_SUFFIX")
+    stamp = build._fingerprint()
+    monkeypatch.setattr(build, "NATIVE_PATH", build.NATIVE_PATH.replace("cpython-3", "cpython-9"))
+    assert build._fingerprint() != stamp
+    assert build.needs_build()
+
+
+def test_an_extension_that_could_not_be_built_is_named(monkeypatch):
+    def no_compiler():
+        raise RuntimeError("no Python.h here")
+
+    _capi.lib()
+    monkeypatch.setattr(build, "needs_build", lambda: True)
+    monkeypatch.setattr(build, "build", no_compiler)
+    for name in ("_lib", "_native", "_build_error"):
+        monkeypatch.setattr(_capi, name, None)
+    monkeypatch.setitem(sys.modules, "fbgemm_b200._native_calls", None)
+    monkeypatch.delattr(F, "_native_calls", raising=False)
+    _capi.lib()
+    with pytest.raises(_capi.Fbgemmb200Error, match="_native_calls.*no Python.h here"):
+        _capi.native()
 
 
 # ---- the extension itself, over stand-ins for the library's functions ------------
