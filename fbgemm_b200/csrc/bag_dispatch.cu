@@ -11,11 +11,14 @@ namespace {
 
 struct VariantInfo {
   int fmt, vb, cpl, g;
+  bool deep_mapped;  // compiled in the deep form with a pruning map alone
 };
 constexpr VariantInfo kVariantInfo[] = {
-#define INFO(FMT, VB, CPL, G) {bag::FMT, VB, CPL, G},
-    FBGEMM_B200_BAG_VARIANTS(INFO)
+#define INFO(FMT, VB, CPL, G) {bag::FMT, VB, CPL, G, false},
+#define INFO_DEEP_MAPPED(FMT, VB, CPL, G) {bag::FMT, VB, CPL, G, true},
+    FBGEMM_B200_BAG_VARIANTS(INFO) FBGEMM_B200_BAG_VARIANTS_DEEP_MAPPED(INFO_DEEP_MAPPED)
 #undef INFO
+#undef INFO_DEEP_MAPPED
 };
 
 // Largest power of two, 16 at most, that divides v.
@@ -79,7 +82,7 @@ int form_of(const BagTable& t) {
   return wide ? bag::kWide : t.flags & kPruned ? bag::kMapped : options || t.data_size == 0 ? bag::kFull : bag::kLean;
 }
 
-// Whole warps per bag while every bag of the launch finds a resident warp: the
+// Whole warps per bag while every bag on the chip finds a resident warp: the
 // fewer lanes share a bag, the longer its rows take, and nothing else is there
 // to run.  Beyond that narrow rows take half warps (one and the same walk serves
 // two bags), the narrowest quarter warps.  Measured, us, on bags of 30 rows at
@@ -89,16 +92,45 @@ int form_of(const BagTable& t) {
 // warps from 8 bags per resident warp on: 33000 bags of 2-bit D = 64 take 39.5 us
 // with them and 33.6 without, 4-bit 40.4 and 38.7, 64 mixed tables of 512 bags
 // 53.3 and 50.6; 100000 bags of 4-bit D = 64 86.5 and 91.9.
+//
+// Launches on other streams (launch_history.h) are on the chip too, but a quarter
+// of their bags counts against whole warps: a small launch spends most of its
+// time in start-up and drain.  us per call on 1, 2, 4, 8, 16 streams with
+// 32 / 16 / 8 lanes, 4-bit D = 64, 4096 bags of 30 rows at 10 M rows:
+//   10.2 / 13.1 / 17.6,  5.7 / 7.1 / 9.2,  4.4 / 4.4 / 5.3,  4.4 / 3.5 / 3.8,  4.0 / 3.3 / 3.2
+// (by its own size alone every such launch took whole warps and the deep form,
+// 5.0 us from four streams on).  Behind a pruning map quarter warps pay from 4
+// bags per resident warp on, 8192 bags of 2-bit D = 128 at 20 M rows, 2, 4 and 16
+// streams: 8.5 / 9.6 / 10.8,  8.3 / 8.9 / 7.6,  7.9 / 8.6 / 7.1.
 constexpr int64_t kResidentWarps = 148 * bag::kBlocksPerSm * bag::kWarps;
 
-int pick_variant(const BagTable& t, int fmt, int64_t bags_in_launch, int* tiles) {
+// Bags that a launch and those beside it keep on the chip at a time.
+int64_t bags_at_a_time(int64_t bags, int64_t beside) {
+  return bags + beside / 4;
+}
+
+int64_t blocks_of(int64_t bags, int variant) {
+  const int64_t per_block = (int64_t)bag::kWarps * (32 / kVariantInfo[variant].g);
+  return (bags + per_block - 1) / per_block;
+}
+
+// Blocks of the deep form that fit the chip at once.
+constexpr int64_t kDeepFit = 148 * bag::kDeepBlocksPerSm;
+
+// `bags` in the launch, `beside` in those on other streams; `single`: one table's launch.
+int pick_variant(const BagTable& t, int fmt, int64_t bags, int64_t beside, bool single, int* tiles) {
   const int align = alignment_of(reinterpret_cast<uintptr_t>(t.data) | (uint64_t)t.stride);
-  const int least_g = bags_in_launch <= kResidentWarps ? 32 : bags_in_launch <= 8 * kResidentWarps ? 16 : 8;
+  const bool mapped = t.flags & kPruned;
+  const int64_t quarter_warps_from = (mapped && beside > 0 ? 4 : 8) * kResidentWarps;
+  const int least_g = bags_at_a_time(bags, beside) <= kResidentWarps ? 32 : bags + beside <= quarter_warps_from ? 16 : 8;
   int best = -1;
   double best_cost = 0;
   for (int i = 0; i < bag::kVariants; ++i) {
     const VariantInfo& v = kVariantInfo[i];
     if (v.fmt != fmt || v.vb > align || v.g < least_g) {
+      continue;
+    }
+    if (v.deep_mapped && !(single && form_of(t) == bag::kMapped && blocks_of(bags, i) <= 2 * kDeepFit)) {
       continue;
     }
     // the last chunk may run into scale,bias behind the payload, but not beyond the row
@@ -120,11 +152,6 @@ int pick_variant(const BagTable& t, int fmt, int64_t bags_in_launch, int* tiles)
     }
   }
   return best;
-}
-
-int64_t blocks_of(const BagTable& t, int variant) {
-  const int64_t per_block = (int64_t)bag::kWarps * (32 / kVariantInfo[variant].g);
-  return (t.bags + per_block - 1) / per_block;
 }
 
 bag::BagFn single_kernel(int variant, int form) {
@@ -168,21 +195,21 @@ cudaError_t launch_bags(const SpmdmParams& p, int bit_rate, cudaStream_t stream)
     c.peers[i] = p.peer_out[i];
   }
   int tiles = 0;
-  const int v = pick_variant(c.t, format_of(p, bit_rate), p.output_size, &tiles);
-  const int64_t blocks = blocks_of(c.t, v);
+  const int v = pick_variant(c.t, format_of(p, bit_rate), p.output_size, p.bags_beside, true, &tiles);
+  const int64_t blocks = blocks_of(p.output_size, v);
   if (blocks <= 0 || blocks > 0x7fffffffLL || tiles > 65535) {
     return cudaErrorInvalidValue;
   }
-  int form = form_of(c.t);
-  form = form == bag::kMapped ? (int)bag::kFull : form;  // one kernel for both
-  // The deep form while the launch fits the chip at once; with a pruning map, one more trip to memory in every stretch,
-  // up to two such launches' worth: 2-bit D = 128, 11000 bags 16.9 against 14.5 us, 14000 20.0 / 18.5, 20000 27.6 / 25.5.
-  // (Dense tables lose there: 8-bit D = 128, 14000 bags 29.7 against 33.6.)
-  const int64_t fit = 148 * bag::kDeepBlocksPerSm * (c.t.flags & kPruned ? 2 : 1);
-  if (form != bag::kWide && blocks * tiles <= fit) {
-    form += 3;
-  }
-  return launch<bag::BagCall>(single_kernel(v, form), dim3((unsigned)blocks, (unsigned)tiles), c, stream);
+  // The deep form while what is on the chip fits it at once.  With a pruning map, one more trip to memory in every
+  // stretch, up to two such launches' worth and whatever runs beside: 2-bit D = 128, 11000 bags 16.9 against 14.5 us,
+  // 14000 20.0 / 18.5, 20000 27.6 / 25.5; quarter warps on 16 streams 9.5 / 7.1.  (Dense tables lose there: 8-bit D = 128,
+  // 14000 bags 29.7 against 33.6; 10000 bags on 16 streams 7.0 against 8.3.  Narrower groups do once anything runs beside
+  // them: 4-bit D = 64, 4096 bags on 16 streams 3.2 against 3.6.)
+  const int form = form_of(c.t);
+  const int64_t bags = kVariantInfo[v].g == 32 ? bags_at_a_time(p.output_size, p.bags_beside) : p.output_size + p.bags_beside;
+  const bool deep = form == bag::kMapped ? blocks * tiles <= 2 * kDeepFit
+                                         : form != bag::kWide && blocks_of(bags, v) * tiles <= kDeepFit;
+  return launch<bag::BagCall>(single_kernel(v, deep ? bag::kDeepForms + form : form), dim3((unsigned)blocks, (unsigned)tiles), c, stream);
 }
 
 // ---- several tables per launch --------------------------------------------------
@@ -218,8 +245,8 @@ cudaError_t build_multi_plan(const SpmdmParams* tables, const int* bit_rates, si
     }
     int tiles = 0;
     bag_table_of(tables[t], &bag_tables[t]);
-    const int v = pick_variant(bag_tables[t], format_of(tables[t], bit_rates[t]), bags, &tiles);
-    const int64_t blocks = blocks_of(bag_tables[t], v);
+    const int v = pick_variant(bag_tables[t], format_of(tables[t], bit_rates[t]), bags, 0, false, &tiles);
+    const int64_t blocks = blocks_of(tables[t].output_size, v);
     if (blocks > 0x7fffffffLL || tiles > 65535) {
       return cudaErrorInvalidValue;
     }

@@ -388,8 +388,7 @@ struct __align__(16) Queue {
 //  kLean  bags by offsets, weights per index, every index a row of the table
 //  kFull  besides: -1 as a pruned index, no_bag, positional
 //         weights, lengths in place of offsets
-//  kMapped  besides: pruning maps (the single-table kernels know no kFull without them; for 64 table-batched tables the
-//         maps' part, unused, cost 4 %)
+//  kMapped  besides: pruning maps (their part, unused, cost 64 table-batched tables 4 %, 3000 bags by lengths 2 %)
 //  kWide  the same where positions, bags (31 bits) or row offsets (32) need more
 // The lean form saves the queue's compaction and half of the tests, a tenth of
 // the time of 65536 bags of 30 rows (8-bit D = 128 76.4 against 83.6 us).
@@ -729,6 +728,9 @@ __device__ __forceinline__ void pool_bags(const BagTable& p, void* const* peers,
         }
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
+          if (MAPS && kDeep && u == 2 && r + 2 >= most) {
+            break;  // half of a stretch's rows are gone: the last group is often half empty (4-bit D = 128, 13.8 / 12.1 us)
+          }
           if constexpr (kQuantized) {
             const ulonglong2 s = q_sb[r + u];
             C::pool(constants, acc, d[g][u], s.x, s.y);
@@ -837,8 +839,14 @@ __global__ void __launch_bounds__(kThreads, kDeepBlocksPerSm) bag_kernel_deep(co
 #define FBGEMM_B200_BAG_VARIANTS(X) \
   FBGEMM_B200_BAG_VARIANTS_8(X) FBGEMM_B200_BAG_VARIANTS_4(X) FBGEMM_B200_BAG_VARIANTS_2(X) FBGEMM_B200_BAG_VARIANTS_PLAIN(X)
 
+// Behind a pruning map, and when launches on other streams fill the chip: 16 columns a lane, which want the deep form's
+// registers (the other forms would spill).
+#define FBGEMM_B200_BAG_VARIANTS_DEEP_MAPPED(X) X(kInt2, 4, 1, 8)
+
 #define FBGEMM_B200_BAG_ID(FMT, VB, CPL, G) id_##FMT##_##VB##_##CPL##_##G,
-enum VariantId : int { FBGEMM_B200_BAG_VARIANTS(FBGEMM_B200_BAG_ID) kVariants };
+enum VariantId : int {
+  FBGEMM_B200_BAG_VARIANTS(FBGEMM_B200_BAG_ID) FBGEMM_B200_BAG_VARIANTS_DEEP_MAPPED(FBGEMM_B200_BAG_ID) kVariants
+};
 #undef FBGEMM_B200_BAG_ID
 
 // Several tables per launch (what the reference's multi-table caller does with
@@ -886,7 +894,8 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm) bag_units_kernel(const
 }
 
 using BagFn = void (*)(const BagCall);
-constexpr int kForms = 5;  // kLean, kMapped, kWide, and the deep forms of kLean and kMapped
+constexpr int kDeepForms = 4;             // kDeepForms + form: its deep form (there is none of kWide)
+constexpr int kForms = 2 * kDeepForms;
 using BagUnitsFn = void (*)(const BagUnits);
 
 }  // namespace bag

@@ -297,7 +297,8 @@ int fbgemm_b200::enqueue_lookup(
     cudaStream_t stream,
     void* const* peer_out,
     int num_peers,
-    int64_t bags_per_peer) {
+    int64_t bags_per_peer,
+    int64_t bags_beside) {
   if (cfg && cfg->out_dtype == FBGEMM_B200_OUT_U8) {
     Derived d;
     const int rc = check_config(cfg, &d);
@@ -354,6 +355,7 @@ int fbgemm_b200::enqueue_lookup(
     flags |= kOff64;
   }
   p.flags = flags;
+  p.bags_beside = bags_beside;
 
   cudaError_t e = launch_spmdm(p, cfg->bit_rate, stream);
   if (e != cudaSuccess) {
@@ -389,16 +391,17 @@ int enqueue_on_stream(
     const int32_t* cit,
     int32_t* status,
     cudaStream_t stream) {
+  const int64_t beside = ctx->history.launched(stream, output_size);
   if (cfg && !cfg->use_offsets && !cfg->no_bag) {
     // Lengths mode: the scanned offsets live in scratch that belongs to the
     // stream, so that launches on different streams never share it.
     std::lock_guard<std::mutex> lock(ctx->mu);
     return enqueue_lookup(cfg, output_size, index_size, data_size, input, indices, offsets_or_lengths, weights, out, cit,
-                          status, scan_scratch_of(ctx, stream), stream);
+                          status, scan_scratch_of(ctx, stream), stream, nullptr, 0, 0, beside);
   }
   DeviceBuffer unused;  // only lengths mode touches the scratch
   return enqueue_lookup(cfg, output_size, index_size, data_size, input, indices, offsets_or_lengths, weights, out, cit,
-                        status, unused, stream);
+                        status, unused, stream, nullptr, 0, 0, beside);
 }
 
 int pruned_lookup(
@@ -737,7 +740,7 @@ int fbgemm_b200_spmdm_launch_sharded(
   DeviceBuffer unused;  // offsets mode: no scratch
   return enqueue_lookup(cfg, output_size, index_size, data_size, input, indices, offsets, weights, nullptr, nullptr,
                         ctx->status + 4 * slot, unused, static_cast<cudaStream_t>(stream), peer_out, num_peers,
-                        bags_per_peer);
+                        bags_per_peer, ctx->history.launched(stream, output_size));
 }
 
 int fbgemm_b200_multi_plan_create(
@@ -936,6 +939,7 @@ int fbgemm_b200_status_read(fbgemm_b200_ctx* ctx, int slot, void* stream, int32_
   if (e != cudaSuccess) {
     return fail_cuda(e, "status read");
   }
+  ctx->history.waited(s);
   int32_t rec[4] = {h[0], h[1], h[2], h[3]};
   if (info) {
     std::memcpy(info, rec, sizeof(rec));
@@ -985,6 +989,7 @@ int fbgemm_b200_spmdm(
   if (e != cudaSuccess) {
     return fail_cuda(e, "lookup");
   }
+  ctx->history.waited(stream);
   return take_record(ctx->sync_status) == 0 ? 1 : 0;
 }
 

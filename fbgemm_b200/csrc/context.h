@@ -8,6 +8,7 @@
 
 #include "host_copy.h"
 #include "internal.h"
+#include "launch_history.h"
 
 namespace fbgemm_b200 {
 
@@ -132,6 +133,7 @@ struct fbgemm_b200_ctx {
   fbgemm_b200::DeviceBuffer remap_scratch;        // fbgemm_b200_compressed_indices_remap (one call at a time, it synchronises)
   std::unordered_map<const void*, fbgemm_b200::ResidentTable> tables;
   std::unordered_set<fbgemm_b200_table_set*> sets;  // made with this context; they lose it when it is destroyed
+  fbgemm_b200::LaunchHistory history;             // single-table launches
   fbgemm_b200::Lane lanes[FBGEMM_B200_HOST_LANES];
 };
 

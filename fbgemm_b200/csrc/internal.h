@@ -45,6 +45,7 @@ struct SpmdmParams {
   int64_t output_stride;      // elements between output rows
   int64_t output_size;        // bags
   int64_t index_size;         // indices
+  int64_t bags_beside;        // bags of other launches that the chip is taken to be busy with
   int32_t block_size;         // D
   int32_t data_bytes;         // packed payload bytes per row
   int32_t data_row_off;       // offset of the payload inside a table row (0, or 4 when scale,bias come first)
@@ -286,7 +287,8 @@ int enqueue_lookup(
     cudaStream_t stream,
     void* const* peer_out = nullptr,
     int num_peers = 0,
-    int64_t bags_per_peer = 0);
+    int64_t bags_per_peer = 0,
+    int64_t bags_beside = 0);
 
 // The validation and parameter set-up half of enqueue_lookup (offsets are left
 // for the caller to fill in).

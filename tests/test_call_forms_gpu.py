@@ -288,3 +288,40 @@ def test_copies_of_an_operator_have_tables_of_their_own(gpu_ctx, oracle):
     np.testing.assert_array_equal(result(deep, indices, offsets), ref)
     k = copy.deepcopy(deep.kernels[0])
     assert C.addressof(k.cfg) != C.addressof(deep.kernels[0].cfg)
+
+
+# ---- overlapping calls of one table ----------------------------------------------------
+
+@pytest.mark.parametrize("bit_rate,dim,batch", [(8, 128, 1000), (8, 86, 301), (8, 128, 4096), (4, 64, 700),
+                                                (4, 33, 4096), (4, 64, 4096), (2, 128, 1024), (2, 128, 4096), (2, 112, 2500),
+                                                (2, 100, 4096)])
+@pytest.mark.parametrize("pruned", [False, True])
+def test_calls_that_overlap_on_several_streams(gpu_ctx, oracle, bit_rate, dim, batch, pruned):
+    """Which kernel takes a call depends on what runs beside it; the rows do not."""
+    rng = np.random.default_rng(bit_rate * dim + batch)
+    rows, calls = 500, 40
+    table = random_fused_table(rng, rows, dim, bit_rate)
+    cit = np.where(rng.random(rows) < 0.4, -1, rng.permutation(rows)).astype(np.int32) if pruned else None
+    n, indices, offsets = bags(rng, batch, rows, 70)
+    if pruned:
+        ok_ref, ref = oracle.spmdm_rowwise_sparse(bit_rate, dim, rows, table, indices, cit, offsets, None, True)
+        k = (F.GenerateEmbeddingSpMDMRowWiseSparse(dim, False, True, index_dtype=np.int64, offset_dtype=np.int64) if bit_rate == 8
+             else F.GenerateEmbeddingSpMDMNBitRowWiseSparse(bit_rate, dim, False, True, index_dtype=np.int64, offset_dtype=np.int64))
+    else:
+        ok_ref, ref = oracle.spmdm(bit_rate, dim, rows, table, indices, offsets, None, True, np.float32)
+        k = (F.GenerateEmbeddingSpMDM(dim, False, True, index_dtype=np.int64, offset_dtype=np.int64) if bit_rate == 8
+             else F.GenerateEmbeddingSpMDMNBit(bit_rate, dim, False, True, index_dtype=np.int64, offset_dtype=np.int64))
+    assert ok_ref
+    args = (dev(table), dev(indices), dev(offsets), None)
+    outs = torch.ones(calls, batch * dim, device="cuda")
+    d_cit = (dev(cit),) if pruned else ()
+    streams = [torch.cuda.Stream() for _ in range(16)]
+    torch.cuda.synchronize()
+    for c in range(calls):          # one stream first, then all of them, then one again
+        s = streams[c % 16 if 8 <= c < 32 else 0]
+        k.launch(batch, n, rows, *args, outs[c], *d_cit, slot=44, stream=s.cuda_stream)
+    torch.cuda.synchronize()
+    assert F.status_read(44)[0]
+    want = bits(ref[:batch * dim])
+    for c in range(calls):
+        np.testing.assert_array_equal(bits(outs[c].cpu().numpy()), want, err_msg=f"call {c}")
