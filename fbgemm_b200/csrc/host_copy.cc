@@ -14,7 +14,6 @@
 #include <cstring>
 #include <mutex>
 #include <thread>
-#include <vector>
 
 #include <unistd.h>
 
@@ -25,6 +24,7 @@ namespace {
 constexpr int kHelpers = 3;
 constexpr size_t kWorthHelp = 512 * 1024;  // waking the helpers costs the copy of a few hundred KB
 constexpr auto kIdle = std::chrono::seconds(1);
+constexpr int kSpins = 2000;  // some 50 us without a slice to copy, then a helper sleeps
 
 class Helpers {
  public:
@@ -37,7 +37,9 @@ class Helpers {
     }
     wake_.notify_all();
     for (auto& t : threads_) {
-      t.join();
+      if (t.joinable()) {
+        t.join();
+      }
     }
   }
 
@@ -52,7 +54,14 @@ class Helpers {
     for (int i = 0; i < count; ++i) {
       bytes += slices[i].bytes;
     }
-    const bool helped = mine.owns_lock() && bytes >= kWorthHelp && open(slices, count, ahead ? count : 0);
+    struct Closing {  // however the copy ends, no helper holds a slice of it afterwards
+      Helpers* helpers = nullptr;
+      ~Closing() {
+        if (helpers) {
+          helpers->close();
+        }
+      }
+    } closing;
     bool ok = true;
     int end = 0;  // slices of the parts so far
     for (int p = 0; p < parts && ok; ++p) {
@@ -62,13 +71,17 @@ class Helpers {
           break;
         }
       }
+      // the helpers are not taken before there is something to copy
+      if (p == 0 && mine.owns_lock() && bytes >= kWorthHelp && open(slices, count, ahead ? count : 0)) {
+        closing.helpers = this;
+      }
       const int begin = end;
       while (end < count && slices[end].part <= p) {
         ++end;
       }
-      if (helped) {
+      if (closing.helpers) {
         if (!ahead) {
-          ready_.store(end, std::memory_order_release);
+          publish(end);
         }
         if (done) {
           while (left_[p].load(std::memory_order_acquire) > 0) {
@@ -84,10 +97,7 @@ class Helpers {
       }
       ok = !done || done(p);
     }
-    if (helped) {
-      while (claim_one()) {
-      }
-      close();
+    while (closing.helpers && claim_one()) {
     }
     return ok;
   }
@@ -136,24 +146,40 @@ class Helpers {
     return false;
   }
 
+  // Slices below `end` may be copied.  (Sequentially consistent, as work()'s counterpart is: either the sleeper is seen
+  // here or it sees the new end.)
+  void publish(int end) {
+    ready_.store(end);
+    if (sleeping_.load() > 0) {
+      { std::lock_guard<std::mutex> l(mu_); }
+      wake_.notify_all();
+    }
+  }
+
   bool open(const CopySlice* slices, int count, int ready) {
     std::lock_guard<std::mutex> l(mu_);
     if (stop_) {
       return false;
     }
-    reap();
-    const unsigned cores = std::thread::hardware_concurrency();
-    const int want = cores > kHelpers + 1 ? kHelpers : 0;
-    while ((int)threads_.size() < want) {
-      try {
-        const size_t slot = threads_.size();
-        gone_[slot] = false;
-        threads_.emplace_back([this, slot] { work(slot); });
-      } catch (...) {
-        break;  // no thread to be had: the callers copy
-      }
+    if (std::thread::hardware_concurrency() <= kHelpers + 1) {
+      return false;
     }
-    if (threads_.empty()) {
+    int have = 0;
+    for (int i = 0; i < kHelpers; ++i) {
+      if (threads_[i].joinable() && gone_[i]) {
+        threads_[i].join();  // left for want of work
+      }
+      if (!threads_[i].joinable()) {
+        try {
+          gone_[i] = false;
+          threads_[i] = std::thread([this, i] { work(i); });
+        } catch (...) {
+          break;  // no thread to be had: fewer helpers, or the caller alone
+        }
+      }
+      ++have;
+    }
+    if (have == 0) {
       return false;
     }
     slices_ = slices;
@@ -174,23 +200,11 @@ class Helpers {
   void close() {
     std::unique_lock<std::mutex> l(mu_);
     open_.store(false, std::memory_order_release);
+    wake_.notify_all();
     done_.wait(l, [this] { return busy_ == 0; });
   }
 
-  // Threads that left for want of work (mu_ held).
-  void reap() {
-    for (size_t i = 0; i < threads_.size(); ++i) {
-      if (!gone_[i]) {
-        return;  // they leave together or not at all worth restarting one by one
-      }
-    }
-    for (auto& t : threads_) {
-      t.join();
-    }
-    threads_.clear();
-  }
-
-  void work(size_t slot) {
+  void work(int slot) {
     std::unique_lock<std::mutex> l(mu_);
     while (true) {
       if (!wake_.wait_for(l, kIdle, [this] { return stop_ || open_.load(std::memory_order_acquire); })) {
@@ -202,9 +216,18 @@ class Helpers {
       }
       ++busy_;
       l.unlock();
-      while (open_.load(std::memory_order_acquire)) {
-        if (!claim_one()) {
+      for (int idle = 0; open_.load(std::memory_order_acquire);) {
+        if (claim_one()) {
+          idle = 0;
+        } else if (++idle < kSpins) {
           pause();
+        } else {
+          l.lock();
+          sleeping_.fetch_add(1);
+          wake_.wait(l, [this] { return !open_.load() || claimed_.load() < ready_.load(); });
+          sleeping_.fetch_sub(1);
+          l.unlock();
+          idle = 0;
         }
       }
       l.lock();
@@ -217,12 +240,12 @@ class Helpers {
   std::mutex in_use_;
   std::mutex mu_;
   std::condition_variable wake_, done_;
-  std::vector<std::thread> threads_;
+  std::thread threads_[kHelpers];
   bool gone_[kHelpers] = {};
   bool stop_ = false;
   int busy_ = 0;
   std::atomic<bool> open_{false};
-  std::atomic<int> claimed_{0}, ready_{0};
+  std::atomic<int> claimed_{0}, ready_{0}, sleeping_{0};
   std::atomic<int> left_[kCopyParts] = {};  // slices of each part that are not copied yet
   const CopySlice* slices_ = nullptr;
 };

@@ -22,6 +22,7 @@ def driver(tmp_path_factory):
 @pytest.mark.parametrize("what", [
     "exact",   # every byte arrives; a copy that ends early leaves nothing behind
     "fork",    # a forked child copies alone and ends
+    "idle",    # waiting for a transfer keeps no core busy
     "again",   # helpers that left for want of work come back
 ])
 def test_copies(driver, what):
