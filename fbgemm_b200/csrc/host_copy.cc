@@ -23,6 +23,12 @@ namespace {
 
 constexpr int kHelpers = 3;
 constexpr size_t kWorthHelp = 512 * 1024;  // waking the helpers costs the copy of a few hundred KB
+// Uploads go past the caches: the GPU alone reads the staging block, and its lines need not be fetched first (253 -> 218 us
+// for the call of 10 000 bags in c_api.cu). So do results from this size on. Smaller ones are left in the caches for the
+// caller, who reads them next; us for the call and a sum over its rows, past / through the caches:
+// 64 KB 67 / 58, 256 KB 104 / 72, 512 KB 146 / 114, 1 MB 235 / 172, 2 MB 405 / 284; 5 MB 812 / 861, 10 MB 1480 / 1430 (the rows
+// then come out of other cores' caches), 75 MB 11500 / 11600.
+constexpr size_t kPastCaches = 4 << 20;
 constexpr auto kIdle = std::chrono::seconds(1);
 constexpr int kSpins = 2000;  // some 100 us without a slice to copy, then a helper sleeps
 
@@ -54,6 +60,7 @@ class Helpers {
     for (int i = 0; i < count; ++i) {
       bytes += slices[i].bytes;
     }
+    const bool past = ahead || bytes >= kPastCaches;
     struct Closing {  // however the copy ends, no helper holds a slice of it afterwards
       Helpers* helpers = nullptr;
       ~Closing() {
@@ -75,7 +82,7 @@ class Helpers {
         }
       }
       // the helpers are not taken before there is something to copy
-      if (p == 0 && mine.owns_lock() && bytes >= kWorthHelp && open(slices, count, ahead ? count : 0)) {
+      if (p == 0 && mine.owns_lock() && bytes >= kWorthHelp && open(slices, count, ahead ? count : 0, past)) {
         closing.helpers = this;
       }
       const int begin = end;
@@ -95,7 +102,7 @@ class Helpers {
         }
       } else {
         for (int i = begin; i < end; ++i) {
-          take(slices[i]);
+          take(slices[i], past);
         }
       }
       ok = !done || done(p);
@@ -106,12 +113,10 @@ class Helpers {
   }
 
  private:
-  // Past the caches: neither side of the copy is read again from them, and the lines of the destination need not be
-  // fetched first (253 -> 218 us for the call of 10 000 bags below).
-  static void take(const CopySlice& s) {
+  static void take(const CopySlice& s, bool past) {
     size_t done = 0;
 #if defined(__x86_64__)
-    if (reinterpret_cast<uintptr_t>(s.dst) % 16 == 0) {
+    if (past && reinterpret_cast<uintptr_t>(s.dst) % 16 == 0) {
       const __m128i* from = static_cast<const __m128i*>(s.src);
       __m128i* to = static_cast<__m128i*>(s.dst);
       for (; done + 64 <= s.bytes; done += 64, from += 4, to += 4) {
@@ -141,7 +146,7 @@ class Helpers {
     int i = claimed_.load(std::memory_order_relaxed);
     while (i < ready_.load(std::memory_order_acquire)) {
       if (claimed_.compare_exchange_weak(i, i + 1, std::memory_order_acq_rel)) {
-        take(slices_[i]);
+        take(slices_[i], past_);
         left_[slices_[i].part].fetch_sub(1, std::memory_order_acq_rel);
         return true;
       }
@@ -195,12 +200,13 @@ class Helpers {
     return have > 0;
   }
 
-  bool open(const CopySlice* slices, int count, int ready) {
+  bool open(const CopySlice* slices, int count, int ready, bool past) {
     std::lock_guard<std::mutex> l(mu_);
     if (stop_ || !start()) {
       return false;
     }
     slices_ = slices;
+    past_ = past;
     for (auto& l : left_) {
       l.store(0, std::memory_order_relaxed);
     }
@@ -277,6 +283,7 @@ class Helpers {
   std::atomic<int> claimed_{0}, ready_{0}, sleeping_{0};
   std::atomic<int> left_[kCopyParts] = {};  // slices of each part that are not copied yet
   const CopySlice* slices_ = nullptr;
+  bool past_ = false;
 };
 
 }  // namespace
