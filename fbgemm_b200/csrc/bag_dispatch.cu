@@ -1,6 +1,7 @@
 // Which bag kernel (bag_kernel.cuh) takes a lookup, and how many tables go into
 // one launch.
 #include <algorithm>
+#include <atomic>
 #include <vector>
 
 #include "bag_kernel.cuh"
@@ -82,6 +83,32 @@ int form_of(const BagTable& t) {
   return wide ? bag::kWide : t.flags & kPruned ? bag::kMapped : options || t.data_size == 0 ? bag::kFull : bag::kLean;
 }
 
+// The current device's SMs.
+int64_t sm_count() {
+  constexpr int kDevices = 64;
+  static std::atomic<int> counts[kDevices];
+  int device = 0, n = 0;
+  if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= kDevices) {
+    return 148;
+  }
+  n = counts[device].load(std::memory_order_relaxed);
+  if (n == 0) {
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || n <= 0) {
+      return 148;
+    }
+    counts[device].store(n, std::memory_order_relaxed);
+  }
+  return n;
+}
+
+// Warps that are resident on `sms` SMs at a time, and blocks of the deep form.
+int64_t resident_warps(int64_t sms) {
+  return sms * bag::kBlocksPerSm * bag::kWarps;
+}
+int64_t deep_fit(int64_t sms) {
+  return sms * bag::kDeepBlocksPerSm;
+}
+
 // Whole warps per bag while every bag on the chip finds a resident warp: the
 // fewer lanes share a bag, the longer its rows take, and nothing else is there
 // to run.  Beyond that narrow rows take half warps (one and the same walk serves
@@ -102,8 +129,6 @@ int form_of(const BagTable& t) {
 // 5.0 us from four streams on).  Behind a pruning map quarter warps pay from 4
 // bags per resident warp on, 8192 bags of 2-bit D = 128 at 20 M rows, 2, 4 and 16
 // streams: 8.5 / 9.6 / 10.8,  8.3 / 8.9 / 7.6,  7.9 / 8.6 / 7.1.
-constexpr int64_t kResidentWarps = 148 * bag::kBlocksPerSm * bag::kWarps;
-
 // Bags that a launch and those beside it keep on the chip at a time.
 int64_t bags_at_a_time(int64_t bags, int64_t beside) {
   return bags + beside / 4;
@@ -114,15 +139,13 @@ int64_t blocks_of(int64_t bags, int variant) {
   return (bags + per_block - 1) / per_block;
 }
 
-// Blocks of the deep form that fit the chip at once.
-constexpr int64_t kDeepFit = 148 * bag::kDeepBlocksPerSm;
-
 // `bags` in the launch, `beside` in those on other streams; `single`: one table's launch.
-int pick_variant(const BagTable& t, int fmt, int64_t bags, int64_t beside, bool single, int* tiles) {
+int pick_variant(const BagTable& t, int fmt, int64_t bags, int64_t beside, bool single, int64_t sms, int* tiles) {
   const int align = alignment_of(reinterpret_cast<uintptr_t>(t.data) | (uint64_t)t.stride);
   const bool mapped = t.flags & kPruned;
-  const int64_t quarter_warps_from = (mapped && beside > 0 ? 4 : 8) * kResidentWarps;
-  const int least_g = bags_at_a_time(bags, beside) <= kResidentWarps ? 32 : bags + beside <= quarter_warps_from ? 16 : 8;
+  const int64_t resident = resident_warps(sms);
+  const int64_t quarter_warps_from = (mapped && beside > 0 ? 4 : 8) * resident;
+  const int least_g = bags_at_a_time(bags, beside) <= resident ? 32 : bags + beside <= quarter_warps_from ? 16 : 8;
   int best = -1;
   double best_cost = 0;
   for (int i = 0; i < bag::kVariants; ++i) {
@@ -130,7 +153,7 @@ int pick_variant(const BagTable& t, int fmt, int64_t bags, int64_t beside, bool 
     if (v.fmt != fmt || v.vb > align || v.g < least_g) {
       continue;
     }
-    if (v.deep_mapped && !(single && form_of(t) == bag::kMapped && blocks_of(bags, i) <= 2 * kDeepFit)) {
+    if (v.deep_mapped && !(single && form_of(t) == bag::kMapped && blocks_of(bags, i) <= 2 * deep_fit(sms))) {
       continue;
     }
     // the last chunk may run into scale,bias behind the payload, but not beyond the row
@@ -194,8 +217,9 @@ cudaError_t launch_bags(const SpmdmParams& p, int bit_rate, cudaStream_t stream)
   for (int i = 0; i < p.num_peers; ++i) {
     c.peers[i] = p.peer_out[i];
   }
+  const int64_t sms = sm_count();
   int tiles = 0;
-  const int v = pick_variant(c.t, format_of(p, bit_rate), p.output_size, p.bags_beside, true, &tiles);
+  const int v = pick_variant(c.t, format_of(p, bit_rate), p.output_size, p.bags_beside, true, sms, &tiles);
   const int64_t blocks = blocks_of(p.output_size, v);
   if (blocks <= 0 || blocks > 0x7fffffffLL || tiles > 65535) {
     return cudaErrorInvalidValue;
@@ -207,8 +231,8 @@ cudaError_t launch_bags(const SpmdmParams& p, int bit_rate, cudaStream_t stream)
   // them: 4-bit D = 64, 4096 bags on 16 streams 3.2 against 3.6.)
   const int form = form_of(c.t);
   const int64_t bags = kVariantInfo[v].g == 32 ? bags_at_a_time(p.output_size, p.bags_beside) : p.output_size + p.bags_beside;
-  const bool deep = form == bag::kMapped ? blocks * tiles <= 2 * kDeepFit
-                                         : form != bag::kWide && blocks_of(bags, v) * tiles <= kDeepFit;
+  const int64_t fit = deep_fit(sms);
+  const bool deep = form == bag::kMapped ? blocks * tiles <= 2 * fit : form != bag::kWide && blocks_of(bags, v) * tiles <= fit;
   return launch<bag::BagCall>(single_kernel(v, deep ? bag::kDeepForms + form : form), dim3((unsigned)blocks, (unsigned)tiles), c, stream);
 }
 
@@ -239,13 +263,14 @@ cudaError_t build_multi_plan(const SpmdmParams* tables, const int* bit_rates, si
   };
   std::vector<Unit> order;
   std::vector<BagTable> bag_tables(count);
+  const int64_t sms = sm_count();
   for (size_t t = 0; t < count; ++t) {
     if (tables[t].output_size <= 0) {
       continue;  // nothing to pool, nothing to store
     }
     int tiles = 0;
     bag_table_of(tables[t], &bag_tables[t]);
-    const int v = pick_variant(bag_tables[t], format_of(tables[t], bit_rates[t]), bags, 0, false, &tiles);
+    const int v = pick_variant(bag_tables[t], format_of(tables[t], bit_rates[t]), bags, 0, false, sms, &tiles);
     const int64_t blocks = blocks_of(tables[t].output_size, v);
     if (blocks > 0x7fffffffLL || tiles > 65535) {
       return cudaErrorInvalidValue;
