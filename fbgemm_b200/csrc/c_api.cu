@@ -3,6 +3,7 @@
 // include/fbgemm_b200/embedding_c_api.h for the contract of each entry point.
 #include <algorithm>
 #include <cstring>
+#include <memory>
 #include <mutex>
 #include <new>
 #include <unordered_map>
@@ -20,6 +21,23 @@ thread_local std::string t_error;
 
 void set_error(const std::string& msg) {
   t_error = msg;
+}
+
+int thrown() noexcept {
+  const char* what = "unexpected exception";
+  int code = FBGEMM_B200_ECUDA;
+  try {
+    throw;
+  } catch (const std::bad_alloc&) {
+    what = "out of host memory";
+    code = FBGEMM_B200_ENOMEM;
+  } catch (...) {
+  }
+  try {
+    set_error(what);
+  } catch (...) {
+  }
+  return code;
 }
 
 int fail_cuda(cudaError_t e, const char* what) {
@@ -687,7 +705,7 @@ int fbgemm_b200_spmdm_launch(
     void* out,
     const int32_t* compressed_indices_table,
     int slot,
-    void* stream) {
+    void* stream) try {
   if (!ctx || slot < 0 || slot >= FBGEMM_B200_USER_SLOTS) {
     set_error("bad context or status slot (callers own slots 0 .. FBGEMM_B200_USER_SLOTS - 1)");
     return FBGEMM_B200_EINVAL;
@@ -711,6 +729,8 @@ int fbgemm_b200_spmdm_launch(
   }
   return enqueue_on_stream(ctx, cfg, output_size, index_size, data_size, input, indices, offsets_or_lengths, weights, out,
                            compressed_indices_table, ctx->status + 4 * slot, static_cast<cudaStream_t>(stream));
+} catch (...) {
+  return thrown();
 }
 
 int fbgemm_b200_spmdm_launch_sharded(
@@ -727,7 +747,7 @@ int fbgemm_b200_spmdm_launch_sharded(
     int num_peers,
     int64_t bags_per_peer,
     int slot,
-    void* stream) {
+    void* stream) try {
   if (!ctx || slot < 0 || slot >= FBGEMM_B200_USER_SLOTS) {
     set_error("bad context or status slot (callers own slots 0 .. FBGEMM_B200_USER_SLOTS - 1)");
     return FBGEMM_B200_EINVAL;
@@ -741,6 +761,8 @@ int fbgemm_b200_spmdm_launch_sharded(
   return enqueue_lookup(cfg, output_size, index_size, data_size, input, indices, offsets, weights, nullptr, nullptr,
                         ctx->status + 4 * slot, unused, static_cast<cudaStream_t>(stream), peer_out, num_peers,
                         bags_per_peer, ctx->history.launched(stream, output_size));
+} catch (...) {
+  return thrown();
 }
 
 int fbgemm_b200_multi_plan_create(
@@ -750,7 +772,7 @@ int fbgemm_b200_multi_plan_create(
     int32_t num_peers,
     int64_t bags_per_peer,
     int slot,
-    fbgemm_b200_multi_plan** out) {
+    fbgemm_b200_multi_plan** out) try {
   if (out) {
     *out = nullptr;
   }
@@ -789,19 +811,16 @@ int fbgemm_b200_multi_plan_create(
     bit_rates[(size_t)t] = c.cfg.bit_rate;
   }
   DeviceGuard guard(ctx->device);
-  auto* plan = new (std::nothrow) fbgemm_b200_multi_plan;
-  if (!plan) {
-    set_error("out of host memory");
-    return FBGEMM_B200_ENOMEM;
-  }
+  auto plan = std::make_unique<fbgemm_b200_multi_plan>();
   plan->device = ctx->device;
   const cudaError_t e = build_multi_plan(params.data(), bit_rates.data(), params.size(), &plan->plan);
   if (e != cudaSuccess) {
-    delete plan;
     return fail_cuda(e, "multi-table plan");
   }
-  *out = plan;
+  *out = plan.release();
   return 0;
+} catch (...) {
+  return thrown();
 }
 
 int fbgemm_b200_multi_plan_launch(fbgemm_b200_multi_plan* plan, void* stream) {
@@ -833,7 +852,7 @@ int fbgemm_b200_table_set_create(
     const fbgemm_b200_table_call* tables,
     const int64_t* out_columns,
     int32_t num_tables,
-    fbgemm_b200_table_set** out) {
+    fbgemm_b200_table_set** out) try {
   if (out) {
     *out = nullptr;
   }
@@ -841,11 +860,7 @@ int fbgemm_b200_table_set_create(
     set_error("table_set_create: bad argument");
     return FBGEMM_B200_EINVAL;
   }
-  auto* set = new (std::nothrow) fbgemm_b200_table_set;
-  if (!set) {
-    set_error("out of host memory");
-    return FBGEMM_B200_ENOMEM;
-  }
+  auto set = std::make_unique<fbgemm_b200_table_set>();
   for (int t = 0; t < num_tables; ++t) {
     const fbgemm_b200_table_call& c = tables[t];
     int rc = fbgemm_b200_spmdm_check_config(&c.cfg);
@@ -857,7 +872,6 @@ int fbgemm_b200_table_set_create(
       rc = FBGEMM_B200_EINVAL;
     }
     if (rc) {
-      delete set;
       return rc;
     }
     set->tables.push_back(c);
@@ -865,11 +879,13 @@ int fbgemm_b200_table_set_create(
   }
   {
     std::lock_guard<std::mutex> lock(ctx->mu);
-    ctx->sets.insert(set);
+    ctx->sets.insert(set.get());
   }
   set->ctx = ctx;
-  *out = set;
+  *out = set.release();
   return 0;
+} catch (...) {
+  return thrown();
 }
 
 int fbgemm_b200_table_set_forward(
@@ -881,7 +897,7 @@ int fbgemm_b200_table_set_forward(
     const float* weights,
     void* out,
     int slot,
-    void* stream) {
+    void* stream) try {
   if (!set || slot < 0 || slot >= FBGEMM_B200_USER_SLOTS || bags < 0 || !offsets || !out) {
     set_error("table_set_forward: bad argument");
     return FBGEMM_B200_EINVAL;
@@ -914,6 +930,8 @@ int fbgemm_b200_table_set_forward(
   DeviceGuard guard(set->ctx->device);
   const cudaError_t e = launch_tables(params.data(), bit_rates.data(), T, static_cast<cudaStream_t>(stream));
   return e == cudaSuccess ? 0 : fail_cuda(e, "table set launch");
+} catch (...) {
+  return thrown();
 }
 
 void fbgemm_b200_table_set_destroy(fbgemm_b200_table_set* set) {
@@ -965,7 +983,7 @@ int fbgemm_b200_spmdm(
     const float* weights,
     void* out,
     const int32_t* compressed_indices_table,
-    void* stream) {
+    void* stream) try {
   if (!ctx) {
     set_error("null context");
     return FBGEMM_B200_EINVAL;
@@ -991,6 +1009,8 @@ int fbgemm_b200_spmdm(
   }
   ctx->history.waited(stream);
   return take_record(ctx->sync_status) == 0 ? 1 : 0;
+} catch (...) {
+  return thrown();
 }
 
 int fbgemm_b200_compressed_indices_remap(
@@ -1194,7 +1214,7 @@ int fbgemm_b200_pruned_hashmap_insert_host(
 
 /* ---- table registry ----------------------------------------------------- */
 
-int fbgemm_b200_table_register(fbgemm_b200_ctx* ctx, const void* host_ptr, size_t bytes) {
+int fbgemm_b200_table_register(fbgemm_b200_ctx* ctx, const void* host_ptr, size_t bytes) try {
   if (!ctx || !host_ptr) {
     set_error("null context or table");
     return FBGEMM_B200_EINVAL;
@@ -1225,6 +1245,8 @@ int fbgemm_b200_table_register(fbgemm_b200_ctx* ctx, const void* host_ptr, size_
     ctx->tables.emplace(host_ptr, entry);
   }
   return 0;
+} catch (...) {
+  return thrown();
 }
 
 int fbgemm_b200_table_unregister(fbgemm_b200_ctx* ctx, const void* host_ptr) {
@@ -1450,7 +1472,7 @@ int fbgemm_b200_spmdm_host_submit(
     const void* offsets_or_lengths,
     const float* weights,
     void* out,
-    const int32_t* cit) {
+    const int32_t* cit) try {
   if (!ctx || lane_id < 0 || lane_id >= FBGEMM_B200_HOST_LANES) {
     set_error("bad context or lane");
     return FBGEMM_B200_EINVAL;
@@ -1689,9 +1711,11 @@ int fbgemm_b200_spmdm_host_submit(
   }
   L.busy = true;
   return 0;
+} catch (...) {
+  return thrown();
 }
 
-int fbgemm_b200_spmdm_host_wait(fbgemm_b200_ctx* ctx, int lane_id) {
+int fbgemm_b200_spmdm_host_wait(fbgemm_b200_ctx* ctx, int lane_id) try {
   if (!ctx || lane_id < 0 || lane_id >= FBGEMM_B200_HOST_LANES) {
     set_error("bad context or lane");
     return FBGEMM_B200_EINVAL;
@@ -1700,6 +1724,19 @@ int fbgemm_b200_spmdm_host_wait(fbgemm_b200_ctx* ctx, int lane_id) {
   if (!L.busy) {
     set_error("lane has nothing in flight");
     return FBGEMM_B200_EINVAL;
+  }
+  const uint8_t* src = static_cast<const uint8_t*>(L.h_out.ptr);
+  uint8_t* dst = static_cast<uint8_t*>(L.user_out);
+  std::vector<CopySlice> slices;  // (before anything else: without memory for it the call can be made again)
+  if (L.out_rows && L.pieces) {
+    constexpr size_t kSlice = 128 * 1024;
+    size_t at = 0;
+    for (int i = 0; i < L.pieces; ++i) {
+      for (; at < L.piece_end[i]; at += kSlice) {
+        slices.push_back({dst + at, src + at, std::min(kSlice, L.piece_end[i] - at), i});
+      }
+      at = L.piece_end[i];
+    }
   }
   L.busy = false;
   if (L.trivially_true) {
@@ -1710,18 +1747,7 @@ int fbgemm_b200_spmdm_host_wait(fbgemm_b200_ctx* ctx, int lane_id) {
   }
   DeviceGuard guard(ctx->device);
   cudaError_t e = cudaSuccess;
-  const uint8_t* src = static_cast<const uint8_t*>(L.h_out.ptr);
-  uint8_t* dst = static_cast<uint8_t*>(L.user_out);
   if (L.out_rows && L.pieces) {
-    std::vector<CopySlice> slices;
-    constexpr size_t kSlice = 128 * 1024;
-    size_t at = 0;
-    for (int i = 0; i < L.pieces; ++i) {
-      for (; at < L.piece_end[i]; at += kSlice) {
-        slices.push_back({dst + at, src + at, std::min(kSlice, L.piece_end[i] - at), i});
-      }
-      at = L.piece_end[i];
-    }
     auto arrived = [&](int i) {
       e = cudaEventSynchronize(L.piece_done[i]);
       return e == cudaSuccess;
@@ -1741,6 +1767,8 @@ int fbgemm_b200_spmdm_host_wait(fbgemm_b200_ctx* ctx, int lane_id) {
     }
   }
   return take_record(static_cast<int32_t*>(L.h_status.ptr)) == 0 ? 1 : 0;
+} catch (...) {
+  return thrown();
 }
 
 int fbgemm_b200_spmdm_host(

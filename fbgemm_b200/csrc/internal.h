@@ -316,6 +316,8 @@ extern std::atomic<int> g_kernel_choice;
 
 // Thread-local error text behind fbgemm_b200_last_error().
 void set_error(const std::string& msg);
+// In an entry point's handler: the code to return for what was thrown.  Nothing is thrown through the C ABI.
+int thrown() noexcept;
 int fail_cuda(cudaError_t e, const char* what);
 
 }  // namespace fbgemm_b200

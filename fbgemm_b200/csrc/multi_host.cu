@@ -17,7 +17,7 @@
 // output buffers pipeline the transfers of one step behind the kernels of the
 // other.
 #include <cstring>
-#include <new>
+#include <memory>
 #include <vector>
 
 #include "context.h"
@@ -127,7 +127,7 @@ int fbgemm_b200_multi_host_create(
     size_t out_bytes,
     const fbgemm_b200_peer_sync* sync,
     int slot,
-    fbgemm_b200_multi_host** out) {
+    fbgemm_b200_multi_host** out) try {
   if (out) {
     *out = nullptr;
   }
@@ -141,11 +141,12 @@ int fbgemm_b200_multi_host_create(
     set_error("multi_host_create: the peer counters must describe the same peers as the lookups");
     return FBGEMM_B200_EINVAL;
   }
-  auto* h = new (std::nothrow) fbgemm_b200_multi_host;
-  if (!h) {
-    set_error("out of host memory");
-    return FBGEMM_B200_ENOMEM;
-  }
+  struct Destroy {
+    void operator()(fbgemm_b200_multi_host* p) const {
+      fbgemm_b200_multi_host_destroy(p);
+    }
+  };
+  std::unique_ptr<fbgemm_b200_multi_host, Destroy> h(new fbgemm_b200_multi_host);
   h->ctx = ctx;
   h->device = ctx->device;
   h->slot = slot;
@@ -164,7 +165,6 @@ int fbgemm_b200_multi_host_create(
       rc = FBGEMM_B200_EINVAL;
     }
     if (rc) {
-      delete h;
       return rc;
     }
     h->calls.push_back(c);
@@ -204,12 +204,12 @@ int fbgemm_b200_multi_host_create(
     e = reserve(h->h_status, 16);
   }
   if (e != cudaSuccess) {
-    const int rc = fail_cuda(e, "multi_host_create");
-    fbgemm_b200_multi_host_destroy(h);
-    return rc;
+    return fail_cuda(e, "multi_host_create");
   }
-  *out = h;
+  *out = h.release();
   return 0;
+} catch (...) {
+  return thrown();
 }
 
 int fbgemm_b200_multi_host_submit(
@@ -218,7 +218,7 @@ int fbgemm_b200_multi_host_submit(
     const void* const* offsets,
     const float* const* weights,
     const int64_t* index_sizes,
-    void* out_host) {
+    void* out_host) try {
   if (!h || !indices || !offsets || !index_sizes || !out_host) {
     set_error("multi_host_submit: bad argument");
     return FBGEMM_B200_EINVAL;
@@ -338,6 +338,8 @@ int fbgemm_b200_multi_host_submit(
   h->step = step;
   h->busy = true;
   return 0;
+} catch (...) {
+  return thrown();
 }
 
 int64_t fbgemm_b200_multi_host_step_device(
@@ -347,7 +349,7 @@ int64_t fbgemm_b200_multi_host_step_device(
     const float* const* weights,
     const int64_t* index_sizes,
     int release,
-    void* stream_) {
+    void* stream_) try {
   if (!h || !indices || !offsets || !index_sizes) {
     set_error("multi_host_step_device: bad argument");
     return FBGEMM_B200_EINVAL;
@@ -396,6 +398,8 @@ int64_t fbgemm_b200_multi_host_step_device(
   }
   h->step = step;
   return (int64_t)step;
+} catch (...) {
+  return thrown();
 }
 
 int fbgemm_b200_multi_host_release(fbgemm_b200_multi_host* h, int64_t step, void* stream) {
