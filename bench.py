@@ -703,17 +703,16 @@ def main_multi(args):
                        weighted=weighted, index_dtype=tnp, offset_dtype=tnp)
     sets = make_input_sets(specs, sl.local, B, alpha, idt, weighted, mean_len, lengths_kind, dev, NUM_SETS)
     bytes_local = float(np.mean([sum(b.index_size * specs[t].row_bytes for t, b in d.items()) for d in sets]))
-    # One lane per output buffer: its own stream (and side streams for the tables' launches), so that the counter
-    # waits and the tail of one global batch overlap with the lookups of the next.
+    # One lane per output buffer: its own stream (and, where a table is a launch of its own, side streams), so that the
+    # counter waits and the tail of one global batch overlap with the lookups of the next.
     lanes = [torch.cuda.Stream(device=dev) for _ in range(nbuf)]
     side = [[torch.cuda.Stream(device=dev) for _ in range(3)] for _ in range(nbuf)]
     bps = max(1, args.batches_per_step)
 
     plans = None
-    if args.launch == "plan":   # one kernel launch per kernel variant instead of one per table
+    if args.launch == "plan":   # built once for every input set and buffer
         plans = {(s, b): sl.make_plan(sets[s], buffer=b, slot=400 + s * nbuf + b) for s in range(NUM_SETS)
                  for b in range(nbuf)}
-    launches_per_batch = (plans[(0, 0)].num_launches if plans else len(sl.local)) + (4 if p2p else 0)
 
     def make_step_calls(lookup):
         """One handle per output buffer that enqueues a whole ordered step with one call from the host, and its
@@ -830,6 +829,7 @@ def main_multi(args):
         torch.cuda.synchronize(dev)
     barrier()
     launches = int(F.launch_count() - before)
+    launches_per_batch = round(launches / (args.steps * bps))
     ms = marks[0].elapsed_time(marks[args.steps])
     per_step_ms = sorted(marks[k].elapsed_time(marks[k + 1]) for k in range(args.steps))
     ok = ok and status_ok()

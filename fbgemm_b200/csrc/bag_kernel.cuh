@@ -12,7 +12,8 @@
 // instruction issue, not bytes.  Hence the layout:
 //  * The columns of a row are spread over the lane group, 1 to 16 bytes of
 //    payload per lane.  A row in flight costs a lane one or two registers, so
-//    8 to 12 rows of a bag are in flight with a full set of warps on the SM.
+//    4 or 8 rows of a bag are in flight with a full set of warps on the SM, 8 or
+//    12 in the deep form (rows_ahead).
 //  * Everything that is per row and not per column is done ONCE per row, by the
 //    lane that owns the row in the walk over the bag's indices (one index per
 //    lane at a time, coalesced): index load, range check, pruning map, weight,

@@ -54,7 +54,8 @@ using namespace fbgemm_b200;
 namespace {
 
 // Status slots: callers own [0, FBGEMM_B200_USER_SLOTS); then one for the
-// index remap; the last FBGEMM_B200_HOST_LANES belong to the host-pointer lanes.
+// index remap; the last FBGEMM_B200_HOST_LANES are reserved (the host-pointer
+// lanes keep their records in Lane::h_status).
 constexpr int kRemapSlot = FBGEMM_B200_USER_SLOTS;
 static_assert(FBGEMM_B200_USER_SLOTS + 1 + FBGEMM_B200_HOST_LANES == FBGEMM_B200_STATUS_SLOTS, "slot ranges");
 

@@ -8,11 +8,12 @@
 // Bound by memory: 4 bytes read per column, 1/4 to 1 written.  Rows follow one
 // another without gaps, so a block takes 16 KB of them as one stretch of bytes,
 // whatever their width: 16-byte asynchronous copies bring them to shared memory,
-// lane groups of 8 (wide rows: 32) quantize row by row from there into the bytes
+// groups of 4 to 32 lanes (launch_quantize) quantize row by row from there into the bytes
 // of the fused rows, and those leave as 16-byte stores of whole sectors.  8 blocks
 // per SM keep 128 KB on their way.  A warp per row that read its row twice and
 // stored single bytes took 248 us for 1 M x 128 columns (8-bit), rows held in
-// registers and stored by words 129 us, this 102 us; memory needs 99 us.
+// registers and stored by words 129 us, this 101 us
+// (a pass of the public call takes 119); memory needs 99 us.
 #include <cuda_fp16.h>
 
 #include "internal.h"

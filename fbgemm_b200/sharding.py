@@ -305,9 +305,8 @@ class ShardedLookup:
 
     def make_plan(self, batches: dict, buffer: int = 0, slot: int = 0):
         """The same lookups as ``launch`` as a multi-table plan
-        (``fbgemm_b200_multi_plan_*``): the local tables grouped by kernel
-        variant, one kernel launch per group, for this input set and output
-        buffer.  Call ``.launch(stream)`` on the result."""
+        (``fbgemm_b200_multi_plan_*``): up to 64 local tables of one form per
+        kernel launch, for this input set and output buffer.  Call ``.launch(stream)`` on the result."""
         from .embedding import MultiTablePlan
 
         calls, peers, col = [], [], 0

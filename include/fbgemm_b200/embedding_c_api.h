@@ -76,7 +76,7 @@ extern "C" {
 /* Number of staging lanes of the host-pointer pipeline. */
 #define FBGEMM_B200_HOST_LANES 16
 /* Status slots a caller may pass: 0 .. FBGEMM_B200_USER_SLOTS - 1.  The rest
- * are the library's (one for the index remap, one per host-pointer lane). */
+ * are the library's (one for the index remap, the others reserved). */
 #define FBGEMM_B200_USER_SLOTS (FBGEMM_B200_STATUS_SLOTS - FBGEMM_B200_HOST_LANES - 1)
 
 typedef struct fbgemm_b200_ctx fbgemm_b200_ctx;
@@ -776,8 +776,8 @@ typedef struct fbgemm_b200_peer_sync {
  * create allocates (staging, streams); submit and wait allocate nothing.
  * fbgemm_b200_multi_host_step_device: the same step for a caller whose index,
  * offset and weight arrays are already on the device: no upload, no download,
- * everything enqueued on the CALLER's `stream` (the handle's side streams fork
- * from it and join it): wait for the peers' acks, the lookups, publish "ready"
+ * everything enqueued on the CALLER's `stream`, one launch for up to 64 tables:
+ * wait for the peers' acks, the lookups, publish "ready"
  * and wait for the peers'; when `stream` gets past it, out_dev holds this rank's
  * rows.  Returns the step number (> 0) or a negative code; errors of the lookups
  * and counter waits go to status slot `slot` (fbgemm_b200_status_read).  With
