@@ -74,11 +74,11 @@ PARITY_BAGS = 64        # bags per table compared with the oracle inside the run
 # (dram__bytes_read.sum + dram__bytes_write.sum; the files under profiles/ say how each was taken).
 TRAFFIC = {
     # single-table workloads: DRAM bytes per functor call of the configuration's batch in the benchmark's steady state
-    0: {"bytes_per_call": 25_902_699 + 5_179_565, "source": "profiles/lookup_kernels__workloads012_steady_state_dram.md"},
-    1: {"bytes_per_call": 10_020_888 + 629_504, "source": "profiles/lookup_kernels__workloads012_steady_state_dram.md"},
-    2: {"bytes_per_call": 13_405_040 + 4_003_784, "source": "profiles/lookup_kernels__workloads012_steady_state_dram.md"},
+    0: {"bytes_per_call": 26_648_021 + 5_329_840, "source": "profiles/lookup_kernels__workloads012_steady_state_dram.md"},
+    1: {"bytes_per_call": 9_872_293 + 778_946, "source": "profiles/lookup_kernels__workloads012_steady_state_dram.md"},
+    2: {"bytes_per_call": 13_888_506 + 4_160_853, "source": "profiles/lookup_kernels__workloads012_steady_state_dram.md"},
     # the 64-table configuration: DRAM bytes of all kernels of one global batch (captured at a quarter of the batch, x 4)
-    3: {"bytes_per_global_batch": 4 * (2_174_574_080 + 178_803_456) / 2, "source": "profiles/lookup_kernels__default_workload_dram.md"},
+    3: {"bytes_per_global_batch": 4 * (2_177_274_880 + 196_862_208) / 2, "source": "profiles/lookup_kernels__default_workload_dram.md"},
 }
 
 
