@@ -6,7 +6,8 @@
 // per output column, rows strictly in index order,
 //     acc = fma(w*scale, q, acc + w*bias)
 // two columns at a time with the packed fp32 instructions of sm_100
-// (add.rn.f32x2, fma.rn.f32x2), which round each half like the scalar forms.
+// (add.rn.f32x2, fma.rn.f32x2), which round each half like the scalar forms;
+// sums are kept scaled by a power of two (see kDown).
 //
 // What bounds a lookup is the chain offsets -> index -> row of every bag and
 // instruction issue, not bytes.  Hence the layout:
@@ -114,61 +115,58 @@ enum : int { kInt8 = 8, kInt4 = 4, kInt2 = 2, kF32 = 32, kF16 = 16, kBf16 = 17, 
 __host__ __device__ constexpr bool is_quantized(int fmt) { return fmt <= 8; }
 __host__ __device__ constexpr int column_bits(int fmt) { return fmt == kBf16 ? 16 : fmt == kFp8 ? 8 : fmt; }
 
-// Integer -> float: column K's bits are planted, where they lie, in the
-// mantissa of the power of two whose last place has their weight, which is then
-// subtracted: one logic instruction per column and half a packed addition.
-// 8-bit columns go through a byte permute (any byte of the word to bits 0-7).
-template <int BITS, int K>
-struct Plant {
-  static constexpr int kPerWord = 32 / BITS;
-  static constexpr int kWord = K / kPerWord;
-  static constexpr int kInWord = K % kPerWord;
-  static constexpr int kHalf = kPerWord / 2;                     // columns per 16 bits
-  static constexpr int kStep = BITS == 8 ? 0 : kInWord % kHalf;  // which power of two
-  static constexpr int kShift = kStep * BITS;                    // where the bits lie in the mantissa
+// Integer -> float without an instruction of its own.  Fewer than 25 bits that
+// lie at bit p of a register and up are, read as fp32, the number q * 2^(p - 149)
+// (subnormal, or of the least exponent, which has the same spacing): one logic
+// instruction cuts a column out where it lies (8-bit: one byte permute takes it
+// to bit 0), and the scale makes up for the power of two.  So that such a scale
+// is an fp32 number the sums are kept as multiples of 2^-kDown of themselves:
+//     acc' = fma(scale * 2^(149 - p - kDown), q * 2^(p - 149), acc' + bias * 2^-kDown)
+// and brought back by an exact multiplication at the end.  Every step rounds as
+// the unscaled one does where neither form leaves fp32's normal range, which holds
+// for all rows whose weighted scale and bias are zero or of magnitude 2^-52 to
+// 2^52: all values are then multiples of 2^-75 (2^-149 scaled: exact where
+// subnormal) and, over 2^31 positions, below 2^92.  A bag with a row of other
+// values (infinite ones, NaN and weights of 1e-20 among them) is pooled once
+// more, unscaled (pool_again).
+// Before, each column's bits were planted in the mantissa of a power of two that
+// a packed addition then subtracted.  One row of 8 columns a lane, issue cycles of
+// a scheduler, rows and scales in shared memory: 8-bit 22.0 / 18.0, 4-bit 25.1 / 19.4.
+// 64 mixed tables of 16 384 bags 1135 / 1069 us, 8 4-bit tables of 65 536 bags 635 / 610.
+constexpr int kDown = 74;
+constexpr float kScaleUp = 1.f * (1ull << 60) * (1 << 15);                          // 2^(149 - kDown)
+constexpr float kBiasDown = 1.f / ((float)(1ull << 60) * (float)(1 << 14));         // 2^-kDown
+constexpr float kSumUp = (float)(1ull << 60) * (float)(1 << 14);                    // 2^kDown
+
+// Whether a weighted scale or bias is one that the scaled sums are not made for.
+__device__ __forceinline__ bool out_of_scale(float x) {
+  const uint32_t magnitude = __float_as_uint(x) << 1;
+  return magnitude != 0 && magnitude - ((127u - 52u) << 24) >= (104u << 24);
+}
+
+// Where column K of a chunk of COLS columns lies: kPlaces columns are cut out of
+// one shifted word, each with a scale of its own.
+template <int BITS, int COLS>
+struct Places {
+  static constexpr int kPlaces = BITS == 8 ? 1 : COLS >= 8 ? 4 : 2;
+  template <int K>
+  __device__ __forceinline__ static float value(const uint32_t* w) {
+    constexpr int at = K * BITS % 32;
+    constexpr int shift = at / (kPlaces * BITS) * (kPlaces * BITS);
+    const uint32_t x = w[K * BITS / 32];
+    if constexpr (BITS == 8) {
+      return __uint_as_float(COLS == 1 ? x : __byte_perm(x, 0u, 0x4440u | (at / 8)));
+    } else {
+      return __uint_as_float((x >> shift) & (((1u << BITS) - 1u) << (at - shift)));
+    }
+  }
 };
 
-// What a format keeps in registers: the powers of two (the logic instruction
-// has room for one immediate, the mask), or how FP8 widens to fp32.
+// How FP8 widens to fp32.
 template <int FMT, int COLS>
 struct Constants {
-  static constexpr int BITS = FMT;
-  static constexpr int kHalf = 16 / BITS;
-  static constexpr int kCount = BITS == 8 ? 1 : (COLS < kHalf ? COLS : kHalf);
-  uint32_t m[kCount];
-  __device__ __forceinline__ void init(const BagTable&) {
-#pragma unroll
-    for (int i = 0; i < kCount; ++i) {
-      asm volatile("mov.b32 %0, %1;" : "=r"(m[i]) : "r"((uint32_t)(127 + 23 - i * (BITS == 8 ? 0 : BITS)) << 23));
-    }
-  }
-  template <int K>
-  __device__ __forceinline__ float plant(const uint32_t* w) const {
-    using P = Plant<BITS, K>;
-    if constexpr (BITS == 8) {
-      return __uint_as_float(__byte_perm(w[P::kWord], m[0], 0x7540u | P::kInWord));
-    } else {
-      const uint32_t x = P::kInWord >= P::kHalf ? w[P::kWord] >> 16 : w[P::kWord];
-      uint32_t r;
-      asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(x), "n"(((1 << BITS) - 1) << P::kShift), "r"(m[P::kStep]));
-      return __uint_as_float(r);
-    }
-  }
-  template <int K>
-  __device__ __forceinline__ static u64 minus() {  // the negated powers of two of columns K, K + 1
-    constexpr float a = -(float)(1u << (23 - Plant<BITS, K>::kShift));
-    constexpr float b = -(float)(1u << (23 - Plant<BITS, K + 1>::kShift));
-    return pack2(a, b);
-  }
-};
-template <int COLS>
-struct Constants<kF32, COLS> {
   __device__ __forceinline__ void init(const BagTable&) {}
 };
-template <int COLS>
-struct Constants<kF16, COLS> : Constants<kF32, COLS> {};
-template <int COLS>
-struct Constants<kBf16, COLS> : Constants<kF32, COLS> {};
 // FP8 -> fp32 as Float8ToFloat_ref (src/RefImplementations.cc:184-215): the seven low bits shifted into fp32's
 // exponent and mantissa, times 2^(127 - bias), sign OR-ed in.
 template <int COLS>
@@ -192,7 +190,7 @@ struct Cols {
   static constexpr int kPairs = kPerChunk * CPL / 2;
   static_assert(kPerChunk * CPL % 2 == 0, "whole pairs");
   static constexpr bool kQuantized = is_quantized(FMT);
-  static constexpr bool kHalfSb = FMT != kInt8;  // with a pruning map: those rows have scale and bias last
+  static constexpr bool kHalfSb = FMT != kInt8;  // 8-bit rows: only with scale and bias first
   using M = Constants<FMT, kPerChunk>;
 
   // Column k of an unquantized chunk.
@@ -209,16 +207,17 @@ struct Cols {
       return __uint_as_float(__float_as_uint(mag) | ((x & 0x80u) << 24));
     }
   }
+  using P = Places<BITS, kPerChunk>;
   template <int K>
-  __device__ __forceinline__ static void pool_chunk(const M& m, u64* acc, const uint32_t* w, u64 s2, u64 b2) {
+  __device__ __forceinline__ static void pool_chunk(u64* acc, const uint32_t* w, u64 s2, u64 further, u64 b2) {
     if constexpr (K < kPerChunk) {
-      const u64 q = add2(pack2(m.template plant<K>(w), m.template plant<K + 1>(w)), M::template minus<K>());
-      acc[K / 2] = fma2(s2, q, add2(acc[K / 2], b2));
-      pool_chunk<K + 2>(m, acc, w, s2, b2);
+      const u64 q = pack2(P::template value<K>(w), P::template value<K + 1>(w));
+      acc[K / 2] = fma2(K % P::kPlaces < 2 ? s2 : further, q, add2(acc[K / 2], b2));
+      pool_chunk<K + 2>(acc, w, s2, further, b2);
     }
   }
-  // One row.  Quantized: acc = fma(scale, q, acc + bias); otherwise acc = fma(w, x, acc) with w in `s2`
-  // (src/RefImplementations.cc:1347-1424, :1543-1615).
+  // One row.  Quantized: acc' = fma(scale', q, acc' + bias'), `s2` the scales of the columns at places 0 and 1;
+  // otherwise acc = fma(w, x, acc) with w in `s2` (src/RefImplementations.cc:1347-1424, :1543-1615).
   __device__ __forceinline__ static void pool(const M& m, u64 (&acc)[kPairs], const Bytes<VB> (&d)[CPL], u64 s2, u64 b2) {
     if constexpr (!is_quantized(FMT)) {
 #pragma unroll
@@ -231,15 +230,27 @@ struct Cols {
     } else if constexpr (kPerChunk == 1) {
 #pragma unroll
       for (int c = 0; c < CPL; c += 2) {
-        const u64 q = add2(pack2(__uint_as_float(d[c].w[0] | m.m[0]), __uint_as_float(d[c + 1].w[0] | m.m[0])),
-                           M::template minus<0>());
+        const u64 q = pack2(P::template value<0>(d[c].w), P::template value<0>(d[c + 1].w));
         acc[c / 2] = fma2(s2, q, add2(acc[c / 2], b2));
       }
     } else {
+      // the scales of places 2 and 3 (one multiplication instead of two shifts more)
+      constexpr float down = 1.f / (1 << (2 * BITS % 32));
+      const u64 further = P::kPlaces > 2 ? mul2(s2, pack2(down, down)) : s2;
 #pragma unroll
       for (int c = 0; c < CPL; ++c) {
-        pool_chunk<0>(m, acc + c * kPerChunk / 2, d[c].w, s2, b2);
+        pool_chunk<0>(acc + c * kPerChunk / 2, d[c].w, s2, further, b2);
       }
+    }
+  }
+  // The same unscaled, column by column (pool_again).
+  __device__ __forceinline__ static void pool_unscaled(float (&acc)[2 * kPairs], const Bytes<VB> (&d)[CPL], float scale,
+                                                       float bias) {
+#pragma unroll
+    for (int k = 0; k < 2 * kPairs; ++k) {
+      const int bit = k % kPerChunk * BITS;
+      const uint32_t q = (d[k / kPerChunk].w[bit / 32] >> (bit % 32)) & ((1u << (BITS % 32)) - 1u);
+      acc[k] = __fmaf_rn(scale, (float)q, __fadd_rn(acc[k], bias));
     }
   }
 };
@@ -451,27 +462,39 @@ __device__ __forceinline__ void bag_from_lengths(const BagTable& p, int64_t firs
   length = bag < p.bags ? at(bag) : 0;
 }
 
-// A bag of a row-wise sparse call whose map names rows beyond 32-bit offsets (several short maps may share one large
-// table), pooled once more from its first position with 64-bit row addresses, one row at a time.  Rare, so it costs the
-// other bags one comparison per mapped row and no registers (11.3 us before and after for 8192 bags of 30 rows, 2-bit
-// D = 128), where 64-bit addresses for every pruned table would cost each of their rows the wide form's extra instructions.
-template <class C, int VB, int CPL, int G>
-__device__ __forceinline__ void pool_far_rows(const BagTable& p, const typename C::M& constants,
-                                              const LaneData<VB, CPL, G, false>& lane_data, int start, int len,
-                                              u64 (&acc)[C::kPairs]) {
+// A bag pooled once more from its first position, one row at a time, with 64-bit row addresses and unscaled sums, where
+// * its row-wise sparse map names rows beyond 32-bit offsets (several short maps may share one large table).  Rare, so it
+//   costs the other bags one comparison per mapped row and no registers (11.3 us before and after for 8192 bags of 30
+//   rows, 2-bit D = 128), where 64-bit addresses for every pruned table would cost each of their rows the wide form's
+//   extra instructions;
+// * a row's weighted scale or bias is out_of_scale.
+template <class C, int VB, int CPL, int G, int MODE, class Lane>
+__device__ __forceinline__ void pool_again(const BagTable& p, const typename C::M& constants, const Lane& lane_data,
+                                           int64_t start, int len, u64 (&acc)[C::kPairs]) {
+  float sum[2 * C::kPairs];
+#pragma unroll
+  for (int k = 0; k < 2 * C::kPairs; ++k) {
+    sum[k] = 0.f;
+  }
 #pragma unroll
   for (int k = 0; k < C::kPairs; ++k) {
     acc[k] = 0ull;
   }
 #pragma unroll 1
   for (int c = 0; c < len; ++c) {
-    const int64_t idx = load_int(p.indices, (int64_t)start + c, p.flags & kIdx64);
-    const int32_t m = idx >= 0 && idx < p.data_size ? __ldg(p.cit + idx) : -1;
-    if (m < 0) {
+    int64_t idx = load_int(p.indices, start + c, p.flags & kIdx64);
+    if (idx < 0 || idx >= p.data_size) {
       continue;
     }
-    const uint8_t* row = p.data + (uint64_t)(uint32_t)m * (uint64_t)p.stride;
-    const float w = p.flags & kWeighted ? __ldg(p.weights + (p.flags & kPositional ? (int64_t)c : (int64_t)start + c)) : 1.f;
+    if (p.flags & kPruned) {
+      const int32_t m = __ldg(p.cit + idx);
+      if (m < 0) {
+        continue;
+      }
+      idx = m;
+    }
+    const uint8_t* row = p.data + (uint64_t)idx * (uint64_t)p.stride;
+    const float w = p.flags & kWeighted ? __ldg(p.weights + (p.flags & kPositional ? (int64_t)c : start + c)) : 1.f;
     Bytes<VB> d[CPL];
 #pragma unroll
     for (int i = 0; i < CPL; ++i) {
@@ -481,7 +504,7 @@ __device__ __forceinline__ void pool_far_rows(const BagTable& p, const typename 
       const uint8_t* sb = row + p.sb_off;
       const uint32_t lo = load_u32(sb, p.sb_align);
       float scale, bias;
-      if (C::kHalfSb) {
+      if (C::kHalfSb || (p.flags & kSbFirst)) {
         scale = __half2float(__ushort_as_half((unsigned short)(lo & 0xffffu)));
         bias = __half2float(__ushort_as_half((unsigned short)(lo >> 16)));
       } else {
@@ -492,9 +515,15 @@ __device__ __forceinline__ void pool_far_rows(const BagTable& p, const typename 
         scale = __fmul_rn(w, scale);
         bias = __fmul_rn(w, bias);
       }
-      C::pool(constants, acc, d, pack2(scale, scale), pack2(bias, bias));
+      C::pool_unscaled(sum, d, scale, bias);
     } else {
       C::pool(constants, acc, d, pack2(w, w), 0ull);
+    }
+  }
+  if constexpr (C::kQuantized) {
+#pragma unroll
+    for (int k = 0; k < C::kPairs; ++k) {
+      acc[k] = pack2(sum[2 * k], sum[2 * k + 1]);
     }
   }
 }
@@ -593,7 +622,7 @@ __device__ __forceinline__ void pool_bags(const BagTable& p, void* const* peers,
     return r;
   };
   uint2 raw = fetch(gl);
-  bool far = false;  // a row of this lane's lies beyond 32-bit offsets
+  bool again = false;  // a row of this lane's lies beyond 32-bit offsets, or is out_of_scale
 #pragma unroll 1
   for (int c0 = 0; c0 < longest; c0 += G) {
     const int c = c0 + gl;
@@ -625,7 +654,7 @@ __device__ __forceinline__ void pool_bags(const BagTable& p, void* const* peers,
       id = keep ? (uint32_t)m : 0u;
       if constexpr (!WIDE) {
         // a table larger than its map: below, with 64-bit row addresses
-        far = far || (keep && id >= p.map_limit);
+        again = again || (keep && id >= p.map_limit);
         keep = keep && id < p.map_limit;
         id = keep ? id : 0u;
       }
@@ -711,7 +740,11 @@ __device__ __forceinline__ void pool_bags(const BagTable& p, void* const* peers,
         scale = __fmul_rn(w, scale);
         bias = __fmul_rn(w, bias);
       }
-      q_sb[at] = make_ulonglong2(pack2(scale, scale), pack2(bias, bias));
+      again = again || out_of_scale(scale) || out_of_scale(bias);
+      scale = __fmul_rn(scale, kScaleUp);
+      bias = __fmul_rn(bias, kBiasDown);
+      const float next = FMT == kInt8 ? scale : __fmul_rn(scale, 1.f / (1 << (FMT % 32)));  // of place 1
+      q_sb[at] = make_ulonglong2(pack2(scale, next), pack2(bias, bias));
     } else {
       q_sb[at].x = pack2(w, w);
     }
@@ -744,9 +777,14 @@ __device__ __forceinline__ void pool_bags(const BagTable& p, void* const* peers,
     __syncwarp();  // the queue is rewritten by the next stretch
   }
 
-  if constexpr (MAPS && !WIDE) {
-    if (pruned && __any_sync(0xffffffffu, far)) {
-      pool_far_rows<C, VB, CPL, G>(p, constants, lane_data, pos - gl - (longest + G - 1) / G * G, len, acc);
+  float up = kQuantized ? kSumUp : 1.f;  // from the scaled sums to the pooled row
+  if constexpr (kQuantized || (MAPS && !WIDE)) {
+    const unsigned lanes = __ballot_sync(0xffffffffu, again);
+    if (lanes != 0) {
+      if ((lanes >> (grp * G)) & kGroupMask) {
+        pool_again<C, VB, CPL, G, MODE>(p, constants, lane_data, pos - gl - (Pos)((longest + G - 1) / G * G), len, acc);
+        up = 1.f;
+      }
     }
   }
 
@@ -761,12 +799,13 @@ __device__ __forceinline__ void pool_bags(const BagTable& p, void* const* peers,
     bag_len = by_lengths ? (int)load_int(p.offsets, bag, off64)
                          : (int)(load_int(p.offsets, (int64_t)bag + 1, off64) - load_int(p.offsets, bag, off64));
   }
-  if (bag_len != 0) {
-    const float inv = __fdiv_rn(1.f, (float)bag_len);
-    const u64 inv2 = pack2(inv, inv);
+  if (kQuantized || bag_len != 0) {
+    // (exact but for the mean's own rounding: a power of two, and no sum is near either end of the range)
+    const float by = bag_len != 0 ? __fmul_rn(__fdiv_rn(1.f, (float)bag_len), up) : up;
+    const u64 by2 = pack2(by, by);
 #pragma unroll
     for (int k = 0; k < C::kPairs; ++k) {
-      acc[k] = mul2(acc[k], inv2);
+      acc[k] = mul2(acc[k], by2);
     }
   }
   char* row;

@@ -1,0 +1,95 @@
+"""Rows and weights at the ends of fp32's range.  The lookup keeps its sums scaled by a power of two, which is exact
+while every weighted scale and bias is zero or of magnitude 2^-52 to 2^52; bags with other values take another path,
+their neighbours in the same warp do not.  Bit for bit against the CPU oracle (NaN where the oracle has NaN)."""
+import numpy as np
+import pytest
+import torch
+
+import fbgemm_b200 as F
+from conftest import bits
+from helpers import random_fused_table, row_bytes
+
+pytestmark = pytest.mark.gpu
+BELOW = np.nextafter(np.float32(1), np.float32(0))
+FLOATS = np.array([0.0, -0.0, 2.0**-52, 2.0**-52 * BELOW, -2.0**-52, 2.0**52, 2.0**52 * BELOW, -2.0**52, 2.0**-53, 1e-20, -1e-20, 1e20,
+                   3e38, -3e38, 1e-44, 2.0**-126, 2.0**-75, 2.0**-74, 2.0**-149, np.inf, -np.inf, np.nan], np.float32)
+HALVES = np.array([0.0, -0.0, 2.0**-24, -2.0**-24, 2.0**-14, 65504.0, -65504.0, np.inf, -np.inf, np.nan], np.float16)
+
+
+def dev(a):
+    return None if a is None else torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+
+def same(got, ref):
+    np.testing.assert_array_equal(np.isnan(got), np.isnan(ref))
+    fine = ~np.isnan(ref)
+    np.testing.assert_array_equal(bits(got)[fine], bits(ref)[fine])
+
+
+def make(rng, bit_rate, dim, batch, weighted, ordinary):
+    """Rows 0 .. 99 are ordinary; each of the others has an odd scale, bias or both, and every fourth bag names one.
+    Rows 200 .. 239 cancel one another: payload 0 and biases b, -b (of sizes that meet in the sums' last places)."""
+    rows = 240
+    t = random_fused_table(rng, rows, dim, bit_rate)
+    odd, kind = (FLOATS, np.float32) if bit_rate == 8 else (HALVES, np.float16)
+    sb = np.ascontiguousarray(t[:, -2 * kind().itemsize:]).view(kind)
+    sb[100:200] = rng.choice(odd, (100, 2))
+    sb[100:140, 0] = sb[:40, 0]
+    sb[140:180, 1] = sb[:40, 1]
+    t[200:, :row_bytes(bit_rate, dim) - 2 * kind().itemsize] = 0
+    size = (2.0 ** rng.integers(-50 if bit_rate == 8 else -14, 51 if bit_rate == 8 else 15, 20)).astype(kind)
+    sb[200::2, 1], sb[201::2, 1] = size, -size
+    t[:, -2 * kind().itemsize:] = sb.view(np.uint8)
+    lengths = rng.integers(0, 40, batch)
+    n = int(lengths.sum())
+    indices = rng.choice(np.concatenate([np.arange(100), np.arange(200, rows)]), n)
+    offsets = np.concatenate([[0], np.cumsum(lengths)]).astype(np.int32)
+    w = rng.standard_normal(n).astype(np.float32) if weighted else None
+    if not ordinary:
+        for b in range(0, batch, 4):
+            if lengths[b]:
+                indices[rng.integers(offsets[b], offsets[b + 1])] = rng.integers(100, 200)
+        for b in range(2, batch, 4):
+            if weighted and lengths[b]:
+                w[rng.integers(offsets[b], offsets[b + 1])] = rng.choice(FLOATS)
+    return rows, t, indices, offsets, w, n
+
+
+@pytest.mark.parametrize("bit_rate", [8, 4, 2])
+@pytest.mark.parametrize("weighted", [False, True])
+@pytest.mark.parametrize("ordinary", [False, True])
+def test_one_table(gpu_ctx, oracle, bit_rate, weighted, ordinary):
+    rng = np.random.default_rng(10 * bit_rate + 2 * weighted + ordinary)
+    for dim in (4, 20, 64, 128, 256, 300):
+        for batch, mean in ((50, False), (50, True), (15_000 if dim <= 128 else 200, False)):
+            rows, t, indices, offsets, w, n = make(rng, bit_rate, dim, batch, weighted, ordinary)
+            with np.errstate(all="ignore"):
+                ok_ref, ref = oracle.spmdm(bit_rate, dim, rows, t, indices, offsets, w, mean, np.float32, False, True,
+                                           output_size=batch, index_size=n)
+            kw = dict(index_dtype=np.int64, offset_dtype=np.int32, out_dtype=np.float32)
+            kern = (F.GenerateEmbeddingSpMDM(dim, weighted, mean, **kw) if bit_rate == 8
+                    else F.GenerateEmbeddingSpMDMNBit(bit_rate, dim, weighted, mean, **kw))
+            out = torch.zeros(batch * dim, device="cuda")
+            assert kern(batch, n, rows, dev(t), dev(indices), dev(offsets), dev(w), out) and ok_ref
+            same(out.cpu().numpy(), ref)
+
+
+@pytest.mark.parametrize("weighted", [False, True])
+def test_several_tables(gpu_ctx, oracle, weighted):
+    rng = np.random.default_rng(3 + weighted)
+    calls, want = [], []
+    for t in range(9):
+        bit_rate, dim, batch = (8, 4, 2)[t % 3], (64, 128, 256)[t // 3], 70 + t
+        rows, table, indices, offsets, w, n = make(rng, bit_rate, dim, batch, weighted, t == 4)
+        want.append(oracle.spmdm(bit_rate, dim, rows, table, indices, offsets, w, False, np.float32, False, True,
+                                 output_size=batch, index_size=n)[1])
+        kw = dict(index_dtype=np.int64, offset_dtype=np.int32, out_dtype=np.float32)
+        kern = (F.GenerateEmbeddingSpMDM(dim, weighted, False, **kw) if bit_rate == 8
+                else F.GenerateEmbeddingSpMDMNBit(bit_rate, dim, weighted, False, **kw))
+        calls.append((kern, batch, n, rows, dev(table), dev(indices), dev(offsets), dev(w), torch.zeros(batch * dim, device="cuda"), None))
+    plan = F.MultiTablePlan(calls)
+    plan.launch()
+    assert F.status_read(0)[0]
+    for c, ref in zip(calls, want):
+        same(c[8].cpu().numpy(), ref)
+    plan.close()
