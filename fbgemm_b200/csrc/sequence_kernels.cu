@@ -28,10 +28,15 @@
 //
 // Bound by memory: rows read once, output rows written once.  Where the 32
 // positions of a warp name rows of one type (all but the warps at a table's
-// border), it walks them several at a time (walk_rows): rows narrower than 128
-// columns side by side, kInFlight loads issued before the first store.  One row
-// at a time 4.2 M rows of 128 int8 columns to fp16 took 519 us, most of it
-// waiting.
+// border), it walks them several at a time (walk_rows): narrow rows side by
+// side, kInFlight loads issued before the first store.  One row at a time 4.2 M
+// rows of 128 int8 columns to fp16 took 519 us, most of it waiting.  16-bit
+// outputs take eight columns a lane where rows allow it: half the shuffles and
+// stores per row.  Integer columns become floats as the lookup's did once (bits
+// planted in a power of two, which a subtraction takes off again): the
+// conversion instruction runs on a unit of 4 lanes a scheduler, and eight of
+// them a row kept that unit 70 % busy.  The same rows: 369 us before, 327 now,
+// of which 7 by 48 registers instead of 64.
 #include <cuda_fp16.h>
 
 #include "internal.h"
@@ -66,7 +71,8 @@ struct SeqArgs {
   int32_t fp8_exponent_bits;
   int32_t fp8_exponent_bias;
   int32_t fill;      // rows that get nothing else are set to zero
-  int32_t by_fours;  // D % 4 == 0 and output rows aligned for 8- / 16-byte stores
+  int32_t by_fours;   // D % 4 == 0 and output rows aligned for 8- / 16-byte stores
+  int32_t by_eights;  // 16-bit output, D % 8 == 0, D >= 64 and output rows aligned for 16-byte stores
 };
 
 __device__ __noinline__ void report(int32_t* st, int code, int64_t table, int64_t pos, int64_t val) {
@@ -77,12 +83,12 @@ __device__ __noinline__ void report(int32_t* st, int code, int64_t table, int64_
   }
 }
 
-__device__ __forceinline__ uint32_t load_bytes(const uint8_t* p, int n) {
-  uint32_t v = 0;
-  for (int i = 0; i < n; ++i) {
-    v |= (uint32_t)__ldg(p + i) << (8 * i);
+// Four bytes at any address.
+__device__ __forceinline__ uint32_t load_word(const uint8_t* p) {
+  if ((reinterpret_cast<uintptr_t>(p) & 3) == 0) {
+    return __ldg(reinterpret_cast<const uint32_t*>(p));
   }
-  return v;
+  return (uint32_t)__ldg(p) | (uint32_t)__ldg(p + 1) << 8 | (uint32_t)__ldg(p + 2) << 16 | (uint32_t)__ldg(p + 3) << 24;
 }
 
 __device__ __forceinline__ uint16_t to_16bit(float v, bool bf16) {
@@ -99,6 +105,15 @@ enum : int { kToF32 = 0, kToF16 = 1, kToBf16 = 2, kCopy = 3 };
 // weights: fma(scale, q, 0 + bias) for quantized rows, fma(1, x, 0) otherwise.
 __device__ __forceinline__ float from_q(uint32_t q, float scale, float start) {
   return __fmaf_rn(scale, (float)(int)q, start);
+}
+// Column K of the word's as a float, exactly: its bits in the mantissa of the power of two whose last place has the
+// weight they have there (8-bit: moved to the lowest byte), less that power.
+template <int BITS, int K>
+__device__ __forceinline__ float column_of(uint32_t w) {
+  constexpr int at = BITS == 8 ? 0 : BITS * K;
+  constexpr uint32_t power = (uint32_t)(127 + 23 - at) << 23;
+  const uint32_t planted = BITS == 8 ? __byte_perm(w, power, 0x7540u | K) : (w & (((1u << BITS) - 1u) << at)) | power;
+  return __fsub_rn(__uint_as_float(planted), (float)(1u << (23 - at)));
 }
 __device__ __forceinline__ float from_x(float x) {
   return __fmaf_rn(1.f, x, 0.f);
@@ -141,29 +156,50 @@ struct Four {
       w[0] = __ldg(reinterpret_cast<const uint32_t*>(data) + u);
     }
   }
-  __device__ __forceinline__ float value(int c, float scale, float start, float fp8_mult, int fp8_shift) const {
-    if constexpr (TYPE == kFP32) {
-      return from_x(__uint_as_float(w[c]));
-    } else if constexpr (TYPE == kFP16) {
-      return from_x(__half2float(__ushort_as_half((unsigned short)(w[c >> 1] >> (16 * (c & 1))))));
-    } else if constexpr (TYPE == kFP8) {
-      return from_fp8((w[0] >> (8 * c)) & 0xffu, fp8_mult, fp8_shift);
-    } else {
+  __device__ __forceinline__ void values(float* v, float scale, float start, float fp8_mult, int fp8_shift) const {
+    if constexpr (TYPE == kINT8 || TYPE == kINT4 || TYPE == kINT2) {
       constexpr int bits = TYPE == kINT8 ? 8 : (TYPE == kINT4 ? 4 : 2);
-      return from_q((w[0] >> (bits * c)) & ((1u << bits) - 1u), scale, start);
+      v[0] = __fmaf_rn(scale, column_of<bits, 0>(w[0]), start);
+      v[1] = __fmaf_rn(scale, column_of<bits, 1>(w[0]), start);
+      v[2] = __fmaf_rn(scale, column_of<bits, 2>(w[0]), start);
+      v[3] = __fmaf_rn(scale, column_of<bits, 3>(w[0]), start);
+    } else {
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        if constexpr (TYPE == kFP32) {
+          v[c] = from_x(__uint_as_float(w[c]));
+        } else if constexpr (TYPE == kFP16) {
+          v[c] = from_x(__half2float(__ushort_as_half((unsigned short)(w[c >> 1] >> (16 * (c & 1))))));
+        } else {
+          v[c] = from_fp8((w[0] >> (8 * c)) & 0xffu, fp8_mult, fp8_shift);
+        }
+      }
     }
   }
 };
 
+// Two columns of a 16-bit output.
 template <int OUT>
-__device__ __forceinline__ void store_four(uint8_t* orow, int u, const float (&v)[4]) {
-  if constexpr (OUT == kToF32) {
-    __stcs(reinterpret_cast<float4*>(orow) + u, make_float4(v[0], v[1], v[2], v[3]));
+__device__ __forceinline__ uint32_t two(float lo, float hi) {
+  if constexpr (OUT == kToBf16) {
+    return (uint32_t)to_16bit(lo, true) | ((uint32_t)to_16bit(hi, true) << 16);
   } else {
-    constexpr bool bf = OUT == kToBf16;
-    __stcs(reinterpret_cast<uint2*>(orow) + u,
-           make_uint2((uint32_t)to_16bit(v[0], bf) | ((uint32_t)to_16bit(v[1], bf) << 16),
-                      (uint32_t)to_16bit(v[2], bf) | ((uint32_t)to_16bit(v[3], bf) << 16)));
+    const __half2 h = __floats2half2_rn(lo, hi);  // one instruction for both
+    return *reinterpret_cast<const uint32_t*>(&h);
+  }
+}
+
+// Columns 4 * FOURS * u onwards of an output row.
+template <int OUT, int FOURS>
+__device__ __forceinline__ void store_fours(uint8_t* orow, int u, const float (&v)[4 * FOURS]) {
+  if constexpr (OUT == kToF32) {
+    static_assert(FOURS == 1, "16 bytes");
+    __stcs(reinterpret_cast<float4*>(orow) + u, make_float4(v[0], v[1], v[2], v[3]));
+  } else if constexpr (FOURS == 1) {
+    __stcs(reinterpret_cast<uint2*>(orow) + u, make_uint2(two<OUT>(v[0], v[1]), two<OUT>(v[2], v[3])));
+  } else {
+    __stcs(reinterpret_cast<uint4*>(orow) + u,
+           make_uint4(two<OUT>(v[0], v[1]), two<OUT>(v[2], v[3]), two<OUT>(v[4], v[5]), two<OUT>(v[6], v[7])));
   }
 }
 
@@ -176,55 +212,79 @@ __device__ __forceinline__ void emit_row_by_fours(const uint8_t* data, uint8_t* 
     Four<TYPE> d;
     d.load(data, u);
     float v[4];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      v[c] = d.value(c, scale, start, fp8_mult, fp8_shift);
-    }
-    store_four<OUT>(orow, u, v);
+    d.values(v, scale, start, fp8_mult, fp8_shift);
+    store_fours<OUT, 1>(orow, u, v);
   }
 }
 
-// All rows of the warp's 32 positions, which are of type TYPE (or pruned: `pruned` has their bits) and take the
-// four-column path: 1 << log_side rows side by side, kInFlight of those at a time.
-template <int TYPE, int OUT>
+// All rows of the warp's 32 positions, which are of type TYPE (or pruned: `pruned` has their bits, scale and start are
+// zero) and take the four-column path: FOURS times four columns a lane, 1 << log_side rows side by side, kInFlight of
+// those at a time.
+template <int TYPE, int OUT, int FOURS>
 __device__ __forceinline__ void walk_rows(const SeqArgs& a, const uint8_t* my_data, float my_scale, float my_start,
                                           unsigned pruned, uint8_t* out_rows, int lane, float fp8_mult, int fp8_shift) {
-  constexpr int kInFlight = TYPE == kFP32 ? 4 : 8;
-  const int units = a.D >> 2;
+  constexpr int kInFlight = TYPE == kFP32 ? 4 / FOURS : TYPE == kFP16 ? 8 / FOURS : 8;
+  constexpr bool kQuantized = TYPE == kINT8 || TYPE == kINT4 || TYPE == kINT2;
+  const int units = a.D / (4 * FOURS);
   const int log_side = units <= 8 ? 2 : (units <= 16 ? 1 : 0);
-  const int lanes = 32 >> log_side;              // per row
-  const int side = lane / lanes, ul = lane - side * lanes;
-  for (int u0 = 0; u0 < units; u0 += lanes) {    // one round for up to 128 columns
+  const int log_lanes = 5 - log_side;            // per row
+  const int side = lane >> log_lanes, ul = lane & ((1 << log_lanes) - 1);
+  for (int u0 = 0; u0 < units; u0 += 1 << log_lanes) {  // one round for up to 128 * FOURS columns
     const int u = u0 + ul;
     const bool in_row = u < units;
 #pragma unroll 1
     for (int i0 = 0; i0 < 32 >> log_side; i0 += kInFlight) {
-      Four<TYPE> d[kInFlight];
+      Four<TYPE> d[kInFlight][FOURS];
 #pragma unroll
       for (int j = 0; j < kInFlight; ++j) {
         const int i = ((i0 + j) << log_side) + side;
         const uint8_t* data = reinterpret_cast<const uint8_t*>(
             __shfl_sync(0xffffffffu, (unsigned long long)reinterpret_cast<uintptr_t>(my_data), i));
         if (in_row) {
-          d[j].load(data, u);
+#pragma unroll
+          for (int f = 0; f < FOURS; ++f) {
+            d[j][f].load(data, u * FOURS + f);
+          }
         }
       }
 #pragma unroll
       for (int j = 0; j < kInFlight; ++j) {
         const int i = ((i0 + j) << log_side) + side;
-        const float scale = __shfl_sync(0xffffffffu, my_scale, i);
-        const float start = __shfl_sync(0xffffffffu, my_start, i);
+        float scale = 0.f, start = 0.f;
+        if constexpr (kQuantized) {
+          scale = __shfl_sync(0xffffffffu, my_scale, i);
+          start = __shfl_sync(0xffffffffu, my_start, i);
+        }
         if (in_row) {
-          float v[4];
+          float v[4 * FOURS];
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            v[c] = (pruned >> i) & 1u ? 0.f : d[j].value(c, scale, start, fp8_mult, fp8_shift);
+          for (int f = 0; f < FOURS; ++f) {
+            d[j][f].values(v + 4 * f, scale, start, fp8_mult, fp8_shift);
           }
-          store_four<OUT>(out_rows + i * a.out_row_bytes, u, v);
+          if (!kQuantized && ((pruned >> i) & 1u)) {
+#pragma unroll
+            for (int c = 0; c < 4 * FOURS; ++c) {
+              v[c] = 0.f;
+            }
+          }
+          store_fours<OUT, FOURS>(out_rows + i * a.out_row_bytes, u, v);
         }
       }
     }
   }
+}
+
+// Eight columns a lane from 64 columns on, so that a quarter of a warp has a row to do.
+template <int TYPE, int OUT>
+__device__ __forceinline__ void walk_rows_of(const SeqArgs& a, const uint8_t* my_data, float my_scale, float my_start,
+                                             unsigned pruned, uint8_t* out_rows, int lane, float fp8_mult, int fp8_shift) {
+  if constexpr (OUT != kToF32) {
+    if (a.by_eights) {
+      walk_rows<TYPE, OUT, 2>(a, my_data, my_scale, my_start, pruned, out_rows, lane, fp8_mult, fp8_shift);
+      return;
+    }
+  }
+  walk_rows<TYPE, OUT, 1>(a, my_data, my_scale, my_start, pruned, out_rows, lane, fp8_mult, fp8_shift);
 }
 
 // Any width and alignment: one column per lane and step.
@@ -240,17 +300,15 @@ __device__ __forceinline__ void emit_row_by_columns(const uint8_t* data, int typ
       store_column<OUT>(orow, j, from_q((byte >> ((j & ((1 << shift_per) - 1)) * bits)) & mask, scale, start));
     }
   } else if (type == kFP32) {
-    const bool aligned = (reinterpret_cast<uintptr_t>(data) & 3) == 0;
     for (int j = lane; j < D; j += 32) {
-      const uint8_t* e = data + 4 * (int64_t)j;
-      store_column<OUT>(orow, j, from_x(__uint_as_float(aligned ? __ldg(reinterpret_cast<const uint32_t*>(e))
-                                                                : load_bytes(e, 4))));
+      store_column<OUT>(orow, j, from_x(__uint_as_float(load_word(data + 4 * (int64_t)j))));
     }
   } else if (type == kFP16) {
     const bool aligned = (reinterpret_cast<uintptr_t>(data) & 1) == 0;
     for (int j = lane; j < D; j += 32) {
       const uint8_t* e = data + 2 * (int64_t)j;
-      const uint32_t h = aligned ? (uint32_t)__ldg(reinterpret_cast<const unsigned short*>(e)) : load_bytes(e, 2);
+      const uint32_t h = aligned ? (uint32_t)__ldg(reinterpret_cast<const unsigned short*>(e))
+                                 : (uint32_t)__ldg(e) | (uint32_t)__ldg(e + 1) << 8;
       store_column<OUT>(orow, j, from_x(__half2float(__ushort_as_half((unsigned short)h))));
     }
   } else {
@@ -261,7 +319,7 @@ __device__ __forceinline__ void emit_row_by_columns(const uint8_t* data, int typ
 }
 
 template <int OUT>
-__global__ void __launch_bounds__(kThreads) sequence_rows_kernel(const SeqArgs a) {
+__global__ void __launch_bounds__(kThreads, 5) sequence_rows_kernel(const SeqArgs a) {
   __shared__ int64_t starts_s[kSharedStarts];
   const int64_t* starts = stage_table_starts(a, starts_s);
   const int lane = threadIdx.x & 31;
@@ -316,10 +374,10 @@ __global__ void __launch_bounds__(kThreads) sequence_rows_kernel(const SeqArgs a
           const uint8_t* sb = my_row + (a.sb_last ? (a.D * bits + 7) / 8 : 0);
           float bias;
           if (my_type == kINT8 && a.sb_last) {
-            my_scale = __uint_as_float(load_bytes(sb, 4));
-            bias = __uint_as_float(load_bytes(sb + 4, 4));
+            my_scale = __uint_as_float(load_word(sb));
+            bias = __uint_as_float(load_word(sb + 4));
           } else {
-            const uint32_t pair = load_bytes(sb, 4);
+            const uint32_t pair = load_word(sb);
             my_scale = __half2float(__ushort_as_half((unsigned short)(pair & 0xffffu)));
             bias = __half2float(__ushort_as_half((unsigned short)(pair >> 16)));
           }
@@ -343,12 +401,12 @@ __global__ void __launch_bounds__(kThreads) sequence_rows_kernel(const SeqArgs a
         const uint8_t* my_data = (my_state == kZeros ? any : my_row) + (quantized && !a.sb_last ? 4 : 0);
         uint8_t* out_rows = a.out + first * a.out_row_bytes;
         switch (type) {
-          case kINT8: walk_rows<kINT8, OUT>(a, my_data, my_scale, my_start, zeros, out_rows, lane, fp8_mult, fp8_shift); break;
-          case kINT4: walk_rows<kINT4, OUT>(a, my_data, my_scale, my_start, zeros, out_rows, lane, fp8_mult, fp8_shift); break;
-          case kINT2: walk_rows<kINT2, OUT>(a, my_data, my_scale, my_start, zeros, out_rows, lane, fp8_mult, fp8_shift); break;
-          case kFP32: walk_rows<kFP32, OUT>(a, my_data, my_scale, my_start, zeros, out_rows, lane, fp8_mult, fp8_shift); break;
-          case kFP16: walk_rows<kFP16, OUT>(a, my_data, my_scale, my_start, zeros, out_rows, lane, fp8_mult, fp8_shift); break;
-          default: walk_rows<kFP8, OUT>(a, my_data, my_scale, my_start, zeros, out_rows, lane, fp8_mult, fp8_shift); break;
+          case kINT8: walk_rows_of<kINT8, OUT>(a, my_data, my_scale, my_start, zeros, out_rows, lane, fp8_mult, fp8_shift); break;
+          case kINT4: walk_rows_of<kINT4, OUT>(a, my_data, my_scale, my_start, zeros, out_rows, lane, fp8_mult, fp8_shift); break;
+          case kINT2: walk_rows_of<kINT2, OUT>(a, my_data, my_scale, my_start, zeros, out_rows, lane, fp8_mult, fp8_shift); break;
+          case kFP32: walk_rows_of<kFP32, OUT>(a, my_data, my_scale, my_start, zeros, out_rows, lane, fp8_mult, fp8_shift); break;
+          case kFP16: walk_rows_of<kFP16, OUT>(a, my_data, my_scale, my_start, zeros, out_rows, lane, fp8_mult, fp8_shift); break;
+          default: walk_rows_of<kFP8, OUT>(a, my_data, my_scale, my_start, zeros, out_rows, lane, fp8_mult, fp8_shift); break;
         }
         return;
       }
@@ -466,6 +524,8 @@ cudaError_t launch_sequence_lookup(
   }
   const int64_t store_bytes = out_kind == FBGEMM_B200_OUT_F32 ? 16 : 8;
   a.by_fours = D % 4 == 0 && reinterpret_cast<uintptr_t>(out) % store_bytes == 0 && out_row_bytes % store_bytes == 0;
+  a.by_eights = out_kind != FBGEMM_B200_OUT_F32 && D % 8 == 0 && D >= 64 && reinterpret_cast<uintptr_t>(out) % 16 == 0 &&
+      out_row_bytes % 16 == 0;
   switch (out_kind) {
     case FBGEMM_B200_OUT_F32: sequence_rows_kernel<kToF32><<<(unsigned)blocks, kThreads, 0, stream>>>(a); break;
     case FBGEMM_B200_OUT_F16: sequence_rows_kernel<kToF16><<<(unsigned)blocks, kThreads, 0, stream>>>(a); break;
