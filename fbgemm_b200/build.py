@@ -24,7 +24,7 @@ LIB_PATH = os.path.join(PKG_DIR, "libfbgemm_b200.so")
 STAMP_PATH = os.path.join(PKG_DIR, "csrc", ".build_stamp")
 
 CUDA_SOURCES = ["bag_units_lean.cu", "bag_units_full.cu", "bag_units_mapped.cu", "bag_units_wide.cu", "bag_kernel_8.cu",
-                "bag_kernel_4.cu", "bag_kernel_2.cu", "bag_kernel_plain.cu", "bag_dispatch.cu", "spmdm_kernels.cu", "rows_copy_kernels.cu", "scan_kernels.cu",
+                "bag_kernel_4.cu", "bag_kernel_2.cu", "bag_kernel_plain.cu", "few_bags_kernel.cu", "bag_dispatch.cu", "spmdm_kernels.cu", "rows_copy_kernels.cu", "scan_kernels.cu",
                 "quantize_kernels.cu", "remap_kernels.cu", "pruned_lookup_kernels.cu", "sequence_kernels.cu", "stage_kernels.cu",
                 "c_api.cu", "noalloc_entry.cu", "peer_sync_kernels.cu", "multi_host.cu"]
 CXX_SOURCES = ["generators.cc", "host_copy.cc"]

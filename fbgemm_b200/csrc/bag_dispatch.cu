@@ -72,6 +72,7 @@ void bag_table_of(const SpmdmParams& p, BagTable* t) {
   t->out_align = (int16_t)alignment_of(o);
   t->fp8_exponent_bits = (int16_t)p.fp8_exponent_bits;
   t->fp8_exponent_bias = (int16_t)p.fp8_exponent_bias;
+  t->data_align = (int16_t)alignment_of(reinterpret_cast<uintptr_t>(t->data) | (uint64_t)t->stride);
 }
 
 // The form of a table's kernel.  (A row-wise sparse call says how many rows its
@@ -141,7 +142,7 @@ int64_t blocks_of(int64_t bags, int variant) {
 
 // `bags` in the launch, `beside` in those on other streams; `single`: one table's launch.
 int pick_variant(const BagTable& t, int fmt, int64_t bags, int64_t beside, bool single, int64_t sms, int* tiles) {
-  const int align = alignment_of(reinterpret_cast<uintptr_t>(t.data) | (uint64_t)t.stride);
+  const int align = t.data_align;
   const bool mapped = t.flags & kPruned;
   const int64_t resident = resident_warps(sms);
   const int64_t quarter_warps_from = (mapped && beside > 0 ? 4 : 8) * resident;
@@ -195,13 +196,13 @@ bag::BagFn single_kernel(int variant, int form) {
 // wait for its results themselves (griddepcontrol.wait).  0.3 to 0.6 us less
 // between launches of 4 to 12 us.
 template <typename Arg>
-cudaError_t launch(void (*fn)(Arg), dim3 grid, const Arg& arg, cudaStream_t stream) {
+cudaError_t launch(void (*fn)(Arg), dim3 grid, const Arg& arg, cudaStream_t stream, int threads = bag::kThreads) {
   cudaLaunchAttribute overlap{};
   overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   overlap.val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
-  cfg.blockDim = dim3(bag::kThreads);
+  cfg.blockDim = dim3((unsigned)threads);
   cfg.stream = stream;
   cfg.attrs = &overlap;
   cfg.numAttrs = 1;
@@ -219,7 +220,23 @@ cudaError_t launch_bags(const SpmdmParams& p, int bit_rate, cudaStream_t stream)
   }
   const int64_t sms = sm_count();
   int tiles = 0;
-  const int v = pick_variant(c.t, format_of(p, bit_rate), p.output_size, p.bags_beside, true, sms, &tiles);
+  const int fmt = format_of(p, bit_rate);
+  // A block per bag and 128 columns, up to four such blocks an SM, eight where bags are long; rows that words cannot copy
+  // only where a bag's walk is long enough to pay for that.  us per call, called and awaited, with a warp per bag / a block
+  // per bag, 8-bit rows at 4 M rows, 10, 100, 590 and 1100 bags:
+  //   D = 64, bags of 4, 30, 64 and 100 rows on average
+  //     12.8 / 12.8  12.9 / 13.1  12.9 / 13.2  12.9 / 13.2 (by a warp)     15.2 / 13.9  15.5 / 14.1  15.8 / 14.3  15.9 / 15.4 (by a warp)
+  //     19.1 / 14.6  19.3 / 14.8  19.9 / 16.0  20.1 / 19.2                 21.5 / 15.0  23.8 / 15.3  24.4 / 17.7  28.5 / 21.6
+  //   D = 86 (halves), bags of 4 and 30 rows, 10, 100 and 590 bags
+  //     13.4 / 14.0  13.7 / 13.9  13.4 / 14.5     16.3 / 15.1  16.8 / 15.5  17.0 / 16.5
+  const int64_t few_tiles = (c.t.cols + bag::kFewColumns - 1) / bag::kFewColumns;
+  const auto rows_per_bag = [&](int64_t rows) { return p.index_size / rows >= p.output_size; };
+  const int64_t few_per_sm = bag::few_by_words(c.t) ? (rows_per_bag(64) ? 8 : 4) : rows_per_bag(16) ? 4 : 0;
+  if (bag::is_quantized(fmt) && p.num_peers <= 0 && !(c.t.flags & kNoBag) && p.output_size > 0 && p.index_size <= 0x7fffff00LL &&
+      (p.output_size + p.bags_beside) * few_tiles <= few_per_sm * sms) {
+    return launch<bag::BagCall>(bag::few_bags(fmt), dim3((unsigned)p.output_size, (unsigned)few_tiles), c, stream, bag::kFewThreads);
+  }
+  const int v = pick_variant(c.t, fmt, p.output_size, p.bags_beside, true, sms, &tiles);
   const int64_t blocks = blocks_of(p.output_size, v);
   if (blocks <= 0 || blocks > 0x7fffffffLL || tiles > 65535) {
     return cudaErrorInvalidValue;

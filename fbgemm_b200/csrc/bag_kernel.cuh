@@ -957,6 +957,15 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm) bag_units_kernel(const
 
 using BagFn = void (*)(const BagCall);
 
+// A handful of bags in one quantized table (few_bags_kernel.cu): a block per bag and kFewColumns columns.
+constexpr int kFewThreads = 256, kFewColumns = 128;
+BagFn few_bags(int fmt);
+// Whether it copies rows in words of four bytes (the last one may run into scale and bias behind the payload, but not
+// beyond the row) or in smaller units.
+__host__ __device__ __forceinline__ bool few_by_words(const BagTable& t) {
+  return t.data_align >= 4 && (t.data_bytes % 4 == 0 || t.sb_off > 0);
+}
+
 constexpr int kDeepForms = 4;             // kDeepForms + form: its deep form (there is none of kWide)
 constexpr int kForms = 2 * kDeepForms;
 using BagUnitsFn = void (*)(const BagUnits);

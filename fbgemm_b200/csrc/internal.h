@@ -106,6 +106,7 @@ struct BagTable {
   int32_t num_peers;
   int16_t fp8_exponent_bits;
   int16_t fp8_exponent_bias;
+  int16_t data_align;         // address alignment of payloads: 16 ... 1
 };
 
 // One lookup kernel launch (spmdm_kernels.cu).  Returns cudaSuccess or the
