@@ -374,7 +374,8 @@ using Row = typename std::conditional<WIDE, unsigned long long, uint32_t>::type;
 // two).  It costs a register or two: not for kernels that have none left.  us
 // without / with: 8-bit 10 000 bags 13.0 / 12.5, pruned 2-bit 8192 bags 9.7 / 9.5,
 // 8 4-bit tables of 65 536 bags 616 / 605, 64 mixed ones of 16 384 1128 / 1121;
-// 8-bit D = 128 on half warps of 40 registers, 65 536 bags of 64 rows, 94.2 / 98.9.
+// 8-bit D = 128 on half warps of 40 registers, 65 536 bags of 64 rows, 94.2 / 98.9;
+// several chunks a lane (8-bit D = 257, 4007 bags of 15 rows) 20.9 / 23.7.
 template <int VB, int CPL, int G, bool WIDE, bool OWN>
 struct LaneData {
   const uint8_t* first;
@@ -577,7 +578,7 @@ __device__ __forceinline__ void pool_bags(const BagTable& p, void* const* peers,
   const bool half_sb = FMT != kInt8 || (p.flags & kSbFirst);
 
   const Pos bag = (Pos)block * (kWarps * (32 / G)) + warp * (32 / G) + grp;
-  constexpr bool kOwn = kDeep || (MODE == kLean && kQuantized && VB * CPL * (kAhead + 1) <= 8);
+  constexpr bool kOwn = CPL == 1 && (kDeep || (MODE == kLean && kQuantized && VB * (kAhead + 1) <= 8));
   LaneData<VB, CPL, G, WIDE, kOwn> lane_data;
   lane_data.init(p.data, tile * kTileBytes, gl, p.data_bytes);
   const uint8_t* sb_data = p.data + p.sb_off;
