@@ -76,7 +76,7 @@ void bag_table_of(const SpmdmParams& p, BagTable* t) {
 }
 
 // The form of a table's kernel.  (A row-wise sparse call says how many rows its
-// map has, not how many its table holds, which may be more: see pool_far_rows.)
+// map has, not how many its table holds, which may be more: see pool_again.)
 int form_of(const BagTable& t) {
   const bool wide = (unsigned __int128)t.data_size * (uint64_t)t.stride > 0xffffffffull || t.bags > 0x7fffff00LL ||
       t.index_size > 0x7fffff00LL;
