@@ -124,24 +124,27 @@ __host__ __device__ constexpr int column_bits(int fmt) { return fmt == kBf16 ? 1
 //     acc' = fma(scale * 2^(149 - p - kDown), q * 2^(p - 149), acc' + bias * 2^-kDown)
 // and brought back by an exact multiplication at the end.  Every step rounds as
 // the unscaled one does where neither form leaves fp32's normal range, which holds
-// for all rows whose weighted scale and bias are zero or of magnitude 2^-52 to
-// 2^52: all values are then multiples of 2^-75 (2^-149 scaled: exact where
-// subnormal) and, over 2^31 positions, below 2^92.  A bag with a row of other
-// values (infinite ones, NaN and weights of 1e-20 among them) is pooled once
-// more, unscaled (pool_again).
+// for all rows whose weighted scale and bias are zero or of magnitude 2^-68
+// (3e-21) to 2^36 (7e10): all values are then multiples of 2^-91 (2^-149 scaled:
+// exact where subnormal) and, over 2^31 positions, below 2^76.  A bag with a row
+// of other values (infinite ones, NaN and weights of 1e-30 among them) is pooled
+// once more, unscaled (pool_again).  kDown moves those 104 powers of two up and
+// down: weights that decay, and softmax weights, are small far more often than
+// embeddings are large.
 // Before, each column's bits were planted in the mantissa of a power of two that
 // a packed addition then subtracted.  One row of 8 columns a lane, issue cycles of
 // a scheduler, rows and scales in shared memory: 8-bit 22.0 / 18.0, 4-bit 25.1 / 19.4.
 // 64 mixed tables of 16 384 bags 1135 / 1069 us, 8 4-bit tables of 65 536 bags 635 / 610.
-constexpr int kDown = 74;
-constexpr float kScaleUp = 1.f * (1ull << 60) * (1 << 15);                          // 2^(149 - kDown)
-constexpr float kBiasDown = 1.f / ((float)(1ull << 60) * (float)(1 << 14));         // 2^-kDown
-constexpr float kSumUp = (float)(1ull << 60) * (float)(1 << 14);                    // 2^kDown
+constexpr int kDown = 58;
+constexpr float kSumUp = (float)(1ull << kDown);                                    // 2^kDown
+constexpr float kBiasDown = 1.f / kSumUp;
+constexpr float kScaleUp = (float)(1ull << 60) * (float)(1ull << (89 - kDown));     // 2^(149 - kDown)
+constexpr int kLeast = kDown - 126, kMost = kDown - 22;                             // powers of two of the range
 
 // Whether a weighted scale or bias is one that the scaled sums are not made for.
 __device__ __forceinline__ bool out_of_scale(float x) {
   const uint32_t magnitude = __float_as_uint(x) << 1;
-  return magnitude != 0 && magnitude - ((127u - 52u) << 24) >= (104u << 24);
+  return magnitude != 0 && magnitude - ((uint32_t)(127 + kLeast) << 24) >= ((uint32_t)(kMost - kLeast) << 24);
 }
 
 // Where column K of a chunk of COLS columns lies: kPlaces columns are cut out of
@@ -489,7 +492,10 @@ __device__ __forceinline__ void bag_from_lengths(const BagTable& p, int64_t firs
 //   costs the other bags one comparison per mapped row and no registers (11.3 us before and after for 8192 bags of 30
 //   rows, 2-bit D = 128), where 64-bit addresses for every pruned table would cost each of their rows the wide form's
 //   extra instructions;
-// * a row's weighted scale or bias is out_of_scale.
+// * a row's weighted scale or bias is out_of_scale.  A chain of two or three loads per row: a launch with one such bag of 20
+//   rows takes 6 us longer, one whose weights are all 1e-30 two to three times as long (us, weights of 1 / 1e-30 and, while
+//   the range was 2^-52 to 2^52, 1e-16 too: 8-bit 10 000 bags of 20 rows 10.1 / 22.5, 4-bit 4096 ragged bags 7.9 / 22.7,
+//   2-bit pruned 8192 bags 9.3 / 30.2, 8 4-bit tables of 16 384 bags 142 / 424).
 template <class C, int VB, int CPL, int G, int MODE, class Lane>
 __device__ __forceinline__ void pool_again(const BagTable& p, const typename C::M& constants, const Lane& lane_data,
                                            int64_t start, int len, u64 (&acc)[C::kPairs]) {
