@@ -371,16 +371,13 @@ template <bool WIDE>
 using Row = typename std::conditional<WIDE, unsigned long long, uint32_t>::type;
 
 // Where a lane finds its chunks of a row; lanes whose chunk lies beyond the
-// payload read chunk 0 instead and do not store.  OWN: a lane's first chunk of
-// row 0 is an address of its own, opaque to the compiler, which otherwise adds
-// row, chunk and table up anew for every row (three instructions instead of
-// two).  It costs a register or two: not for kernels that have none left.  us
-// without / with: 8-bit 10 000 bags 13.0 / 12.5, pruned 2-bit 8192 bags 9.7 / 9.5,
-// 8 4-bit tables of 65 536 bags 616 / 605, 64 mixed ones of 16 384 1128 / 1121;
-// 8-bit D = 128 on half warps of 40 registers, 65 536 bags of 64 rows, 94.2 / 98.9;
-// several chunks a lane (8-bit D = 257, 4007 bags of 15 rows) 20.9 / 23.7.
+// payload read chunk 0 instead and do not store.  OWN (one chunk a lane): where
+// row 0 has the lane's chunk is an address of its own, opaque to the compiler,
+// which otherwise adds row, chunk and table up anew for every row (three
+// instructions instead of two).  It costs a register or two: see own_address.
 template <int VB, int CPL, int G, bool WIDE, bool OWN>
 struct LaneData {
+  static_assert(!OWN || CPL == 1, "one address");
   const uint8_t* first;
   uint32_t at[CPL];  // from there
   __device__ __forceinline__ void init(const uint8_t* data, int tile_at, int gl, int data_bytes) {
@@ -392,24 +389,16 @@ struct LaneData {
     }
     if constexpr (OWN) {
       asm volatile("mov.b64 %0, %1;" : "=l"(first) : "l"(data + at[0]));
-#pragma unroll
-      for (int c = CPL - 1; c >= 0; --c) {
-        at[c] = at[c] > at[0] ? c * G * VB : 0;
-      }
     }
   }
   // Chunk c of the row whose payload starts at `row`.
   __device__ __forceinline__ const uint8_t* chunk(const uint8_t* row, const uint8_t* data, int c) const {
-    return OWN ? first + (row - data) + at[c] : row + at[c];
+    return OWN ? first + (row - data) : row + at[c];
   }
   __device__ __forceinline__ void load(Bytes<VB> (&d)[CPL], Row<WIDE> row) const {
 #pragma unroll
     for (int c = 0; c < CPL; ++c) {
-      if (OWN && c == 0) {
-        d[c].load(first + row);
-      } else {
-        d[c].load(first + (Row<WIDE>)(row + at[c]));
-      }
+      d[c].load(OWN ? first + row : first + (Row<WIDE>)(row + at[c]));
     }
   }
 };
@@ -437,6 +426,17 @@ enum : int { kLean = 0, kFull = 1, kWide = 2, kMapped = 3 };
 // registers each (kDeep) take one more with whole warps.
 __host__ __device__ constexpr int rows_ahead(int fmt, int g, bool deep) {
   return g == 32 ? (deep ? 2 : 1) : deep ? 1 : g == 16 && (fmt == kInt8 || fmt == kInt2) ? 1 : 0;
+}
+
+// Whether lanes keep an address of their own: kernels whose rows in flight leave registers for it.  us per call without /
+// with: 8-bit 10 000 bags 13.0 / 12.5, pruned 2-bit 8192 bags 9.7 / 9.5, fp16 D = 64 1500 bags 3.15 / 2.92, 8 4-bit tables
+// of 65 536 bags 616 / 605, 64 mixed ones of 16 384 1128 / 1121.  Beyond the line: 8-bit D = 128 on half warps of 40
+// registers, 65 536 bags of 64 rows, 94.2 / 98.9; in the deep form fp32 D = 128 4000 bags 7.9 / 8.5, 8-bit D = 256 by lengths
+// 1500 bags 5.7 / 6.3 (their rows in flight spill); several chunks a lane (8-bit D = 257, 4007 bags of 15 rows) 20.9 / 23.7.
+__host__ __device__ constexpr bool own_address(int fmt, int vb, int cpl, int g, int mode, bool deep) {
+  const int bytes_in_flight = vb * (rows_ahead(fmt, g, deep) + 1);
+  const int most = deep ? (is_quantized(fmt) && mode != kLean ? 16 : 24) : is_quantized(fmt) && mode == kLean ? 8 : 0;
+  return cpl == 1 && bytes_in_flight <= most;
 }
 
 // The stream's next launch may be set up while this one drains; it waits here until all results of this one are there.
@@ -496,7 +496,7 @@ __device__ __forceinline__ void bag_from_lengths(const BagTable& p, int64_t firs
 //   rows takes 6 us longer, one whose weights are all 1e-30 two to three times as long (us, weights of 1 / 1e-30 and, while
 //   the range was 2^-52 to 2^52, 1e-16 too: 8-bit 10 000 bags of 20 rows 10.1 / 22.5, 4-bit 4096 ragged bags 7.9 / 22.7,
 //   2-bit pruned 8192 bags 9.3 / 30.2, 8 4-bit tables of 16 384 bags 142 / 424).
-template <class C, int VB, int CPL, int G, int MODE, class Lane>
+template <class C, int VB, int CPL, class Lane>
 __device__ __forceinline__ void pool_again(const BagTable& p, const typename C::M& constants, const Lane& lane_data,
                                            int64_t start, int len, u64 (&acc)[C::kPairs]) {
   float sum[2 * C::kPairs];
@@ -584,8 +584,7 @@ __device__ __forceinline__ void pool_bags(const BagTable& p, void* const* peers,
   const bool half_sb = FMT != kInt8 || (p.flags & kSbFirst);
 
   const Pos bag = (Pos)block * (kWarps * (32 / G)) + warp * (32 / G) + grp;
-  constexpr bool kOwn = CPL == 1 && (kDeep || (MODE == kLean && kQuantized && VB * (kAhead + 1) <= 8));
-  LaneData<VB, CPL, G, WIDE, kOwn> lane_data;
+  LaneData<VB, CPL, G, WIDE, own_address(FMT, VB, CPL, G, MODE, kDeep)> lane_data;
   lane_data.init(p.data, tile * kTileBytes, gl, p.data_bytes);
   const uint8_t* sb_data = p.data + p.sb_off;
   typename C::M constants;
@@ -811,7 +810,7 @@ __device__ __forceinline__ void pool_bags(const BagTable& p, void* const* peers,
     const unsigned lanes = __ballot_sync(0xffffffffu, again);
     if (lanes != 0) {
       if ((lanes >> (grp * G)) & kGroupMask) {
-        pool_again<C, VB, CPL, G, MODE>(p, constants, lane_data, pos - gl - (Pos)((longest + G - 1) / G * G), len, acc);
+        pool_again<C, VB, CPL>(p, constants, lane_data, pos - gl - (Pos)((longest + G - 1) / G * G), len, acc);
         up = 1.f;
       }
     }
