@@ -5,6 +5,7 @@
 #include <vector>
 
 #include "bag_kernel.cuh"
+#include "few_bags_rule.h"
 
 namespace fbgemm_b200 {
 
@@ -221,22 +222,22 @@ cudaError_t launch_bags(const SpmdmParams& p, int bit_rate, cudaStream_t stream)
   const int64_t sms = sm_count();
   int tiles = 0;
   const int fmt = format_of(p, bit_rate);
-  // A block per bag and 128 columns, up to four such blocks an SM, eight where bags are long; rows that words cannot copy
-  // only where a bag's walk is long enough to pay for that.  us per call, called and awaited, with a warp per bag / a block
-  // per bag, 8-bit rows at 4 M rows, 10, 100, 590 and 1100 bags:
-  //   D = 64, bags of 4, 30, 64 and 100 rows on average
-  //     12.8 / 12.8  12.9 / 13.1  12.9 / 13.2  12.9 / 13.2 (by a warp)     15.2 / 13.9  15.5 / 14.1  15.8 / 14.3  15.9 / 15.4 (by a warp)
-  //     19.1 / 14.6  19.3 / 14.8  19.9 / 16.0  20.1 / 19.2                 21.5 / 15.0  23.8 / 15.3  24.4 / 17.7  28.5 / 21.6
-  //   D = 86 (halves), bags of 4 and 30 rows, 10, 100 and 590 bags
-  //     13.4 / 14.0  13.7 / 13.9  13.4 / 14.5     16.3 / 15.1  16.8 / 15.5  17.0 / 16.5
-  const int64_t few_tiles = (c.t.cols + bag::kFewColumns - 1) / bag::kFewColumns;
-  const auto rows_per_bag = [&](int64_t rows) { return p.index_size / rows >= p.output_size; };
-  const int64_t few_per_sm = bag::few_by_words(c.t) ? (rows_per_bag(64) ? 8 : 4) : rows_per_bag(16) ? 4 : 0;
-  if (bag::is_quantized(fmt) && p.num_peers <= 0 && !(c.t.flags & kNoBag) && p.output_size > 0 && p.index_size <= 0x7fffff00LL &&
-      (p.output_size + p.bags_beside) * few_tiles <= few_per_sm * sms) {
-    return launch<bag::BagCall>(bag::few_bags(fmt), dim3((unsigned)p.output_size, (unsigned)few_tiles), c, stream, bag::kFewThreads);
-  }
   const int v = pick_variant(c.t, fmt, p.output_size, p.bags_beside, true, sms, &tiles);
+  if (bag::is_quantized(fmt) && p.num_peers <= 0 && !(c.t.flags & kNoBag) && p.index_size <= 0x7fffff00LL) {
+    FewBagsCall few{};
+    few.bits = fmt;
+    few.words = bag::few_by_words(c.t);
+    few.units = bag::few_units(c.t, fmt);
+    few.warp_chunks = kVariantInfo[v].cpl;
+    few.mapped = c.t.flags & kPruned;
+    few.tiles = (c.t.cols + bag::kFewColumns - 1) / bag::kFewColumns;
+    few.bags = p.output_size;
+    few.beside = p.bags_beside;
+    few.rows = p.index_size;
+    if (few_bags_pay(few, sms)) {
+      return launch<bag::BagCall>(bag::few_bags(fmt), dim3((unsigned)p.output_size, (unsigned)few.tiles), c, stream, bag::kFewThreads);
+    }
+  }
   const int64_t blocks = blocks_of(p.output_size, v);
   if (blocks <= 0 || blocks > 0x7fffffffLL || tiles > 65535) {
     return cudaErrorInvalidValue;

@@ -971,6 +971,15 @@ BagFn few_bags(int fmt);
 __host__ __device__ __forceinline__ bool few_by_words(const BagTable& t) {
   return t.data_align >= 4 && (t.data_bytes % 4 == 0 || t.sb_off > 0);
 }
+// Of those, by halves where rows allow it.
+__host__ __device__ __forceinline__ bool few_by_halves(const BagTable& t) {
+  return t.data_align >= 2 && (t.data_bytes % 2 == 0 || t.sb_off > 0);
+}
+// Units that a row's widest tile takes.
+inline int few_units(const BagTable& t, int fmt) {
+  const int bytes = t.data_bytes < kFewColumns * fmt / 8 ? t.data_bytes : kFewColumns * fmt / 8;
+  return few_by_halves(t) ? (bytes + 1) / 2 : bytes;
+}
 
 constexpr int kDeepForms = 4;             // kDeepForms + form: its deep form (there is none of kWide)
 constexpr int kForms = 2 * kDeepForms;

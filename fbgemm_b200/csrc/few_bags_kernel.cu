@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(kFewThreads) few_bags_kernel(const __grid_cons
 
   // Whole words: the last one may run into scale and bias behind the payload, but not beyond the row.
   const bool by_words = few_by_words(p);
-  const bool by_halves = p.data_align >= 2 && (p.data_bytes % 2 == 0 || p.sb_off > 0);
+  const bool by_halves = few_by_halves(p);
   const int col = blockIdx.y * kPitch + tid;
   float acc = 0.f;
   for (int c0 = 0; c0 < len; c0 += kRows) {
