@@ -805,15 +805,26 @@ __device__ __forceinline__ void pool_bags(const BagTable& p, void* const* peers,
     __syncwarp();  // the queue is rewritten by the next stretch
   }
 
+  constexpr bool kAgain = kQuantized || (MAPS && !WIDE);
+  // Pooled again before the row is stored; with eight bytes a lane and whole warps of the lean deep form after it, and stored
+  // again: the walk's code is better with it there.  us, before / after the store: 8-bit D = 256, 590 bags of 16 rows
+  // 4.17 / 3.88, 1500 of 20 rows 5.59 / 5.28; D = 512, 100 bags of 16 rows 4.09 / 3.79; D = 1024, 1100 bags of 2 rows
+  // 4.13 / 3.82.  (8-bit D = 64 3.32 / 3.36, pruned D = 256 4.59 / 4.71; the 40-register forms spill, 4-bit D = 128, 15 000
+  // bags 12.6 / 16.5.)
+  constexpr bool kAgainLast = kAgain && kDeep && G == 32 && VB == 8 && MODE == kLean;
   float up = kQuantized ? kSumUp : 1.f;  // from the scaled sums to the pooled row
-  if constexpr (kQuantized || (MAPS && !WIDE)) {
-    const unsigned lanes = __ballot_sync(0xffffffffu, again);
-    if (lanes != 0) {
-      if ((lanes >> (grp * G)) & kGroupMask) {
-        pool_again<C, VB, CPL>(p, constants, lane_data, pos - gl - (Pos)((longest + G - 1) / G * G), len, acc);
-        up = 1.f;
-      }
+  unsigned lanes = 0;                    // of the group's, those that met a row for pool_again
+  if constexpr (kAgain) {
+    lanes = __ballot_sync(0xffffffffu, again);
+  }
+  auto pool_anew = [&] {
+    if (lanes != 0 && ((lanes >> (grp * G)) & kGroupMask)) {
+      pool_again<C, VB, CPL>(p, constants, lane_data, pos - gl - (Pos)((longest + G - 1) / G * G), len, acc);
+      up = 1.f;
     }
+  };
+  if constexpr (kAgain && !kAgainLast) {
+    pool_anew();
   }
 
   if constexpr (!kDeep) {
@@ -822,38 +833,46 @@ __device__ __forceinline__ void pool_bags(const BagTable& p, void* const* peers,
   if (bag >= (Pos)p.bags) {
     return;
   }
-  int bag_len = 0;
-  if (p.flags & kNormalize) {
-    bag_len = by_lengths ? (int)load_int(p.offsets, bag, off64)
-                         : (int)(load_int(p.offsets, (int64_t)bag + 1, off64) - load_int(p.offsets, bag, off64));
-  }
-  if (kQuantized || bag_len != 0) {
-    // (exact but for the mean's own rounding: a power of two, and no sum is near either end of the range)
-    const float by = bag_len != 0 ? __fmul_rn(__fdiv_rn(1.f, (float)bag_len), up) : up;
-    const u64 by2 = pack2(by, by);
+#pragma unroll 1
+  for (;;) {
+    int bag_len = 0;
+    if (p.flags & kNormalize) {
+      bag_len = by_lengths ? (int)load_int(p.offsets, bag, off64)
+                           : (int)(load_int(p.offsets, (int64_t)bag + 1, off64) - load_int(p.offsets, bag, off64));
+    }
+    if (kQuantized || bag_len != 0) {
+      // (exact but for the mean's own rounding: a power of two, and no sum is near either end of the range)
+      const float by = bag_len != 0 ? __fmul_rn(__fdiv_rn(1.f, (float)bag_len), up) : up;
+      const u64 by2 = pack2(by, by);
+#pragma unroll
+      for (int k = 0; k < C::kPairs; ++k) {
+        acc[k] = mul2(acc[k], by2);
+      }
+    }
+    char* row;
+    if (p.num_peers > 0) {
+      const int64_t d = bag / p.bags_per_peer;
+      row = static_cast<char*>(peers[d]) + (bag - d * p.bags_per_peer) * p.out_pitch;
+    } else {
+      row = static_cast<char*>(p.out) + bag * p.out_pitch;
+    }
+    float v[2 * C::kPairs];
 #pragma unroll
     for (int k = 0; k < C::kPairs; ++k) {
-      acc[k] = mul2(acc[k], by2);
+      unpack2(acc[k], v[2 * k], v[2 * k + 1]);
     }
-  }
-  char* row;
-  if (p.num_peers > 0) {
-    const int64_t d = bag / p.bags_per_peer;
-    row = static_cast<char*>(peers[d]) + (bag - d * p.bags_per_peer) * p.out_pitch;
-  } else {
-    row = static_cast<char*>(p.out) + bag * p.out_pitch;
-  }
-  float v[2 * C::kPairs];
 #pragma unroll
-  for (int k = 0; k < C::kPairs; ++k) {
-    unpack2(acc[k], v[2 * k], v[2 * k + 1]);
-  }
-#pragma unroll
-  for (int c = 0; c < CPL; ++c) {
-    const int col = tile * (kTileBytes * 8 / C::BITS) + (c * G + gl) * C::kPerChunk;
-    if (col < p.cols) {
-      store_columns<C::kPerChunk>(p, row, col, v + c * C::kPerChunk);
+    for (int c = 0; c < CPL; ++c) {
+      const int col = tile * (kTileBytes * 8 / C::BITS) + (c * G + gl) * C::kPerChunk;
+      if (col < p.cols) {
+        store_columns<C::kPerChunk>(p, row, col, v + c * C::kPerChunk);
+      }
     }
+    if (!kAgainLast || lanes == 0) {
+      return;
+    }
+    pool_anew();
+    lanes = 0;
   }
 }
 
