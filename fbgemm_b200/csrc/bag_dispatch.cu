@@ -167,9 +167,16 @@ int pick_variant(const BagTable& t, int fmt, int64_t bags, int64_t beside, bool 
     if (n > 1 && v.g < 32) {
       continue;
     }
-    // instructions per row: what a row costs besides its columns, its loads, and 2.5 per column of a lane
+    // Instructions per row: what a row costs besides its columns, its loads, and per column of a lane one that cuts it out,
+    // half a packed addition and half a packed multiply-add (unquantized rows, whose conversions differ, 2.5 in all).  Half
+    // an instruction more where four chunks a lane make the rows in flight spill, and for a few bags, whose warps do not
+    // fill the chip and rather have more tiles.  us with 2.5 throughout / so: 8-bit D = 150 (two tiles of 4 columns a lane
+    // for three of 2), 4007, 15 000 and 60 000 bags 9.4 / 9.6, 30.5 / 27.5, 120 / 103, 700 bags if they did too 5.6 / 6.0;
+    // 8-bit D = 301 (five tiles of 2 for three of 4), 700, 1500, 4007 and 15 000 bags 9.1 / 6.4, 12.2 / 12.4, 18.9 / 16.0,
+    // 71 / 59; 4-bit D = 802 (seven for four), 700 and 15 000 bags 10.0 / 7.3, 119 / 89.
     const double cols = (double)v.vb * v.cpl * 8 / bag::column_bits(fmt);
-    const double cost = n * (6.0 + 1.5 * v.cpl + 2.5 * cols) * v.g;
+    const double per_column = !bag::is_quantized(fmt) ? 2.5 : 2.0 + (v.cpl >= 4 ? 0.5 : 0.0) + (bags + beside <= 8 * sms ? 0.5 : 0.0);
+    const double cost = n * (6.0 + 1.5 * v.cpl + per_column * cols) * v.g;
     if (best < 0 || cost < best_cost) {
       best = i;
       best_cost = cost;
