@@ -51,11 +51,13 @@ def check(oracle, rng, bit_rate, dim, batch, sb_last, pad, weighted=True, rows=1
 
 @pytest.mark.parametrize("bit_rate", [8, 4, 2])
 @pytest.mark.parametrize("sb_last", [True, False])
-def test_row_widths_and_alignments(gpu_ctx, oracle, bit_rate, sb_last):
+@pytest.mark.parametrize("batch", [40, 1500])
+def test_row_widths_and_alignments(gpu_ctx, oracle, bit_rate, sb_last, batch):
+    """40 bags are partly for a block each (few_bags_kernel.cu), 1500 for a warp each."""
     rng = np.random.default_rng(100 * bit_rate + sb_last)
-    for dim in (1, 2, 15, 16, 17, 31, 32, 33, 63, 64, 65, 127, 128, 129, 255, 256, 257, 300, 520, 1024):
+    for dim in (1, 2, 15, 16, 17, 31, 32, 33, 63, 64, 65, 127, 128, 129, 150, 192, 193, 255, 256, 257, 300, 320, 321, 520, 1024):
         for pad in (0, 1, 2, 4):
-            check(oracle, rng, bit_rate, dim, 40, sb_last, pad, weighted=(dim + pad) % 2 == 0)
+            check(oracle, rng, bit_rate, dim, batch, sb_last, pad, weighted=(dim + pad) % 2 == 0)
 
 
 @pytest.mark.parametrize("bit_rate", [8, 4, 2])
@@ -67,16 +69,18 @@ def test_lanes_per_bag(gpu_ctx, oracle, bit_rate, batch):
 
 
 @pytest.mark.parametrize("bit_rate", [8, 4])
-def test_rows_beyond_4gb(gpu_ctx, oracle, bit_rate):
-    """Few rows, far apart: the table's pitch puts them beyond 32-bit offsets."""
+@pytest.mark.parametrize("batch", [50, 2000])
+def test_rows_beyond_4gb(gpu_ctx, oracle, bit_rate, batch):
+    """Few rows, far apart: the table's pitch puts them beyond 32-bit offsets.  50 bags are for a block each, 2000 for a warp;
+    then beside a small table in one launch."""
     rng = np.random.default_rng(bit_rate)
-    dim, rows, stride, batch = 64, 70_000, 65_536, 50
+    dim, rows, stride = 64, 70_000, 65_536
     used = np.sort(rng.choice(rows, 64, replace=False))
     used[-1] = rows - 1
     compact = random_fused_table(rng, len(used), dim, bit_rate)
     table = torch.zeros(rows * stride, dtype=torch.uint8, device="cuda").view(rows, stride)
     table[torch.from_numpy(used).cuda(), :row_bytes(bit_rate, dim)] = dev(compact)
-    lengths = rng.choice(EDGE_LENGTHS, batch)
+    lengths = rng.choice(EDGE_LENGTHS[-6:] if batch == 50 else EDGE_LENGTHS, batch)
     n = int(lengths.sum())
     pick = rng.integers(0, len(used), n)
     offsets = np.concatenate([[0], np.cumsum(lengths)]).astype(np.int32)
@@ -87,6 +91,15 @@ def test_rows_beyond_4gb(gpu_ctx, oracle, bit_rate):
     kern = generate(bit_rate, dim, True, True, stride)
     assert kern(batch, n, rows, table, dev(used[pick]), dev(offsets), dev(w), out) and ok_ref
     np.testing.assert_array_equal(bits(out.cpu().numpy()), bits(ref))
+    out2, out3 = torch.zeros_like(out), torch.zeros_like(out)
+    plan = F.MultiTablePlan([(kern, batch, n, rows, table, dev(used[pick]), dev(offsets), dev(w), out2, None),
+                             (generate(bit_rate, dim, True, True, -1), batch, n, len(used), dev(compact), dev(pick), dev(offsets),
+                              dev(w), out3, None)])
+    plan.launch()
+    assert F.status_read(0)[0]
+    np.testing.assert_array_equal(bits(out2.cpu().numpy()), bits(ref))
+    np.testing.assert_array_equal(bits(out3.cpu().numpy()), bits(ref))
+    plan.close()
     bad = used[pick].copy()
     bad[0] = rows
     assert not kern(batch, n, rows, table, dev(bad), dev(offsets), dev(w), out)
