@@ -19,8 +19,9 @@
 //    lane that owns the row in the walk over the bag's indices (one index per
 //    lane at a time, coalesced): index load, range check, pruning map, weight,
 //    scale and bias load, their conversion and weighting.  The results go
-//    through shared memory: where the row lies, and {scale, scale, bias, bias}
-//    ready for the packed instructions - one 16-byte broadcast load per row.
+//    through shared memory: where the row lies, and ready for the packed
+//    instructions {scale, scale of the second column, bias, bias} (see Places) -
+//    one 16-byte broadcast load per row.
 //  * Rows that an index does not name (pruned, -1, out of range) drop out of
 //    that queue by ballot and popcount, so the row loop knows no skipped rows.
 //  * Row loads are issued ahead of the arithmetic, four rows at a time.
@@ -407,7 +408,7 @@ struct LaneData {
 template <bool WIDE>
 struct __align__(16) Queue {
   Row<WIDE> row[32];
-  ulonglong2 sb[32];  // {scale, scale}, {bias, bias}; {weight, weight} of unquantized rows
+  ulonglong2 sb[32];  // {scale of place 0, of place 1}, {bias, bias}; {weight, weight} of unquantized rows
 };
 
 // What a kernel is compiled for.
@@ -493,9 +494,11 @@ __device__ __forceinline__ void bag_from_lengths(const BagTable& p, int64_t firs
 //   rows, 2-bit D = 128), where 64-bit addresses for every pruned table would cost each of their rows the wide form's
 //   extra instructions;
 // * a row's weighted scale or bias is out_of_scale.  A chain of two or three loads per row: a launch with one such bag of 20
-//   rows takes 6 us longer, one whose weights are all 1e-30 two to three times as long (us, weights of 1 / 1e-30 and, while
-//   the range was 2^-52 to 2^52, 1e-16 too: 8-bit 10 000 bags of 20 rows 10.1 / 22.5, 4-bit 4096 ragged bags 7.9 / 22.7,
-//   2-bit pruned 8192 bags 9.3 / 30.2, 8 4-bit tables of 16 384 bags 142 / 424).
+//   rows takes 5 us longer, one whose weights are all 1e-30 two to three times as long (us, weights of 1 / 1e-30 and, while
+//   the range was 2^-52 to 2^52, 1e-16 too: 8-bit 10 000 bags of 20 rows 10.1 / 20.5, 4-bit 4096 ragged bags 7.3 / 22.7,
+//   2-bit pruned 8192 bags 9.2 / 30.0, 8 4-bit tables of 16 384 bags 142 / 424, 64 mixed ones of 512 49 / 83).  Kept small:
+//   its instructions arrive with the first bag that needs them.  Four rows at a time 4096 ragged bags of which one is such
+//   take 17.6 us instead of 14.5.
 template <class C, int VB, int CPL, class Lane>
 __device__ __forceinline__ void pool_again(const BagTable& p, const typename C::M& constants, const Lane& lane_data,
                                            int64_t start, int len, u64 (&acc)[C::kPairs]) {

@@ -19,12 +19,12 @@
 // bisection over the T+1 table starts, the index, the bounds check, the row
 // address, scale and bias - so that this chain of dependent loads is paid once
 // per 32 positions; then the warp walks the positions (the lane's findings
-// broadcast by shuffles): lane l produces columns 4l .. 4l+3 (+128, ...) from one
-// load of the 1-16 bytes that hold them and one 8- or 16-byte store, by code
-// compiled for the row type and the output type, so that the stores - which
-// are most of the traffic, 4 or 2 bytes per column against 1/4 to 4 read - are
-// coalesced and wide; widths that are no multiple of 4 and unaligned rows go
-// column by column.
+// broadcast by shuffles): a lane produces four columns, eight of a 16-bit output
+// of 64 columns and more, from the 1 to 16 bytes of each four and with one 8- or
+// 16-byte store, by code compiled for the row type and the output type, so that
+// the stores - which are most of the traffic, 4 or 2 bytes per column against 1/4
+// to 4 read - are coalesced and wide; widths that are no multiple of 4 and
+// unaligned rows go column by column.
 //
 // Bound by memory: rows read once, output rows written once.  Where the 32
 // positions of a warp name rows of one type (all but the warps at a table's
